@@ -392,10 +392,10 @@ extern "C" NqpuError nqpu_expectation_z_all(const NqpuState* state, double* out,
   return NQPU_OK;
 }
 
-static NqpuError pauli_expect(const StateImpl* s, uint64_t xm, uint64_t zm, uint64_t ym, double* out) {
-  double r[2];
-  NQ_TRY(state_pauli(s, xm, zm, ym, r));
-  *out = r[0];
+static NqpuError pauli_expect(const StateImpl* s, const std::vector<PauliString>& strings, double* out) {
+  double r = 0.0;
+  NQ_TRY(state_pauli_sum(const_cast<StateImpl*>(s), strings, &r));
+  *out = r;
   return NQPU_OK;
 }
 
@@ -403,14 +403,14 @@ extern "C" NqpuError nqpu_expectation_x(const NqpuState* state, uint32_t qubit, 
   if (!state || !out) return NQPU_NULL_POINTER;
   const StateImpl* s = S(state);
   if (qubit >= s->n) return NQPU_INVALID_QUBIT;
-  return pauli_expect(s, 1ull << qubit, 0, 0, out);
+  return pauli_expect(s, {PauliString{1ull << qubit, 0, 0, 1.0}}, out);
 }
 
 extern "C" NqpuError nqpu_expectation_y(const NqpuState* state, uint32_t qubit, double* out) {
   if (!state || !out) return NQPU_NULL_POINTER;
   const StateImpl* s = S(state);
   if (qubit >= s->n) return NQPU_INVALID_QUBIT;
-  return pauli_expect(s, 1ull << qubit, 1ull << qubit, 1ull << qubit, out);
+  return pauli_expect(s, {PauliString{1ull << qubit, 1ull << qubit, 1ull << qubit, 1.0}}, out);
 }
 
 extern "C" NqpuError nqpu_expectation_pauli_sum(const NqpuState* state, const char* paulis,
@@ -420,7 +420,7 @@ extern "C" NqpuError nqpu_expectation_pauli_sum(const NqpuState* state, const ch
   const StateImpl* s = S(state);
   const uint32_t n = s->n;
   // Parse all terms first (invalid characters -> InvalidParameter, nothing runs).
-  std::vector<std::tuple<uint64_t, uint64_t, uint64_t>> masks(num_terms);
+  std::vector<PauliString> strings(num_terms);
   for (uint32_t t = 0; t < num_terms; ++t) {
     uint64_t xm = 0, zm = 0, ym = 0;
     for (uint32_t q = 0; q < n; ++q) {
@@ -434,17 +434,9 @@ extern "C" NqpuError nqpu_expectation_pauli_sum(const NqpuState* state, const ch
       }
     }
     if (!is_finite_param(coeffs[t])) return NQPU_INVALID_PARAMETER;
-    masks[t] = std::make_tuple(xm, zm, ym);
+    strings[t] = PauliString{xm, zm, ym, coeffs[t]};
   }
-  double total = 0.0;
-  for (uint32_t t = 0; t < num_terms; ++t) {
-    double v = 0.0;
-    NqpuError e = pauli_expect(s, std::get<0>(masks[t]), std::get<1>(masks[t]), std::get<2>(masks[t]), &v);
-    if (e != NQPU_OK) return e;
-    total += coeffs[t] * v;
-  }
-  *out = total;
-  return NQPU_OK;
+  return pauli_expect(s, strings, out);
 }
 
 extern "C" NqpuError nqpu_fidelity(const NqpuState* a, const NqpuState* b, double* out) {

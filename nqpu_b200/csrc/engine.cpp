@@ -55,8 +55,8 @@ StateImpl* state_new(uint32_t n, DType dt) {
   bool ok = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaMalloc(&s->amp, s->bytes) == cudaSuccess;
   ok = ok && cudaMalloc(reinterpret_cast<void**>(&s->scratch), reduce_scratch_bytes(int(n))) == cudaSuccess;
-  ok = ok && cudaMalloc(reinterpret_cast<void**>(&s->d_small), 512 * sizeof(double)) == cudaSuccess;
-  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&s->h_small), 512 * sizeof(double)) == cudaSuccess;
+  ok = ok && cudaMalloc(reinterpret_cast<void**>(&s->d_small), kSmallDoubles * sizeof(double)) == cudaSuccess;
+  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&s->h_small), kSmallDoubles * sizeof(double)) == cudaSuccess;
   ok = ok && launch_set_basis(dt, s->amp, int(n), 0, s->stream, device_sms()) == cudaSuccess;
   ok = ok && cudaStreamSynchronize(s->stream) == cudaSuccess;
   if (!ok) {
@@ -74,6 +74,7 @@ void state_free(StateImpl* s) {
   if (s->scratch) cudaFree(s->scratch);
   if (s->d_small) cudaFree(s->d_small);
   if (s->h_small) cudaFreeHost(s->h_small);
+  if (s->d_tab) cudaFree(s->d_tab);
   if (s->d_uni) cudaFree(s->d_uni);
   if (s->d_shots) cudaFree(s->d_shots);
   if (s->run_norm) cudaFree(s->run_norm);
@@ -112,9 +113,7 @@ cudaError_t state_run_error(StateImpl* s) {
 
 cudaError_t state_zsums(const StateImpl* s, double* zs, double* total) {
   const int n = int(s->n);
-  cudaError_t e = launch_zsums(s->dt, s->amp, n, s->scratch, s->d_small, s->stream, device_sms());
-  if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(s->h_small, s->d_small, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, s->stream);
+  cudaError_t e = launch_zsums(s->dt, s->amp, n, s->scratch, s->h_small, s->stream, device_sms());
   if (e != cudaSuccess) return e;
   e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return e;
@@ -149,24 +148,62 @@ cudaError_t state_reset_qubit(StateImpl* s, uint32_t qubit) {
   return launch_collapse(s->dt, s->amp, int(s->n), int(qubit), 0, f, s->stream, device_sms());
 }
 
-cudaError_t state_pauli(const StateImpl* s, uint64_t xm, uint64_t zm, uint64_t ym, double* out2) {
-  cudaError_t e = launch_pauli(s->dt, s->amp, int(s->n), xm, zm, ym, s->scratch, s->d_small, s->stream, device_sms());
-  if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(s->h_small, s->d_small, 2 * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-  if (e != cudaSuccess) return e;
-  e = cudaStreamSynchronize(s->stream);
-  if (e != cudaSuccess) return e;
-  out2[0] = s->h_small[0];
-  out2[1] = s->h_small[1];
+// One string that no register set holds (or a state of fewer than four qubits).
+static cudaError_t pauli_direct(const StateImpl* s, const PauliString& p, double* out) {
+  cudaError_t e = launch_pauli(s->dt, s->amp, int(s->n), p.x, p.z, p.y, s->scratch, s->h_small, s->stream, device_sms());
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  if (e == cudaSuccess) *out += p.c * s->h_small[0];
+  return e;
+}
+
+cudaError_t state_pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out) {
+  *out = 0.0;
+  cudaError_t e;
+  if (s->n < 4) {
+    for (const PauliString& p : strings)
+      if ((e = pauli_direct(s, p, out)) != cudaSuccess) return e;
+    return cudaSuccess;
+  }
+  PauliPlan plan;
+  std::vector<PauliString> wide;
+  for (size_t lo = 0; lo < strings.size(); lo += kPauliMaxTerms) {
+    pauli_plan(strings.data() + lo, std::min<size_t>(kPauliMaxTerms, strings.size() - lo), int(s->n), &plan, &wide);
+    for (const PauliString& p : wide)
+      if ((e = pauli_direct(s, p, out)) != cudaSuccess) return e;
+    if (plan.sets.empty()) continue;
+    // tables: terms (16 bytes each), then the sets
+    const size_t tb = plan.terms.size() * sizeof(PauliTerm), bytes = tb + plan.sets.size() * sizeof(PauliSet);
+    char* dev = reinterpret_cast<char*>(s->d_small + kSmallTable);
+    std::vector<char> big;
+    char* host = reinterpret_cast<char*>(s->h_small + kSmallTable);
+    if (bytes > (kSmallDoubles - kSmallTable) * sizeof(double)) {
+      if (s->tab_cap < bytes) {
+        if (s->d_tab) cudaFree(s->d_tab);  // earlier sums have returned, so nothing queued reads it
+        s->d_tab = nullptr;
+        s->tab_cap = 0;
+        if ((e = cudaMalloc(&s->d_tab, bytes)) != cudaSuccess) return e;
+        s->tab_cap = bytes;
+      }
+      dev = static_cast<char*>(s->d_tab);
+      big.resize(bytes);
+      host = big.data();
+    }
+    std::memcpy(host, plan.terms.data(), tb);
+    std::memcpy(host + tb, plan.sets.data(), bytes - tb);
+    if ((e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) return e;
+    e = launch_pauli_sum(s->dt, s->amp, int(s->n), reinterpret_cast<const PauliSet*>(dev + tb), plan,
+                         reinterpret_cast<const PauliTerm*>(dev), s->scratch, s->h_small, s->stream, device_sms());
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return e;
+    *out += s->h_small[0];
+  }
   return cudaSuccess;
 }
 
 cudaError_t state_inner(const StateImpl* a, const StateImpl* b, double* out2) {
   cudaError_t e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return e;
-  e = launch_inner(a->dt, a->amp, b->dt, b->amp, int(a->n), a->scratch, a->d_small, a->stream, device_sms());
-  if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(a->h_small, a->d_small, 2 * sizeof(double), cudaMemcpyDeviceToHost, a->stream);
+  e = launch_inner(a->dt, a->amp, b->dt, b->amp, int(a->n), a->scratch, a->h_small, a->stream, device_sms());
   if (e != cudaSuccess) return e;
   e = cudaStreamSynchronize(a->stream);
   if (e != cudaSuccess) return e;

@@ -8,6 +8,7 @@
 #include <tuple>
 #include <vector>
 #include "../../include/nqpu_b200.h"
+#include "kernels.h"
 #include "planner.h"
 #include "sv_types.h"
 
@@ -20,6 +21,8 @@ double next_random_f64();
 bool device_ready();
 int device_sms();
 
+constexpr size_t kSmallDoubles = 2048, kSmallTable = 64;
+
 struct StateImpl {
   uint32_t n = 0;
   DType dt = DType::C128;
@@ -27,8 +30,13 @@ struct StateImpl {
   size_t bytes = 0;
   cudaStream_t stream = nullptr;
   double* scratch = nullptr;   // reduction scratch (reduce_scratch_bytes)
-  double* d_small = nullptr;   // small device outputs (256 doubles)
-  double* h_small = nullptr;   // pinned host mirror of d_small
+  // small buffers (kSmallDoubles each): reduction results are written by the
+  // kernels into h_small[0, kSmallTable), pinned host memory; small tables of a
+  // call are staged behind them and copied to the same place of d_small
+  double* d_small = nullptr;
+  double* h_small = nullptr;
+  void* d_tab = nullptr;       // tables that do not fit d_small, grown on demand
+  size_t tab_cap = 0;
   double* d_uni = nullptr;     // sampling uniforms
   uint64_t* d_shots = nullptr; // sampling outcomes
   uint32_t shot_cap = 0;
@@ -50,7 +58,9 @@ cudaError_t state_run_scratch(StateImpl* s, size_t doubles, double** norm, int**
 cudaError_t state_run_error(StateImpl* s);
 // out (n+1 values): [0] = sum|a|^2, [1+q] = sum over bit q set; either pointer may be null.
 cudaError_t state_zsums(const StateImpl* s, double* zs, double* total);
-cudaError_t state_pauli(const StateImpl* s, uint64_t xm, uint64_t zm, uint64_t ym, double* out2);
+// sum_t c_t <P_t> (one launch per kPauliMaxTerms strings plus one per string
+// that spans more than four X|Y positions).
+cudaError_t state_pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out);
 cudaError_t state_inner(const StateImpl* a, const StateImpl* b, double* out2);
 cudaError_t state_sample(const StateImpl* s, const double* uniforms, uint32_t shots, uint64_t* out);
 cudaError_t state_probabilities(const StateImpl* s, double* out);

@@ -46,31 +46,67 @@ cudaError_t launch_convert(DType src_dt, const void* src, DType dst_dt, void* ds
                            cudaStream_t s, int num_sms);
 
 // --- FP64 reductions ---------------------------------------------------------
-// Layout of the all-<Z_i> scratch (doubles): kZsMaxBlocks x kZsBlkVals
-// per-block low-bit partials, then one total per segment of kZsSegVecs 128-bit
-// vectors (room is kept for kZsSegSlots per segment).
-constexpr int kZsBlkVals = 16;
+// All-<Z_i>: a warp works on chunks of kZsChunkVecs 128-bit vectors; the scratch
+// holds one row per value (n + 1 of them) of at most kZsMaxBlocks block partials.
+constexpr uint64_t kZsChunkVecs = 32 * 8;  // lanes x vectors per lane
 constexpr int kZsMaxBlocks = 1024;
-constexpr uint64_t kZsSegVecs = 256 * 16;  // threads per block x vectors per thread
-constexpr int kZsSegSlots = 8;
-// Doubles of all-<Z_i> scratch for a state of 2^vec_log2 128-bit vectors.
-constexpr size_t zsums_scratch_doubles(int vec_log2) {
-  return size_t(kZsMaxBlocks) * kZsBlkVals +
-         size_t(((uint64_t(1) << vec_log2) + kZsSegVecs - 1) / kZsSegVecs) * kZsSegSlots;
-}
+// Doubles of all-<Z_i> scratch for an n-qubit state.
+constexpr size_t zsums_scratch_doubles(int n) { return size_t(kZsMaxBlocks) * size_t(n + 1); }
 // Scratch bytes every reduction below needs on an n-qubit state.
 size_t reduce_scratch_bytes(int n);
+// out[v] = sum over b < nblk of part[v * nblk + b] (one block, fixed order).
+cudaError_t launch_sum_rows(const double* part, int nvals, int nblk, double* out, cudaStream_t s);
 // out[0] = sum |a|^2, out[1+q] = sum over amplitudes with bit q set of |a|^2, q < n.
+// `out` here and in launch_inner is device memory or pinned host memory.
 cudaError_t launch_zsums(DType dt, const void* amp, int n, double* scratch, double* out,
                          cudaStream_t s, int num_sms);
 // out[0..1] = sum conj(a) b (re, im)
 cudaError_t launch_inner(DType dta, const void* a, DType dtb, const void* b, int n,
                          double* scratch, double* out, cudaStream_t s, int num_sms);
 // Pauli-string expectation (R/lib.rs:465 semantics): xmask = X|Y positions,
-// zmask = Z|Y positions, ny = number of Y factors.  out[0] = real part.
+// zmask = Z|Y positions, ymask = Y positions.  out[0] = real part.
 cudaError_t launch_pauli(DType dt, const void* amp, int n, uint64_t xmask, uint64_t zmask,
                          uint64_t ymask, double* scratch, double* out, cudaStream_t s,
                          int num_sms);
+
+// --- Pauli sums (kernels_pauli.cu) -------------------------------------------
+struct PauliString {
+  uint64_t x, z, y;  // X|Y positions, Z|Y positions, Y positions
+  double c;
+};
+// A register set of the Pauli-sum kernel: a thread holds the 16 amplitudes that
+// differ in the four index bits rbit (ascending) and evaluates on them every
+// term whose X|Y positions lie in those bits.  Terms [beg[m], beg[m + 1]) have
+// X|Y positions m (a mask over rbit); beg[0]..beg[1] are diagonal terms, sorted
+// by their Z positions within rbit, dbeg[k] the first with positions >= k.
+struct PauliSet {
+  uint16_t beg[17];
+  uint16_t dbeg[17];
+  uint16_t xused, dused;  // bit m: the list of X|Y (diagonal: Z) positions m is not empty
+  uint8_t rbit[4];
+};
+// One term: z = Z|Y positions outside the set's bits | those inside << 60 |
+// (odd number of Y's) << 59; c = coefficient with the pair factor and the sign
+// of i^ny folded in.
+struct PauliTerm {
+  uint64_t z;
+  double c;
+};
+constexpr int kPauliMaxTerms = 65535;  // of one launch (16-bit offsets)
+struct PauliPlan {
+  std::vector<PauliSet> sets;
+  std::vector<PauliTerm> terms;
+};
+// Split a Pauli sum on n >= 4 qubits into register sets; terms whose X|Y
+// positions span more than four qubits are left in `wide` (at most
+// kPauliMaxTerms strings per call).
+void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan,
+                std::vector<PauliString>* wide);
+// out[0] = the plan's sum over the state; d_sets / d_terms are the plan's tables
+// in device memory.
+cudaError_t launch_pauli_sum(DType dt, const void* amp, int n, const PauliSet* d_sets, const PauliPlan& plan,
+                             const PauliTerm* d_terms, double* scratch, double* out, cudaStream_t s, int num_sms);
+
 // Sampling with given uniforms: out[s] = first i with u[s] < cumsum_i, else 2^n-1.
 cudaError_t launch_sample(DType dt, const void* amp, int n, const double* d_uniforms,
                           uint32_t shots, double* scratch, uint64_t* d_out, cudaStream_t s,

@@ -1,0 +1,258 @@
+// Pauli sums: sum_t c_t <P_t> of many Pauli strings in one launch
+// (expectation_pauli_string / expectation of a Hamiltonian, R/lib.rs:465,518).
+//
+// With coeff(i) = i^ny (-1)^popcount(i & z), a string contributes
+// sum_i Re(conj(a_i) coeff(i) a_{i ^ x}).  For x = 0 that is |a_i|^2 with a
+// sign; for x != 0 the amplitudes i and i ^ x contribute the same value, so one
+// term per pair is enough: 2 (-1)^{ny/2} (-1)^{pc(i & z)} Re(conj(a_i) a_{i^x})
+// for an even number of Y's and -+2 (...) Im(...) for an odd one.
+//
+// The host groups the strings into register sets of four qubits (pauli_plan): a
+// thread loads the 16 amplitudes that differ in a set's qubits, converts them to
+// FP64 once, and evaluates every string whose X|Y positions lie inside the set on
+// them.  Diagonal strings take a Walsh-Hadamard transform of the 16
+// probabilities: the sum of |a|^2 over the block with any sign pattern on its
+// four qubits is one of its 16 outputs, so a string costs one sign and one
+// addition per 16 amplitudes.
+//
+// Bound: an n-qubit Ising Hamiltonian takes ceil(n / 4) sets, each a read of the
+// state.  The sets whose qubits lie below kPauliChunkBits run chunk by chunk, so
+// all but the first of them find the chunk in L2.  FP64 conversion (two per
+// complex64 amplitude and set) comes second.  Before, each string was a launch
+// of its own that read the state with 4-byte loads (and its partner amplitudes
+// again) and ended in a host synchronisation.
+#include "reduce_device.cuh"
+
+namespace nqpu {
+
+// 2^22 amplitudes are 32 MB (complex64) / 64 MB (complex128): well inside the L2.
+constexpr int kPauliChunkBits = 22;
+
+void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan,
+                std::vector<PauliString>* wide) {
+  plan->sets.clear();
+  plan->terms.clear();
+  wide->clear();
+  struct Group {
+    uint64_t bits = 0;
+    std::vector<size_t> idx;
+  };
+  std::vector<Group> groups;
+  std::vector<size_t> diag;
+  for (size_t t = 0; t < count; ++t) {
+    const uint64_t x = strings[t].x;
+    if (x == 0) { diag.push_back(t); continue; }
+    if (__builtin_popcountll(x) > 4) { wide->push_back(strings[t]); continue; }
+    Group* g = nullptr;
+    for (Group& h : groups)
+      if (__builtin_popcountll(h.bits | x) <= 4) { g = &h; break; }
+    if (!g) { groups.emplace_back(); g = &groups.back(); }
+    g->bits |= x;
+    g->idx.push_back(t);
+  }
+  if (!diag.empty()) {
+    if (groups.empty()) groups.emplace_back();
+    groups[0].idx.insert(groups[0].idx.end(), diag.begin(), diag.end());
+  }
+  // fill every set to four qubits, highest first (a set without low qubits loads
+  // whole lines per warp)
+  for (Group& g : groups)
+    for (int q = std::min(n, kPauliChunkBits) - 1; q >= 0 && __builtin_popcountll(g.bits) < 4; --q) g.bits |= 1ull << q;
+  std::stable_sort(groups.begin(), groups.end(), [](const Group& a, const Group& b) {
+    return (a.bits >> kPauliChunkBits != 0) < (b.bits >> kPauliChunkBits != 0);
+  });
+  for (const Group& g : groups) {
+    PauliSet S{};
+    int nb = 0;
+    for (int q = 0; q < n; ++q)
+      if ((g.bits >> q) & 1) S.rbit[nb++] = uint8_t(q);
+    auto inside = [&](uint64_t m) {
+      int v = 0;
+      for (int b = 0; b < 4; ++b) v |= int((m >> S.rbit[b]) & 1) << b;
+      return v;
+    };
+    // (X positions, Z positions) within the set order the terms
+    std::vector<std::pair<int, size_t>> order;
+    for (size_t t : g.idx) order.push_back({inside(strings[t].x) * 16 + inside(strings[t].z), t});
+    std::stable_sort(order.begin(), order.end(),
+                     [](const std::pair<int, size_t>& a, const std::pair<int, size_t>& b) { return a.first < b.first; });
+    size_t k = 0;
+    for (int m = 0; m <= 16; ++m) {
+      while (k < order.size() && order[k].first < 16 * m) ++k;
+      S.beg[m] = uint16_t(plan->terms.size() + k);
+      if (m > 0 && S.beg[m] > S.beg[m - 1] && m - 1 > 0) S.xused |= uint16_t(1u << (m - 1));
+    }
+    k = 0;
+    for (int m = 0; m <= 16; ++m) {
+      while (k < order.size() && order[k].first < m) ++k;
+      S.dbeg[m] = uint16_t(plan->terms.size() + k);
+      if (m > 0 && S.dbeg[m] > S.dbeg[m - 1]) S.dused |= uint16_t(1u << (m - 1));
+    }
+    for (const auto& o : order) {
+      const PauliString& P = strings[o.second];
+      const int ny = __builtin_popcountll(P.y) & 3;
+      PauliTerm T;
+      T.z = (P.z & ~g.bits) | (uint64_t(inside(P.z)) << 60) | (uint64_t(ny & 1) << 59);
+      T.c = P.x == 0 ? P.c : 2.0 * P.c * ((ny == 1 || ny == 2) ? -1.0 : 1.0);
+      plan->terms.push_back(T);
+    }
+    plan->sets.push_back(S);
+  }
+}
+
+__device__ __forceinline__ double flip(double v, uint32_t bit) {  // -v when bit 0 of `bit` is set
+  return __hiloint2double(__double2hiint(v) ^ int(bit << 31), __double2loint(v));
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(kRedThreads, 2)
+    k_pauli_sum(const Real* __restrict__ amp, int n, const PauliSet* __restrict__ sets, int nlow, int nsets,
+                const PauliTerm* __restrict__ terms, double* __restrict__ part, double* __restrict__ out) {
+  using C = typename Tr<Real>::C;
+  const C* a = reinterpret_cast<const C*>(amp);
+  const int hbits = n < kPauliChunkBits ? n : kPauliChunkBits;
+  // work units of kRedThreads threads: first (chunk, low set, tile), then (high set, tile)
+  const int lt_low = max(0, hbits - 4 - 8), lt_high = max(0, n - 4 - 8);
+  const uint64_t low_units = (uint64_t(nlow) << lt_low) << (n - hbits);
+  const uint64_t units = low_units + (uint64_t(nsets - nlow) << lt_high);
+  KSum acc;
+  for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    int si;
+    uint64_t w, chunk = 0;
+    int span;  // index bits the unit's threads run over
+    if (u < low_units) {
+      const uint64_t t = u >> lt_low;
+      chunk = t / unsigned(nlow);
+      si = int(t - chunk * unsigned(nlow));
+      w = ((u & ((1ull << lt_low) - 1)) << 8) + threadIdx.x;
+      span = hbits;
+    } else {
+      const uint64_t v = u - low_units;
+      si = nlow + int(v >> lt_high);
+      w = ((v & ((1ull << lt_high) - 1)) << 8) + threadIdx.x;
+      span = n;
+    }
+    if (w >> (span - 4)) continue;  // fewer work items than threads
+    const PauliSet* S = sets + si;
+    uint64_t base = w, off[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      base = insert_zero_bit(base, S->rbit[b]);
+      off[b] = 1ull << S->rbit[b];
+    }
+    base += chunk << hbits;
+    C v[16];
+    auto idx = [&](int r) {
+      return base + ((r & 1) ? off[0] : 0) + ((r & 2) ? off[1] : 0) + ((r & 4) ? off[2] : 0) + ((r & 8) ? off[3] : 0);
+    };
+    if (sizeof(Real) == 4 && off[0] == 1) {  // qubit 0 in the set: pairs as 128-bit loads
+#pragma unroll
+      for (int r = 0; r < 16; r += 2) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(a + idx(r)));
+        v[r].x = x.x; v[r].y = x.y; v[r + 1].x = x.z; v[r + 1].y = x.w;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = __ldg(a + idx(r));
+    }
+    double re[16], im[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      re[r] = v[r].x;
+      im[r] = v[r].y;
+    }
+    double item = 0.0;
+    auto term = [&](int t, double* c) {
+      const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(terms + t));
+      *c = __longlong_as_double((long long)x.y);
+      return x.x;
+    };
+    constexpr uint64_t kOutside = (1ull << 59) - 1;
+    const uint32_t dused = S->dused, xused = S->xused;
+    if (dused) {
+      double W[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) W[r] = re[r] * re[r] + im[r] * im[r];
+#pragma unroll
+      for (int b = 1; b < 16; b <<= 1)
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (!(r & b)) {
+            const double x = W[r], y = W[r | b];
+            W[r] = x + y;
+            W[r | b] = x - y;
+          }
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        if (!((dused >> m) & 1)) continue;
+        const int e = S->dbeg[m + 1];
+        double cs = 0.0;
+        for (int t = S->dbeg[m]; t < e; ++t) {
+          double c;
+          const uint64_t z = term(t, &c);
+          cs += flip(c, uint32_t(__popcll(base & z & kOutside)));
+        }
+        item += W[m] * cs;
+      }
+    }
+#pragma unroll
+    for (int m = 1; m < 16; ++m) {
+      if (!((xused >> m) & 1)) continue;
+      const int top = m >= 8 ? 8 : m >= 4 ? 4 : m >= 2 ? 2 : 1;
+      const int e = S->beg[m + 1];
+      for (int t = S->beg[m]; t < e; ++t) {
+        double c;
+        const uint64_t z = term(t, &c);
+        const uint32_t zr = uint32_t(z >> 60);
+        // bit r: parity of r & zr
+        const uint32_t pat = ((zr & 1) ? 0xAAAAu : 0u) ^ ((zr & 2) ? 0xCCCCu : 0u) ^ ((zr & 4) ? 0xF0F0u : 0u) ^
+                             ((zr & 8) ? 0xFF00u : 0u);
+        double s = 0.0;
+        if ((z >> 59) & 1) {
+#pragma unroll
+          for (int r = 0; r < 16; ++r)
+            if (!(r & top)) s += flip(re[r] * im[r ^ m] - im[r] * re[r ^ m], pat >> r);
+        } else if (zr == 0) {
+#pragma unroll
+          for (int r = 0; r < 16; ++r)
+            if (!(r & top)) s += re[r] * re[r ^ m] + im[r] * im[r ^ m];
+        } else {
+#pragma unroll
+          for (int r = 0; r < 16; ++r)
+            if (!(r & top)) s += flip(re[r] * re[r ^ m] + im[r] * im[r ^ m], pat >> r);
+        }
+        item += flip(c * s, uint32_t(__popcll(base & z & kOutside)));
+      }
+    }
+    acc.add(item);
+  }
+  __shared__ double sh[kRedWarps];
+  const double r = warp_sum(acc.s);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) sh[warp] = r;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < kRedWarps; ++w) t += sh[w];
+    if (gridDim.x == 1) out[0] = t;
+    else part[blockIdx.x] = t;
+  }
+}
+
+cudaError_t launch_pauli_sum(DType dt, const void* amp, int n, const PauliSet* d_sets, const PauliPlan& plan,
+                             const PauliTerm* d_terms, double* scratch, double* out, cudaStream_t s, int num_sms) {
+  int nlow = 0;
+  for (const PauliSet& S : plan.sets) nlow += S.rbit[3] < kPauliChunkBits;
+  const int nsets = int(plan.sets.size());
+  const uint64_t units = (uint64_t(nsets) << n) >> 12;  // of 256 threads x 16 amplitudes
+  const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(std::max<uint64_t>(units, uint64_t(nsets)),
+                                                                       uint64_t(num_sms) * 2)));
+  if (dt == DType::C64)
+    k_pauli_sum<float><<<g, kRedThreads, 0, s>>>(static_cast<const float*>(amp), n, d_sets, nlow, nsets, d_terms, scratch, out);
+  else
+    k_pauli_sum<double><<<g, kRedThreads, 0, s>>>(static_cast<const double*>(amp), n, d_sets, nlow, nsets, d_terms, scratch, out);
+  if (g > 1) return launch_sum_rows(scratch, 1, int(g), out, s);
+  return cudaGetLastError();
+}
+
+}  // namespace nqpu

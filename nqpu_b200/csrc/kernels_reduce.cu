@@ -7,181 +7,119 @@
 // as a serial loop per qubit or per term; here every reduction is one coalesced
 // pass with FP64 accumulation: per-thread Kahan sums, warp-shuffle trees, and a
 // final single-block FP64 combine, so results are deterministic for a given
-// state and launch shape.
-#include "sv_device.cuh"
-#include "kernels.h"
+// state and launch shape.  Pauli sums are in kernels_pauli.cu.
+#include "reduce_device.cuh"
 
 namespace nqpu {
 
-struct KSum {
-  double s = 0.0, c = 0.0;
-  __device__ __forceinline__ void add(double x) {
-    double y = x - c;
-    double t = s + y;
-    c = (t - s) - y;
-    s = t;
+// out[v] = sum over the blocks of part[v * nblk + b]: one warp per value, fixed
+// order.  Values are strided by block so a warp's loads are coalesced.
+__global__ void __launch_bounds__(1024)
+    k_sum_rows(const double* __restrict__ part, int nvals, int nblk, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int v = warp; v < nvals; v += int(blockDim.x >> 5)) {
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += part[size_t(v) * nblk + b];
+    s = warp_sum(s);
+    if (lane == 0) out[v] = s;
   }
-};
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
-constexpr int kRedThreads = 256;
-constexpr int kRedVecPerThread = 16;  // a segment = 256 * 16 vectors
-
-template <typename Real>
-__device__ __forceinline__ void vec_probs(const typename Tr<Real>::V& v, double* p);
-template <>
-__device__ __forceinline__ void vec_probs<float>(const float4& v, double* p) {
-  p[0] = double(v.x) * double(v.x) + double(v.y) * double(v.y);
-  p[1] = double(v.z) * double(v.z) + double(v.w) * double(v.w);
-}
-template <>
-__device__ __forceinline__ void vec_probs<double>(const double2& v, double* p) {
-  p[0] = v.x * v.x + v.y * v.y;
+cudaError_t launch_sum_rows(const double* part, int nvals, int nblk, double* out, cudaStream_t s) {
+  k_sum_rows<<<1, 32 * std::min(nvals, 32), 0, s>>>(part, nvals, nblk, out);
+  return cudaGetLastError();
 }
 
-// Layout of the zsums scratch (doubles, kernels.h):
-//   [0, nblk*kBlkVals)            per-block low-bit partials
-//   [kZsMaxBlocks*kBlkVals, + nseg) per-segment totals
-constexpr int kBlkVals = kZsBlkVals;  // tot, bit0(c64), 8 thread bits, 4 j bits, (pad)
-static_assert(kZsSegVecs == uint64_t(kRedThreads) * kRedVecPerThread, "segment size");
-
+// ---- all <Z_q> --------------------------------------------------------------
+// A warp's work unit is a chunk of 32 lanes x 8 vectors (kZsChunkVecs).  Vector
+// index bits 0..4 are lanes, 5..7 the thread's vectors, 8.. the chunk number.
+// Per chunk a thread sums its 8 probabilities in a tree that also yields the
+// sums over each of its three vector bits; only those five sums go through the
+// compensated accumulators.  Lane b of the warp accumulates the chunk totals
+// whose chunk bit b is set, so no per-segment array goes through memory and the
+// final step adds (n + 1) rows of one value per block.
+//
+// Bound: HBM (the state is read once), FP64 issue close behind: 11 FP64
+// operations per 128-bit vector here.  The earlier form took 22 (a compensated
+// add per vector bit and vector), wrote one total per 4096 vectors and folded
+// those in one block, which alone cost about 30 us of the 38 us of a 10-qubit
+// call.
 template <typename Real>
 __global__ void __launch_bounds__(kRedThreads)
-    k_zsums(const Real* __restrict__ amp, int n, uint64_t nseg, double* __restrict__ blk_part,
-            double* __restrict__ seg_part) {
+    k_zsums(const Real* __restrict__ amp, int n, uint64_t nchunks, double* __restrict__ part,
+            double* __restrict__ out) {
   using V = typename Tr<Real>::V;
   constexpr int VB = Tr<Real>::kVecBit;
-  constexpr int APV = Tr<Real>::kAmpsPerVec;
-  const uint64_t nvec_total = (1ull << n) >> VB;
+  constexpr int NV = int(kZsChunkVecs / 32);
+  static_assert(NV == 8, "the tree below sums 8 vectors");
+  const uint64_t nvec = (1ull << n) >> VB;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  KSum tot, b0;
-  KSum jb[4];
+  KSum tot, b0, j0, j1, j2, hi;
   const V* vp = reinterpret_cast<const V*>(amp);
-  static_assert(kRedThreads == 256, "segment total sums 8 warps");
-  __shared__ double seg_red[kRedThreads / 32];
-  for (uint64_t seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
-    const uint64_t vbase = seg * (kRedThreads * kRedVecPerThread);
-    V v[kRedVecPerThread];
+  const uint64_t nwarps = uint64_t(gridDim.x) * kRedWarps;
+  for (uint64_t ch = uint64_t(blockIdx.x) * kRedWarps + warp; ch < nchunks; ch += nwarps) {
+    const uint64_t vb = ch * kZsChunkVecs + lane;
+    V v[NV];
+    if (vb - lane + kZsChunkVecs <= nvec) {
 #pragma unroll
-    for (int j = 0; j < kRedVecPerThread; ++j) {
-      const uint64_t vi = vbase + tid + j * kRedThreads;
-      if (vi < nvec_total) v[j] = __ldcs(vp + vi);
-    }
-    double segp = 0.0;
+      for (int j = 0; j < NV; ++j) v[j] = __ldcs(vp + vb + 32 * j);
+    } else {  // a state of less than one chunk
 #pragma unroll
-    for (int j = 0; j < kRedVecPerThread; ++j) {
-      const uint64_t vi = vbase + tid + j * kRedThreads;
-      if (vi < nvec_total) {
-        double p[2];
-        vec_probs<Real>(v[j], p);
-        double pv = p[0];
-        if (APV == 2) {
-          pv += p[1];
-          b0.add(p[1]);
-        }
-        tot.add(pv);
-        segp += pv;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (j & (1 << q)) jb[q].add(pv);
+      for (int j = 0; j < NV; ++j) {
+        v[j] = V{};
+        if (vb + 32 * j < nvec) v[j] = __ldcs(vp + vb + 32 * j);
       }
     }
-    segp = warp_sum(segp);
-    if (lane == 0) seg_red[warp] = segp;
-    __syncthreads();
-    if (tid == 0)
-      seg_part[seg] = ((seg_red[0] + seg_red[1]) + (seg_red[2] + seg_red[3])) +
-                      ((seg_red[4] + seg_red[5]) + (seg_red[6] + seg_red[7]));
-    __syncthreads();
+    double p[NV], odd = 0.0;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      double q[2];
+      vec_probs<Real>(v[j], q);
+      p[j] = q[0];
+      if (VB == 1) {
+        p[j] += q[1];
+        odd += q[1];
+      }
+    }
+    const double s01 = p[0] + p[1], s23 = p[2] + p[3], s45 = p[4] + p[5], s67 = p[6] + p[7];
+    const double top = s45 + s67, t = (s01 + s23) + top;
+    tot.add(t);
+    if (VB == 1) b0.add(odd);
+    j0.add((p[1] + p[3]) + (p[5] + p[7]));
+    j1.add(s23 + s67);
+    j2.add(top);
+    const double w = warp_sum(t);
+    if ((ch >> lane) & 1) hi.add(w);
   }
-  // Per-block partials of the low bits: thread bits come from the per-thread totals.
-  __shared__ double red[kRedThreads / 32][kBlkVals];
-  double vals[kBlkVals];
+  // row v of the block: 0 total, 1 + q the sum over amplitudes with bit q set
+  __shared__ double red[kRedWarps][kMaxQubits + 2];
   const double t = tot.s;
-  vals[0] = t;
-  vals[1] = b0.s;
+  double vals[6 + 5] = {t, b0.s, j0.s, j1.s, j2.s, 0.0};
 #pragma unroll
-  for (int b = 0; b < 8; ++b) vals[2 + b] = ((tid >> b) & 1) ? t : 0.0;
+  for (int b = 0; b < 5; ++b) vals[5 + b] = ((lane >> b) & 1) ? t : 0.0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) vals[10 + q] = jb[q].s;
-  vals[14] = vals[15] = 0.0;
+  for (int i = 0; i < 10; ++i) vals[i] = warp_sum(vals[i]);
+  if (lane == 0) {
+    red[warp][0] = vals[0];
+    if (VB == 1) red[warp][1] = vals[1];
 #pragma unroll
-  for (int i = 0; i < kBlkVals; ++i) vals[i] = warp_sum(vals[i]);
-  if (lane == 0)
-    for (int i = 0; i < kBlkVals; ++i) red[warp][i] = vals[i];
+    for (int b = 0; b < 5; ++b) red[warp][1 + VB + b] = vals[5 + b];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) red[warp][1 + VB + 5 + b] = vals[2 + b];
+  }
+  // chunk bits: qubits VB + 8 .. n - 1 (kMaxQubits of them at most)
+  if (VB + 8 + lane < n) red[warp][1 + VB + 8 + lane] = hi.s;
   __syncthreads();
-  if (tid < kBlkVals) {
+  if (tid <= n) {
     double s = 0.0;
-    for (int w = 0; w < kRedThreads / 32; ++w) s += red[w][tid];
-    blk_part[blockIdx.x * kBlkVals + tid] = s;
+    for (int w = 0; w < kRedWarps; ++w) s += red[w][tid];
+    if (gridDim.x == 1) out[tid] = s;
+    else part[size_t(tid) * gridDim.x + blockIdx.x] = s;
   }
 }
-
-// Final combine: one block.  Low bits from block partials, high bits from
-// segment partials (segment index bit b <-> amplitude bit H + b).
-template <int VB>
-__global__ void __launch_bounds__(1024)
-    k_zsums_final(int n, int nblk, uint64_t nseg, int H, const double* __restrict__ blk_part,
-                  double* __restrict__ seg_part, double* __restrict__ out) {
-  __shared__ double sh[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto block_sum = [&](double v) -> double {
-    v = warp_sum(v);
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (warp == 0) {
-      r = (lane < int(blockDim.x / 32)) ? sh[lane] : 0.0;
-      r = warp_sum(r);
-    }
-    return r;  // valid in thread 0
-  };
-  // low-bit values: index 0 = total, then per amplitude bit
-  // complex64: amp bit 0 -> vals[1]; amp bits 1..8 -> vals[2..9]; bits 9..12 -> vals[10..13]
-  // complex128: amp bits 0..7 -> vals[2..9]; bits 8..11 -> vals[10..13]
-  for (int vi = 0; vi < 14; ++vi) {
-    double s = 0.0;
-    for (int b = tid; b < nblk; b += blockDim.x) s += blk_part[b * kBlkVals + vi];
-    s = block_sum(s);
-    if (tid == 0) {
-      int qbit;
-      if (vi == 0) qbit = -1;
-      else if (vi == 1) qbit = (VB == 1) ? 0 : -2;
-      else if (vi < 10) qbit = VB + (vi - 2);
-      else qbit = VB + 8 + (vi - 10);
-      if (qbit == -1) out[0] = s;
-      else if (qbit >= 0 && qbit < n && qbit < H) out[1 + qbit] = s;
-    }
-  }
-  // High bits: nseg is a power of two (2^(n-H)).  Fold the segment totals in
-  // half, top bit first: at level b the upper half A[2^b .. 2^(b+1)) sums to the
-  // weight of amplitude bit H + b, and A[i] += A[i + 2^b] leaves A[0 .. 2^b)
-  // indexed by the lower segment bits.  In place: at each level every i is
-  // read and written by one thread only; block_sum's barriers order the levels.
-  double* A = seg_part;
-  for (int b = n - H - 1; b >= 0; --b) {
-    const uint64_t half = 1ull << b;
-    KSum acc;
-    for (uint64_t i = tid; i < half; i += blockDim.x) {
-      const double u = A[i + half];
-      acc.add(u);
-      A[i] += u;
-    }
-    const double s = block_sum(acc.s);
-    if (tid == 0) out[1 + H + b] = s;
-  }
-}
-
-static uint64_t seg_vecs() { return kZsSegVecs; }
+static_assert(1 + 1 + 8 <= kMaxQubits + 2, "the chunk's own bits fit the row");
 
 size_t reduce_scratch_bytes(int n) {
-  // worst case complex128: one vector per amplitude
   size_t zs = sizeof(double) * zsums_scratch_doubles(n);
   size_t samp = sizeof(double) * (2 * ((1ull << n) / 4096 + 2) + 64);
   size_t inner = sizeof(double) * (2 * 4096 + 64);
@@ -191,18 +129,15 @@ size_t reduce_scratch_bytes(int n) {
 template <typename Real>
 static cudaError_t zsums_t(const Real* amp, int n, double* scratch, double* out, cudaStream_t s,
                            int num_sms) {
-  constexpr int VB = Tr<Real>::kVecBit;
-  const uint64_t nvec = (1ull << n) >> VB;
-  const uint64_t nvec_eff = nvec ? nvec : 1;
-  const uint64_t nseg = (nvec_eff + seg_vecs() - 1) / seg_vecs();
-  int nblk = int(std::min<uint64_t>(nseg, uint64_t(num_sms) * 4));
-  nblk = std::min(nblk, kZsMaxBlocks);
-  double* blk_part = scratch;
-  double* seg_part = scratch + size_t(kZsMaxBlocks) * kBlkVals;
-  // segment = 4096 vectors = 2^(12 + VB) amplitudes
-  const int H = 12 + VB;
-  k_zsums<Real><<<nblk, kRedThreads, 0, s>>>(amp, n, nseg, blk_part, seg_part);
-  k_zsums_final<VB><<<1, 1024, 0, s>>>(n, nblk, nseg, H, blk_part, seg_part, out);
+  const uint64_t nvec = (1ull << n) >> Tr<Real>::kVecBit;
+  const uint64_t nchunks = std::max<uint64_t>(1, (nvec + kZsChunkVecs - 1) / kZsChunkVecs);
+  // Up to four chunks per warp one block does it all (the second launch costs
+  // about as much as three more chunks per warp); otherwise at least one chunk
+  // per warp, at most three blocks per SM (96 KB of loads in flight per SM).
+  uint64_t nblk = nchunks <= 4 * kRedWarps ? 1 : (nchunks + kRedWarps - 1) / kRedWarps;
+  nblk = std::min<uint64_t>(nblk, std::min<uint64_t>(uint64_t(num_sms) * 3, kZsMaxBlocks));
+  k_zsums<Real><<<unsigned(nblk), kRedThreads, 0, s>>>(amp, n, nchunks, scratch, out);
+  if (nblk > 1) return launch_sum_rows(scratch, n + 1, int(nblk), out, s);
   return cudaGetLastError();
 }
 
@@ -213,54 +148,80 @@ cudaError_t launch_zsums(DType dt, const void* amp, int n, double* scratch, doub
 }
 
 // ---- inner product ----------------------------------------------------------
+// Two consecutive amplitudes of either precision in FP64.
+__device__ __forceinline__ void load_pair(const float* p, uint64_t pair, double* v) {
+  const float4 x = __ldcs(reinterpret_cast<const float4*>(p) + pair);
+  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void load_pair(const double* p, uint64_t pair, double* v) {
+  const double2 x = __ldcs(reinterpret_cast<const double2*>(p) + 2 * pair);
+  const double2 y = __ldcs(reinterpret_cast<const double2*>(p) + 2 * pair + 1);
+  v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+}
+
+// Bound: HBM (both states are read once).  Four pairs of amplitudes per state
+// in flight per thread as 128-bit loads; the eight products of a step are
+// summed plainly and go through the compensated accumulators as one value.
 template <typename RA, typename RB>
 __global__ void __launch_bounds__(kRedThreads)
-    k_inner(const RA* __restrict__ a, const RB* __restrict__ b, uint64_t dim,
-            double* __restrict__ part) {
+    k_inner(const RA* __restrict__ a, const RB* __restrict__ b, uint64_t npairs,
+            double* __restrict__ part, double* __restrict__ out) {
   KSum re, im;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < dim; i += stride) {
-    const double ar = a[2 * i], ai = a[2 * i + 1];
-    const double br = b[2 * i], bi = b[2 * i + 1];
-    re.add(ar * br + ai * bi);
-    im.add(ar * bi - ai * br);
+  const uint64_t stride = uint64_t(gridDim.x) * kRedThreads;
+  uint64_t i = uint64_t(blockIdx.x) * kRedThreads + threadIdx.x;
+  auto step = [&](const double* x, const double* y, double& r, double& m) {
+    r += (x[0] * y[0] + x[1] * y[1]) + (x[2] * y[2] + x[3] * y[3]);
+    m += (x[0] * y[1] - x[1] * y[0]) + (x[2] * y[3] - x[3] * y[2]);
+  };
+  for (; i + 3 * stride < npairs; i += 4 * stride) {
+    double x[4][4], y[4][4], r = 0.0, m = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      load_pair(a, i + k * stride, x[k]);
+      load_pair(b, i + k * stride, y[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) step(x[k], y[k], r, m);
+    re.add(r);
+    im.add(m);
   }
-  __shared__ double sh[2][kRedThreads / 32];
-  double r = warp_sum(re.s), m = warp_sum(im.s);
+  for (; i < npairs; i += stride) {
+    double x[4], y[4], r = 0.0, m = 0.0;
+    load_pair(a, i, x);
+    load_pair(b, i, y);
+    step(x, y, r, m);
+    re.add(r);
+    im.add(m);
+  }
+  __shared__ double sh[2][kRedWarps];
+  const double r = warp_sum(re.s), m = warp_sum(im.s);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) { sh[0][warp] = r; sh[1][warp] = m; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double sr = 0, sm = 0;
-    for (int w = 0; w < kRedThreads / 32; ++w) { sr += sh[0][w]; sm += sh[1][w]; }
-    part[2 * blockIdx.x] = sr;
-    part[2 * blockIdx.x + 1] = sm;
+  if (threadIdx.x < 2) {
+    double t = 0.0;
+    for (int w = 0; w < kRedWarps; ++w) t += sh[threadIdx.x][w];
+    if (gridDim.x == 1) out[threadIdx.x] = t;
+    else part[size_t(threadIdx.x) * gridDim.x + blockIdx.x] = t;
   }
-}
-
-__global__ void k_sum_pairs(const double* __restrict__ part, int nblk, double* __restrict__ out) {
-  // single warp, deterministic order
-  double r = 0, m = 0;
-  for (int i = threadIdx.x; i < nblk; i += 32) { r += part[2 * i]; m += part[2 * i + 1]; }
-  r = warp_sum(r);
-  m = warp_sum(m);
-  if (threadIdx.x == 0) { out[0] = r; out[1] = m; }
 }
 
 cudaError_t launch_inner(DType dta, const void* a, DType dtb, const void* b, int n, double* scratch,
                          double* out, cudaStream_t s, int num_sms) {
-  const uint64_t dim = 1ull << n;
-  int nblk = int(std::min<uint64_t>((dim + kRedThreads - 1) / kRedThreads, uint64_t(num_sms) * 8));
-  nblk = std::max(1, std::min(nblk, 4096));
+  const uint64_t npairs = (1ull << n) >> 1;
+  // one block up to 8 pairs per thread, else at least 4 per thread (one step)
+  uint64_t nblk = npairs <= 8 * kRedThreads ? 1 : (npairs + 4 * kRedThreads - 1) / (4 * kRedThreads);
+  nblk = std::min<uint64_t>(nblk, std::min<uint64_t>(uint64_t(num_sms) * 4, 4096));
+  const unsigned g = unsigned(nblk);
   if (dta == DType::C64 && dtb == DType::C64)
-    k_inner<float, float><<<nblk, kRedThreads, 0, s>>>(static_cast<const float*>(a), static_cast<const float*>(b), dim, scratch);
+    k_inner<float, float><<<g, kRedThreads, 0, s>>>(static_cast<const float*>(a), static_cast<const float*>(b), npairs, scratch, out);
   else if (dta == DType::C64)
-    k_inner<float, double><<<nblk, kRedThreads, 0, s>>>(static_cast<const float*>(a), static_cast<const double*>(b), dim, scratch);
+    k_inner<float, double><<<g, kRedThreads, 0, s>>>(static_cast<const float*>(a), static_cast<const double*>(b), npairs, scratch, out);
   else if (dtb == DType::C64)
-    k_inner<double, float><<<nblk, kRedThreads, 0, s>>>(static_cast<const double*>(a), static_cast<const float*>(b), dim, scratch);
+    k_inner<double, float><<<g, kRedThreads, 0, s>>>(static_cast<const double*>(a), static_cast<const float*>(b), npairs, scratch, out);
   else
-    k_inner<double, double><<<nblk, kRedThreads, 0, s>>>(static_cast<const double*>(a), static_cast<const double*>(b), dim, scratch);
-  k_sum_pairs<<<1, 32, 0, s>>>(scratch, nblk, out);
+    k_inner<double, double><<<g, kRedThreads, 0, s>>>(static_cast<const double*>(a), static_cast<const double*>(b), npairs, scratch, out);
+  if (g > 1) return launch_sum_rows(scratch, 2, int(g), out, s);
   return cudaGetLastError();
 }
 
@@ -298,8 +259,7 @@ __global__ void __launch_bounds__(kRedThreads)
   if (threadIdx.x == 0) {
     double sr = 0;
     for (int w = 0; w < kRedThreads / 32; ++w) sr += sh[w];
-    part[2 * blockIdx.x] = sr;
-    part[2 * blockIdx.x + 1] = 0.0;
+    part[blockIdx.x] = sr;
   }
 }
 
@@ -314,75 +274,119 @@ cudaError_t launch_pauli(DType dt, const void* amp, int n, uint64_t xmask, uint6
     k_pauli<float><<<nblk, kRedThreads, 0, s>>>(static_cast<const float*>(amp), dim, xmask, zmask, ny, scratch);
   else
     k_pauli<double><<<nblk, kRedThreads, 0, s>>>(static_cast<const double*>(amp), dim, xmask, zmask, ny, scratch);
-  k_sum_pairs<<<1, 32, 0, s>>>(scratch, nblk, out);
-  return cudaGetLastError();
+  return launch_sum_rows(scratch, 1, nblk, out, s);
 }
 
 // ---- sampling ---------------------------------------------------------------
 constexpr int kSampSegBits = 12;  // 4096 amplitudes per CDF segment
 
+// Segment sums.  Bound: HBM.  A full segment is 256 threads x 16 amplitudes, all
+// of a thread's 128-bit loads in flight at once (complex64 8, complex128 16);
+// the scalar form moved one 4- or 8-byte load per step.
 template <typename Real>
-__global__ void __launch_bounds__(256)
-    k_seg_probs(const Real* __restrict__ amp, uint64_t dim, uint64_t nseg, int segbits,
-                double* __restrict__ seg_sum) {
-  __shared__ double sh[8];
+__global__ void __launch_bounds__(kRedThreads)
+    k_seg_probs(const Real* __restrict__ amp, uint64_t nseg, int segbits, double* __restrict__ seg_sum) {
+  using V = typename Tr<Real>::V;
+  constexpr int VB = Tr<Real>::kVecBit;
+  constexpr int NV = (1 << (kSampSegBits - VB)) / kRedThreads;
+  __shared__ double sh[kRedWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t seglen = 1ull << segbits;
+  const uint64_t segvec = (1ull << segbits) >> VB;
+  const V* vp = reinterpret_cast<const V*>(amp);
   for (uint64_t sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
-    double acc = 0.0;
-    for (uint64_t k = threadIdx.x; k < seglen; k += blockDim.x) {
-      const uint64_t i = sg * seglen + k;
-      if (i < dim) {
-        const double ar = amp[2 * i], ai = amp[2 * i + 1];
-        acc += ar * ar + ai * ai;
+    V v[NV];
+    const uint64_t b = sg * segvec;
+    if (segvec == uint64_t(NV) * kRedThreads) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[j] = __ldcs(vp + b + threadIdx.x + j * kRedThreads);
+    } else {  // a state of less than one segment
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const uint64_t k = threadIdx.x + uint64_t(j) * kRedThreads;
+        v[j] = V{};
+        if (k < segvec) v[j] = __ldg(vp + b + k);
       }
+    }
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      double p[2];
+      vec_probs<Real>(v[j], p);
+      acc += VB == 1 ? p[0] + p[1] : p[0];
     }
     acc = warp_sum(acc);
     if (lane == 0) sh[warp] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0;
-      for (int w = 0; w < 8; ++w) t += sh[w];
+      for (int w = 0; w < kRedWarps; ++w) t += sh[w];
       seg_sum[sg] = t;
     }
     __syncthreads();
   }
 }
 
-// Inclusive scan of seg_sum into seg_incl (single block, FP64, deterministic).
+// Inclusive scan of seg_sum into seg_incl (single block, FP64, deterministic):
+// tiles of 4 consecutive values per thread with a running carry, so every load
+// is coalesced and a state of 2^24 amplitudes is one tile.
 __global__ void __launch_bounds__(1024)
     k_seg_scan(const double* __restrict__ seg_sum, uint64_t nseg, double* __restrict__ seg_incl) {
-  __shared__ double sh[1024];
-  const uint64_t per = (nseg + blockDim.x - 1) / blockDim.x;
-  const uint64_t b = threadIdx.x * per;
-  const uint64_t e = b + per < nseg ? b + per : nseg;
-  double local = 0.0;
-  for (uint64_t i = b; i < e; ++i) local += seg_sum[i];
-  sh[threadIdx.x] = local;
-  __syncthreads();
-  // Hillis-Steele inclusive scan over the 1024 chunk totals
-  for (int off = 1; off < 1024; off <<= 1) {
-    double v = (threadIdx.x >= unsigned(off)) ? sh[threadIdx.x - off] : 0.0;
+  __shared__ double sh[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double carry = 0.0;
+  for (uint64_t t0 = 0; t0 < nseg; t0 += 4096) {
+    const uint64_t b = t0 + uint64_t(threadIdx.x) * 4;
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = b + k < nseg ? seg_sum[b + k] : 0.0;
+    v[1] += v[0];
+    v[2] += v[1];
+    v[3] += v[2];
+    double sc = v[3];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, sc, o);
+      if (lane >= o) sc += t;
+    }
+    if (lane == 31) sh[warp] = sc;
     __syncthreads();
-    sh[threadIdx.x] += v;
-    __syncthreads();
-  }
-  double run = threadIdx.x ? sh[threadIdx.x - 1] : 0.0;
-  for (uint64_t i = b; i < e; ++i) {
-    run += seg_sum[i];
-    seg_incl[i] = run;
+    double ws = sh[lane];  // every warp scans the 32 warp totals
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, ws, o);
+      if (lane >= o) ws += t;
+    }
+    const double before_warp = __shfl_sync(0xffffffffu, ws, warp ? warp - 1 : 0);
+    const double before_lane = __shfl_up_sync(0xffffffffu, sc, 1);
+    double base = carry;
+    if (warp) base += before_warp;
+    if (lane) base += before_lane;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (b + k < nseg) seg_incl[b + k] = base + v[k];
+    carry += __shfl_sync(0xffffffffu, ws, 31);
+    __syncthreads();  // sh is rewritten by the next tile
   }
 }
 
-// One warp per shot.
+// One warp per shot.  In a segment a step covers 32 lanes x 8 vectors: each lane
+// loads 8 consecutive vectors at once, sums its probabilities serially, and the
+// warp scans the 32 lane totals; the lane whose range holds r then picks the
+// amplitude from its own prefix.  A segment is 8 (complex64) or 16 (complex128)
+// dependent steps instead of 128 of one amplitude per lane.
 template <typename Real>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
     k_sample(const Real* __restrict__ amp, uint64_t dim, int segbits, uint64_t nseg,
              const double* __restrict__ seg_sum, const double* __restrict__ seg_incl,
              const double* __restrict__ u, uint32_t shots, uint64_t* __restrict__ out) {
+  using V = typename Tr<Real>::V;
+  constexpr int VB = Tr<Real>::kVecBit;
+  constexpr int NV = 8, NP = NV << VB;  // vectors and amplitudes of a lane's step
+  const V* vp = reinterpret_cast<const V*>(amp);
   const int lane = threadIdx.x & 31;
   const uint64_t warp_id = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
   const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  const uint64_t nvec = dim >> VB;
   for (uint64_t sh = warp_id; sh < shots; sh += nwarps) {
     const double r = u[sh];
     // first segment whose inclusive prefix exceeds r
@@ -392,39 +396,54 @@ __global__ void __launch_bounds__(256)
       if (seg_incl[mid] > r) hi = mid; else lo = mid + 1;
     }
     uint64_t result = dim - 1;
-    if (lo < nseg) {
-      double run = seg_incl[lo] - seg_sum[lo];
-      bool found = false;
-      for (uint64_t sg = lo; sg < nseg && !found; ++sg) {
-        if (sg != lo) run = seg_incl[sg] - seg_sum[sg];
-        const uint64_t s0 = sg << segbits;
-        const uint64_t s1 = (s0 + (1ull << segbits)) < dim ? s0 + (1ull << segbits) : dim;
-        for (uint64_t base = s0; base < s1; base += 32) {
-          const uint64_t i = base + lane;
-          double p = 0.0;
-          if (i < s1) {
-            const double ar = amp[2 * i], ai = amp[2 * i + 1];
-            p = ar * ar + ai * ai;
-          }
-          // inclusive warp scan
-          double sc = p;
+    bool found = false;
+    for (uint64_t sg = lo; sg < nseg && !found; ++sg) {
+      double run = seg_incl[sg] - seg_sum[sg];
+      const uint64_t v0 = (sg << segbits) >> VB;
+      const uint64_t seg_end = v0 + ((1ull << segbits) >> VB);
+      const uint64_t v1 = seg_end < nvec ? seg_end : nvec;
+      for (uint64_t b = v0; b < v1; b += 32 * NV) {
+        const uint64_t k = b + uint64_t(lane) * NV;
+        V v[NV];
+        if (b + 32 * NV <= v1) {
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            double t = __shfl_up_sync(0xffffffffu, sc, o);
-            if (lane >= o) sc += t;
+          for (int j = 0; j < NV; ++j) v[j] = __ldg(vp + k + j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NV; ++j) {
+            v[j] = V{};
+            if (k + j < v1) v[j] = __ldg(vp + k + j);
           }
-          const double cum = run + sc;
-          const unsigned hit = __ballot_sync(0xffffffffu, (i < s1) && (r < cum));
-          if (hit) {
-            result = base + (__ffs(hit) - 1);
-            found = true;
-            break;
-          }
-          run += __shfl_sync(0xffffffffu, sc, 31);
         }
+        double p[NP];  // inclusive prefix within the lane
+#pragma unroll
+        for (int j = 0; j < NV; ++j) vec_probs<Real>(v[j], p + (j << VB));
+#pragma unroll
+        for (int j = 1; j < NP; ++j) p[j] += p[j - 1];
+        double sc = p[NP - 1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double t = __shfl_up_sync(0xffffffffu, sc, o);
+          if (lane >= o) sc += t;
+        }
+        const double excl = __shfl_up_sync(0xffffffffu, sc, 1);
+        const double base = lane ? run + excl : run;
+        const unsigned hit = __ballot_sync(0xffffffffu, k < v1 && r < base + p[NP - 1]);
+        if (hit) {
+          const int src = __ffs(hit) - 1;
+          int first = NP - 1;
+#pragma unroll
+          for (int j = NP - 2; j >= 0; --j)
+            if (r < base + p[j]) first = j;
+          const uint64_t i = (k << VB) + unsigned(first);
+          result = __shfl_sync(0xffffffffu, i, src);
+          found = true;
+          break;
+        }
+        run += __shfl_sync(0xffffffffu, sc, 31);
       }
     }
-    if (lane == 0) out[sh] = result;
+    if (lane == 0) out[sh] = result < dim ? result : dim - 1;
   }
 }
 
@@ -436,11 +455,11 @@ cudaError_t launch_sample(DType dt, const void* amp, int n, const double* d_unif
   const uint64_t nseg = dim >> segbits;
   double* seg_sum = scratch;
   double* seg_incl = scratch + nseg + 1;
-  const int g1 = int(std::min<uint64_t>(nseg, uint64_t(num_sms) * 8));
+  const int g1 = int(std::min<uint64_t>(nseg, uint64_t(num_sms) * 6));
   if (dt == DType::C64)
-    k_seg_probs<float><<<g1, 256, 0, s>>>(static_cast<const float*>(amp), dim, nseg, segbits, seg_sum);
+    k_seg_probs<float><<<g1, kRedThreads, 0, s>>>(static_cast<const float*>(amp), nseg, segbits, seg_sum);
   else
-    k_seg_probs<double><<<g1, 256, 0, s>>>(static_cast<const double*>(amp), dim, nseg, segbits, seg_sum);
+    k_seg_probs<double><<<g1, kRedThreads, 0, s>>>(static_cast<const double*>(amp), nseg, segbits, seg_sum);
   k_seg_scan<<<1, 1024, 0, s>>>(seg_sum, nseg, seg_incl);
   if (shots == 0) return cudaGetLastError();
   const uint64_t warps = shots;

@@ -35,7 +35,7 @@ namespace nqpu {
 // comes from zsums_scratch_doubles) plus 64 doubles at the end for the n+1 sums.
 constexpr int kNoAllocMaxVecLog2 = 27;
 constexpr size_t kNoAllocSumSlots = 64;
-constexpr size_t kNoAllocScratchDoubles = zsums_scratch_doubles(kNoAllocMaxVecLog2) + kNoAllocSumSlots;
+constexpr size_t kNoAllocScratchDoubles = zsums_scratch_doubles(kNoAllocMaxVecLog2 + 1) + kNoAllocSumSlots;
 static_assert(kNoAllocSumSlots >= size_t(kMaxQubits) + 1, "room for the n+1 sums");
 static_assert(kNoAllocScratchDoubles * sizeof(double) <= (size_t(3) << 20), "modest fixed footprint");
 

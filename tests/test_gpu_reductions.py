@@ -1,0 +1,97 @@
+"""Reductions at the edges of their launch shapes, against plain numpy in FP64.
+
+All sums run in FP64 over at most 2^23 values in trees and compensated
+accumulators; numpy's pairwise sum of the same values is good to a few 2^-53 of
+the sum of magnitudes, and 1e-13 of it leaves two orders of room for either.
+"""
+import numpy as np
+import pytest
+
+from nqpu_b200.state import StateVector
+
+pytestmark = pytest.mark.gpu
+
+
+def random_state(n, dtype, seed):
+    rng = np.random.default_rng(seed)
+    a = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    a *= rng.random(1 << n) < 0.7  # some zero amplitudes
+    a[0] = 1.0
+    a /= np.linalg.norm(a)
+    a = a.astype(np.complex64 if dtype == "c64" else np.complex128).astype(np.complex128)
+    sv = StateVector(n, dtype)
+    sv.set_amplitudes(a)
+    return a, sv
+
+
+# one chunk and less, one block, the step to several blocks, the full grid
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 10, 13, 14, 15, 16, 20, 22])
+def test_z_and_fidelity(n, dtype):
+    a, sv = random_state(n, dtype, n)
+    p = np.abs(a) ** 2
+    idx = np.arange(1 << n)
+    want = [p[(idx >> q) & 1 == 0].sum() - p[(idx >> q) & 1 == 1].sum() for q in range(n)]
+    np.testing.assert_allclose(sv.expectation_z_all(), want, rtol=0, atol=1e-13)
+    for other in ("c64", "c128"):
+        b, sb = random_state(n, other, n + 100)
+        assert abs(sv.fidelity(sb) - abs(np.vdot(a, b)) ** 2) <= 1e-13
+        sb.close()
+    sv.close()
+
+
+# less than a segment, one segment, several, more than one tile of the scan
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 11, 12, 13, 18])
+def test_sample_picks_the_bin(n, dtype):
+    a, sv = random_state(n, dtype, n)
+    p = np.abs(a) ** 2
+    cum = np.cumsum(p)
+    rng = np.random.default_rng(n)
+    pick = np.concatenate([[0], rng.choice(np.nonzero(p)[0], size=500)])
+    u = cum[pick] - 0.5 * p[pick]  # the middle of the bin: 1e-9 from its edges at least
+    pick, u = pick[p[pick] > 1e-9], u[p[pick] > 1e-9]
+    np.testing.assert_array_equal(sv.sample_with_uniforms(u), pick.astype(np.uint64))
+    np.testing.assert_array_equal(sv.sample_with_uniforms([1.0 - 1e-17, 2.0]), [(1 << n) - 1] * 2)
+    sv.close()
+
+
+def pauli_value(a, s):
+    n = len(s)
+    idx = np.arange(1 << n)
+    x = sum(1 << q for q in range(n) if s[q] in "XY")
+    z = sum(1 << q for q in range(n) if s[q] in "ZY")
+    par = idx & z
+    for sh in (16, 8, 4, 2, 1):
+        par = par ^ (par >> sh)
+    v = np.conj(a) * (1 - 2 * (par & 1)) * a[idx ^ x]
+    return float((1j ** s.count("Y") * v.sum()).real)
+
+
+def random_strings(rng, n, count):
+    out = []
+    for i in range(count):
+        w = int(rng.integers(0, min(n, 7) + 1))
+        s = ["I"] * n
+        for q in rng.choice(n, size=w, replace=False):
+            s[q] = "XYZ"[int(rng.integers(3))]
+        out.append("".join(s))
+    return out
+
+
+# fewer qubits than a register set, less than a unit of work, several chunks;
+# 900 strings need more table than the small buffers hold
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n,count", [(1, 8), (3, 20), (4, 60), (5, 60), (8, 900), (11, 60), (12, 60), (13, 60), (23, 12)])
+def test_pauli_sum(n, count, dtype):
+    a, sv = random_state(n, dtype, n)
+    rng = np.random.default_rng(n)
+    strings = random_strings(rng, n, count) + ["I" * n, "Z" * n, "Y" + "Z" * (n - 1), "I" * (n - 1) + "X"]
+    c = rng.normal(size=len(strings))
+    want = np.array([pauli_value(a, s) for s in strings])
+    scale = np.abs(c).sum()
+    assert abs(sv.expectation_pauli_sum(list(zip(c, strings))) - c @ want) <= 1e-13 * scale
+    for s, w in list(zip(strings, want))[-6:]:
+        assert abs(sv.expectation_pauli_string(s) - w) <= 1e-13
+    assert abs(sv.expectation_x(n - 1) - want[-1]) <= 1e-13
+    sv.close()
