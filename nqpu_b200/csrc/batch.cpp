@@ -17,6 +17,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "planner.h"
+#include "tileprog.h"
 
 namespace nqpu {
 
@@ -39,10 +40,9 @@ struct BatchImpl {
   float* d_arena = nullptr;
   BatchCirc* d_circs = nullptr;
   BatchTask* d_tasks = nullptr;
-  unsigned char* d_tables = nullptr;  // one allocation: passes, stages, ops, Ising terms
+  unsigned char* d_tables = nullptr;  // one allocation: passes, programs, Ising terms
   PassRec* d_passes = nullptr;        // (interior pointers of d_tables)
-  StageRec* d_stages = nullptr;
-  TileOp<float>* d_ops = nullptr;
+  ProgWord* d_prog = nullptr;
   double* d_obs = nullptr;
   uint32_t* d_counters = nullptr;
   double* d_partials = nullptr;
@@ -72,7 +72,7 @@ static void batch_release(BatchImpl* b) {
   if (b->h_err) cudaFreeHost(b->h_err);
   b->graph = nullptr;
   b->d_arena = nullptr; b->d_circs = nullptr; b->d_tasks = nullptr; b->d_tables = nullptr; b->d_passes = nullptr;
-  b->d_stages = nullptr; b->d_ops = nullptr; b->d_obs = nullptr; b->d_counters = nullptr;
+  b->d_prog = nullptr; b->d_obs = nullptr; b->d_counters = nullptr;
   b->d_partials = nullptr; b->d_results = nullptr; b->d_cursor = nullptr; b->d_err = nullptr;
   b->h_results = nullptr; b->h_err = nullptr;
   b->built = false;
@@ -133,7 +133,7 @@ static cudaError_t batch_build(BatchImpl* b) {
   uint32_t counters = 0, partials = 0;
   b->n_small = 0;
   // per-circuit tiled plans (independent: built on host threads), then
-  // concatenated with rebased stage/op indices
+  // concatenated with rebased program offsets
   const size_t nc = b->entries.size();
   std::vector<TilePlan> plans(nc);
   std::vector<char> plan_ok(nc, 0);
@@ -143,28 +143,28 @@ static cudaError_t batch_build(BatchImpl* b) {
       const bool small = E.n <= b->small_max;
       const int kmax = small ? 13 : std::min(b->plan_kmax, 13);
       std::string err;
-      plan_ok[ci] = build_tile_plan(lower_circuit(E.gates), E.n, DType::C64, kmax, &plans[ci], &err) &&
+      const std::vector<Op> ops = lower_circuit(E.gates);
+      plan_ok[ci] = build_tile_plan(ops, E.n, DType::C64, kmax, &plans[ci], &err) &&
                     (!small || plans[ci].passes.size() == 1);
+      if (plan_ok[ci]) build_tile_prog(ops, &plans[ci]);
     }
   });
   b->prep_us[0] = since_us(clk);
   // the concatenated tables: offsets per circuit first, then every circuit's
-  // records copied (with rebased stage / op indices) on host threads into
+  // records copied (with rebased program offsets) on host threads into
   // arrays allocated without initialisation
-  std::vector<size_t> pbase(nc + 1, 0), sbase(nc + 1, 0), obase(nc + 1, 0), jbase(nc + 1, 0);
+  std::vector<size_t> pbase(nc + 1, 0), obase(nc + 1, 0), jbase(nc + 1, 0);
   for (size_t ci = 0; ci < nc; ++ci) {
     if (!plan_ok[ci]) return cudaErrorInvalidValue;
     pbase[ci + 1] = pbase[ci] + plans[ci].passes.size();
-    sbase[ci + 1] = sbase[ci] + plans[ci].stages.size();
-    obase[ci + 1] = obase[ci] + plans[ci].ops_f.size();
+    obase[ci + 1] = obase[ci] + plans[ci].prog.size();
     jbase[ci + 1] = jbase[ci] + b->entries[ci].J.size() + b->entries[ci].h.size();
   }
-  if (sbase[nc] > size_t(INT32_MAX) || obase[nc] > size_t(INT32_MAX) || jbase[nc] > size_t(INT32_MAX))
+  if (obase[nc] > size_t(INT32_MAX) || jbase[nc] > size_t(INT32_MAX))
     return cudaErrorInvalidValue;  // the device records index tables with 32-bit offsets
   auto align256 = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t off_s = align256(pbase[nc] * sizeof(PassRec));
-  const size_t off_o = off_s + align256(sbase[nc] * sizeof(StageRec));
-  const size_t off_j = off_o + align256(obase[nc] * sizeof(TileOp<float>));
+  const size_t off_o = align256(pbase[nc] * sizeof(PassRec));
+  const size_t off_j = off_o + align256(obase[nc] * sizeof(ProgWord));
   const size_t table_bytes = off_j + align256(std::max<size_t>(1, jbase[nc]) * sizeof(double));
   std::unique_lock<std::mutex> stage_lock(g_stage.mu);
   if (g_stage.cap < table_bytes) {
@@ -176,8 +176,7 @@ static cudaError_t batch_build(BatchImpl* b) {
     g_stage.cap = table_bytes;
   }
   PassRec* passes = reinterpret_cast<PassRec*>(g_stage.p);
-  StageRec* stages = reinterpret_cast<StageRec*>(g_stage.p + off_s);
-  TileOp<float>* ops = reinterpret_cast<TileOp<float>*>(g_stage.p + off_o);
+  ProgWord* prog = reinterpret_cast<ProgWord*>(g_stage.p + off_o);
   double* obs = reinterpret_cast<double*>(g_stage.p + off_j);
   parallel_ranges(nc, 16, [&](size_t lo, size_t hi) {
     for (size_t ci = lo; ci < hi; ++ci) {
@@ -185,16 +184,9 @@ static cudaError_t batch_build(BatchImpl* b) {
       PassRec* pd = passes + pbase[ci];
       for (size_t i = 0; i < tp.passes.size(); ++i) {
         pd[i] = tp.passes[i];
-        pd[i].stage_begin += int32_t(sbase[ci]);
-        pd[i].stage_end += int32_t(sbase[ci]);
+        pd[i].prog_begin += int32_t(obase[ci]);
       }
-      StageRec* sd = stages + sbase[ci];
-      for (size_t i = 0; i < tp.stages.size(); ++i) {
-        sd[i] = tp.stages[i];
-        sd[i].op_begin += int32_t(obase[ci]);
-        sd[i].op_end += int32_t(obase[ci]);
-      }
-      if (!tp.ops_f.empty()) std::memcpy(ops + obase[ci], tp.ops_f.data(), tp.ops_f.size() * sizeof(TileOp<float>));
+      std::copy(tp.prog.begin(), tp.prog.end(), prog + obase[ci]);
       const BatchEntry& E = b->entries[ci];
       std::copy(E.J.begin(), E.J.end(), obs + jbase[ci]);
       std::copy(E.h.begin(), E.h.end(), obs + jbase[ci] + E.J.size());
@@ -273,8 +265,7 @@ static cudaError_t batch_build(BatchImpl* b) {
   if ((e = upload(&b->d_tasks, tasks)) != cudaSuccess) return e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_tables), table_bytes)) != cudaSuccess) return e;
   b->d_passes = reinterpret_cast<PassRec*>(b->d_tables);
-  b->d_stages = reinterpret_cast<StageRec*>(b->d_tables + off_s);
-  b->d_ops = reinterpret_cast<TileOp<float>*>(b->d_tables + off_o);
+  b->d_prog = reinterpret_cast<ProgWord*>(b->d_tables + off_o);
   b->d_obs = reinterpret_cast<double*>(b->d_tables + off_j);
   if ((e = cudaMemcpyAsync(b->d_tables, g_stage.p, table_bytes, cudaMemcpyHostToDevice, b->stream)) != cudaSuccess)
     return e;
@@ -282,8 +273,8 @@ static cudaError_t batch_build(BatchImpl* b) {
   if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return e;
   stage_lock.unlock();
   b->upload_bytes = circs.size() * sizeof(BatchCirc) + tasks.size() * sizeof(BatchTask) +
-                    pbase[nc] * sizeof(PassRec) + sbase[nc] * sizeof(StageRec) +
-                    obase[nc] * sizeof(TileOp<float>) + jbase[nc] * sizeof(double);
+                    pbase[nc] * sizeof(PassRec) +
+                    obase[nc] * sizeof(ProgWord) + jbase[nc] * sizeof(double);
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_counters), sizeof(uint32_t) * b->n_counters)) != cudaSuccess) return e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_partials), sizeof(double) * std::max<uint32_t>(1, partials))) != cudaSuccess) return e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_results), sizeof(double) * std::max<size_t>(1, circs.size()))) != cudaSuccess) return e;
@@ -296,7 +287,7 @@ static cudaError_t batch_build(BatchImpl* b) {
   // capture: reset counters/cursor/error, the persistent launch, result copies
   BatchLaunch L;
   L.arena = b->d_arena; L.circs = b->d_circs; L.tasks = b->d_tasks; L.n_tasks = b->n_tasks;
-  L.passes = b->d_passes; L.stages = b->d_stages; L.ops = b->d_ops; L.obs = b->d_obs;
+  L.passes = b->d_passes; L.prog = b->d_prog; L.obs = b->d_obs;
   L.counters = b->d_counters; L.partials = b->d_partials; L.results = b->d_results;
   L.cursor = b->d_cursor; L.err = b->d_err;
   L.grid = unsigned(std::max(1, device_sms() * b->ctas_per_sm));

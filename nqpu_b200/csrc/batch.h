@@ -34,8 +34,7 @@ struct BatchLaunch {
   const BatchTask* tasks;
   uint32_t n_tasks;
   const PassRec* passes;
-  const StageRec* stages;
-  const TileOp<float>* ops;
+  const ProgWord* prog;
   const double* obs;
   uint32_t* counters;
   double* partials;

@@ -10,6 +10,7 @@
 #include "kernels.h"
 #include "tcpass.h"
 #include "tcrun.h"
+#include "tileprog.h"
 
 namespace nqpu {
 
@@ -299,9 +300,7 @@ cudaError_t state_upload_c128(StateImpl* s, const NqpuComplex* in) {
 // ---------------------------------------------------------------------------
 static void plan_free(DevicePlan* p) {
   if (!p) return;
-  if (p->d_passes) cudaFree(p->d_passes);
-  if (p->d_stages) cudaFree(p->d_stages);
-  if (p->d_ops) cudaFree(p->d_ops);
+  if (p->d_prog) cudaFree(p->d_prog);
   if (p->fused) fused_plan_free(p->fused);
   if (p->tc) tc_plan_free(p->tc);
   delete p;
@@ -337,8 +336,9 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
   p->stats = PlanStats{};
   if (mode == NQPU_MODE_TILED && int(n) >= tile_min_qubits(dt)) {
     std::string err;
-    p->kmax = tile_kmax_for(dt);
-    if (!build_tile_plan(p->ops, int(n), dt, p->kmax, &p->tile, &err)) return false;
+    p->tile_cfg = tile_config_raw(dt);
+    if (!build_tile_plan_for(p->ops, int(n), dt, &p->tile, &err)) return false;
+    build_tile_prog(p->ops, &p->tile);
     p->stats = p->tile.stats;
   } else if (mode == NQPU_MODE_FUSED) {
     p->stats.ops = p->ops.size();
@@ -375,7 +375,7 @@ int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt) {
   if (!tc_plan_stats(ops, int(n), dt, &ts)) return NQPU_MODE_TILED;
   TilePlan tp;
   std::string err;
-  if (!build_tile_plan(ops, int(n), dt, tile_kmax_for(dt), &tp, &err)) return NQPU_MODE_TENSOR;
+  if (!build_tile_plan_for(ops, int(n), dt, &tp, &err)) return NQPU_MODE_TENSOR;
   double work = 0.0;
   for (const Op& op : ops) {
     switch (op.kind) {
@@ -441,23 +441,16 @@ cudaError_t run_ops_pergate(StateImpl* s, const std::vector<Op>& ops) {
   return cudaSuccess;
 }
 
-static cudaError_t upload_tile(DevicePlan* p) {
-  const TilePlan& t = p->tile;
-  cudaError_t e;
-  const size_t np = std::max<size_t>(1, t.passes.size());
-  const size_t ns = std::max<size_t>(1, t.stages.size());
-  const size_t opsz = t.dt == DType::C64 ? sizeof(TileOp<float>) : sizeof(TileOp<double>);
-  const size_t nops = t.dt == DType::C64 ? t.ops_f.size() : t.ops_d.size();
-  if ((e = cudaMalloc(reinterpret_cast<void**>(&p->d_passes), np * sizeof(PassRec))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(reinterpret_cast<void**>(&p->d_stages), ns * sizeof(StageRec))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&p->d_ops, std::max<size_t>(1, nops) * opsz)) != cudaSuccess) return e;
-  if (!t.passes.empty() && (e = cudaMemcpy(p->d_passes, t.passes.data(), t.passes.size() * sizeof(PassRec), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  if (!t.stages.empty() && (e = cudaMemcpy(p->d_stages, t.stages.data(), t.stages.size() * sizeof(StageRec), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  if (nops) {
-    const void* src = t.dt == DType::C64 ? static_cast<const void*>(t.ops_f.data()) : static_cast<const void*>(t.ops_d.data());
-    if ((e = cudaMemcpy(p->d_ops, src, nops * opsz, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+// The copy is ordered on the stream the plan runs on first and has landed when
+// this returns, so every stream may run the plan afterwards (a plain cudaMemcpy
+// of pageable memory may return before its data reaches the device, and the
+// states' non-blocking streams do not wait for the default stream).
+static cudaError_t upload_tile(DevicePlan* p, cudaStream_t st) {
+  const size_t bytes = p->tile.prog.size() * sizeof(ProgWord);
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p->d_prog), std::max<size_t>(16, bytes));
+  if (e != cudaSuccess || bytes == 0) return e;
+  e = cudaMemcpyAsync(p->d_prog, p->tile.prog.data(), bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
 static cudaError_t mark(std::vector<cudaEvent_t>* ev, cudaStream_t st) {
@@ -515,7 +508,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   const auto key = std::make_tuple(s->n, int(s->dt), effective, si);
   DevicePlan*& p = c->plans[key];
   // rebuild when the circuit changed or the tiled kernel's tile size did
-  if (p && (p->version != c->version || (effective == NQPU_MODE_TILED && p->kmax != tile_kmax_for(s->dt)))) {
+  if (p && (p->version != c->version || (effective == NQPU_MODE_TILED && p->tile_cfg != tile_config_raw(s->dt)))) {
     cudaStreamSynchronize(s->stream);
     plan_free(p);
     p = nullptr;
@@ -528,7 +521,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
       return cudaErrorInvalidValue;
     }
     if (effective == NQPU_MODE_TILED) {
-      cudaError_t e = upload_tile(p);
+      cudaError_t e = upload_tile(p, s->stream);
       if (e != cudaSuccess) {
         plan_free(p);
         p = nullptr;
@@ -557,8 +550,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
     return state_run_error(s);  // bounded-wait expiry flag
   }
   for (size_t i = 0; i < p->tile.passes.size(); ++i) {
-    e = launch_tile_pass(s->dt, s->amp, int(s->n), p->tile.passes[i], p->d_passes, p->d_stages,
-                         p->d_ops, int(i), s->stream, device_sms());
+    e = launch_tile_pass(s->dt, s->amp, p->tile.passes[i], p->d_prog, s->stream, device_sms());
     if (e != cudaSuccess) return e;
     if ((e = mark(events, s->stream)) != cudaSuccess) return e;
   }

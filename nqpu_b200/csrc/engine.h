@@ -72,12 +72,10 @@ struct DevicePlan {
   uint64_t version = ~0ull;
   TilePlan tile;
   std::vector<Op> ops;         // lowered ops (per-gate mode)
-  PassRec* d_passes = nullptr;
-  StageRec* d_stages = nullptr;
-  void* d_ops = nullptr;
+  ProgWord* d_prog = nullptr;
   void* fused = nullptr;       // fused-mode plan (owned by the fused module)
   void* tc = nullptr;          // tensor-core pass plan (owned by tcpass.cu)
-  int kmax = 0;                // tile bits the tiled plan was built for
+  int tile_cfg = 0;            // tile configuration the tiled plan was built for
   PlanStats stats;
 };
 

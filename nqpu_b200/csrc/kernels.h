@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <vector>
+#include "planner.h"
 #include "sv_types.h"
 
 namespace nqpu {
@@ -23,14 +24,17 @@ struct PGArgs {
 cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, cudaStream_t s, int num_sms);
 
 // --- tiled pass path ---------------------------------------------------------
-int tile_kmax_for(DType dt);
-// CTA configuration of the tiled pass kernel (1: one CTA/SM, double-buffered
-// tiles; 2: two CTAs/SM, single-buffered).
+// CTA configuration of the tiled pass kernel (1: one CTA per SM, double-buffered
+// tiles; 2: two CTAs per SM, single-buffered; 4: four on half-size tiles).  get
+// names the default while none is set; raw is 0 then.
 void tile_config_set(DType dt, int minb);
 int tile_config_get(DType dt);
-cudaError_t launch_tile_pass(DType dt, void* amp, int n, const PassRec& host_pass,
-                             const PassRec* d_passes, const StageRec* d_stages, const void* d_ops,
-                             int pass_idx, cudaStream_t stream, int num_sms);
+int tile_config_raw(DType dt);
+// Tiled plan of the tile size in force for the dtype.
+bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err);
+// One pass; d_prog is the plan's program table in device memory.
+cudaError_t launch_tile_pass(DType dt, void* amp, const PassRec& host_pass, const ProgWord* d_prog,
+                             cudaStream_t stream, int num_sms);
 
 // --- state utilities ---------------------------------------------------------
 cudaError_t launch_set_basis(DType dt, void* amp, int n, uint64_t index, cudaStream_t s, int num_sms);

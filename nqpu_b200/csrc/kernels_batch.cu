@@ -33,6 +33,9 @@ namespace nqpu {
 
 constexpr int kBatchK = 13;                       // complex64 tile bits
 constexpr uint32_t kBatchVec = 1u << (kBatchK - 1);
+// Words of a pass's program kept in shared memory (a longer one is read from
+// global memory): what two CTAs per SM leave.
+constexpr int kBatchProgWords = 1152;
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   uint32_t v;
@@ -116,8 +119,8 @@ __device__ __forceinline__ double ising_tile(const float4* __restrict__ sv, int 
 
 __global__ void __launch_bounds__(kTileThreads, 2)
     k_batch(float* __restrict__ arena, const BatchCirc* __restrict__ circs, const BatchTask* __restrict__ tasks,
-            uint32_t n_tasks, const PassRec* __restrict__ passes, const StageRec* __restrict__ stages,
-            const TileOp<float>* __restrict__ ops, const double* __restrict__ obs, uint32_t* __restrict__ counters,
+            uint32_t n_tasks, const PassRec* __restrict__ passes,
+            const uint4* __restrict__ progs, const double* __restrict__ obs, uint32_t* __restrict__ counters,
             double* __restrict__ partials, double* __restrict__ results, uint32_t* __restrict__ cursor,
             int* __restrict__ err, uint32_t spin_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -127,6 +130,13 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   double* hq = lut + 768;                                           // h_i, i < n
   uint32_t* tabs = reinterpret_cast<uint32_t*>(hq + 64);            // stage tables of the current pass
   __shared__ PassRec P;
+  // program of the current pass: behind its stage tables in shared memory, where it fits
+  auto tab_words = [&]() { return (P.stage_end - P.stage_begin) * (kStageTabWords / 4); };
+  auto prog_words = [&]() { return P.prog_words - tab_words(); };
+  auto prog = [&]() -> const uint4* {
+    return prog_words() <= kBatchProgWords ? reinterpret_cast<const uint4*>(tabs) + tab_words()
+                                           : progs + P.prog_begin + tab_words();
+  };
   __shared__ int s_pass;  // global index of the pass whose tables are loaded (-1: none)
   __shared__ uint32_t s_task;
   __shared__ int s_flag;
@@ -154,7 +164,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     for (uint32_t u = tid; u < nvec; u += blockDim.x)
       sv[swz(u)] = (one && u == 0) ? make_float4(1.f, 0.f, 0.f, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  // Pass record, high-offset table and stage tables; consecutive tasks of the
+  // Pass record, high-offset table, stage tables and program; consecutive tasks of the
   // same pass on this CTA reuse them.
   auto load_pass = [&](const BatchCirc& C, int p) {
     const int gp = C.pass_base + p;
@@ -170,7 +180,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         if ((hh >> j) & 1) off |= 1ull << P.qhi[j];
       hi_off[hh] = off;
     }
-    build_pass_tabs<float>(P, stages, tabs);  // ends with a barrier
+    load_pass_prog(P, progs, prog_words() <= kBatchProgWords ? prog_words() : 0, reinterpret_cast<uint4*>(tabs));
     if (tid == 0) s_pass = gp;
     __syncthreads();
   };
@@ -195,7 +205,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       const uint32_t nvec = 1u << (P.k - 1);
       init_tile(nvec, true);
       __syncthreads();
-      run_tile_stages<float, true>(sv, P, tabs, ops, 0u);
+      run_tile_stages<float>(sv, P, tabs, prog(), 0u);
       double jtot;
       load_obs(C, &jtot);
       __syncthreads();
@@ -233,7 +243,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         cp_async_wait0();
       }
       __syncthreads();
-      run_tile_stages<float, true>(sv, P, tabs, ops, ext);
+      run_tile_stages<float>(sv, P, tabs, prog(), ext);
       for (uint32_t u = tid; u < nvec; u += blockDim.x) {
         const uint32_t t = u << 1;
         const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
@@ -279,7 +289,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
 
 size_t batch_smem_bytes() {
   return sizeof(float4) * kBatchVec + sizeof(uint64_t) * kHiOffEntries + sizeof(double) * (768 + 64) +
-         sizeof(uint32_t) * kMaxPassStages * kStageTabWords;
+         sizeof(uint32_t) * kMaxPassStages * kStageTabWords + sizeof(uint4) * kBatchProgWords;
 }
 
 cudaError_t launch_batch(const BatchLaunch& L, cudaStream_t s) {
@@ -292,7 +302,7 @@ cudaError_t launch_batch(const BatchLaunch& L, cudaStream_t s) {
   e = attr.get(dev, [&] { return cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); },
                cudaErrorInvalidDevice);
   if (e != cudaSuccess) return e;
-  k_batch<<<L.grid, kTileThreads, smem, s>>>(L.arena, L.circs, L.tasks, L.n_tasks, L.passes, L.stages, L.ops,
+  k_batch<<<L.grid, kTileThreads, smem, s>>>(L.arena, L.circs, L.tasks, L.n_tasks, L.passes, reinterpret_cast<const uint4*>(L.prog),
                                             L.obs, L.counters, L.partials, L.results, L.cursor, L.err,
                                             L.spin_limit ? L.spin_limit : kBatchSpinLimit);
   return cudaGetLastError();

@@ -24,16 +24,16 @@
 namespace nqpu {
 
 // Dynamic shared memory: [tile buffer 0 | tile buffer 1 | hi_off table
-// (2^(k-c) <= kHiOffEntries u64) | stage tables (kMaxPassStages x kStageTabWords u32)].
+// (2^(k-c) <= kHiOffEntries u64) | stage tables of the pass (kStageTabWords u32
+// each) | the pass's program, prog_smem words (0: read from global memory)].
 // MINB = 1: one persistent CTA per SM; while the stages of tile i run on one
 // buffer, the cp.async copies of tile i+1 stream into the other.  MINB > 1:
 // MINB CTAs per SM with one buffer each hide each other's copies.  Each thread
 // holds 16 vectors, so a CTA has 2^KMAX / (16 x amplitudes per vector) threads.
 template <typename Real, int KMAX, int MINB>
 __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
-    k_tile_pass(Real* __restrict__ amp, const PassRec* __restrict__ passes,
-                const StageRec* __restrict__ stages, const TileOp<Real>* __restrict__ ops,
-                int pass_idx, uint64_t n_tiles) {
+    k_tile_pass(Real* __restrict__ amp, const __grid_constant__ PassRec P, const uint4* __restrict__ progs,
+                int prog_smem, uint64_t n_tiles) {
   using T = Tr<Real>;
   using V = typename T::V;
   constexpr int VB = T::kVecBit;
@@ -46,15 +46,7 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
   V* buf1 = kDoubleBuffer ? buf0 + kMaxVec : buf0;
   uint64_t* hi_off = reinterpret_cast<uint64_t*>(smem_raw + (kDoubleBuffer ? 2 : 1) * sizeof(V) * kMaxVec);
   uint32_t* tabs = reinterpret_cast<uint32_t*>(hi_off + kHiOffEntries);
-  __shared__ PassRec P;
-
   const int tid = threadIdx.x;
-  {
-    const int32_t* src = reinterpret_cast<const int32_t*>(passes + pass_idx);
-    int32_t* dst = reinterpret_cast<int32_t*>(&P);
-    for (int i = tid; i < int(sizeof(PassRec) / 4); i += blockDim.x) dst[i] = src[i];
-  }
-  __syncthreads();
   const int k = P.k, c = P.c;
   const uint32_t nvec = 1u << (k - VB);
   const int nhi = k - c;
@@ -64,7 +56,14 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
       if ((h >> j) & 1) off |= 1ull << P.qhi[j];
     hi_off[h] = off;
   }
-  build_pass_tabs<Real>(P, stages, tabs);  // ends with a barrier
+  load_pass_prog(P, progs, prog_smem, reinterpret_cast<uint4*>(tabs));
+  const int tab_words = (P.stage_end - P.stage_begin) * (kStageTabWords / 4);
+  const uint4* prog = prog_smem ? reinterpret_cast<const uint4*>(tabs) + tab_words : progs + P.prog_begin + tab_words;
+  __syncthreads();
+  // everything above read only the plan's tables: the previous pass of the
+  // state may still be running up to here
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t lowmask = (1u << c) - 1u;
 
   // HBM -> shared, asynchronous (consecutive threads take consecutive vectors).
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
     for (int j = 0; j < P.n_ext; ++j)
       if ((base >> P.ext[j]) & 1ull) ext |= 1u << (k + j);
 
-    run_tile_stages<Real>(sv, P, tabs, ops, ext);
+    run_tile_stages<Real>(sv, P, tabs, prog, ext);
 
     // shared -> HBM
 #pragma unroll
@@ -125,10 +124,19 @@ template <typename Real>
 constexpr int tile_kmax_full() { return sizeof(Real) == 4 ? 13 : 12; }
 
 template <typename Real, int KMAX>
-static size_t tile_smem_bytes(int minb) {
+static size_t tile_smem_base(int minb) {
   using V = typename Tr<Real>::V;
   return (minb == 1 ? 2 : 1) * sizeof(V) * (size_t(1) << (KMAX - Tr<Real>::kVecBit)) +
-         sizeof(uint64_t) * kHiOffEntries + sizeof(uint32_t) * kMaxPassStages * kStageTabWords;
+         sizeof(uint64_t) * kHiOffEntries;
+}
+// Most dynamic shared memory of a CTA when MINB of them share an SM's 227 KB
+// (1 KB each goes to the system, under 1 KB to the static arrays); enough for
+// the tables of the longest pass.
+template <typename Real, int KMAX>
+static size_t tile_smem_max(int minb) {
+  const size_t need = tile_smem_base<Real, KMAX>(minb) + sizeof(uint32_t) * kMaxPassStages * kStageTabWords;
+  const size_t share = size_t(227 * 1024) / size_t(minb) - 2048;
+  return std::max(need, share);
 }
 
 // CTA configuration of the tiled pass kernel per dtype (CTAs per SM):
@@ -136,21 +144,26 @@ static size_t tile_smem_bytes(int minb) {
 //   2: two 64 KB-tile CTAs per SM, one buffer each;
 //   4: four CTAs per SM on 32 KB tiles (one tile bit fewer, half the threads):
 //      more independent CTAs to overlap each other's barriers and copies, at
-//      the price of more passes.
-// Plans are built for the configuration's tile size (tile_kmax_for).
-// Defaults measured on B200 (28-qubit brickwork): complex64 runs fastest with
-// four 32 KB-tile CTAs per SM, complex128 with one double-buffered CTA (its
-// 2-CTA build spills registers).
-static int g_tile_minb[2] = {4, 1};
+//      the price of more passes;
+//   0: not set: chosen per plan and launch.
+//     complex64: 4, or 2 for a plan on 13-bit tiles (build_tile_plan_for).
+//     complex128: 1 while there is at most one tile per SM (no spills at 218
+//     registers: a 13-qubit ansatz takes 123 us against 134), else 2 (four warps
+//     per scheduler instead of two hide the dependency waits: 25-qubit ansatz
+//     6.6 against 9.1 ms, 20-qubit brickwork 618 against 718 us).
+static int g_tile_minb[2] = {0, 0};
 
 void tile_config_set(DType dt, int minb) {
   g_tile_minb[dt == DType::C64 ? 0 : 1] = (minb == 4) ? 4 : (minb == 2) ? 2 : 1;
 }
-int tile_config_get(DType dt) { return g_tile_minb[dt == DType::C64 ? 0 : 1]; }
+int tile_config_raw(DType dt) { return g_tile_minb[dt == DType::C64 ? 0 : 1]; }
+int tile_config_get(DType dt) {
+  const int c = tile_config_raw(dt);
+  return c ? c : dt == DType::C64 ? 4 : 1;
+}
 
 template <typename Real, int KMAX, int MINB>
-cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const PassRec* d_passes,
-                                 const StageRec* d_stages, const TileOp<Real>* d_ops, int pass_idx,
+cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const ProgWord* d_prog,
                                  cudaStream_t stream, int num_sms) {
   // a plan built for larger tiles than this kernel holds must not run on it,
   // nor one whose tables exceed the shared-memory copies
@@ -159,11 +172,19 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Pass
     return cudaErrorInvalidValue;
   auto kern = k_tile_pass<Real, KMAX, MINB>;
   constexpr int kThreads = (1 << (KMAX - Tr<Real>::kVecBit)) / kVecPerThread;
-  // shared memory of this launch: the tile buffer(s), the high-offset table and
-  // the stage tables of this pass only (more CTAs fit when passes are short)
-  const size_t smem_max = tile_smem_bytes<Real, KMAX>(MINB);
-  const size_t smem = smem_max - sizeof(uint32_t) * kStageTabWords *
-                                     size_t(kMaxPassStages - (host_pass.stage_end - host_pass.stage_begin));
+  // shared memory of this launch: the tile buffer(s), the high-offset table, the
+  // stage tables of this pass and, where it fits beside them in MINB CTAs per
+  // SM, its program (a single-tile CTA would wait for each op's first read
+  // from L2 otherwise)
+  const size_t smem_max = tile_smem_max<Real, KMAX>(MINB);
+  size_t smem = tile_smem_base<Real, KMAX>(MINB) +
+                sizeof(uint32_t) * kStageTabWords * size_t(host_pass.stage_end - host_pass.stage_begin);
+  const int words = host_pass.prog_words - (host_pass.stage_end - host_pass.stage_begin) * (kStageTabWords / 4);
+  int prog_smem = 0;
+  if (smem + sizeof(ProgWord) * size_t(words) <= smem_max) {
+    prog_smem = words;
+    smem += sizeof(ProgWord) * size_t(prog_smem);
+  }
   // the shared-memory limit is a per-device attribute: set once per device
   static PerDeviceOnce<cudaError_t> attr;
   int dev = 0;
@@ -175,42 +196,65 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Pass
   const uint64_t n_tiles = 1ull << host_pass.n_out;
   const uint64_t max_ctas = uint64_t(num_sms) * MINB;
   const unsigned grid = unsigned(n_tiles < max_ctas ? n_tiles : max_ctas);
-  kern<<<grid, kThreads, smem, stream>>>(amp, d_passes, d_stages, d_ops, pass_idx, n_tiles);
-  return cudaGetLastError();
+  // The pass may start while the kernel before it on the stream drains (its CTAs
+  // load their tables, then wait for that kernel to complete).
+  cudaLaunchAttribute pdl{};
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, amp, host_pass, reinterpret_cast<const uint4*>(d_prog), prog_smem, n_tiles);
 }
 
 template <typename Real>
-cudaError_t launch_tile_pass_t(Real* amp, int n, const PassRec& host_pass, const PassRec* d_passes,
-                               const StageRec* d_stages, const TileOp<Real>* d_ops, int pass_idx,
-                               cudaStream_t stream, int num_sms) {
-  (void)n;
+static cudaError_t launch_tile_pass_t(Real* amp, const PassRec& host_pass, const ProgWord* d_prog,
+                                      cudaStream_t stream, int num_sms) {
   constexpr int K = tile_kmax_full<Real>();
-  switch (g_tile_minb[sizeof(Real) == 4 ? 0 : 1]) {
-    case 4:
-      return launch_tile_pass_cfg<Real, K - 1, 4>(amp, host_pass, d_passes, d_stages, d_ops, pass_idx, stream,
-                                                  num_sms);
-    case 2:
-      return launch_tile_pass_cfg<Real, K, 2>(amp, host_pass, d_passes, d_stages, d_ops, pass_idx, stream, num_sms);
-    default:
-      return launch_tile_pass_cfg<Real, K, 1>(amp, host_pass, d_passes, d_stages, d_ops, pass_idx, stream, num_sms);
+  int cfg = g_tile_minb[sizeof(Real) == 4 ? 0 : 1];
+  if (cfg == 0) {
+    if (sizeof(Real) == 4) cfg = host_pass.k == K ? 2 : 4;
+    else cfg = (1ull << host_pass.n_out) <= uint64_t(num_sms) ? 1 : 2;
+  }
+  switch (cfg) {
+    case 4: return launch_tile_pass_cfg<Real, K - 1, 4>(amp, host_pass, d_prog, stream, num_sms);
+    case 2: return launch_tile_pass_cfg<Real, K, 2>(amp, host_pass, d_prog, stream, num_sms);
+    default: return launch_tile_pass_cfg<Real, K, 1>(amp, host_pass, d_prog, stream, num_sms);
   }
 }
 
-cudaError_t launch_tile_pass(DType dt, void* amp, int n, const PassRec& host_pass,
-                             const PassRec* d_passes, const StageRec* d_stages, const void* d_ops,
-                             int pass_idx, cudaStream_t stream, int num_sms) {
-  if (dt == DType::C64)
-    return launch_tile_pass_t<float>(static_cast<float*>(amp), n, host_pass, d_passes, d_stages,
-                                     static_cast<const TileOp<float>*>(d_ops), pass_idx, stream,
-                                     num_sms);
-  return launch_tile_pass_t<double>(static_cast<double*>(amp), n, host_pass, d_passes, d_stages,
-                                    static_cast<const TileOp<double>*>(d_ops), pass_idx, stream,
-                                    num_sms);
+cudaError_t launch_tile_pass(DType dt, void* amp, const PassRec& host_pass, const ProgWord* d_prog,
+                             cudaStream_t stream, int num_sms) {
+  if (dt == DType::C64) return launch_tile_pass_t<float>(static_cast<float*>(amp), host_pass, d_prog, stream, num_sms);
+  return launch_tile_pass_t<double>(static_cast<double*>(amp), host_pass, d_prog, stream, num_sms);
 }
 
-int tile_kmax_for(DType dt) {
+static int tile_kmax_for(DType dt) {
   const int full = dt == DType::C64 ? 13 : 12;
   return tile_config_get(dt) == 4 ? full - 1 : full;
+}
+
+// From this size on a complex64 pass is long enough (32 MB of state) for its HBM
+// time to matter and for a second plan to be worth building.
+constexpr int kWideTileMinQubits = 22;
+
+// Complex64 tiles of 2^12 amplitudes are the better ones per pass (four CTAs of
+// 128 threads against two of 256: 3 % on a 24-qubit brickwork of 13 / 12 passes),
+// 2^13 save passes: taken when they save at least a fifth (27-qubit phase
+// estimation 7 instead of 10 passes, 7.5 against 8.3 ms; 25-qubit Ising
+// evolution 7 instead of 9, 3.35 against 3.53 ms; a 26-qubit brickwork, 13
+// instead of 15, would lose 2.5 %).
+bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err) {
+  if (!build_tile_plan(ops, n, dt, tile_kmax_for(dt), out, err)) return false;
+  if (dt != DType::C64 || tile_config_raw(dt) != 0 || n < kWideTileMinQubits || out->passes.size() < 2) return true;
+  TilePlan wide;
+  if (build_tile_plan(ops, n, dt, 13, &wide, err) && 5 * wide.passes.size() <= 4 * out->passes.size())
+    *out = std::move(wide);
+  return true;
 }
 
 }  // namespace nqpu

@@ -263,28 +263,6 @@ static TileOp<Real> encode_op(const Op& o, const int* tile_pos, const int* reg_o
     t.m[2 * i] = Real(o.m[i].real());
     t.m[2 * i + 1] = Real(o.m[i].imag());
   }
-  // flat dispatch code: 1 + b for a dense 1q gate on register bit b without
-  // register controls, 8 + 8 b + v for X on register bit b with at most one
-  // register control (v = 0: none, else its register bit + 1)
-  if (o.kind == OP_U1 && t.creg == 0) t.fast = uint8_t(1 + t.rb0);
-  if (o.kind == OP_X1 && (t.creg & (t.creg - 1)) == 0) {
-    int v = 0;
-    if (t.creg) {
-      v = 1;
-      while (!((t.creg >> (v - 1)) & 1u)) ++v;
-    }
-    t.fast = uint8_t(8 + 8 * t.rb0 + v);
-  }
-  // Diagonal shapes (read by the batch executor, whose HEA circuits are two
-  // thirds diagonal ops; d = register bit, nrb for a thread-level bit):
-  //   48 + d           diag(d0, d1) on bit d, no controls
-  //   128 + creg       phase on register mask creg (controls outside the registers: tc)
-  //   160 + 8 d0 + d1  diagonal on bits (d0, d1), no controls
-  const int nrb = sizeof(Real) == 4 ? 5 : 4;
-  auto dbit = [&](uint8_t d) { return d == 0xFF ? nrb : int(d); };
-  if (o.kind == OP_D1 && t.creg == 0 && t.cnr == 0) t.fast2 = uint8_t(48 + dbit(t.dreg0));
-  if (o.kind == OP_PH) t.fast2 = uint8_t(128 + t.creg);
-  if (o.kind == OP_D2 && t.creg == 0 && t.cnr == 0) t.fast2 = uint8_t(160 + 8 * dbit(t.dreg0) + dbit(t.dreg1));
   return t;
 }
 
@@ -297,6 +275,8 @@ bool build_tile_plan(const std::vector<Op>& ops, int n, DType dt, int kmax, Tile
   out->stages.clear();
   out->ops_f.clear();
   out->ops_d.clear();
+  out->op_src.clear();
+  out->prog.clear();
   if (n < tile_min_qubits(dt)) {
     if (err) *err = "state too small for the tiled kernel";
     return false;
@@ -527,6 +507,7 @@ bool build_tile_plan(const std::vector<Op>& ops, int n, DType dt, int kmax, Tile
       for (size_t i = 0; i < order.size(); ++i) S.tpos[i] = order[i];
       S.op_begin = int(dt == DType::C64 ? out->ops_f.size() : out->ops_d.size());
       for (int idx : sops) {
+        out->op_src.push_back(idx);
         if (dt == DType::C64)
           out->ops_f.push_back(encode_op<float>(ops[idx], tile_pos, reg_of_tile, ext_of_qubit, k));
         else

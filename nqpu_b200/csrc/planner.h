@@ -65,6 +65,8 @@ struct TilePlan {
   std::vector<StageRec> stages;
   std::vector<TileOp<float>> ops_f;
   std::vector<TileOp<double>> ops_d;
+  std::vector<int32_t> op_src;  // the op each entry of ops_f / ops_d encodes
+  std::vector<ProgWord> prog;   // compiled stages (build_tile_prog)
   PlanStats stats;
 };
 

@@ -41,6 +41,7 @@
 #include "kernels.h"
 #include "planner.h"
 #include "tcrun.h"
+#include "tileprog.h"
 
 namespace nqpu {
 namespace {
@@ -115,8 +116,8 @@ struct Request {
   TcPlan tcplan;
   std::vector<size_t> bmat_off;        // B operands of each pass, in halves after off_stages
   std::vector<Op> ops;                 // per-gate path (states below the tiled minimum)
-  std::vector<unsigned char> tables;   // passes | stages | ops, kTableAlign-aligned parts
-  size_t off_stages = 0, off_ops = 0;
+  std::vector<unsigned char> tables;   // tensor: passes | B operands (kTableAlign-aligned); tiled: programs
+  size_t off_stages = 0;
   double t_submit = 0, t_admit = 0, t_done = 0;
   std::vector<double> z;
   std::vector<uint64_t> outcomes;
@@ -219,13 +220,9 @@ cudaError_t launch_request(ServerImpl* sv, Lane& L, Request& r) {
     if ((e = cudaMemcpyAsync(L.h_tcerr, L.d_tcerr, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return e;
   } else if (r.tiled) {
-    const PassRec* dp = reinterpret_cast<const PassRec*>(L.d_tab);
-    const StageRec* ds = reinterpret_cast<const StageRec*>(L.d_tab + r.off_stages);
-    const void* dops = L.d_tab + r.off_ops;
-    for (size_t i = 0; i < r.plan.passes.size(); ++i)
-      if ((e = launch_tile_pass(DType::C64, amp, int(r.n), r.plan.passes[i], dp, ds, dops, int(i), st,
-                                sv->sms)) != cudaSuccess)
-        return e;
+    const ProgWord* dprog = reinterpret_cast<const ProgWord*>(L.d_tab);
+    for (const PassRec& P : r.plan.passes)
+      if ((e = launch_tile_pass(DType::C64, amp, P, dprog, st, sv->sms)) != cudaSuccess) return e;
   } else {
     for (const Op& op : r.ops)
       if ((e = launch_pergate(DType::C64, amp, int(r.n), op, st, sv->sms)) != cudaSuccess) return e;
@@ -489,19 +486,13 @@ extern "C" NqpuError nqpu_server_submit(NqpuServer* server, const NqpuCircuit* c
     r->tcplan.bmats.shrink_to_fit();
   } else if (int(c->n) >= tile_min_qubits(DType::C64)) {
     std::string err;
-    if (!build_tile_plan(ops, int(c->n), DType::C64, tile_kmax_for(DType::C64), &r->plan, &err))
+    if (!build_tile_plan_for(ops, int(c->n), DType::C64, &r->plan, &err))
       return NQPU_INVALID_PARAMETER;
+    build_tile_prog(ops, &r->plan);
     r->tiled = true;
-    const TilePlan& p = r->plan;
-    const size_t bp = p.passes.size() * sizeof(PassRec);
-    const size_t bs = p.stages.size() * sizeof(StageRec);
-    const size_t bo = p.ops_f.size() * sizeof(TileOp<float>);
-    r->off_stages = align_up(bp);
-    r->off_ops = r->off_stages + align_up(bs);
-    r->tables.assign(r->off_ops + std::max<size_t>(bo, 1), 0);
-    if (bp) std::memcpy(r->tables.data(), p.passes.data(), bp);
-    if (bs) std::memcpy(r->tables.data() + r->off_stages, p.stages.data(), bs);
-    if (bo) std::memcpy(r->tables.data() + r->off_ops, p.ops_f.data(), bo);
+    const size_t bytes = r->plan.prog.size() * sizeof(ProgWord);
+    r->tables.assign(std::max<size_t>(bytes, 1), 0);
+    if (bytes) std::memcpy(r->tables.data(), r->plan.prog.data(), bytes);
   } else {
     r->ops = std::move(ops);
   }

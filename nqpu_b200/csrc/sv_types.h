@@ -93,7 +93,7 @@ struct PassRec {
   int32_t n_ext;
   int32_t ext[32];           // qubit of virtual bit k+j
   int32_t stage_begin, stage_end;
-  int32_t pad[2];
+  int32_t prog_begin, prog_words;  // stage tables and programs (in the ProgWord table)
 };
 
 // Permutation ops (X, CNOT with at most one control, SWAP) are not executed in
@@ -114,13 +114,18 @@ struct StageRec {
   int32_t n_tbits;           // thread-index bits in use
   int32_t tpos[24];          // tile-local VECTOR bit position of thread-index bit j
   int32_t op_begin, op_end;  // range in the op table
-  int32_t pad;
+  int32_t prog_begin;        // program words, relative to the pass's first
   int32_t scol[5];
   int32_t sbx;
   int32_t ncond;
   uint32_t cond_cnr[kMaxCondPerm];
   int32_t cond_w[kMaxCondPerm];
-  int32_t pad2;
+  int32_t prog_end;
+};
+
+// One word of the stage programs the tile kernels run (encoding: tileprog.h).
+struct alignas(16) ProgWord {
+  uint32_t w[4];
 };
 
 // Device op of a stage.  Register-bit numbering: complex64 register bit 0 is
@@ -132,8 +137,7 @@ struct TileOp {
   uint8_t rb0, rb1;     // register target bits (dense ops)
   uint8_t creg;         // mask over register bits: controls held in registers
   uint8_t dreg0, dreg1; // register bit of diagonal qubit 0/1, 0xFF when not a register bit
-  uint8_t fast;         // flat dispatch code of the common cases (0: decode the fields)
-  uint8_t fast2;        // flat dispatch code of the diagonal shapes (read by the batch executor)
+  uint8_t pad0[2];
   uint32_t cnr;         // virtual-index mask of controls not in registers
   uint32_t dv0, dv1;    // virtual-index mask of diagonal qubit 0/1 when not a register bit
   uint32_t pad1[3];     // header is 32 B so m[] is 16-byte aligned

@@ -3,6 +3,7 @@
 // executor and async-copy helpers.  Included by .cu files only.
 #pragma once
 #include "sv_device.cuh"
+#include "tileprog.h"
 
 namespace nqpu {
 
@@ -37,14 +38,14 @@ __device__ __forceinline__ void ldc2(const Real* __restrict__ p, typename Tr<Rea
                                      typename Tr<Real>::C& b);
 template <>
 __device__ __forceinline__ void ldc2<float>(const float* __restrict__ p, float2& a, float2& b) {
-  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  const float4 v = *reinterpret_cast<const float4*>(p);
   a = make_float2(v.x, v.y);
   b = make_float2(v.z, v.w);
 }
 template <>
 __device__ __forceinline__ void ldc2<double>(const double* __restrict__ p, double2& a, double2& b) {
-  a = __ldg(reinterpret_cast<const double2*>(p));
-  b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  a = *reinterpret_cast<const double2*>(p);
+  b = *(reinterpret_cast<const double2*>(p) + 1);
 }
 
 // complex product on a register amplitude: packed FFMA2 form for complex64
@@ -149,76 +150,76 @@ __device__ __forceinline__ void dispatch_x1_ctrl(C (&a)[NA], uint32_t creg, bool
   }
 }
 
+// real 2x2 (RY, H, ...): no re/im mixing, two packed operations per amplitude
+template <typename C, int NA, int B>
+__device__ __forceinline__ void rb_u1_real(C (&a)[NA], decltype(C::x) m00, decltype(C::x) m01, decltype(C::x) m10,
+                                           decltype(C::x) m11) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    if (i & (1 << B)) continue;
+    const int j = i | (1 << B);
+    const C x = a[i], y = a[j];
+    if constexpr (sizeof(m00) == 4) {
+      a[i] = __ffma2_rn(make_float2(m01, m01), y, __fmul2_rn(make_float2(m00, m00), x));
+      a[j] = __ffma2_rn(make_float2(m11, m11), y, __fmul2_rn(make_float2(m10, m10), x));
+    } else {
+      a[i].x = m00 * x.x + m01 * y.x;
+      a[i].y = m00 * x.y + m01 * y.y;
+      a[j].x = m10 * x.x + m11 * y.x;
+      a[j].y = m10 * x.y + m11 * y.y;
+    }
+  }
+}
+
+// 2x2 with a real diagonal and an imaginary off-diagonal i m01, i m10 (RX, Y)
+template <typename C, int NA, int B>
+__device__ __forceinline__ void rb_u1_cross(C (&a)[NA], decltype(C::x) m00, decltype(C::x) m01, decltype(C::x) m10,
+                                            decltype(C::x) m11) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    if (i & (1 << B)) continue;
+    const int j = i | (1 << B);
+    const C x = a[i], y = a[j];
+    if constexpr (sizeof(m00) == 4) {
+      a[i] = __ffma2_rn(make_float2(-m01, m01), swap_ri(y), __fmul2_rn(make_float2(m00, m00), x));
+      a[j] = __ffma2_rn(make_float2(-m10, m10), swap_ri(x), __fmul2_rn(make_float2(m11, m11), y));
+    } else {
+      a[i].x = m00 * x.x - m01 * y.y;
+      a[i].y = m00 * x.y + m01 * y.x;
+      a[j].x = m11 * y.x - m10 * x.y;
+      a[j].y = m11 * y.y + m10 * x.x;
+    }
+  }
+}
+
 // phase m on the register amplitudes whose bits CMASK are all set
 template <typename C, int NA, int CMASK>
-__device__ __forceinline__ void rb_ph(C (&a)[NA], C m, bool neg) {
+__device__ __forceinline__ void rb_ph(C (&a)[NA], C m) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i)
+    if ((i & CMASK) == CMASK) a[i] = rmul(m, a[i]);
+}
+
+// diag(d0, d1) on register bit B
+template <typename C, int NA, int B>
+__device__ __forceinline__ void rb_d1(C (&a)[NA], C d0, C d1) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i) a[i] = rmul((i & (1 << B)) ? d1 : d0, a[i]);
+}
+
+// sign flip (s = 0 or the sign bit) of the register amplitudes with bits CMASK
+template <typename C, int NA, int CMASK>
+__device__ __forceinline__ void rb_sign(C (&a)[NA], uint32_t s) {
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
     if ((i & CMASK) != CMASK) continue;
-    if (neg) {
-      a[i].x = -a[i].x;
-      a[i].y = -a[i].y;
+    if constexpr (sizeof(a[0].x) == 4) {
+      a[i].x = __uint_as_float(__float_as_uint(a[i].x) ^ s);
+      a[i].y = __uint_as_float(__float_as_uint(a[i].y) ^ s);
     } else {
-      a[i] = rmul(m, a[i]);
+      a[i].x = __hiloint2double(__double2hiint(a[i].x) ^ int(s), __double2loint(a[i].x));
+      a[i].y = __hiloint2double(__double2hiint(a[i].y) ^ int(s), __double2loint(a[i].y));
     }
-  }
-}
-
-// diag(d0, d1) selected by register bit DB (DB == NA_BITS: the thread-level bit tb)
-template <typename C, int NA, int DB, int NRB>
-__device__ __forceinline__ void rb_d1(C (&a)[NA], C d0, C d1, uint32_t tb) {
-  if constexpr (DB >= NRB) {
-    const C d = csel(tb != 0, d1, d0);
-#pragma unroll
-    for (int i = 0; i < NA; ++i) a[i] = rmul(d, a[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < NA; ++i) a[i] = rmul((i & (1 << DB)) ? d1 : d0, a[i]);
-  }
-}
-
-// diag on two bits (register bit or thread-level bit when >= NRB)
-template <typename C, int NA, int D0, int D1, int NRB>
-__device__ __forceinline__ void rb_d2(C (&a)[NA], const C* m, uint32_t tb0, uint32_t tb1) {
-  if constexpr (D0 >= NRB && D1 >= NRB) {
-    const C lo = csel(tb0 != 0, m[1], m[0]);
-    const C hi = csel(tb0 != 0, m[3], m[2]);
-    const C d = csel(tb1 != 0, hi, lo);
-#pragma unroll
-    for (int i = 0; i < NA; ++i) a[i] = rmul(d, a[i]);
-  } else if constexpr (D0 >= NRB) {
-    const C lo = csel(tb0 != 0, m[1], m[0]);
-    const C hi = csel(tb0 != 0, m[3], m[2]);
-#pragma unroll
-    for (int i = 0; i < NA; ++i) a[i] = rmul((i & (1 << D1)) ? hi : lo, a[i]);
-  } else if constexpr (D1 >= NRB) {
-    const C lo = csel(tb1 != 0, m[2], m[0]);
-    const C hi = csel(tb1 != 0, m[3], m[1]);
-#pragma unroll
-    for (int i = 0; i < NA; ++i) a[i] = rmul((i & (1 << D0)) ? hi : lo, a[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      const int k = ((i >> D0) & 1) | (((i >> D1) & 1) << 1);
-      a[i] = rmul(m[k], a[i]);
-    }
-  }
-}
-
-// generic diagonal with controls: d selected per amplitude at run time
-template <typename C, int NA>
-__device__ __forceinline__ void rb_diag_generic(C (&a)[NA], const C* m, int nd, uint32_t dreg0,
-                                                uint32_t dreg1, uint32_t tb0, uint32_t tb1, bool tc,
-                                                uint32_t creg) {
-#pragma unroll
-  for (int i = 0; i < NA; ++i) {
-    const bool cond = tc && ((uint32_t(i) & creg) == creg);
-    const uint32_t b0 = (dreg0 != 0xFF) ? ((uint32_t(i) >> dreg0) & 1u) : tb0;
-    const uint32_t b1 = (nd > 1) ? ((dreg1 != 0xFF) ? ((uint32_t(i) >> dreg1) & 1u) : tb1) : 0u;
-    const C lo = csel(b0 != 0, m[1], m[0]);
-    const C hi = csel(b0 != 0, m[3], m[2]);
-    const C d = csel(b1 != 0, hi, lo);
-    a[i] = csel(cond, cmul(d, a[i]), a[i]);
   }
 }
 
@@ -263,29 +264,6 @@ __device__ __forceinline__ void rb_sw(C (&a)[NA], bool tc, uint32_t creg) {
 // ---- dispatch helpers ------------------------------------------------------
 #define NQ_REG_CASES(M, ...) M(0, __VA_ARGS__) M(1, __VA_ARGS__) M(2, __VA_ARGS__) M(3, __VA_ARGS__) M(4, __VA_ARGS__)
 
-template <typename C, int NA, int NRB>
-__device__ __forceinline__ void dispatch_ph(C (&a)[NA], uint32_t creg, C m, bool neg) {
-  switch (creg) {
-#define NQ_PHC(V) case V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, m, neg); break;
-    NQ_PHC(0) NQ_PHC(1) NQ_PHC(2) NQ_PHC(3) NQ_PHC(4) NQ_PHC(5) NQ_PHC(6) NQ_PHC(7)
-    NQ_PHC(8) NQ_PHC(9) NQ_PHC(10) NQ_PHC(11) NQ_PHC(12) NQ_PHC(13) NQ_PHC(14) NQ_PHC(15)
-    NQ_PHC(16) NQ_PHC(17) NQ_PHC(18) NQ_PHC(19) NQ_PHC(20) NQ_PHC(21) NQ_PHC(22) NQ_PHC(23)
-    NQ_PHC(24) NQ_PHC(25) NQ_PHC(26) NQ_PHC(27) NQ_PHC(28) NQ_PHC(29) NQ_PHC(30) NQ_PHC(31)
-#undef NQ_PHC
-    default: break;
-  }
-}
-
-template <typename C, int NA, int NRB, int D0>
-__device__ __forceinline__ void dispatch_d2_b(C (&a)[NA], int d1, const C* m, uint32_t tb0, uint32_t tb1) {
-  switch (d1) {
-#define NQ_D2B(V) case V: if constexpr (V <= NRB && (V != D0 || V == NRB)) rb_d2<C, NA, D0, V, NRB>(a, m, tb0, tb1); break;
-    NQ_D2B(0) NQ_D2B(1) NQ_D2B(2) NQ_D2B(3) NQ_D2B(4) NQ_D2B(5)
-#undef NQ_D2B
-    default: break;
-  }
-}
-
 template <typename Real, typename C, int NA, int NRB, int B0>
 __device__ __forceinline__ void dispatch_u2_b(C (&a)[NA], int b1, const Real* mp, bool tc, uint32_t creg) {
   switch (b1) {
@@ -306,207 +284,183 @@ __device__ __forceinline__ void dispatch_sw_b(C (&a)[NA], int b1, bool tc, uint3
   }
 }
 
-// Apply ops [ob, oe) of a stage to the thread's register block.
-// vbase = virtual index of register amplitude 0 (register bits are zero in it).
-template <typename Real, int NA, int NRB, bool kDiagFlat = false>
-__device__ __forceinline__ void apply_stage_ops(typename Tr<Real>::C (&a)[NA],
-                                                const TileOp<Real>* __restrict__ ops, int ob,
-                                                int oe, uint32_t vbase) {
+// Ops a stage program holds as TileOp records: 1q gates with register controls,
+// X with register controls in the middle of a stage, SWAP and 4x4 matrices.
+template <typename Real, int NA, int NRB>
+__device__ __forceinline__ void apply_record(typename Tr<Real>::C (&a)[NA], const TileOp<Real>* op, uint32_t vbase) {
   using C = typename Tr<Real>::C;
-  // software pipeline: the next op's header and first four matrix entries are
-  // loaded while the current op runs
-  uint4 nh = make_uint4(0, 0, 0, 0);
-  uint32_t ndv1 = 0;
-  C nm[4];
-  auto fetch = [&](int o) {
-    const TileOp<Real>* op = ops + o;
-    nh = __ldg(reinterpret_cast<const uint4*>(op));
-    ndv1 = __ldg(reinterpret_cast<const uint32_t*>(op) + 4);
-    ldc2<Real>(op->m, nm[0], nm[1]);
-    ldc2<Real>(op->m + 4, nm[2], nm[3]);
-  };
-  if (ob < oe) fetch(ob);
-  for (int o = ob; o < oe; ++o) {
-    const TileOp<Real>* op = ops + o;
-    const uint4 h0 = nh;
-    const uint32_t dv1 = ndv1;
-    const C pm0 = nm[0], pm1 = nm[1], pm2 = nm[2], pm3 = nm[3];
-    if (o + 1 < oe) fetch(o + 1);
-    const uint32_t kind = h0.x & 0xFF;
-    const uint32_t rb0 = (h0.x >> 8) & 0xFF;
-    const uint32_t rb1 = (h0.x >> 16) & 0xFF;
-    const uint32_t creg = (h0.x >> 24) & 0xFF;
-    const uint32_t dreg0 = h0.y & 0xFF;
-    const uint32_t dreg1 = (h0.y >> 8) & 0xFF;
-    const uint32_t cnr = h0.z;
-    const uint32_t dv0 = h0.w;
-    const bool tc = (vbase & cnr) == cnr;
-    const Real* mp = op->m;
-    // the common cases (dense 1q gate, X / CNOT with at most one register
-    // control) through one flat switch on a code the planner precomputed
-    const uint32_t fast = (h0.y >> 16) & 0xFF;
-    if (fast != 0) {
-      switch (fast) {
-#define NQ_FU1(B, _) case 1 + B: if constexpr (B < NRB) { if (tc) rb_u1<C, NA, B>(a, pm0, pm1, pm2, pm3); } break;
-        NQ_REG_CASES(NQ_FU1, 0)
-#undef NQ_FU1
-#define NQ_FX1V(B, V) case 8 + 8 * B + V: \
-        if constexpr (B < NRB && (V == 0 || (V - 1 < NRB && V - 1 != B))) \
-          rb_x1_fixed<C, NA, B, (V == 0 ? 0 : (1 << (V - 1))), false>(a, tc); \
-        break;
-#define NQ_FX1(B, _) NQ_FX1V(B, 0) NQ_FX1V(B, 1) NQ_FX1V(B, 2) NQ_FX1V(B, 3) NQ_FX1V(B, 4) NQ_FX1V(B, 5)
-        NQ_REG_CASES(NQ_FX1, 0)
-#undef NQ_FX1
-#undef NQ_FX1V
+  const uint32_t rb0 = op->rb0, rb1 = op->rb1, creg = op->creg, cnr = op->cnr;
+  const bool tc = (vbase & cnr) == cnr;
+  const Real* mp = op->m;
+  switch (op->kind) {
+    case OP_U1: {
+      C m0, m1, m2, m3;
+      ldc2<Real>(mp, m0, m1);
+      ldc2<Real>(mp + 4, m2, m3);
+      switch (rb0) {
+#define NQ_U1C(B, _) case B: if constexpr (B < NRB) rb_u1_ctrl<C, NA, B>(a, m0, m1, m2, m3, tc, creg); break;
+        NQ_REG_CASES(NQ_U1C, 0)
+#undef NQ_U1C
         default: break;
       }
-      continue;
+      break;
     }
-    // the batch executor's variant also takes the diagonal shapes through a
-    // flat switch (TileOp::fast2); measured +1 % there, while the tiled pass
-    // kernel ran QFT passes 1 % slower with it
-    if constexpr (kDiagFlat) {
-      const uint32_t fast2 = (h0.y >> 24) & 0xFF;
-      if (fast2 != 0) {
-        switch (fast2) {
-#define NQ_FD1(B) case 48 + B: \
-          if constexpr (B <= NRB) rb_d1<C, NA, B, NRB>(a, pm0, pm1, (vbase & dv0) ? 1u : 0u); \
-          break;
-          NQ_FD1(0) NQ_FD1(1) NQ_FD1(2) NQ_FD1(3) NQ_FD1(4) NQ_FD1(5)
-#undef NQ_FD1
-#define NQ_FPH(V) case 128 + V: \
-          if constexpr (V < (1 << NRB)) { \
-            if (tc) rb_ph<C, NA, V>(a, pm0, (pm0.x == Real(-1)) && (pm0.y == Real(0))); \
-          } \
-          break;
-          NQ_FPH(0) NQ_FPH(1) NQ_FPH(2) NQ_FPH(3) NQ_FPH(4) NQ_FPH(5) NQ_FPH(6) NQ_FPH(7)
-          NQ_FPH(8) NQ_FPH(9) NQ_FPH(10) NQ_FPH(11) NQ_FPH(12) NQ_FPH(13) NQ_FPH(14) NQ_FPH(15)
-          NQ_FPH(16) NQ_FPH(17) NQ_FPH(18) NQ_FPH(19) NQ_FPH(20) NQ_FPH(21) NQ_FPH(22) NQ_FPH(23)
-          NQ_FPH(24) NQ_FPH(25) NQ_FPH(26) NQ_FPH(27) NQ_FPH(28) NQ_FPH(29) NQ_FPH(30) NQ_FPH(31)
-#undef NQ_FPH
-#define NQ_FD2V(D0, D1) case 160 + 8 * D0 + D1: \
-          if constexpr (D0 <= NRB && D1 <= NRB && (D0 != D1 || D0 == NRB)) { \
-            const C m[4] = {pm0, pm1, pm2, pm3}; \
-            rb_d2<C, NA, D0, D1, NRB>(a, m, (vbase & dv0) ? 1u : 0u, (vbase & dv1) ? 1u : 0u); \
-          } \
-          break;
-#define NQ_FD2(D0) NQ_FD2V(D0, 0) NQ_FD2V(D0, 1) NQ_FD2V(D0, 2) NQ_FD2V(D0, 3) NQ_FD2V(D0, 4) NQ_FD2V(D0, 5)
-          NQ_FD2(0) NQ_FD2(1) NQ_FD2(2) NQ_FD2(3) NQ_FD2(4) NQ_FD2(5)
-#undef NQ_FD2
-#undef NQ_FD2V
-          default: break;
-        }
-        continue;
-      }
-    }
-    switch (kind) {
-      case OP_U1: {
-        const C m0 = pm0, m1 = pm1, m2 = pm2, m3 = pm3;
-        if (creg == 0) {
-          if (!tc) break;
-          switch (rb0) {
-#define NQ_U1(B, _) case B: if constexpr (B < NRB) rb_u1<C, NA, B>(a, m0, m1, m2, m3); break;
-            NQ_REG_CASES(NQ_U1, 0)
-#undef NQ_U1
-            default: break;
-          }
-        } else {
-          switch (rb0) {
-#define NQ_U1C(B, _) case B: if constexpr (B < NRB) rb_u1_ctrl<C, NA, B>(a, m0, m1, m2, m3, tc, creg); break;
-            NQ_REG_CASES(NQ_U1C, 0)
-#undef NQ_U1C
-            default: break;
-          }
-        }
+    case OP_X1: {
+      // X / CNOT kept in registers because later ops of the stage act on
+      // its qubits (the others are deferred into the write-back map).  At
+      // most one register control: a fixed register permutation; more
+      // (Toffoli): generic per-amplitude selects.
+      if (creg & (creg - 1)) {
+        rb_x1_generic<C, NA>(a, int(rb0), tc, creg);
         break;
       }
-      case OP_X1: {
-        // X / CNOT kept in registers because later ops of the stage act on
-        // its qubits (the others are deferred into the write-back map).  At
-        // most one register control: a fixed register permutation; more
-        // (Toffoli): generic per-amplitude selects.
-        if (creg & (creg - 1)) {
-          rb_x1_generic<C, NA>(a, int(rb0), tc, creg);
-          break;
-        }
-        // selects even when tc is always true: a compile-time register
-        // permutation here would make the allocator shuffle (and spill) the
-        // register block on every other op's path
-        switch (rb0) {
+      // selects even when tc is always true: a compile-time register
+      // permutation here would make the allocator shuffle (and spill) the
+      // register block on every other op's path
+      switch (rb0) {
 #define NQ_X1(B, _) case B: \
-          if constexpr (B < NRB) dispatch_x1_ctrl<C, NA, NRB, B, false>(a, creg, tc); \
-          break;
-          NQ_REG_CASES(NQ_X1, 0)
+        if constexpr (B < NRB) dispatch_x1_ctrl<C, NA, NRB, B, false>(a, creg, tc); \
+        break;
+        NQ_REG_CASES(NQ_X1, 0)
 #undef NQ_X1
-          default: break;
-        }
-        break;
+        default: break;
       }
-      case OP_PH: {
-        if (!tc) break;
-        const C m0 = pm0;
-        const bool neg = (m0.x == Real(-1)) && (m0.y == Real(0));
-        dispatch_ph<C, NA, NRB>(a, creg, m0, neg);
-        break;
-      }
-      case OP_D1: {
-        C m[4];
-        m[0] = pm0;
-        m[1] = pm1;
-        const uint32_t tb = (vbase & dv0) ? 1u : 0u;
-        if (creg == 0 && cnr == 0) {
-          switch (dreg0 == 0xFF ? NRB : int(dreg0)) {
-#define NQ_D1(B, _) case B: if constexpr (B <= NRB) rb_d1<C, NA, B, NRB>(a, m[0], m[1], tb); break;
-            NQ_REG_CASES(NQ_D1, 0)
-            case 5: if constexpr (NRB == 5) rb_d1<C, NA, 5, NRB>(a, m[0], m[1], tb); break;
-#undef NQ_D1
-            default: break;
-          }
-        } else {
-          m[2] = m[0];
-          m[3] = m[1];
-          rb_diag_generic<C, NA>(a, m, 1, dreg0, 0xFF, tb, 0, tc, creg);
-        }
-        break;
-      }
-      case OP_D2: {
-        C m[4] = {pm0, pm1, pm2, pm3};
-        const uint32_t tb0 = (vbase & dv0) ? 1u : 0u;
-        const uint32_t tb1 = (vbase & dv1) ? 1u : 0u;
-        if (creg == 0 && cnr == 0) {
-          const int d0 = dreg0 == 0xFF ? NRB : int(dreg0);
-          const int d1 = dreg1 == 0xFF ? NRB : int(dreg1);
-          switch (d0) {
-#define NQ_D2A(V) case V: if constexpr (V <= NRB) dispatch_d2_b<C, NA, NRB, V>(a, d1, m, tb0, tb1); break;
-            NQ_D2A(0) NQ_D2A(1) NQ_D2A(2) NQ_D2A(3) NQ_D2A(4) NQ_D2A(5)
-#undef NQ_D2A
-            default: break;
-          }
-        } else {
-          rb_diag_generic<C, NA>(a, m, 2, dreg0, dreg1, tb0, tb1, tc, creg);
-        }
-        break;
-      }
-      case OP_U2: {
-        switch (rb0) {
+      break;
+    }
+    case OP_U2: {
+      switch (rb0) {
 #define NQ_U2A(B, _) case B: if constexpr (B < NRB) dispatch_u2_b<Real, C, NA, NRB, B>(a, rb1, mp, tc, creg); break;
-          NQ_REG_CASES(NQ_U2A, 0)
+        NQ_REG_CASES(NQ_U2A, 0)
 #undef NQ_U2A
-          default: break;
-        }
-        break;
+        default: break;
       }
-      case OP_SW: {
-        switch (rb0) {
+      break;
+    }
+    case OP_SW: {
+      switch (rb0) {
 #define NQ_SWA(B, _) case B: if constexpr (B < NRB) dispatch_sw_b<C, NA, NRB, B>(a, rb1, tc, creg); break;
-          NQ_REG_CASES(NQ_SWA, 0)
+        NQ_REG_CASES(NQ_SWA, 0)
 #undef NQ_SWA
-          default: break;
-        }
-        break;
+        default: break;
       }
-      default:
-        break;
+      break;
+    }
+    default:
+      break;
+  }
+}
+
+// The phase of a list of (mask, phase) entries for this thread; *p moves past it.
+// complex64: exact sums of angles in 2^-32 turns and one sine / cosine, at any
+// list length within about one rounding of the true phase (a running product of
+// rounded factors would lose one per entry).  complex128: a product.
+__device__ __forceinline__ uint32_t list_angle(const uint4*& p, uint32_t cnt, uint32_t angle, uint32_t vbase) {
+  for (uint32_t i = 0; i < cnt; i += 2) {
+    const uint4 e = *p++;
+    if ((vbase & e.x) == e.x) angle += e.y;
+    if ((vbase & e.z) == e.z) angle += e.w;  // an odd list ends in (0, 0)
+  }
+  return angle;
+}
+__device__ __forceinline__ float2 phase_of(uint32_t angle) {
+  float2 v;
+  sincospif(float(int32_t(angle)) * 0x1p-31f, &v.y, &v.x);
+  return v;
+}
+__device__ __forceinline__ double2 list_phase(const uint4*& p, uint32_t cnt, double2 v, uint32_t vbase) {
+  for (uint32_t i = 0; i < cnt; ++i, p += 2) {
+    const uint32_t m = p->x;
+    const double2 f = *reinterpret_cast<const double2*>(p + 1);
+    if ((vbase & m) == m) v = cmul(f, v);
+  }
+  return v;
+}
+
+// Run a stage's program (tileprog.h) on the thread's register block.
+// vbase = virtual index of register amplitude 0 (register bits are zero in it).
+template <typename Real, int NA, int NRB>
+__device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], const uint4* p,
+                                                 const uint4* const end, uint32_t vbase) {
+  using C = typename Tr<Real>::C;
+  constexpr bool F32 = sizeof(Real) == 4;
+  while (p < end) {
+    const uint4 h = *p;
+    const uint32_t code = h.x & 0xFFFFu;
+    const uint4* q = p + 1;
+    p += max(h.x >> 16, 1u);  // ends on any contents
+    C d0, d1;  // phases
+    uint32_t sign = 0;
+    if (code < TC_D) {
+      if ((vbase & h.y) != h.y) continue;  // a 2x2 with a control outside the registers
+    } else if (code < TC_PH) {
+      if constexpr (F32) {
+        const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
+        d0 = phase_of(g);
+        d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
+      } else {
+        d0 = *reinterpret_cast<const double2*>(q);
+        d1 = *reinterpret_cast<const double2*>(q + 1);
+        q += 2;
+        d0 = list_phase(q, h.y & 0xFFFFu, d0, vbase);
+        d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
+      }
+    } else if (code < TC_SG) {
+      if constexpr (F32) {
+        if (code < TC_PU) d0 = phase_of(list_angle(q, h.y, h.z, vbase));
+        else d0 = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
+      } else {
+        d0 = *reinterpret_cast<const double2*>(q);
+        ++q;
+        d0 = list_phase(q, h.y, d0, vbase);
+      }
+    } else if (code < TC_LEG) {
+      sign = h.z;
+      for (uint32_t i = 0; i < h.y; i += 4) {
+        const uint4 e = *q++;
+        sign += (vbase & e.x) == e.x;
+        if (i + 1 < h.y) sign += (vbase & e.y) == e.y;
+        if (i + 2 < h.y) sign += (vbase & e.z) == e.z;
+        if (i + 3 < h.y) sign += (vbase & e.w) == e.w;
+      }
+      sign <<= 31;
+    }
+    switch (code) {
+#define NQ_B(B, _) \
+      case TC_R + B: \
+        if constexpr (B < NRB) { \
+          C u, v; \
+          ldc2<Real>(reinterpret_cast<const Real*>(q), u, v); \
+          rb_u1_real<C, NA, B>(a, u.x, u.y, v.x, v.y); \
+        } \
+        break; \
+      case TC_X + B: \
+        if constexpr (B < NRB) { \
+          C u, v; \
+          ldc2<Real>(reinterpret_cast<const Real*>(q), u, v); \
+          rb_u1_cross<C, NA, B>(a, u.x, u.y, v.x, v.y); \
+        } \
+        break; \
+      case TC_G + B: \
+        if constexpr (B < NRB) { \
+          C m0, m1, m2, m3; \
+          ldc2<Real>(reinterpret_cast<const Real*>(q), m0, m1); \
+          ldc2<Real>(reinterpret_cast<const Real*>(q) + 4, m2, m3); \
+          rb_u1<C, NA, B>(a, m0, m1, m2, m3); \
+        } \
+        break; \
+      case TC_D + B: if constexpr (B < NRB) rb_d1<C, NA, B>(a, d0, d1); break;
+      NQ_REG_CASES(NQ_B, 0)
+#undef NQ_B
+#define NQ_A(V) \
+      case TC_PH + V: case TC_PU + V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d0); break; \
+      case TC_SG + V: if constexpr (V < (1 << NRB)) rb_sign<C, NA, V>(a, sign); break;
+      NQ_A(0) NQ_A(1) NQ_A(2) NQ_A(3) NQ_A(4) NQ_A(5) NQ_A(6) NQ_A(7)
+      NQ_A(8) NQ_A(9) NQ_A(10) NQ_A(11) NQ_A(12) NQ_A(13) NQ_A(14) NQ_A(15)
+      NQ_A(16) NQ_A(17) NQ_A(18) NQ_A(19) NQ_A(20) NQ_A(21) NQ_A(22) NQ_A(23)
+      NQ_A(24) NQ_A(25) NQ_A(26) NQ_A(27) NQ_A(28) NQ_A(29) NQ_A(30) NQ_A(31)
+#undef NQ_A
+      case TC_LEG: apply_record<Real, NA, NRB>(a, reinterpret_cast<const TileOp<Real>*>(q), vbase); break;
+      default: break;
     }
   }
 }
@@ -555,94 +509,24 @@ __device__ __forceinline__ uint64_t tile_base(const PassRec& P, uint64_t tile) {
 }
 
 
-// Per-stage constants derived from a StageRec, kept in shared memory for the
-// whole pass (kStageTabWords words per stage; built once per pass by
-// build_stage_tab, so the per-tile stage loop does no bit-by-bit work):
-//   S..S+3     slot offsets swz(vector bit of free register bit i)
-//   CW..CW+3   slot offsets of the write-back images of the free register bits
-//   HB         bit i: the image of free register bit i flips amplitude bit 0 (complex64)
-//   MZ         image of register bit 0 (complex64; 1 = bit 0 stays bit 0)
-//   CZ, HZ     slot offset and bit 0 of MZ's image
-//   WS, WH     slot offset and bit 0 of the constant translation sbx
-//   NC, OB, OE conditional translations, op range
-//   CC, CS, CH per conditional translation: control mask, slot offset, bit 0
-//   UL, UH     deposit of thread-index bits 0..3 / 4..7 into the vector index
-//   SL, SH     the same deposits through the swizzle (swz is linear over XOR)
-struct StageTab {
-  enum : int { S = 0, CW = 4, HB = 8, MZ = 9, CZ = 10, HZ = 11, WS = 12, WH = 13, NC = 14, OB = 15, OE = 16,
-               CC = 17, CS = 21, CH = 25, UL = 32, UH = 48, SL = 64, SH = 80 };
-};
-static_assert(StageTab::SH + 16 <= kStageTabWords, "stage table layout");
-
-template <int VB>
-__device__ void build_stage_tab(const StageRec* __restrict__ S, uint32_t* __restrict__ t) {
-  uint32_t s[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) s[i] = swz(1u << (S->rpos[i] - VB));
-  auto regslot = [&](uint32_t m) {
-    uint32_t x = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if ((m >> (VB + i)) & 1u) x ^= s[i];
-    return x;
-  };
-  uint32_t hb = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t m = uint32_t(S->scol[VB + i]);
-    t[StageTab::S + i] = s[i];
-    t[StageTab::CW + i] = regslot(m);
-    hb |= (VB == 1 ? (m & 1u) : 0u) << i;
-  }
-  const uint32_t mz = VB == 1 ? uint32_t(S->scol[0]) : 1u;
-  t[StageTab::HB] = hb;
-  t[StageTab::MZ] = mz;
-  t[StageTab::CZ] = regslot(mz);
-  t[StageTab::HZ] = VB == 1 ? (mz & 1u) : 0u;
-  t[StageTab::WS] = regslot(uint32_t(S->sbx));
-  t[StageTab::WH] = VB == 1 ? (uint32_t(S->sbx) & 1u) : 0u;
-  t[StageTab::NC] = uint32_t(S->ncond);
-  t[StageTab::OB] = uint32_t(S->op_begin);
-  t[StageTab::OE] = uint32_t(S->op_end);
-  for (int i = 0; i < kMaxCondPerm; ++i) {
-    const uint32_t w = uint32_t(S->cond_w[i]);
-    t[StageTab::CC + i] = S->cond_cnr[i];
-    t[StageTab::CS + i] = regslot(w);
-    t[StageTab::CH + i] = VB == 1 ? (w & 1u) : 0u;
-  }
-  const int ntb = S->n_tbits;
-  for (int v = 0; v < 16; ++v) {
-    uint32_t lo = 0, hi = 0;
-    for (int j = 0; j < 4; ++j) {
-      if (j < ntb && ((v >> j) & 1)) lo |= 1u << S->tpos[j];
-      if (j + 4 < ntb && ((v >> j) & 1)) hi |= 1u << S->tpos[j + 4];
-    }
-    t[StageTab::UL + v] = lo;
-    t[StageTab::UH + v] = hi;
-    t[StageTab::SL + v] = swz(lo);
-    t[StageTab::SH + v] = swz(hi);
-  }
-}
-
-// Build the stage tables of pass P into `tabs` (every thread of the CTA calls
-// it; it ends with a block barrier).
-template <typename Real>
-__device__ __forceinline__ void build_pass_tabs(const PassRec& P, const StageRec* __restrict__ stages,
-                                                uint32_t* __restrict__ tabs) {
-  const int nst = P.stage_end - P.stage_begin;
-  for (int i = threadIdx.x; i < nst; i += blockDim.x)
-    build_stage_tab<Tr<Real>::kVecBit>(stages + P.stage_begin + i, tabs + i * kStageTabWords);
-  __syncthreads();
+// Copy a pass's stage tables (StageTab, tileprog.h) and, behind them, the first
+// `words` words of its program into shared memory; every thread of the CTA calls
+// it, and a barrier has to follow.
+__device__ __forceinline__ void load_pass_prog(const PassRec& P, const uint4* __restrict__ progs, int words,
+                                               uint4* __restrict__ dst) {
+  const uint4* src = progs + P.prog_begin;
+  const int n = (P.stage_end - P.stage_begin) * (kStageTabWords / 4) + words;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
 // Run stages [P.stage_begin, P.stage_end) of a pass on the tile held in shared
 // memory `sv` (swizzled vector slots), with the pass's stage tables in `tabs`.
 // Every thread of the CTA must call it (it contains block barriers); threads
 // >= nvec/16 only take part in them.
-template <typename Real, bool kDiagFlat = false>
+template <typename Real>
 __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict__ sv, const PassRec& P,
                                                 const uint32_t* __restrict__ tabs,
-                                                const TileOp<Real>* __restrict__ ops, uint32_t ext) {
+                                                const uint4* prog, uint32_t ext) {
   using T = Tr<Real>;
   using C = typename T::C;
   constexpr int VB = T::kVecBit;
@@ -652,6 +536,7 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
   const int tid = threadIdx.x;
   const uint32_t active_threads = (1u << (P.k - VB)) / kVecPerThread;
   const int nst = P.stage_end - P.stage_begin;
+  const uint32_t words = uint32_t(P.prog_words - nst * (kStageTabWords / 4));
   for (int si = 0; si < nst; ++si) {
     const uint32_t* Tb = tabs + si * kStageTabWords;
     if (uint32_t(tid) < active_threads) {
@@ -669,7 +554,7 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
         unpack_vec<Real>(sv[slot], a + r * APV);
       }
       const uint32_t vbase = (ub << VB) | ext;
-      apply_stage_ops<Real, NA, NRB, kDiagFlat>(a, ops, int(Tb[StageTab::OB]), int(Tb[StageTab::OE]), vbase);
+      apply_stage_prog<Real, NA, NRB>(a, prog + Tb[StageTab::OB], prog + min(Tb[StageTab::OE], words), vbase);
       // Write-back through the stage's deferred permutation pi(p) = A p ^ w:
       // register amplitude p goes to the slot of logical index pi(p).  Slot
       // offsets are linear in the free register bits (register bits
