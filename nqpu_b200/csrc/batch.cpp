@@ -143,7 +143,7 @@ static cudaError_t batch_build(BatchImpl* b) {
       const bool small = E.n <= b->small_max;
       const int kmax = small ? 13 : std::min(b->plan_kmax, 13);
       std::string err;
-      const std::vector<Op> ops = lower_circuit(E.gates);
+      const std::vector<Op> ops = carry_phases(lower_circuit(E.gates));
       plan_ok[ci] = build_tile_plan(ops, E.n, DType::C64, kmax, &plans[ci], &err) &&
                     (!small || plans[ci].passes.size() == 1);
       if (plan_ok[ci]) build_tile_prog(ops, &plans[ci]);

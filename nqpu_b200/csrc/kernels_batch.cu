@@ -33,9 +33,11 @@ namespace nqpu {
 
 constexpr int kBatchK = 13;                       // complex64 tile bits
 constexpr uint32_t kBatchVec = 1u << (kBatchK - 1);
-// Words of a pass's program kept in shared memory (a longer one is read from
-// global memory): what two CTAs per SM leave.
-constexpr int kBatchProgWords = 1152;
+// Words of a pass's stage tables and program kept in shared memory (a longer
+// program is read from global memory): what two CTAs per SM leave, and never less
+// than the tables of the longest pass.
+constexpr int kBatchProgWords = 2496;
+static_assert(kBatchProgWords * 4 >= kMaxPassStages * kStageTabWords, "stage tables fit");
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   uint32_t v;
@@ -132,10 +134,11 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   __shared__ PassRec P;
   // program of the current pass: behind its stage tables in shared memory, where it fits
   auto tab_words = [&]() { return (P.stage_end - P.stage_begin) * (kStageTabWords / 4); };
-  auto prog_words = [&]() { return P.prog_words - tab_words(); };
-  auto prog = [&]() -> const uint4* {
-    return prog_words() <= kBatchProgWords ? reinterpret_cast<const uint4*>(tabs) + tab_words()
-                                           : progs + P.prog_begin + tab_words();
+  auto run_stages = [&](uint32_t ext) {
+    if (P.prog_words <= kBatchProgWords)
+      run_tile_stages<float>(sv, P, tabs, reinterpret_cast<const uint4*>(tabs) + tab_words(), ext);
+    else
+      run_tile_stages<float>(sv, P, tabs, progs + P.prog_begin + tab_words(), ext);
   };
   __shared__ int s_pass;  // global index of the pass whose tables are loaded (-1: none)
   __shared__ uint32_t s_task;
@@ -173,6 +176,8 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     int32_t* dst = reinterpret_cast<int32_t*>(&P);
     for (int i = tid; i < int(sizeof(PassRec) / 4); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
+    load_pass_prog(P, progs, P.prog_words <= kBatchProgWords ? P.prog_words - tab_words() : 0,
+                   reinterpret_cast<uint4*>(tabs));
     const int nhi = P.k - P.c;
     for (int hh = tid; hh < (1 << nhi); hh += blockDim.x) {
       uint64_t off = 0;
@@ -180,7 +185,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         if ((hh >> j) & 1) off |= 1ull << P.qhi[j];
       hi_off[hh] = off;
     }
-    load_pass_prog(P, progs, prog_words() <= kBatchProgWords ? prog_words() : 0, reinterpret_cast<uint4*>(tabs));
+    cp_async_wait0();
     if (tid == 0) s_pass = gp;
     __syncthreads();
   };
@@ -205,7 +210,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       const uint32_t nvec = 1u << (P.k - 1);
       init_tile(nvec, true);
       __syncthreads();
-      run_tile_stages<float>(sv, P, tabs, prog(), 0u);
+      run_stages(0u);
       double jtot;
       load_obs(C, &jtot);
       __syncthreads();
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         cp_async_wait0();
       }
       __syncthreads();
-      run_tile_stages<float>(sv, P, tabs, prog(), ext);
+      run_stages(ext);
       for (uint32_t u = tid; u < nvec; u += blockDim.x) {
         const uint32_t t = u << 1;
         const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
 
 size_t batch_smem_bytes() {
   return sizeof(float4) * kBatchVec + sizeof(uint64_t) * kHiOffEntries + sizeof(double) * (768 + 64) +
-         sizeof(uint32_t) * kMaxPassStages * kStageTabWords + sizeof(uint4) * kBatchProgWords;
+         sizeof(uint4) * kBatchProgWords;
 }
 
 cudaError_t launch_batch(const BatchLaunch& L, cudaStream_t s) {

@@ -50,15 +50,17 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
   const int k = P.k, c = P.c;
   const uint32_t nvec = 1u << (k - VB);
   const int nhi = k - c;
+  load_pass_prog(P, progs, prog_smem, reinterpret_cast<uint4*>(tabs));
   for (int h = tid; h < (1 << nhi); h += blockDim.x) {
     uint64_t off = 0;
     for (int j = 0; j < nhi; ++j)
       if ((h >> j) & 1) off |= 1ull << P.qhi[j];
     hi_off[h] = off;
   }
-  load_pass_prog(P, progs, prog_smem, reinterpret_cast<uint4*>(tabs));
   const int tab_words = (P.stage_end - P.stage_begin) * (kStageTabWords / 4);
-  const uint4* prog = prog_smem ? reinterpret_cast<const uint4*>(tabs) + tab_words : progs + P.prog_begin + tab_words;
+  const uint4* prog_s = reinterpret_cast<const uint4*>(tabs) + tab_words;
+  const uint4* prog_g = progs + P.prog_begin + tab_words;
+  cp_async_wait0();
   __syncthreads();
   // everything above read only the plan's tables: the previous pass of the
   // state may still be running up to here
@@ -103,7 +105,9 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
     for (int j = 0; j < P.n_ext; ++j)
       if ((base >> P.ext[j]) & 1ull) ext |= 1u << (k + j);
 
-    run_tile_stages<Real>(sv, P, tabs, prog, ext);
+    // two copies, so that the usual one reads the program by shared-memory loads
+    if (prog_smem) run_tile_stages<Real>(sv, P, tabs, prog_s, ext);
+    else run_tile_stages<Real>(sv, P, tabs, prog_g, ext);
 
     // shared -> HBM
 #pragma unroll

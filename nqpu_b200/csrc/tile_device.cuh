@@ -48,13 +48,6 @@ __device__ __forceinline__ void ldc2<double>(const double* __restrict__ p, doubl
   b = *(reinterpret_cast<const double2*>(p) + 1);
 }
 
-// complex product on a register amplitude: packed FFMA2 form for complex64
-template <typename C>
-__device__ __forceinline__ C rmul(C m, C x) {
-  if constexpr (sizeof(m.x) == 4) return pcmul(pack_coef(m), x);
-  else return cmul(m, x);
-}
-
 // dense 2x2, no controls
 template <typename C, int NA, int B>
 __device__ __forceinline__ void rb_u1(C (&a)[NA], C m0, C m1, C m2, C m3) {
@@ -150,46 +143,51 @@ __device__ __forceinline__ void dispatch_x1_ctrl(C (&a)[NA], uint32_t creg, bool
   }
 }
 
-// real 2x2 (RY, H, ...): no re/im mixing, two packed operations per amplitude
+// real rotation as three shears in place (t = tan(phi / 2), s = sin(phi))
 template <typename C, int NA, int B>
-__device__ __forceinline__ void rb_u1_real(C (&a)[NA], decltype(C::x) m00, decltype(C::x) m01, decltype(C::x) m10,
-                                           decltype(C::x) m11) {
+__device__ __forceinline__ void rb_rot(C (&a)[NA], decltype(C::x) t, decltype(C::x) s) {
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
     if (i & (1 << B)) continue;
-    const int j = i | (1 << B);
-    const C x = a[i], y = a[j];
-    if constexpr (sizeof(m00) == 4) {
-      a[i] = __ffma2_rn(make_float2(m01, m01), y, __fmul2_rn(make_float2(m00, m00), x));
-      a[j] = __ffma2_rn(make_float2(m11, m11), y, __fmul2_rn(make_float2(m10, m10), x));
+    C &x = a[i], &y = a[i | (1 << B)];
+    if constexpr (sizeof(t) == 4) {
+      const float2 nt = make_float2(-t, -t), ss = make_float2(s, s);
+      x = __ffma2_rn(nt, y, x);
+      y = __ffma2_rn(ss, x, y);
+      x = __ffma2_rn(nt, y, x);
     } else {
-      a[i].x = m00 * x.x + m01 * y.x;
-      a[i].y = m00 * x.y + m01 * y.y;
-      a[j].x = m10 * x.x + m11 * y.x;
-      a[j].y = m10 * x.y + m11 * y.y;
+      x.x = fma(-t, y.x, x.x);
+      x.y = fma(-t, y.y, x.y);
+      y.x = fma(s, x.x, y.x);
+      y.y = fma(s, x.y, y.y);
+      x.x = fma(-t, y.x, x.x);
+      x.y = fma(-t, y.y, x.y);
     }
   }
 }
 
-// 2x2 with a real diagonal and an imaginary off-diagonal i m01, i m10 (RX, Y)
+// RX(2 phi): the rotation of (x.re, y.im) by -phi and of (x.im, y.re) by phi
 template <typename C, int NA, int B>
-__device__ __forceinline__ void rb_u1_cross(C (&a)[NA], decltype(C::x) m00, decltype(C::x) m01, decltype(C::x) m10,
-                                            decltype(C::x) m11) {
+__device__ __forceinline__ void rb_cross(C (&a)[NA], decltype(C::x) t, decltype(C::x) s) {
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
     if (i & (1 << B)) continue;
-    const int j = i | (1 << B);
-    const C x = a[i], y = a[j];
-    if constexpr (sizeof(m00) == 4) {
-      a[i] = __ffma2_rn(make_float2(-m01, m01), swap_ri(y), __fmul2_rn(make_float2(m00, m00), x));
-      a[j] = __ffma2_rn(make_float2(-m10, m10), swap_ri(x), __fmul2_rn(make_float2(m11, m11), y));
-    } else {
-      a[i].x = m00 * x.x - m01 * y.y;
-      a[i].y = m00 * x.y + m01 * y.x;
-      a[j].x = m11 * y.x - m10 * x.y;
-      a[j].y = m11 * y.y + m10 * x.x;
-    }
+    C &x = a[i], &y = a[i | (1 << B)];
+    x.x = fma(t, y.y, x.x);
+    x.y = fma(-t, y.x, x.y);
+    y.y = fma(-s, x.x, y.y);
+    y.x = fma(s, x.y, y.x);
+    x.x = fma(t, y.y, x.x);
+    x.y = fma(-t, y.x, x.y);
   }
+}
+
+// m * x in place, scalar: four operations and no re/im swap
+template <typename C>
+__device__ __forceinline__ void cmul_in(C m, C& v) {
+  const auto u = m.y * v.y, w = m.y * v.x;
+  v.x = fma(m.x, v.x, -u);
+  v.y = fma(m.x, v.y, w);
 }
 
 // phase m on the register amplitudes whose bits CMASK are all set
@@ -197,14 +195,26 @@ template <typename C, int NA, int CMASK>
 __device__ __forceinline__ void rb_ph(C (&a)[NA], C m) {
 #pragma unroll
   for (int i = 0; i < NA; ++i)
-    if ((i & CMASK) == CMASK) a[i] = rmul(m, a[i]);
+    if ((i & CMASK) == CMASK) cmul_in(m, a[i]);
+}
+
+// one phase per register amplitude
+template <typename Real, typename C, int NA>
+__device__ __forceinline__ void rb_table(C (&a)[NA], const uint4* q) {
+#pragma unroll
+  for (int i = 0; i < NA; i += 2) {
+    C u, v;
+    ldc2<Real>(reinterpret_cast<const Real*>(q) + 2 * i, u, v);
+    cmul_in(u, a[i]);
+    cmul_in(v, a[i + 1]);
+  }
 }
 
 // diag(d0, d1) on register bit B
 template <typename C, int NA, int B>
 __device__ __forceinline__ void rb_d1(C (&a)[NA], C d0, C d1) {
 #pragma unroll
-  for (int i = 0; i < NA; ++i) a[i] = rmul((i & (1 << B)) ? d1 : d0, a[i]);
+  for (int i = 0; i < NA; ++i) cmul_in((i & (1 << B)) ? d1 : d0, a[i]);
 }
 
 // sign flip (s = 0 or the sign bit) of the register amplitudes with bits CMASK
@@ -385,61 +395,49 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
   constexpr bool F32 = sizeof(Real) == 4;
   while (p < end) {
     const uint4 h = *p;
-    const uint32_t code = h.x & 0xFFFFu;
     const uint4* q = p + 1;
+    uint32_t code = h.x & 0xFFFFu;
+    C d0;  // the instruction's two reals
+    if constexpr (F32) d0 = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
+    else d0 = *reinterpret_cast<const double2*>(q);  // (the word table ends in a spare word)
+    C d1 = d0;
+    uint32_t sign = 0x80000000u;
     p += max(h.x >> 16, 1u);  // ends on any contents
-    C d0, d1;  // phases
-    uint32_t sign = 0;
-    if (code < TC_D) {
-      if ((vbase & h.y) != h.y) continue;  // a 2x2 with a control outside the registers
-    } else if (code < TC_PH) {
-      if constexpr (F32) {
-        const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
-        d0 = phase_of(g);
-        d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
-      } else {
-        d0 = *reinterpret_cast<const double2*>(q);
-        d1 = *reinterpret_cast<const double2*>(q + 1);
-        q += 2;
-        d0 = list_phase(q, h.y & 0xFFFFu, d0, vbase);
-        d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
+    if (code >= TC_LIST) {
+      if (code < TC_SL) {
+        if constexpr (F32) d0 = phase_of(list_angle(q, h.y, h.z, vbase));
+        else d0 = list_phase(++q, h.y, d0, vbase);
+        code += TC_PU - TC_PH;
+      } else if (code < TC_D) {
+        sign = h.z;
+        for (uint32_t i = 0; i < h.y; i += 4) {
+          const uint4 e = *q++;
+          sign += (vbase & e.x) == e.x;
+          if (i + 1 < h.y) sign += (vbase & e.y) == e.y;
+          if (i + 2 < h.y) sign += (vbase & e.z) == e.z;
+          if (i + 3 < h.y) sign += (vbase & e.w) == e.w;
+        }
+        sign <<= 31;
+        code += TC_SG - TC_SL;
+      } else if (code < TC_LEG) {
+        if constexpr (F32) {
+          const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
+          d0 = phase_of(g);
+          d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
+        } else {
+          d1 = *reinterpret_cast<const double2*>(q + 1);
+          q += 2;
+          d0 = list_phase(q, h.y & 0xFFFFu, d0, vbase);
+          d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
+        }
       }
-    } else if (code < TC_SG) {
-      if constexpr (F32) {
-        if (code < TC_PU) d0 = phase_of(list_angle(q, h.y, h.z, vbase));
-        else d0 = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
-      } else {
-        d0 = *reinterpret_cast<const double2*>(q);
-        ++q;
-        d0 = list_phase(q, h.y, d0, vbase);
-      }
-    } else if (code < TC_LEG) {
-      sign = h.z;
-      for (uint32_t i = 0; i < h.y; i += 4) {
-        const uint4 e = *q++;
-        sign += (vbase & e.x) == e.x;
-        if (i + 1 < h.y) sign += (vbase & e.y) == e.y;
-        if (i + 2 < h.y) sign += (vbase & e.z) == e.z;
-        if (i + 3 < h.y) sign += (vbase & e.w) == e.w;
-      }
-      sign <<= 31;
+    } else if (code < TC_T && (vbase & h.y) != h.y) {
+      continue;  // a 2x2 with a control outside the registers
     }
     switch (code) {
 #define NQ_B(B, _) \
-      case TC_R + B: \
-        if constexpr (B < NRB) { \
-          C u, v; \
-          ldc2<Real>(reinterpret_cast<const Real*>(q), u, v); \
-          rb_u1_real<C, NA, B>(a, u.x, u.y, v.x, v.y); \
-        } \
-        break; \
-      case TC_X + B: \
-        if constexpr (B < NRB) { \
-          C u, v; \
-          ldc2<Real>(reinterpret_cast<const Real*>(q), u, v); \
-          rb_u1_cross<C, NA, B>(a, u.x, u.y, v.x, v.y); \
-        } \
-        break; \
+      case TC_R + B: if constexpr (B < NRB) rb_rot<C, NA, B>(a, d0.x, d0.y); break; \
+      case TC_X + B: if constexpr (B < NRB) rb_cross<C, NA, B>(a, d0.x, d0.y); break; \
       case TC_G + B: \
         if constexpr (B < NRB) { \
           C m0, m1, m2, m3; \
@@ -451,8 +449,9 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
       case TC_D + B: if constexpr (B < NRB) rb_d1<C, NA, B>(a, d0, d1); break;
       NQ_REG_CASES(NQ_B, 0)
 #undef NQ_B
+      case TC_T: rb_table<Real, C, NA>(a, q); break;
 #define NQ_A(V) \
-      case TC_PH + V: case TC_PU + V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d0); break; \
+      case TC_PU + V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d0); break; \
       case TC_SG + V: if constexpr (V < (1 << NRB)) rb_sign<C, NA, V>(a, sign); break;
       NQ_A(0) NQ_A(1) NQ_A(2) NQ_A(3) NQ_A(4) NQ_A(5) NQ_A(6) NQ_A(7)
       NQ_A(8) NQ_A(9) NQ_A(10) NQ_A(11) NQ_A(12) NQ_A(13) NQ_A(14) NQ_A(15)
@@ -510,13 +509,15 @@ __device__ __forceinline__ uint64_t tile_base(const PassRec& P, uint64_t tile) {
 
 
 // Copy a pass's stage tables (StageTab, tileprog.h) and, behind them, the first
-// `words` words of its program into shared memory; every thread of the CTA calls
-// it, and a barrier has to follow.
+// `words` words of its program into shared memory, asynchronously: every thread
+// of the CTA calls it, then waits for its copies (cp_async_wait0) and the CTA
+// meets at a barrier.
 __device__ __forceinline__ void load_pass_prog(const PassRec& P, const uint4* __restrict__ progs, int words,
-                                               uint4* __restrict__ dst) {
+                                               uint4* dst) {
   const uint4* src = progs + P.prog_begin;
   const int n = (P.stage_end - P.stage_begin) * (kStageTabWords / 4) + words;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) cp_async16(dst + i, src + i);
+  cp_async_commit();
 }
 
 // Run stages [P.stage_begin, P.stage_end) of a pass on the tile held in shared

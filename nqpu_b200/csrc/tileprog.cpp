@@ -24,14 +24,15 @@ struct Phase {
   }
 };
 
-struct Instr {
-  enum Kind { DENSE, PHASE, PAIR, LEGACY } kind = DENSE;
-  int bit = 0;         // DENSE, PAIR
-  uint32_t cnr = 0;    // DENSE
-  cplx m[4];           // DENSE
-  uint32_t A = 0;      // PHASE
-  Phase a, b;          // PHASE: a; PAIR: all amplitudes, amplitudes with `bit`
-  size_t op = 0;       // LEGACY: index into the plan's ops
+// An op of a stage, or a part of one, before scheduling.
+struct Item {
+  enum Kind { PHASE, ROT, CROSS, GENERIC, RECORD } kind = PHASE;
+  uint32_t diag = 0, dense = 0;  // register bits it reads (commutes with phases) / changes
+  uint32_t cnr = 0;              // virtual-index mask: a phase's condition, a 2x2's control
+  cplx m[4];                     // PHASE: m[0]; GENERIC: the matrix
+  double t = 0, s = 0;           // ROT, CROSS
+  size_t op = 0;                 // RECORD: index into the plan's ops
+  bool done = false;
 };
 
 // Angle in 2^-32 turns of a unit complex number.
@@ -49,7 +50,7 @@ class Writer {
     return begin_;
   }
   void end() { (*out_)[begin_].w[0] |= uint32_t(out_->size() - begin_) << 16; }
-  ProgWord& head() { return (*out_)[begin_]; }
+  ProgWord& head() { return (*out_)[begin_]; }  // valid until more is written
   void reals(const double* v, int n) {
     if (f32_) {
       std::vector<float> f(v, v + n);
@@ -87,99 +88,127 @@ template <typename Real>
 class StageCompiler {
  public:
   StageCompiler(const std::vector<Op>& ops, const TilePlan& plan, const std::vector<TileOp<Real>>& enc)
-      : ops_(ops), plan_(plan), enc_(enc) {}
+      : ops_(ops), plan_(plan), enc_(enc), W_(nullptr, sizeof(Real) == 4) {}
 
   // Compile stage S; `global` is the phase common to all amplitudes, carried from
   // stage to stage and applied by the last one.
   void run(const StageRec& S, bool last, cplx* global, std::vector<ProgWord>* out) {
-    code_.clear();
+    W_ = Writer(out, sizeof(Real) == 4);
+    items_.clear();
     for (Phase& p : pend_) p = Phase();
-    for (int& o : open_) o = -1;
+    for (bool& h : have_) h = false;
     for (int o = S.op_begin; o < S.op_end; ++o) add(size_t(o));
+    for (int b = 0; b < kBits; ++b) settle(b);
+    schedule();
     *global *= pend_[0].uniform;
     pend_[0].uniform = last ? *global : cplx(1.0, 0.0);
     finish();
-    emit(out);
   }
 
  private:
-  static constexpr int kBits = sizeof(Real) == 4 ? 5 : 4;
+  static constexpr bool kF32 = sizeof(Real) == 4;
+  static constexpr int kBits = kF32 ? 5 : 4;
+  static constexpr uint32_t kAll = 1u << kBits;
 
+  // ---- ops to items -------------------------------------------------------
+  // 2x2s on a register bit and constant phases on it alone multiply up in acc_
+  // until something that does not commute with them arrives.
   void phase(uint32_t A, uint32_t B, cplx p) {
-    Phase& P = pend_[A];
-    P.used = true;
-    if (B == 0) { P.uniform *= p; return; }
-    for (size_t i = 0; i < P.list.size(); ++i)
-      if (P.list[i].mask == B) {
-        P.list[i].p *= p;
-        if (P.list[i].p == cplx(1.0, 0.0)) P.list.erase(P.list.begin() + long(i));
-        return;
-      }
-    P.list.push_back(Entry{B, p});
-  }
-
-  // Emit the pending phases that do not commute with a dense op on bits `t`.
-  void flush(uint32_t t) {
-    for (uint32_t A = 1; A < (1u << kBits); ++A) {
-      if (!(A & t) || !pend_[A].used) continue;
-      put(A, pend_[A]);
-      pend_[A] = Phase();
-    }
-  }
-
-  void put(uint32_t A, const Phase& P) {
-    if (P.trivial()) return;
-    // a constant phase on one bit goes into the complex matrix before it
-    if ((A & (A - 1)) == 0 && A != 0 && P.list.empty()) {
-      const int o = open_[ctz(A)];
-      if (o >= 0 && code_[size_t(o)].cnr == 0 && generic(code_[size_t(o)].m)) {
-        code_[size_t(o)].m[2] *= P.uniform;
-        code_[size_t(o)].m[3] *= P.uniform;
-        return;
-      }
+    if ((A & (A - 1)) == 0 && A != 0 && B == 0 && have_[ctz(A)]) {
+      acc_[ctz(A)][2] *= p;
+      acc_[ctz(A)][3] *= p;
+      return;
     }
     for (int b = 0; b < kBits; ++b)
-      if ((A >> b) & 1) open_[b] = -1;
-    Instr I;
-    I.kind = Instr::PHASE;
-    I.A = A;
-    I.a = P;
-    code_.push_back(I);
+      if ((A >> b) & 1) settle(b);
+    push_phase(A, B, p);
+  }
+  void push_phase(uint32_t A, uint32_t B, cplx p) {
+    if (p == cplx(1.0, 0.0)) return;
+    Item I;
+    I.diag = A;
+    I.cnr = B;
+    I.m[0] = p;
+    items_.push_back(I);
   }
 
-  // Stage end: what is left; the phase on all amplitudes joins a one-bit phase.
-  void finish() {
-    const Phase all = pend_[0];
-    int join = -1;
-    if (!all.trivial())
-      for (int b = 0; b < kBits && join < 0; ++b) {
-        const Phase& P = pend_[1u << b];
-        if (P.used && !P.trivial() && !P.signs()) join = b;
+  void settle(int b) {
+    if (!have_[b]) return;
+    have_[b] = false;
+    dense(b, 0, acc_[b]);
+  }
+
+  // A 2x2 as items: phase x rotation x phase where it is unitary, else as it is.
+  void dense(int b, uint32_t cnr, const cplx* m) {
+    Item I;
+    I.dense = 1u << b;
+    I.cnr = cnr;
+    const double eps = 1e-12;
+    const cplx m11 = std::abs(m[0]) > std::abs(m[1]) ? std::conj(m[0]) * det(m) : m[3];
+    const bool unitary = std::abs(std::norm(m[0]) + std::norm(m[2]) - 1.0) < eps &&
+                         std::abs(std::norm(m[1]) + std::norm(m[3]) - 1.0) < eps &&
+                         std::abs(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) < eps && std::abs(m11 - m[3]) < 1e-9;
+    if (!unitary || cnr != 0) {
+      I.kind = Item::GENERIC;
+      for (int i = 0; i < 4; ++i) I.m[i] = m[i];
+      items_.push_back(I);
+      return;
+    }
+    // RX: cos and -i sin
+    if (m[0].imag() == 0 && m[3].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[0].real() == m[3].real() &&
+        m[1].imag() == m[2].imag()) {
+      const double sg = m[0].real() < 0 ? -1.0 : 1.0;  // |phi| <= pi/2 up to a common sign
+      push_phase(0, 0, cplx(sg, 0.0));
+      shears(sg * m[0].real(), -sg * m[1].imag(), &I);
+      I.kind = Item::CROSS;
+      if (I.s != 0.0) items_.push_back(I);
+      return;
+    }
+    const double c = std::abs(m[0]), s = std::abs(m[2]);
+    const cplx one(1.0, 0.0);
+    if (s < kTiny || c < kTiny) {  // a phase, or a rotation by pi/2 with phases
+      const cplx p0 = s < kTiny ? m[0] : -m[1], p1 = s < kTiny ? m[3] / m[0] : m[2] / -m[1];
+      push_phase(0, 0, p0 / std::abs(p0));
+      if (c < kTiny) {
+        shears(0.0, 1.0, &I);
+        I.kind = Item::ROT;
+        items_.push_back(I);
       }
-    for (uint32_t A = 1; A < (1u << kBits); ++A) {
-      if (!pend_[A].used || (join >= 0 && A == (1u << join))) continue;
-      put(A, pend_[A]);
+      push_phase(1u << b, 0, clean(p1 / std::abs(p1)));
+      return;
     }
-    if (join >= 0) {
-      Instr I;
-      I.kind = Instr::PAIR;
-      I.bit = join;
-      I.a = all;
-      I.b = pend_[1u << join];
-      code_.push_back(I);
-    } else {
-      put(0, all);
+    // e^{ia} diag(1, after) [[c, -s], [s, c]] diag(1, before)
+    const cplx a = m[0] / c;
+    // (`before` from the larger of the entries that fix it: a small off-diagonal
+    // has no precise phase, and only its product with `after` matters then)
+    cplx after = (m[2] / s) / a, before = s > c ? (-m[1] / s) / a : (m[3] / c) / a / after;
+    after /= std::abs(after);
+    before /= std::abs(before);
+    double sn = s;
+    if (std::abs(after + one) < kTiny) {  // a rotation the other way
+      sn = -s;
+      after = -after;
+      before = -before;
     }
+    push_phase(0, 0, a);
+    push_phase(1u << b, 0, clean(before));
+    shears(c, sn, &I);
+    I.kind = Item::ROT;
+    items_.push_back(I);
+    push_phase(1u << b, 0, clean(after));
   }
-
-  static int ctz(uint32_t v) { return __builtin_ctz(v); }
-  static bool real(const cplx* m) {
-    return m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0;
+  // A phase that is 1 or -1 up to the rounding of its making.
+  static constexpr double kTiny = 1e-15;
+  static cplx clean(cplx p) {
+    if (std::abs(p - cplx(1.0, 0.0)) < kTiny) return cplx(1.0, 0.0);
+    return std::abs(p + cplx(1.0, 0.0)) < kTiny ? cplx(-1.0, 0.0) : p;
   }
-  static bool cross(const cplx* m) {
-    return m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
+  static cplx det(const cplx* m) { return m[0] * m[3] - m[1] * m[2]; }
+  static void shears(double c, double s, Item* I) {  // c >= 0
+    const double h = std::hypot(c, s);
+    I->t = (s / h) / (1.0 + c / h);
+    I->s = s / h;
   }
-  static bool generic(const cplx* m) { return !real(m) && !cross(m); }
 
   void add(size_t oi) {
     const TileOp<Real>& t = enc_[oi];
@@ -203,128 +232,235 @@ class StageCompiler {
         return;
       }
       case OP_U1:
-        if (t.creg == 0) { dense(t.rb0, t.cnr, o.m); return; }
-        break;
+        if (t.creg != 0) break;
+        if (t.cnr != 0) {
+          settle(t.rb0);
+          dense(t.rb0, t.cnr, o.m);
+          return;
+        }
+        if (have_[t.rb0]) {
+          const cplx* p = acc_[t.rb0];
+          const cplx r[4] = {o.m[0] * p[0] + o.m[1] * p[2], o.m[0] * p[1] + o.m[1] * p[3],
+                             o.m[2] * p[0] + o.m[3] * p[2], o.m[2] * p[1] + o.m[3] * p[3]};
+          for (int i = 0; i < 4; ++i) acc_[t.rb0][i] = r[i];
+        } else {
+          have_[t.rb0] = true;
+          for (int i = 0; i < 4; ++i) acc_[t.rb0][i] = o.m[i];
+        }
+        return;
       default:
         break;
     }
-    uint32_t touched = 1u << t.rb0;
-    if (t.kind == OP_U2 || t.kind == OP_SW) touched |= 1u << t.rb1;
-    flush(touched);
-    // the op reads its register controls: it stays after what wrote them
-    touched |= t.creg;
-    for (int b = 0; b < kBits; ++b)
-      if ((touched >> b) & 1) open_[b] = -1;
-    Instr I;
-    I.kind = Instr::LEGACY;
+    Item I;
+    I.kind = Item::RECORD;
     I.op = oi;
-    code_.push_back(I);
+    I.dense = 1u << t.rb0;
+    if (t.kind == OP_U2 || t.kind == OP_SW) I.dense |= 1u << t.rb1;
+    I.diag = t.creg;
+    for (int b = 0; b < kBits; ++b)
+      if (((I.dense | I.diag) >> b) & 1) settle(b);
+    items_.push_back(I);
   }
 
-  void dense(int b, uint32_t cnr, const cplx* m) {
-    // phases on this bit alone and constant: into the matrix where that makes
-    // the product no dearer (it is complex already, or the gate before it on
-    // this bit is still open to take it)
-    cplx M[4] = {m[0], m[1], m[2], m[3]};
-    Phase& P = pend_[1u << b];
-    const bool merge = open_[b] >= 0 && code_[size_t(open_[b])].cnr == cnr;
-    bool others = false;
-    for (uint32_t A = 1; A < (1u << kBits); ++A)
-      if ((A >> b) & 1 && A != (1u << b) && pend_[A].used && !pend_[A].trivial()) others = true;
-    if (P.used && P.list.empty() && cnr == 0 && (generic(M) || (merge && !others))) {
-      M[1] *= P.uniform;
-      M[3] *= P.uniform;
-      P = Phase();
-    }
-    if (merge && !others && (!P.used || P.trivial())) {
-      cplx* p = code_[size_t(open_[b])].m;
-      const cplx r[4] = {M[0] * p[0] + M[1] * p[2], M[0] * p[1] + M[1] * p[3],
-                         M[2] * p[0] + M[3] * p[2], M[2] * p[1] + M[3] * p[3]};
-      std::memcpy(p, r, sizeof(r));
-      return;
-    }
-    flush(1u << b);
-    Instr I;
-    I.kind = Instr::DENSE;
-    I.bit = b;
-    I.cnr = cnr;
-    for (int i = 0; i < 4; ++i) I.m[i] = M[i];
-    open_[b] = int(code_.size());
-    code_.push_back(I);
-  }
-
-  void emit(std::vector<ProgWord>* out) {
-    constexpr bool f32 = sizeof(Real) == 4;
-    Writer W(out, f32);
-    for (const Instr& I : code_) {
-      switch (I.kind) {
-        case Instr::DENSE: {
-          if (real(I.m)) {
-            const double v[4] = {I.m[0].real(), I.m[1].real(), I.m[2].real(), I.m[3].real()};
-            W.header(TC_R + uint32_t(I.bit), I.cnr);
-            W.reals(v, 4);
-          } else if (cross(I.m)) {
-            const double v[4] = {I.m[0].real(), I.m[1].imag(), I.m[2].imag(), I.m[3].real()};
-            W.header(TC_X + uint32_t(I.bit), I.cnr);
-            W.reals(v, 4);
-          } else {
-            double v[8];
-            for (int i = 0; i < 4; ++i) { v[2 * i] = I.m[i].real(); v[2 * i + 1] = I.m[i].imag(); }
-            W.header(TC_G + uint32_t(I.bit), I.cnr);
-            W.reals(v, 8);
-          }
-          break;
+  // ---- scheduling ---------------------------------------------------------
+  // Rounds of: take every phase that no earlier open dense item blocks, then emit
+  // every dense item with nothing open before it on its bits.  Phases gather
+  // as long as they can, so that a layer's join in one instruction.
+  void schedule() {
+    size_t left = items_.size();
+    while (left) {
+      uint32_t open = 0;
+      for (Item& I : items_) {
+        if (I.done) continue;
+        if (I.kind == Item::PHASE && !(I.diag & open)) {
+          pend(I.diag, I.cnr, I.m[0]);
+          I.done = true;
+          --left;
+        } else {
+          open |= I.dense;
         }
-        case Instr::PHASE: {
-          const Phase& P = I.a;
-          const double u[2] = {P.uniform.real(), P.uniform.imag()};
-          if (P.signs()) {
-            W.header(TC_SG + I.A, uint32_t(P.list.size()));
-            W.head().w[2] = P.uniform.real() < 0 ? 1u : 0u;
-            std::vector<uint32_t> v;
-            for (const Entry& e : P.list) v.push_back(e.mask);
-            while (v.size() % 4) v.push_back(~0u);  // never matched: counted off by header.y
-            if (!v.empty()) W.bytes(v.data(), v.size() * 4);
-          } else if (f32 && P.list.empty()) {
-            W.header(TC_PU + I.A);
-            const float f[2] = {float(u[0]), float(u[1])};
-            std::memcpy(&W.head().w[2], f, 8);
-          } else {
-            W.header(TC_PH + I.A, uint32_t(P.list.size()));
-            if (f32) W.head().w[2] = turns(P.uniform);
-            else W.reals(u, 2);
-            W.list(P.list);
-          }
-          break;
-        }
-        case Instr::PAIR: {
-          W.header(TC_D + uint32_t(I.bit), uint32_t(I.a.list.size()) | uint32_t(I.b.list.size()) << 16);
-          if (f32) {
-            W.head().w[2] = turns(I.a.uniform);
-            W.head().w[3] = turns(I.b.uniform);
-          } else {
-            const double u[4] = {I.a.uniform.real(), I.a.uniform.imag(), I.b.uniform.real(), I.b.uniform.imag()};
-            W.reals(u, 4);
-          }
-          W.list(I.a.list);
-          W.list(I.b.list);
-          break;
-        }
-        case Instr::LEGACY:
-          W.header(TC_LEG);
-          W.bytes(&enc_[I.op], sizeof(TileOp<Real>));
-          break;
       }
-      W.end();
+      uint32_t dense_open = 0, diag_open = 0, bits = 0;
+      std::vector<size_t> batch;
+      for (size_t i = 0; i < items_.size(); ++i) {
+        const Item& I = items_[i];
+        if (I.done) continue;
+        if (I.kind != Item::PHASE && !(I.dense & (dense_open | diag_open)) && !(I.diag & dense_open)) {
+          batch.push_back(i);
+          bits |= I.dense;
+        }
+        dense_open |= I.dense;
+        diag_open |= I.diag;
+      }
+      if (batch.empty()) break;  // only phases were left
+      flush(bits);
+      for (size_t i : batch) {
+        emit(items_[i]);
+        items_[i].done = true;
+        --left;
+      }
     }
   }
+
+  void pend(uint32_t A, uint32_t B, cplx p) {
+    Phase& P = pend_[A];
+    P.used = true;
+    if (B == 0) { P.uniform *= p; return; }
+    for (size_t i = 0; i < P.list.size(); ++i)
+      if (P.list[i].mask == B) {
+        P.list[i].p *= p;
+        if (P.list[i].p == cplx(1.0, 0.0)) P.list.erase(P.list.begin() + long(i));
+        return;
+      }
+    P.list.push_back(Entry{B, p});
+  }
+
+  // ---- emission -----------------------------------------------------------
+  // Constant phases among the sets `which`: one table of all pending ones when
+  // that is cheaper than one instruction each (per amplitude: 4 operations and
+  // half a load in the table, 4 alone, 2 for a sign; 30 for an instruction).
+  void join_constant(const std::vector<uint32_t>& which) {
+    long alone = 0;
+    for (uint32_t A : which) {
+      const Phase& P = pend_[A];
+      if (P.uniform == cplx(1.0, 0.0) || !P.list.empty()) continue;
+      alone += 30 + (P.uniform == cplx(-1.0, 0.0) ? 2L : 4L) * long(kAll >> __builtin_popcount(A));
+    }
+    if (alone <= 30 + 9L * long(kAll) / 2) return;
+    std::vector<double> v(2 * kAll);
+    for (uint32_t r = 0; r < kAll; ++r) {
+      cplx p(1.0, 0.0);
+      for (uint32_t A = 0; A < kAll; ++A)
+        if ((r & A) == A) p *= pend_[A].uniform;
+      v[2 * r] = p.real();
+      v[2 * r + 1] = p.imag();
+    }
+    for (uint32_t A = 0; A < kAll; ++A) {
+      pend_[A].uniform = cplx(1.0, 0.0);
+      if (pend_[A].list.empty()) pend_[A] = Phase();
+    }
+    W_.header(TC_T);
+    W_.reals(v.data(), int(v.size()));
+    W_.end();
+  }
+
+  // Emit the pending phases that do not commute with a dense item on bits `t`.
+  void flush(uint32_t t) {
+    std::vector<uint32_t> which;
+    for (uint32_t A = 1; A < kAll; ++A)
+      if ((A & t) && pend_[A].used) which.push_back(A);
+    // the phase on all amplitudes can wait: it goes with the stage's last ones
+    const cplx all = pend_[0].uniform;
+    pend_[0].uniform = cplx(1.0, 0.0);
+    join_constant(which);
+    pend_[0].uniform = all;
+    for (uint32_t A : which) {
+      put(A, pend_[A]);
+      pend_[A] = Phase();
+    }
+  }
+
+  // Stage end: what is left; a list on all amplitudes joins one on a bit.
+  void finish() {
+    std::vector<uint32_t> which;
+    for (uint32_t A = 0; A < kAll; ++A) which.push_back(A);
+    join_constant(which);
+    const Phase all = pend_[0];
+    int join = -1;
+    if (!all.trivial())
+      for (int b = 0; b < kBits && join < 0; ++b) {
+        const Phase& P = pend_[1u << b];
+        if (P.used && !P.trivial() && !P.signs()) join = b;
+      }
+    for (uint32_t A = 1; A < kAll; ++A)
+      if (pend_[A].used && (join < 0 || A != (1u << join))) put(A, pend_[A]);
+    if (join < 0) put(0, all);
+    else pair(join, all, pend_[1u << join]);
+  }
+
+  void put(uint32_t A, const Phase& P) {
+    if (P.trivial()) return;
+    const double u[2] = {P.uniform.real(), P.uniform.imag()};
+    if (P.signs()) {
+      if (P.list.empty()) {
+        W_.header(TC_SG + A);
+      } else {
+        W_.header(TC_SL + A, uint32_t(P.list.size()));
+        W_.head().w[2] = u[0] < 0 ? 1u : 0u;
+        std::vector<uint32_t> v;
+        for (const Entry& e : P.list) v.push_back(e.mask);
+        W_.bytes(v.data(), v.size() * 4);
+      }
+    } else if (P.list.empty()) {
+      W_.header(TC_PU + A);
+      pair_of(u);
+    } else {
+      W_.header(TC_PH + A, uint32_t(P.list.size()));
+      if (kF32) W_.head().w[2] = turns(P.uniform);
+      else W_.reals(u, 2);
+      W_.list(P.list);
+    }
+    W_.end();
+  }
+
+  void pair(int b, const Phase& all, const Phase& bit) {
+    W_.header(TC_D + uint32_t(b), uint32_t(all.list.size()) | uint32_t(bit.list.size()) << 16);
+    if (kF32) {
+      W_.head().w[2] = turns(all.uniform);
+      W_.head().w[3] = turns(bit.uniform);
+    } else {
+      const double u[4] = {all.uniform.real(), all.uniform.imag(), bit.uniform.real(), bit.uniform.imag()};
+      W_.reals(u, 4);
+    }
+    W_.list(all.list);
+    W_.list(bit.list);
+    W_.end();
+  }
+
+  // Two reals of an instruction: in the header (complex64) or the next word.
+  void pair_of(const double* v) {
+    if (kF32) {
+      const float f[2] = {float(v[0]), float(v[1])};
+      std::memcpy(&W_.head().w[2], f, 8);
+    } else {
+      W_.reals(v, 2);
+    }
+  }
+
+  void emit(const Item& I) {
+    switch (I.kind) {
+      case Item::ROT:
+      case Item::CROSS: {
+        const double v[2] = {I.t, I.s};
+        W_.header((I.kind == Item::ROT ? TC_R : TC_X) + uint32_t(ctz(I.dense)), I.cnr);
+        pair_of(v);
+        break;
+      }
+      case Item::GENERIC: {
+        double v[8];
+        for (int i = 0; i < 4; ++i) { v[2 * i] = I.m[i].real(); v[2 * i + 1] = I.m[i].imag(); }
+        W_.header(TC_G + uint32_t(ctz(I.dense)), I.cnr);
+        W_.reals(v, 8);
+        break;
+      }
+      default:
+        W_.header(TC_LEG);
+        W_.bytes(&enc_[I.op], sizeof(TileOp<Real>));
+        break;
+    }
+    W_.end();
+  }
+
+  static int ctz(uint32_t v) { return __builtin_ctz(v); }
 
   const std::vector<Op>& ops_;
   const TilePlan& plan_;
   const std::vector<TileOp<Real>>& enc_;
-  std::vector<Instr> code_;
+  Writer W_;
+  std::vector<Item> items_;
   Phase pend_[32];
-  int open_[5];
+  cplx acc_[5][4];
+  bool have_[5];
 };
 
 // Shared-memory slot of vector u (the kernels' swz).
@@ -397,11 +533,80 @@ void compile(const std::vector<Op>& ops, TilePlan* plan, const std::vector<TileO
       std::memcpy(static_cast<void*>(plan->prog.data() + tabs + size_t(s - P.stage_begin) * (kStageTabWords / 4)), tab,
                   sizeof(tab));
     }
+    plan->prog.push_back(ProgWord{{0, 0, 0, 0}});  // the kernel reads one word past a header
     P.prog_words = int32_t(plan->prog.size() - tabs);
   }
 }
 
+// A complex unitary 2x2 without controls that is neither real nor of RX's form.
+bool takes_carry(const Op& o) {
+  if (o.kind != OP_U1 || o.nctrl != 0) return false;
+  const cplx* m = o.m;
+  const double eps = 1e-12;
+  if (std::abs(std::norm(m[0]) + std::norm(m[2]) - 1.0) > eps || std::abs(std::norm(m[1]) + std::norm(m[3]) - 1.0) > eps ||
+      std::abs(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) > eps)
+    return false;
+  const bool real = m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0;
+  const bool cross = m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
+  return !real && !cross && std::abs(m[0]) > 1e-6 && std::abs(m[2]) > 1e-6;
+}
+
+void times(const cplx* a, const cplx* b, cplx* out) {
+  const cplx r[4] = {a[0] * b[0] + a[1] * b[2], a[0] * b[1] + a[1] * b[3], a[2] * b[0] + a[3] * b[2],
+                     a[2] * b[1] + a[3] * b[3]};
+  std::memcpy(static_cast<void*>(out), r, sizeof(r));
+}
+
 }  // namespace
+
+std::vector<Op> carry_phases(const std::vector<Op>& in) {
+  std::vector<Op> ops(in);
+  std::vector<std::vector<size_t>> on(kMaxQubits);
+  for (size_t i = 0; i < ops.size(); ++i)
+    for (int q = 0; q < kMaxQubits; ++q)
+      if ((ops[i].qubit_mask() >> q) & 1) on[size_t(q)].push_back(i);
+  std::vector<size_t> at(kMaxQubits, 0);  // ops of the qubit met so far
+  for (size_t i = 0; i < ops.size(); ++i) {
+    const uint64_t qm = ops[i].qubit_mask();
+    for (int q = 0; q < kMaxQubits; ++q)
+      if ((qm >> q) & 1) ++at[size_t(q)];
+    if (!takes_carry(ops[i])) continue;
+    const int q = ops[i].t0;
+    const std::vector<size_t>& list = on[size_t(q)];
+    bool z = true, x = true, found = false;
+    size_t e = 0;
+    for (size_t k = at[size_t(q)]; k < list.size() && (z || x); ++k) {
+      const Op& o = ops[list[k]];
+      if (takes_carry(o)) {
+        e = list[k];
+        found = true;
+        break;
+      }
+      if (o.diagonal() || ((o.ctrl_mask() >> q) & 1)) x = false;
+      else if (o.kind == OP_X1 && o.t0 == q) z = false;
+      else z = x = false;
+    }
+    if (!found || z == x) continue;  // none, or nothing between: the compiler merges the two
+    cplx* m = ops[i].m;
+    cplx w[4] = {m[0], m[1], m[2], m[3]}, c[4] = {1.0, 0.0, 0.0, 1.0};
+    if (z) {
+      const cplx p = (m[2] / std::abs(m[2])) / (m[0] / std::abs(m[0]));
+      c[3] = p;
+      w[2] = m[2] / p;
+      w[3] = m[3] / p;
+    } else {
+      // RX(al) rotation phase: RX(-al) m has a real ratio in its first column
+      const double al = std::atan2(-2.0 * (std::conj(m[0]) * m[2]).imag(), std::norm(m[0]) - std::norm(m[2]));
+      const double ch = std::cos(al / 2), sh = std::sin(al / 2);
+      const cplx rx[4] = {ch, cplx(0, -sh), cplx(0, -sh), ch}, inv[4] = {ch, cplx(0, sh), cplx(0, sh), ch};
+      std::memcpy(static_cast<void*>(c), rx, sizeof(c));
+      times(inv, m, w);
+    }
+    std::memcpy(static_cast<void*>(m), w, sizeof(w));
+    times(ops[e].m, c, ops[e].m);
+  }
+  return ops;
+}
 
 void build_tile_prog(const std::vector<Op>& ops, TilePlan* plan) {
   plan->prog.clear();

@@ -5,30 +5,38 @@
 // One instruction is a header word and its operands:
 //
 //   header.x   code | words << 16 (words of the instruction, header included)
-//   R + b      real 2x2 on register bit b: header.y = virtual-index mask that must
-//   X + b      be set; the matrix entries (m00, m01, m10, m11) follow, real for R,
-//              real diagonal and imaginary off-diagonal for X, complex for G
-//   G + b
-//   PH + A     phase on the register amplitudes whose bits A are all set.  The
-//              phase is a product over a list of (mask, phase): an entry counts
-//              when the thread's virtual index has all bits of mask set.
-//              header.y = entries.  complex64: angles in 2^-32 turns, header.z =
-//              constant part, two (mask, angle) per word.  complex128: complex
-//              factors, one word constant part, two words (mask) (re, im) each.
-//   PU + A     the same with a constant phase (complex64: re, im in header.z, .w)
+//   R + b      real rotation on register bit b as three shears (t = tan(phi / 2),
+//              s = sin(phi), |phi| <= pi/2): header.y = virtual-index mask that must
+//              be set; t, s in header.z, .w (complex64) or the next word
+//   X + b      the same with the imaginary off-diagonal of RX
+//   G + b      any complex 2x2: the entries m00, m01, m10, m11 follow
+//   T          one constant phase per register amplitude: 2^(register bits) entries
+//   PU + A     constant phase on the register amplitudes whose bits A are all set
+//              (re, im in header.z, .w or the next word)
+//   SG + A     sign flip of those amplitudes
+//   PH + A     phase on those amplitudes that is a product over a list of (mask,
+//              phase): an entry counts when the thread's virtual index has all
+//              bits of mask set.  header.y = entries.  complex64: angles in
+//              2^-32 turns, header.z = constant part, two (mask, angle) per word.
+//              complex128: complex factors, one word constant part, two words
+//              (mask) (re, im) each.
 //   D + b      PH on all amplitudes and PH on those with bit b, one multiplication
 //              per amplitude: header.y = entries of the first | of the second
 //              << 16; constant parts in header.z, .w (complex64) or two words
-//   SG + A     sign flips on the amplitudes with bits A: header.y = masks, header.z
-//              = constant parity; four masks per word
+//   SL + A     sign flips: header.y = masks, header.z = constant parity; four
+//              masks per word
 //   LEG        any other op: its TileOp record follows
 //
-// Why a program and not the ops themselves: the tile kernels are bound by issue
-// (FP32) and by the FP64 pipe, and diagonal gates commute, so all phases of a
-// stage that multiply the same register amplitudes are one multiplication whose
-// factor a thread works out once instead of once per amplitude and gate.  A
-// controlled phase costs a list entry (4 instructions) where it took 16 complex
-// products; RY, H and RX need half or less of a complex 2x2 product.
+// Why a program and not the ops themselves: the tile kernels are bound by
+// instructions (every one costs a warp about seven cycles at any occupancy the
+// register block allows) and, for complex128, by the FP64 pipe.  Diagonal gates
+// commute, so all phases of a stage that multiply the same register amplitudes are
+// one multiplication whose factor a thread works out once; a controlled phase
+// costs a list entry (4 instructions) where it took 16 complex products.  Every
+// unitary 2x2 is phase x real rotation x phase: the rotation takes three fused
+// multiply-adds per pair and component in place (a complex 2x2 takes eight and
+// the re / im swaps), and the phases before and after the rotations of a layer
+// join in one T.
 #pragma once
 #include <cstdint>
 #include <vector>
@@ -57,8 +65,17 @@ struct StageTab {
 static_assert(StageTab::SH + 16 <= kStageTabWords && kStageTabWords % 4 == 0, "stage table layout");
 
 enum TileCode : uint32_t {
-  TC_R = 0, TC_X = 8, TC_G = 16, TC_D = 24, TC_PH = 32, TC_PU = 64, TC_SG = 96, TC_LEG = 128,
+  TC_R = 0, TC_X = 8, TC_G = 16, TC_T = 24, TC_PU = 32, TC_SG = 64,
+  TC_LIST = 96,  // from here on the thread evaluates a list first
+  TC_PH = 96, TC_SL = 128, TC_D = 160, TC_LEG = 168,
 };
+
+// The op list with every complex 2x2 reduced to rotation x phase where a later 2x2
+// on its qubit can take the rest: a phase passes through controls and diagonal
+// ops, an RX through X targets, so before a CNOT each of the two qubits hands one
+// of its three Euler angles on.  A layer's gates then need one phase table per
+// stage instead of two.  Same length, same qubits per op.
+std::vector<Op> carry_phases(const std::vector<Op>& ops);
 
 // Compile every stage of `plan` (built from `ops`) into plan->prog and set the
 // word ranges in its pass and stage records: per pass the stage tables, then the

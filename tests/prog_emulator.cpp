@@ -72,15 +72,18 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
     const ProgWord* q = p + 1;
     const ProgWord& h = *p;
     if (len == 0 || p + len > end) return -2;
-    if (code < TC_D) {
+    const cd two = F32 ? cget<float>(p, 1) : cget<double>(q, 0);  // the instruction's two reals
+    if (code < TC_T) {
       const uint32_t b = 1u << (code & 7u);
       if (b >= a.size()) return -3;
       cd m[4];
       if (code >= TC_G) {
         for (int i = 0; i < 4; ++i) m[i] = cget<Real>(q, i);
       } else {
-        const cd u = cget<Real>(q, 0), v = cget<Real>(q, 1), off = code >= TC_X ? cd(0, 1) : cd(1, 0);
-        m[0] = u.real(); m[1] = off * u.imag(); m[2] = off * v.real(); m[3] = v.imag();
+        // the three shears as one matrix
+        const double t = two.real(), s = two.imag(), c = 1 - t * s, o = t * (2 - t * s);
+        const cd f = code >= TC_X ? cd(0, 1) : cd(1, 0);
+        m[0] = c; m[1] = -f * o; m[2] = (code >= TC_X ? -f : f) * s; m[3] = c;
       }
       for (uint32_t i = 0; hit(h.w[1]) && i < a.size(); ++i) {
         if (i & b) continue;
@@ -88,33 +91,28 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
         a[i] = m[0] * x + m[1] * y;
         a[i | b] = m[2] * x + m[3] * y;
       }
-    } else if (code < TC_PH) {
+    } else if (code == TC_T) {
+      for (uint32_t i = 0; i < a.size(); ++i) a[i] *= cget<Real>(q, int(i));
+    } else if (code < TC_SG) {
+      for (uint32_t i = 0; i < a.size(); ++i)
+        if ((i & (code & 31u)) == (code & 31u)) a[i] *= two;
+    } else if (code < TC_LIST || (code >= TC_SL && code < TC_D)) {
+      uint32_t s = code < TC_LIST ? 1u : h.w[2];
+      for (uint32_t i = 0; code >= TC_SL && i < h.w[1]; ++i) s += hit(q[i / 4].w[i & 3]);
+      for (uint32_t i = 0; i < a.size(); ++i)
+        if ((i & (code & 31u)) == (code & 31u) && (s & 1)) a[i] = -a[i];
+    } else if (code < TC_SL) {
+      if (!F32) ++q;
+      const cd v = list(q, h.w[1], F32 ? turn(h.w[2]) : two);
+      for (uint32_t i = 0; i < a.size(); ++i)
+        if ((i & (code & 31u)) == (code & 31u)) a[i] *= v;
+    } else if (code < TC_LEG) {
       const uint32_t b = 1u << (code - TC_D);
-      cd d0, d1;
-      if (F32) {
-        d0 = turn(h.w[2]);
-        d1 = turn(h.w[3]);
-      } else {
-        d0 = cget<double>(q, 0);
-        d1 = cget<double>(q, 1);
-        q += 2;
-      }
+      cd d0 = F32 ? turn(h.w[2]) : two, d1 = F32 ? turn(h.w[3]) : cget<double>(q, 1);
+      if (!F32) q += 2;
       d0 = list(q, h.w[1] & 0xFFFFu, d0);
       d1 = d0 * list(q, h.w[1] >> 16, d1);
       for (uint32_t i = 0; i < a.size(); ++i) a[i] *= (i & b) ? d1 : d0;
-    } else if (code < TC_SG) {
-      const uint32_t A = code & 31u;
-      cd v(1, 0);
-      if (code >= TC_PU) v = cget<float>(p, 1);
-      else if (F32) v = list(q, h.w[1], turn(h.w[2]));
-      else { v = cget<double>(q, 0); ++q; v = list(q, h.w[1], v); }
-      for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & A) == A) a[i] *= v;
-    } else if (code < TC_LEG) {
-      uint32_t s = h.w[2];
-      for (uint32_t i = 0; i < h.w[1]; ++i) s += hit(q[i / 4].w[i & 3]);
-      for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & (code & 31u)) == (code & 31u) && (s & 1)) a[i] = -a[i];
     } else {
       TileOp<Real> t;
       std::memcpy(&t, q, sizeof(t));
@@ -193,7 +191,7 @@ extern "C" int prog_run(int n, int c64, int kmax, const double* flat, int ngates
   const int vb = c64 ? 1 : 0, nrb = vb + kRegFree;
   TilePlan plan;
   std::string err;
-  const std::vector<Op> ops = lower_circuit(gates);
+  const std::vector<Op> ops = carry_phases(lower_circuit(gates));
   if (!build_tile_plan(ops, n, dt, kmax, &plan, &err)) return -1;
   build_tile_prog(ops, &plan);
   stats[0] = int64_t(plan.op_src.size());
@@ -204,7 +202,7 @@ extern "C" int prog_run(int n, int c64, int kmax, const double* flat, int ngates
   for (size_t i = 0; i < dim; ++i) st[i] = cd(state[2 * i], state[2 * i + 1]);
   for (const PassRec& P : plan.passes) {
     const size_t tw = size_t(P.stage_end - P.stage_begin) * (kStageTabWords / 4);
-    for (size_t i = tw; i < size_t(P.prog_words); i += plan.prog[size_t(P.prog_begin) + i].w[0] >> 16) ++stats[1];
+    for (size_t i = tw; i + 1 < size_t(P.prog_words); i += plan.prog[size_t(P.prog_begin) + i].w[0] >> 16) ++stats[1];
     auto qubit = [&](int tb) { return tb < P.c ? tb : P.qhi[tb - P.c]; };
     for (int s = P.stage_begin; s < P.stage_end; ++s) {
       const StageRec& S = plan.stages[size_t(s)];
