@@ -336,7 +336,7 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
   p->stats = PlanStats{};
   if (mode == NQPU_MODE_TILED && int(n) >= tile_min_qubits(dt)) {
     std::string err;
-    p->ops = carry_phases(p->ops);
+    p->ops = carry_phases(std::move(p->ops));
     p->tile_cfg = tile_config_raw(dt);
     if (!build_tile_plan_for(p->ops, int(n), dt, &p->tile, &err)) return false;
     build_tile_prog(p->ops, &p->tile);

@@ -486,7 +486,7 @@ extern "C" NqpuError nqpu_server_submit(NqpuServer* server, const NqpuCircuit* c
     r->tcplan.bmats.shrink_to_fit();
   } else if (int(c->n) >= tile_min_qubits(DType::C64)) {
     std::string err;
-    ops = carry_phases(ops);
+    ops = carry_phases(std::move(ops));
     if (!build_tile_plan_for(ops, int(c->n), DType::C64, &r->plan, &err))
       return NQPU_INVALID_PARAMETER;
     build_tile_prog(ops, &r->plan);

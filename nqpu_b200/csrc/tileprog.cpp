@@ -15,6 +15,11 @@ struct Phase {
   bool used = false;
   cplx uniform{1.0, 0.0};
   std::vector<Entry> list;
+  void clear() {  // keeps the list's memory
+    used = false;
+    uniform = cplx(1.0, 0.0);
+    list.clear();
+  }
   bool trivial() const { return list.empty() && uniform == cplx(1.0, 0.0); }
   bool signs() const {  // only factors of +1 and -1
     if (uniform != cplx(1.0, 0.0) && uniform != cplx(-1.0, 0.0)) return false;
@@ -51,10 +56,11 @@ class Writer {
   }
   void end() { (*out_)[begin_].w[0] |= uint32_t(out_->size() - begin_) << 16; }
   ProgWord& head() { return (*out_)[begin_]; }  // valid until more is written
-  void reals(const double* v, int n) {
+  void reals(const double* v, int n) {  // at most 64
     if (f32_) {
-      std::vector<float> f(v, v + n);
-      bytes(f.data(), sizeof(float) * size_t(n));
+      float f[64];
+      for (int i = 0; i < n; ++i) f[i] = float(v[i]);
+      bytes(f, sizeof(float) * size_t(n));
     } else {
       bytes(v, sizeof(double) * size_t(n));
     }
@@ -66,9 +72,10 @@ class Writer {
   }
   void list(const std::vector<Entry>& l) {
     if (f32_) {
-      std::vector<uint32_t> v;
-      for (const Entry& e : l) { v.push_back(e.mask); v.push_back(turns(e.p)); }
-      if (!v.empty()) bytes(v.data(), v.size() * 4);
+      for (size_t i = 0; i < l.size(); i += 2) {
+        const bool two = i + 1 < l.size();
+        out_->push_back(ProgWord{{l[i].mask, turns(l[i].p), two ? l[i + 1].mask : 0u, two ? turns(l[i + 1].p) : 0u}});
+      }
     } else {
       for (const Entry& e : l) {
         out_->push_back(ProgWord{{e.mask, 0, 0, 0}});
@@ -95,7 +102,8 @@ class StageCompiler {
   void run(const StageRec& S, bool last, cplx* global, std::vector<ProgWord>* out) {
     W_ = Writer(out, sizeof(Real) == 4);
     items_.clear();
-    for (Phase& p : pend_) p = Phase();
+    for (Phase& p : pend_) p.clear();
+    used_ = 0;
     for (bool& h : have_) h = false;
     for (int o = S.op_begin; o < S.op_end; ++o) add(size_t(o));
     for (int b = 0; b < kBits; ++b) settle(b);
@@ -281,7 +289,8 @@ class StageCompiler {
         }
       }
       uint32_t dense_open = 0, diag_open = 0, bits = 0;
-      std::vector<size_t> batch;
+      std::vector<size_t>& batch = batch_;
+      batch.clear();
       for (size_t i = 0; i < items_.size(); ++i) {
         const Item& I = items_[i];
         if (I.done) continue;
@@ -305,6 +314,7 @@ class StageCompiler {
   void pend(uint32_t A, uint32_t B, cplx p) {
     Phase& P = pend_[A];
     P.used = true;
+    used_ |= 1u << A;
     if (B == 0) { P.uniform *= p; return; }
     for (size_t i = 0; i < P.list.size(); ++i)
       if (P.list[i].mask == B) {
@@ -319,61 +329,68 @@ class StageCompiler {
   // Constant phases among the sets `which`: one table of all pending ones when
   // that is cheaper than one instruction each (per amplitude: 4 operations and
   // half a load in the table, 4 alone, 2 for a sign; 30 for an instruction).
-  void join_constant(const std::vector<uint32_t>& which) {
+  void join_constant(uint32_t which) {
     long alone = 0;
-    for (uint32_t A : which) {
+    for (uint32_t w = which; w; w &= w - 1) {
+      const uint32_t A = uint32_t(ctz(w));
       const Phase& P = pend_[A];
       if (P.uniform == cplx(1.0, 0.0) || !P.list.empty()) continue;
       alone += 30 + (P.uniform == cplx(-1.0, 0.0) ? 2L : 4L) * long(kAll >> __builtin_popcount(A));
     }
     if (alone <= 30 + 9L * long(kAll) / 2) return;
-    std::vector<double> v(2 * kAll);
-    for (uint32_t r = 0; r < kAll; ++r) {
-      cplx p(1.0, 0.0);
-      for (uint32_t A = 0; A < kAll; ++A)
-        if ((r & A) == A) p *= pend_[A].uniform;
-      v[2 * r] = p.real();
-      v[2 * r + 1] = p.imag();
-    }
-    for (uint32_t A = 0; A < kAll; ++A) {
+    cplx v[32];
+    for (cplx& x : v) x = cplx(1.0, 0.0);
+    for (uint32_t w = used_; w; w &= w - 1) {
+      const uint32_t A = uint32_t(ctz(w));
+      const cplx u = pend_[A].uniform;
+      if (u != cplx(1.0, 0.0))
+        for (uint32_t r = A; r < kAll; r = (r + 1) | A) v[r] *= u;
       pend_[A].uniform = cplx(1.0, 0.0);
-      if (pend_[A].list.empty()) pend_[A] = Phase();
+      if (pend_[A].list.empty()) drop(A);
+    }
+    double d[64];
+    for (uint32_t r = 0; r < kAll; ++r) {
+      d[2 * r] = v[r].real();
+      d[2 * r + 1] = v[r].imag();
     }
     W_.header(TC_T);
-    W_.reals(v.data(), int(v.size()));
+    W_.reals(d, 2 * int(kAll));
     W_.end();
+  }
+  void drop(uint32_t A) {
+    pend_[A].clear();
+    used_ &= ~(1u << A);
   }
 
   // Emit the pending phases that do not commute with a dense item on bits `t`.
   void flush(uint32_t t) {
-    std::vector<uint32_t> which;
-    for (uint32_t A = 1; A < kAll; ++A)
-      if ((A & t) && pend_[A].used) which.push_back(A);
+    uint32_t which = 0;
+    for (uint32_t w = used_ & ~1u; w; w &= w - 1)
+      if (uint32_t(ctz(w)) & t) which |= w & (~w + 1);
     // the phase on all amplitudes can wait: it goes with the stage's last ones
     const cplx all = pend_[0].uniform;
     pend_[0].uniform = cplx(1.0, 0.0);
     join_constant(which);
-    pend_[0].uniform = all;
-    for (uint32_t A : which) {
-      put(A, pend_[A]);
-      pend_[A] = Phase();
+    if (all != cplx(1.0, 0.0)) pend(0, 0, all);
+    for (uint32_t w = which & used_; w; w &= w - 1) {
+      put(uint32_t(ctz(w)), pend_[ctz(w)]);
+      drop(uint32_t(ctz(w)));
     }
   }
 
   // Stage end: what is left; a list on all amplitudes joins one on a bit.
   void finish() {
-    std::vector<uint32_t> which;
-    for (uint32_t A = 0; A < kAll; ++A) which.push_back(A);
-    join_constant(which);
-    const Phase all = pend_[0];
+    if (pend_[0].uniform != cplx(1.0, 0.0)) used_ |= 1u;
+    join_constant(used_);
+    const Phase& all = pend_[0];
     int join = -1;
     if (!all.trivial())
       for (int b = 0; b < kBits && join < 0; ++b) {
         const Phase& P = pend_[1u << b];
         if (P.used && !P.trivial() && !P.signs()) join = b;
       }
-    for (uint32_t A = 1; A < kAll; ++A)
-      if (pend_[A].used && (join < 0 || A != (1u << join))) put(A, pend_[A]);
+    for (uint32_t w = used_ & ~1u; w; w &= w - 1)
+      if (join < 0 || ctz(w) != (1 << join)) put(uint32_t(ctz(w)), pend_[ctz(w)]);
     if (join < 0) put(0, all);
     else pair(join, all, pend_[1u << join]);
   }
@@ -458,7 +475,9 @@ class StageCompiler {
   const std::vector<TileOp<Real>>& enc_;
   Writer W_;
   std::vector<Item> items_;
+  std::vector<size_t> batch_;
   Phase pend_[32];
+  uint32_t used_ = 0;  // pend_ entries in use
   cplx acc_[5][4];
   bool have_[5];
 };
@@ -559,26 +578,40 @@ void times(const cplx* a, const cplx* b, cplx* out) {
 
 }  // namespace
 
-std::vector<Op> carry_phases(const std::vector<Op>& in) {
-  std::vector<Op> ops(in);
-  std::vector<std::vector<size_t>> on(kMaxQubits);
-  for (size_t i = 0; i < ops.size(); ++i)
-    for (int q = 0; q < kMaxQubits; ++q)
-      if ((ops[i].qubit_mask() >> q) & 1) on[size_t(q)].push_back(i);
-  std::vector<size_t> at(kMaxQubits, 0);  // ops of the qubit met so far
+std::vector<Op> carry_phases(std::vector<Op> ops) {
+  size_t takers = 0;
+  for (const Op& o : ops) takers += takes_carry(o);
+  if (takers < 2) return ops;
+  // the op after op i on each of its (at most five) qubits, from a backward walk
+  struct Next {
+    int8_t q[5];
+    int32_t op[5];
+    int n = 0;
+  };
+  std::vector<Next> next(ops.size());
+  int32_t seen[64];
+  for (int32_t& v : seen) v = -1;
+  for (size_t i = ops.size(); i-- > 0;)
+    for (uint64_t m = ops[i].qubit_mask(); m; m &= m - 1) {
+      const int q = __builtin_ctzll(m);
+      next[i].q[next[i].n] = int8_t(q);
+      next[i].op[next[i].n++] = seen[q];
+      seen[q] = int32_t(i);
+    }
+  auto after = [&](size_t i, int q) {
+    for (int k = 0; k < next[i].n; ++k)
+      if (next[i].q[k] == q) return next[i].op[k];
+    return -1;
+  };
   for (size_t i = 0; i < ops.size(); ++i) {
-    const uint64_t qm = ops[i].qubit_mask();
-    for (int q = 0; q < kMaxQubits; ++q)
-      if ((qm >> q) & 1) ++at[size_t(q)];
     if (!takes_carry(ops[i])) continue;
     const int q = ops[i].t0;
-    const std::vector<size_t>& list = on[size_t(q)];
     bool z = true, x = true, found = false;
     size_t e = 0;
-    for (size_t k = at[size_t(q)]; k < list.size() && (z || x); ++k) {
-      const Op& o = ops[list[k]];
+    for (int32_t k = after(i, q); k >= 0 && (z || x); k = after(size_t(k), q)) {
+      const Op& o = ops[size_t(k)];
       if (takes_carry(o)) {
-        e = list[k];
+        e = size_t(k);
         found = true;
         break;
       }

@@ -75,7 +75,7 @@ enum TileCode : uint32_t {
 // ops, an RX through X targets, so before a CNOT each of the two qubits hands one
 // of its three Euler angles on.  A layer's gates then need one phase table per
 // stage instead of two.  Same length, same qubits per op.
-std::vector<Op> carry_phases(const std::vector<Op>& ops);
+std::vector<Op> carry_phases(std::vector<Op> ops);
 
 // Compile every stage of `plan` (built from `ops`) into plan->prog and set the
 // word ranges in its pass and stage records: per pass the stage tables, then the
