@@ -244,12 +244,29 @@ __device__ __forceinline__ void rb_u2(C (&a)[NA], const Real* __restrict__ mp, b
     const bool cond = tc && ((uint32_t(i) & creg) == creg);
     const C x0 = a[i], x1 = a[i | M0], x2 = a[i | M1], x3 = a[i | M0 | M1];
     C y[4];
+    if constexpr (sizeof(Real) == 4) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      C m[4];
-      ldc2<Real>(mp + 8 * r, m[0], m[1]);
-      ldc2<Real>(mp + 8 * r + 4, m[2], m[3]);
-      y[r] = cmac4(m, x0, x1, x2, x3);
+      for (int r = 0; r < 4; ++r) {
+        C m[4];
+        ldc2<Real>(mp + 8 * r, m[0], m[1]);
+        ldc2<Real>(mp + 8 * r + 4, m[2], m[3]);
+        y[r] = cmac4(m, x0, x1, x2, x3);
+      }
+    } else {
+      // one entry at a time: the 128-register build has no room for a row
+      auto mac = [&](int k, const C& x, C& acc) {
+        const C m = reinterpret_cast<const C*>(mp)[k];
+        acc.x = fma(m.x, x.x, fma(-m.y, x.y, acc.x));
+        acc.y = fma(m.x, x.y, fma(m.y, x.x, acc.y));
+      };
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        y[r].x = y[r].y = 0;
+        mac(4 * r, x0, y[r]);
+        mac(4 * r + 1, x1, y[r]);
+        mac(4 * r + 2, x2, y[r]);
+        mac(4 * r + 3, x3, y[r]);
+      }
     }
     a[i] = csel(cond, y[0], x0);
     a[i | M0] = csel(cond, y[1], x1);
@@ -386,29 +403,73 @@ __device__ __forceinline__ double2 list_phase(const uint4*& p, uint32_t cnt, dou
   return v;
 }
 
+template <typename Real, int NA, int NRB>
+__device__ __forceinline__ void rotate_bits(typename Tr<Real>::C (&a)[NA], uint32_t bits, const uint4& h,
+                                            const uint4* q, bool cross) {
+  using C = typename Tr<Real>::C;
+  auto par = [&](int b) {  // t, s of bit b
+    C v;
+    if constexpr (sizeof(Real) == 4) {
+      if (b == 0) v = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
+      else v = reinterpret_cast<const float2*>(q)[b - 1];
+    } else {
+      v = reinterpret_cast<const double2*>(q)[b];
+    }
+    return v;
+  };
+#define NQ_ROT(B, _) \
+  if constexpr (B < NRB) { \
+    if (bits & (1u << B)) { \
+      const C v = par(B); \
+      if (cross) rb_cross<C, NA, B>(a, v.x, v.y); \
+      else rb_rot<C, NA, B>(a, v.x, v.y); \
+    } \
+  }
+  NQ_REG_CASES(NQ_ROT, 0)
+#undef NQ_ROT
+}
+
 // Run a stage's program (tileprog.h) on the thread's register block.
 // vbase = virtual index of register amplitude 0 (register bits are zero in it).
+// Whole warps run it: the headers are made warp-uniform values, so that the
+// dispatch compiles to uniform branches.
 template <typename Real, int NA, int NRB>
 __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], const uint4* p,
                                                  const uint4* const end, uint32_t vbase) {
   using C = typename Tr<Real>::C;
   constexpr bool F32 = sizeof(Real) == 4;
   while (p < end) {
-    const uint4 h = *p;
+    uint4 h = *p;
     const uint4* q = p + 1;
-    uint32_t code = h.x & 0xFFFFu;
-    C d0;  // the instruction's two reals
-    if constexpr (F32) d0 = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
-    else d0 = *reinterpret_cast<const double2*>(q);  // (the word table ends in a spare word)
-    C d1 = d0;
-    uint32_t sign = 0x80000000u;
+    h.x = __shfl_sync(0xffffffffu, h.x, 0);
+    const uint32_t code = h.x & 0xFFu, arg = (h.x >> 8) & 0xFFu;
     p += max(h.x >> 16, 1u);  // ends on any contents
-    if (code >= TC_LIST) {
-      if (code < TC_SL) {
-        if constexpr (F32) d0 = phase_of(list_angle(q, h.y, h.z, vbase));
-        else d0 = list_phase(++q, h.y, d0, vbase);
-        code += TC_PU - TC_PH;
-      } else if (code < TC_D) {
+    if (code <= TC_X) {
+      const uint32_t bits = __shfl_sync(0xffffffffu, h.y, 0);
+      if (code == TC_R) rotate_bits<Real, NA, NRB>(a, bits, h, q, false);
+      else rotate_bits<Real, NA, NRB>(a, bits, h, q, true);
+    } else if (code == TC_T) {
+      rb_table<Real, C, NA>(a, q);
+    } else if (code <= TC_PH) {
+      C d;
+      if constexpr (F32) {
+        if (code == TC_PU) d = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
+        else d = phase_of(list_angle(q, h.y, h.z, vbase));
+      } else {
+        d = *reinterpret_cast<const double2*>(q);
+        if (code == TC_PH) d = list_phase(++q, h.y, d, vbase);
+      }
+      switch (arg) {
+#define NQ_A(V) case V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d); break;
+#define NQ_SETS(M) M(0) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) \
+        M(16) M(17) M(18) M(19) M(20) M(21) M(22) M(23) M(24) M(25) M(26) M(27) M(28) M(29) M(30) M(31)
+        NQ_SETS(NQ_A)
+#undef NQ_A
+        default: break;
+      }
+    } else if (code <= TC_SL) {
+      uint32_t sign = 1u;
+      if (code == TC_SL) {
         sign = h.z;
         for (uint32_t i = 0; i < h.y; i += 4) {
           const uint4 e = *q++;
@@ -417,49 +478,47 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
           if (i + 2 < h.y) sign += (vbase & e.z) == e.z;
           if (i + 3 < h.y) sign += (vbase & e.w) == e.w;
         }
-        sign <<= 31;
-        code += TC_SG - TC_SL;
-      } else if (code < TC_LEG) {
-        if constexpr (F32) {
-          const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
-          d0 = phase_of(g);
-          d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
-        } else {
-          d1 = *reinterpret_cast<const double2*>(q + 1);
-          q += 2;
-          d0 = list_phase(q, h.y & 0xFFFFu, d0, vbase);
-          d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
-        }
       }
-    } else if (code < TC_T && (vbase & h.y) != h.y) {
-      continue;  // a 2x2 with a control outside the registers
-    }
-    switch (code) {
-#define NQ_B(B, _) \
-      case TC_R + B: if constexpr (B < NRB) rb_rot<C, NA, B>(a, d0.x, d0.y); break; \
-      case TC_X + B: if constexpr (B < NRB) rb_cross<C, NA, B>(a, d0.x, d0.y); break; \
-      case TC_G + B: \
-        if constexpr (B < NRB) { \
-          C m0, m1, m2, m3; \
-          ldc2<Real>(reinterpret_cast<const Real*>(q), m0, m1); \
-          ldc2<Real>(reinterpret_cast<const Real*>(q) + 4, m2, m3); \
-          rb_u1<C, NA, B>(a, m0, m1, m2, m3); \
-        } \
-        break; \
-      case TC_D + B: if constexpr (B < NRB) rb_d1<C, NA, B>(a, d0, d1); break;
-      NQ_REG_CASES(NQ_B, 0)
-#undef NQ_B
-      case TC_T: rb_table<Real, C, NA>(a, q); break;
-#define NQ_A(V) \
-      case TC_PU + V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d0); break; \
-      case TC_SG + V: if constexpr (V < (1 << NRB)) rb_sign<C, NA, V>(a, sign); break;
-      NQ_A(0) NQ_A(1) NQ_A(2) NQ_A(3) NQ_A(4) NQ_A(5) NQ_A(6) NQ_A(7)
-      NQ_A(8) NQ_A(9) NQ_A(10) NQ_A(11) NQ_A(12) NQ_A(13) NQ_A(14) NQ_A(15)
-      NQ_A(16) NQ_A(17) NQ_A(18) NQ_A(19) NQ_A(20) NQ_A(21) NQ_A(22) NQ_A(23)
-      NQ_A(24) NQ_A(25) NQ_A(26) NQ_A(27) NQ_A(28) NQ_A(29) NQ_A(30) NQ_A(31)
+      sign <<= 31;
+      switch (arg) {
+#define NQ_A(V) case V: if constexpr (V < (1 << NRB)) rb_sign<C, NA, V>(a, sign); break;
+        NQ_SETS(NQ_A)
 #undef NQ_A
-      case TC_LEG: apply_record<Real, NA, NRB>(a, reinterpret_cast<const TileOp<Real>*>(q), vbase); break;
-      default: break;
+#undef NQ_SETS
+        default: break;
+      }
+    } else if (code == TC_D) {
+      C d0, d1;
+      if constexpr (F32) {
+        const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
+        d0 = phase_of(g);
+        d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
+      } else {
+        d0 = *reinterpret_cast<const double2*>(q);
+        d1 = *reinterpret_cast<const double2*>(q + 1);
+        q += 2;
+        d0 = list_phase(q, h.y & 0xFFFFu, d0, vbase);
+        d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
+      }
+      switch (arg) {
+#define NQ_B(B, _) case B: if constexpr (B < NRB) rb_d1<C, NA, B>(a, d0, d1); break;
+        NQ_REG_CASES(NQ_B, 0)
+#undef NQ_B
+        default: break;
+      }
+    } else if (code == TC_G) {
+      C m0, m1, m2, m3;
+      ldc2<Real>(reinterpret_cast<const Real*>(q), m0, m1);
+      ldc2<Real>(reinterpret_cast<const Real*>(q) + 4, m2, m3);
+      const bool tc = (vbase & h.y) == h.y;  // controls outside the registers
+      switch (arg) {
+#define NQ_B(B, _) case B: if constexpr (B < NRB) { if (tc) rb_u1<C, NA, B>(a, m0, m1, m2, m3); } break;
+        NQ_REG_CASES(NQ_B, 0)
+#undef NQ_B
+        default: break;
+      }
+    } else {
+      apply_record<Real, NA, NRB>(a, reinterpret_cast<const TileOp<Real>*>(q), vbase);
     }
   }
 }
@@ -522,8 +581,10 @@ __device__ __forceinline__ void load_pass_prog(const PassRec& P, const uint4* __
 
 // Run stages [P.stage_begin, P.stage_end) of a pass on the tile held in shared
 // memory `sv` (swizzled vector slots), with the pass's stage tables in `tabs`.
-// Every thread of the CTA must call it (it contains block barriers); threads
-// >= nvec/16 only take part in them.
+// Every thread of the CTA must call it (it contains block barriers); warps
+// beyond nvec/16 threads only take part in them, and in a warp that is only partly
+// needed the other lanes run along on an earlier thread's amplitudes without
+// writing.
 template <typename Real>
 __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict__ sv, const PassRec& P,
                                                 const uint32_t* __restrict__ tabs,
@@ -540,11 +601,13 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
   const uint32_t words = uint32_t(P.prog_words - nst * (kStageTabWords / 4));
   for (int si = 0; si < nst; ++si) {
     const uint32_t* Tb = tabs + si * kStageTabWords;
-    if (uint32_t(tid) < active_threads) {
-      const uint32_t ub = Tb[StageTab::UL + (tid & 15)] | Tb[StageTab::UH + (tid >> 4)];
+    if (uint32_t(tid & ~31) < active_threads) {
+      const bool writes = uint32_t(tid) < active_threads;
+      const int tid_ = writes ? tid : tid & int(active_threads - 1);
+      const uint32_t ub = Tb[StageTab::UL + (tid_ & 15)] | Tb[StageTab::UH + (tid_ >> 4)];
       // swz is linear over XOR and ub, vm_i have disjoint bits, so
       // swz(ub | sum vm_i) = swz(ub) ^ xor_i swz(vm_i).
-      const uint32_t sb = Tb[StageTab::SL + (tid & 15)] ^ Tb[StageTab::SH + (tid >> 4)];
+      const uint32_t sb = Tb[StageTab::SL + (tid_ & 15)] ^ Tb[StageTab::SH + (tid_ >> 4)];
       const uint4 sq = *reinterpret_cast<const uint4*>(Tb + StageTab::S);
       const uint32_t s0 = sq.x, s1 = sq.y, s2 = sq.z, s3 = sq.w;
       C a[NA];
@@ -556,67 +619,69 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
       }
       const uint32_t vbase = (ub << VB) | ext;
       apply_stage_prog<Real, NA, NRB>(a, prog + Tb[StageTab::OB], prog + min(Tb[StageTab::OE], words), vbase);
-      // Write-back through the stage's deferred permutation pi(p) = A p ^ w:
-      // register amplitude p goes to the slot of logical index pi(p).  Slot
-      // offsets are linear in the free register bits (register bits
-      // VB..VB+3); for complex64, bit 0 of pi(p) selects the 8-byte half.
-      uint32_t wslot = Tb[StageTab::WS], hw = Tb[StageTab::WH];
-      const int nc = int(Tb[StageTab::NC]);
-      for (int i = 0; i < nc; ++i) {
-        const uint32_t cm = Tb[StageTab::CC + i];
-        if ((vbase & cm) == cm) {
-          wslot ^= Tb[StageTab::CS + i];
-          hw ^= Tb[StageTab::CH + i];
+      if (writes) {
+        // Write-back through the stage's deferred permutation pi(p) = A p ^ w:
+        // register amplitude p goes to the slot of logical index pi(p).  Slot
+        // offsets are linear in the free register bits (register bits
+        // VB..VB+3); for complex64, bit 0 of pi(p) selects the 8-byte half.
+        uint32_t wslot = Tb[StageTab::WS], hw = Tb[StageTab::WH];
+        const int nc = int(Tb[StageTab::NC]);
+        for (int i = 0; i < nc; ++i) {
+          const uint32_t cm = Tb[StageTab::CC + i];
+          if ((vbase & cm) == cm) {
+            wslot ^= Tb[StageTab::CS + i];
+            hw ^= Tb[StageTab::CH + i];
+          }
         }
-      }
-      const uint4 cq = *reinterpret_cast<const uint4*>(Tb + StageTab::CW);
-      const uint32_t c0 = cq.x, c1 = cq.y, c2 = cq.z, c3 = cq.w;
-      const uint32_t sw = sb ^ wslot;
-      if constexpr (VB == 1) {
-        const uint32_t mz = Tb[StageTab::MZ], hb = Tb[StageTab::HB];
-        const uint32_t h0 = hb & 1u, h1 = (hb >> 1) & 1u, h2 = (hb >> 2) & 1u, h3 = (hb >> 3) & 1u;
-        if (mz == 1u) {
-          // bit 0 stays bit 0: each vector keeps its pair, halves swap when
-          // bit 0 of pi is flipped by the other register bits or by w
-          if ((hb | hw) == 0u) {
-            // no deferred flip of qubit 0 in this stage: whole vectors, no selects
+        const uint4 cq = *reinterpret_cast<const uint4*>(Tb + StageTab::CW);
+        const uint32_t c0 = cq.x, c1 = cq.y, c2 = cq.z, c3 = cq.w;
+        const uint32_t sw = sb ^ wslot;
+        if constexpr (VB == 1) {
+          const uint32_t mz = Tb[StageTab::MZ], hb = Tb[StageTab::HB];
+          const uint32_t h0 = hb & 1u, h1 = (hb >> 1) & 1u, h2 = (hb >> 2) & 1u, h3 = (hb >> 3) & 1u;
+          if (mz == 1u) {
+            // bit 0 stays bit 0: each vector keeps its pair, halves swap when
+            // bit 0 of pi is flipped by the other register bits or by w
+            if ((hb | hw) == 0u) {
+              // no deferred flip of qubit 0 in this stage: whole vectors, no selects
 #pragma unroll
-            for (int r = 0; r < kVecPerThread; ++r) {
-              const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
-                                    ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
-              sv[slot] = pack_vec<Real>(a[2 * r], a[2 * r + 1]);
+              for (int r = 0; r < kVecPerThread; ++r) {
+                const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
+                                      ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
+                sv[slot] = pack_vec<Real>(a[2 * r], a[2 * r + 1]);
+              }
+            } else {
+#pragma unroll
+              for (int r = 0; r < kVecPerThread; ++r) {
+                const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
+                                      ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
+                const uint32_t hs = hw ^ ((r & 1) ? h0 : 0u) ^ ((r & 2) ? h1 : 0u) ^
+                                    ((r & 4) ? h2 : 0u) ^ ((r & 8) ? h3 : 0u);
+                const C lo = a[2 * r], hi = a[2 * r + 1];
+                sv[slot] = hs ? pack_vec<Real>(hi, lo) : pack_vec<Real>(lo, hi);
+              }
             }
           } else {
+            // bit 0 moves into other bits: store each amplitude separately
+            const uint32_t cz = Tb[StageTab::CZ], hz = Tb[StageTab::HZ];
+            C* sa = reinterpret_cast<C*>(sv);
 #pragma unroll
             for (int r = 0; r < kVecPerThread; ++r) {
               const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
                                     ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
               const uint32_t hs = hw ^ ((r & 1) ? h0 : 0u) ^ ((r & 2) ? h1 : 0u) ^
                                   ((r & 4) ? h2 : 0u) ^ ((r & 8) ? h3 : 0u);
-              const C lo = a[2 * r], hi = a[2 * r + 1];
-              sv[slot] = hs ? pack_vec<Real>(hi, lo) : pack_vec<Real>(lo, hi);
+              sa[2 * slot + hs] = a[2 * r];
+              sa[2 * (slot ^ cz) + (hs ^ hz)] = a[2 * r + 1];
             }
           }
         } else {
-          // bit 0 moves into other bits: store each amplitude separately
-          const uint32_t cz = Tb[StageTab::CZ], hz = Tb[StageTab::HZ];
-          C* sa = reinterpret_cast<C*>(sv);
 #pragma unroll
           for (int r = 0; r < kVecPerThread; ++r) {
             const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
                                   ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
-            const uint32_t hs = hw ^ ((r & 1) ? h0 : 0u) ^ ((r & 2) ? h1 : 0u) ^
-                                ((r & 4) ? h2 : 0u) ^ ((r & 8) ? h3 : 0u);
-            sa[2 * slot + hs] = a[2 * r];
-            sa[2 * (slot ^ cz) + (hs ^ hz)] = a[2 * r + 1];
+            sv[slot] = pack_vec<Real>(a + r * APV);
           }
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < kVecPerThread; ++r) {
-          const uint32_t slot = sw ^ ((r & 1) ? c0 : 0u) ^ ((r & 2) ? c1 : 0u) ^
-                                ((r & 4) ? c2 : 0u) ^ ((r & 8) ? c3 : 0u);
-          sv[slot] = pack_vec<Real>(a + r * APV);
         }
       }
     }

@@ -49,9 +49,9 @@ uint32_t turns(cplx p) {
 class Writer {
  public:
   explicit Writer(std::vector<ProgWord>* out, bool f32) : out_(out), f32_(f32) {}
-  size_t header(uint32_t code, uint32_t y = 0) {
+  size_t header(uint32_t code, uint32_t arg, uint32_t y = 0) {
     begin_ = out_->size();
-    out_->push_back(ProgWord{{code, y, 0, 0}});
+    out_->push_back(ProgWord{{code | arg << 8, y, 0, 0}});
     return begin_;
   }
   void end() { (*out_)[begin_].w[0] |= uint32_t(out_->size() - begin_) << 16; }
@@ -303,6 +303,8 @@ class StageCompiler {
       }
       if (batch.empty()) break;  // only phases were left
       flush(bits);
+      emit_rotations(Item::ROT);
+      emit_rotations(Item::CROSS);
       for (size_t i : batch) {
         emit(items_[i]);
         items_[i].done = true;
@@ -353,7 +355,7 @@ class StageCompiler {
       d[2 * r] = v[r].real();
       d[2 * r + 1] = v[r].imag();
     }
-    W_.header(TC_T);
+    W_.header(TC_T, 0);
     W_.reals(d, 2 * int(kAll));
     W_.end();
   }
@@ -400,19 +402,19 @@ class StageCompiler {
     const double u[2] = {P.uniform.real(), P.uniform.imag()};
     if (P.signs()) {
       if (P.list.empty()) {
-        W_.header(TC_SG + A);
+        W_.header(TC_SG, A);
       } else {
-        W_.header(TC_SL + A, uint32_t(P.list.size()));
+        W_.header(TC_SL, A, uint32_t(P.list.size()));
         W_.head().w[2] = u[0] < 0 ? 1u : 0u;
         std::vector<uint32_t> v;
         for (const Entry& e : P.list) v.push_back(e.mask);
         W_.bytes(v.data(), v.size() * 4);
       }
     } else if (P.list.empty()) {
-      W_.header(TC_PU + A);
+      W_.header(TC_PU, A);
       pair_of(u);
     } else {
-      W_.header(TC_PH + A, uint32_t(P.list.size()));
+      W_.header(TC_PH, A, uint32_t(P.list.size()));
       if (kF32) W_.head().w[2] = turns(P.uniform);
       else W_.reals(u, 2);
       W_.list(P.list);
@@ -421,7 +423,7 @@ class StageCompiler {
   }
 
   void pair(int b, const Phase& all, const Phase& bit) {
-    W_.header(TC_D + uint32_t(b), uint32_t(all.list.size()) | uint32_t(bit.list.size()) << 16);
+    W_.header(TC_D, uint32_t(b), uint32_t(all.list.size()) | uint32_t(bit.list.size()) << 16);
     if (kF32) {
       W_.head().w[2] = turns(all.uniform);
       W_.head().w[3] = turns(bit.uniform);
@@ -444,28 +446,36 @@ class StageCompiler {
     }
   }
 
-  void emit(const Item& I) {
-    switch (I.kind) {
-      case Item::ROT:
-      case Item::CROSS: {
-        const double v[2] = {I.t, I.s};
-        W_.header((I.kind == Item::ROT ? TC_R : TC_X) + uint32_t(ctz(I.dense)), I.cnr);
-        pair_of(v);
-        break;
-      }
-      case Item::GENERIC: {
-        double v[8];
-        for (int i = 0; i < 4; ++i) { v[2 * i] = I.m[i].real(); v[2 * i + 1] = I.m[i].imag(); }
-        W_.header(TC_G + uint32_t(ctz(I.dense)), I.cnr);
-        W_.reals(v, 8);
-        break;
-      }
-      default:
-        W_.header(TC_LEG);
-        W_.bytes(&enc_[I.op], sizeof(TileOp<Real>));
-        break;
+  // The rotations of a batch (distinct bits) as one instruction.
+  void emit_rotations(Item::Kind kind) {
+    uint32_t bits = 0;
+    double v[5][2] = {};
+    for (size_t i : batch_) {
+      const Item& I = items_[i];
+      if (I.kind != kind) continue;
+      bits |= I.dense;
+      v[ctz(I.dense)][0] = I.t;
+      v[ctz(I.dense)][1] = I.s;
     }
+    if (!bits) return;
+    W_.header(kind == Item::ROT ? TC_R : TC_X, 0, bits);
+    if (kF32) pair_of(v[0]);
+    W_.reals(kF32 ? v[1] : v[0], kF32 ? 2 * (kBits - 1) : 2 * kBits);
     W_.end();
+  }
+
+  void emit(const Item& I) {
+    if (I.kind == Item::GENERIC) {
+      double v[8];
+      for (int i = 0; i < 4; ++i) { v[2 * i] = I.m[i].real(); v[2 * i + 1] = I.m[i].imag(); }
+      W_.header(TC_G, uint32_t(ctz(I.dense)), I.cnr);
+      W_.reals(v, 8);
+      W_.end();
+    } else if (I.kind == Item::RECORD) {
+      W_.header(TC_LEG, 0);
+      W_.bytes(&enc_[I.op], sizeof(TileOp<Real>));
+      W_.end();
+    }
   }
 
   static int ctz(uint32_t v) { return __builtin_ctz(v); }

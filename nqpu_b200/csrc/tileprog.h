@@ -4,26 +4,29 @@
 // 16-byte words (plain C++, no CUDA headers, so the CPU tests can interpret it).
 // One instruction is a header word and its operands:
 //
-//   header.x   code | words << 16 (words of the instruction, header included)
-//   R + b      real rotation on register bit b as three shears (t = tan(phi / 2),
-//              s = sin(phi), |phi| <= pi/2): header.y = virtual-index mask that must
-//              be set; t, s in header.z, .w (complex64) or the next word
-//   X + b      the same with the imaginary off-diagonal of RX
-//   G + b      any complex 2x2: the entries m00, m01, m10, m11 follow
+//   header.x   code | arg << 8 | words << 16 (words of the instruction, header
+//              included); A = a set of register bits, b = one of them
+//   R          real rotations on the register bits of header.y, each as three
+//              shears (t = tan(phi / 2), s = sin(phi), |phi| <= pi/2): t, s per bit
+//              at a fixed place, bit 0 in header.z, .w and two bits per word
+//              after it (complex64) or one bit per word (complex128)
+//   X          the same with the imaginary off-diagonal of RX
+//   G b        any complex 2x2: header.y = virtual-index mask that must be set; the
+//              entries m00, m01, m10, m11 follow
 //   T          one constant phase per register amplitude: 2^(register bits) entries
-//   PU + A     constant phase on the register amplitudes whose bits A are all set
+//   PU A       constant phase on the register amplitudes whose bits A are all set
 //              (re, im in header.z, .w or the next word)
-//   SG + A     sign flip of those amplitudes
-//   PH + A     phase on those amplitudes that is a product over a list of (mask,
+//   SG A       sign flip of those amplitudes
+//   PH A       phase on those amplitudes that is a product over a list of (mask,
 //              phase): an entry counts when the thread's virtual index has all
 //              bits of mask set.  header.y = entries.  complex64: angles in
 //              2^-32 turns, header.z = constant part, two (mask, angle) per word.
 //              complex128: complex factors, one word constant part, two words
 //              (mask) (re, im) each.
-//   D + b      PH on all amplitudes and PH on those with bit b, one multiplication
+//   D b        PH on all amplitudes and PH on those with bit b, one multiplication
 //              per amplitude: header.y = entries of the first | of the second
 //              << 16; constant parts in header.z, .w (complex64) or two words
-//   SL + A     sign flips: header.y = masks, header.z = constant parity; four
+//   SL A       sign flips: header.y = masks, header.z = constant parity; four
 //              masks per word
 //   LEG        any other op: its TileOp record follows
 //
@@ -64,11 +67,7 @@ struct StageTab {
 };
 static_assert(StageTab::SH + 16 <= kStageTabWords && kStageTabWords % 4 == 0, "stage table layout");
 
-enum TileCode : uint32_t {
-  TC_R = 0, TC_X = 8, TC_G = 16, TC_T = 24, TC_PU = 32, TC_SG = 64,
-  TC_LIST = 96,  // from here on the thread evaluates a list first
-  TC_PH = 96, TC_SL = 128, TC_D = 160, TC_LEG = 168,
-};
+enum TileCode : uint32_t { TC_R, TC_X, TC_T, TC_PU, TC_PH, TC_SG, TC_SL, TC_D, TC_G, TC_LEG };
 
 // The op list with every complex 2x2 reduced to rotation x phase where a later 2x2
 // on its qubit can take the rest: a phase passes through controls and diagonal

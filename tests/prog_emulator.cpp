@@ -68,46 +68,51 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
     return v;
   };
   while (p < end) {
-    const uint32_t code = p->w[0] & 0xFFFFu, len = p->w[0] >> 16;
+    const uint32_t code = p->w[0] & 0xFFu, arg = (p->w[0] >> 8) & 0xFFu, len = p->w[0] >> 16;
     const ProgWord* q = p + 1;
     const ProgWord& h = *p;
     if (len == 0 || p + len > end) return -2;
     const cd two = F32 ? cget<float>(p, 1) : cget<double>(q, 0);  // the instruction's two reals
-    if (code < TC_T) {
-      const uint32_t b = 1u << (code & 7u);
-      if (b >= a.size()) return -3;
-      cd m[4];
-      if (code >= TC_G) {
-        for (int i = 0; i < 4; ++i) m[i] = cget<Real>(q, i);
-      } else {
-        // the three shears as one matrix
-        const double t = two.real(), s = two.imag(), c = 1 - t * s, o = t * (2 - t * s);
-        const cd f = code >= TC_X ? cd(0, 1) : cd(1, 0);
-        m[0] = c; m[1] = -f * o; m[2] = (code >= TC_X ? -f : f) * s; m[3] = c;
-      }
-      for (uint32_t i = 0; hit(h.w[1]) && i < a.size(); ++i) {
+    auto two_by_two = [&](uint32_t b, const cd* m) {
+      for (uint32_t i = 0; i < a.size(); ++i) {
         if (i & b) continue;
         const cd x = a[i], y = a[i | b];
         a[i] = m[0] * x + m[1] * y;
         a[i | b] = m[2] * x + m[3] * y;
       }
+    };
+    if (code == TC_R || code == TC_X) {
+      if (h.w[1] >= a.size()) return -3;
+      for (int b = 0; (1u << b) < a.size(); ++b) {
+        if (!((h.w[1] >> b) & 1)) continue;
+        // the three shears as one matrix
+        const cd ts = F32 ? (b ? cget<float>(q, b - 1) : two) : cget<double>(q, b);
+        const double t = ts.real(), s = ts.imag(), c = 1 - t * s, o = t * (2 - t * s);
+        const cd f = code == TC_X ? cd(0, 1) : cd(1, 0);
+        const cd m[4] = {c, -f * o, (code == TC_X ? -f : f) * s, c};
+        two_by_two(1u << b, m);
+      }
+    } else if (code == TC_G) {
+      cd m[4];
+      for (int i = 0; i < 4; ++i) m[i] = cget<Real>(q, i);
+      if (hit(h.w[1])) two_by_two(1u << arg, m);
     } else if (code == TC_T) {
       for (uint32_t i = 0; i < a.size(); ++i) a[i] *= cget<Real>(q, int(i));
-    } else if (code < TC_SG) {
+    } else if (code == TC_PU) {
       for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & (code & 31u)) == (code & 31u)) a[i] *= two;
-    } else if (code < TC_LIST || (code >= TC_SL && code < TC_D)) {
-      uint32_t s = code < TC_LIST ? 1u : h.w[2];
-      for (uint32_t i = 0; code >= TC_SL && i < h.w[1]; ++i) s += hit(q[i / 4].w[i & 3]);
+        if ((i & arg) == arg) a[i] *= two;
+    } else if (code == TC_SG || code == TC_SL) {
+      uint32_t s = code == TC_SG ? 1u : h.w[2];
+      for (uint32_t i = 0; code == TC_SL && i < h.w[1]; ++i) s += hit(q[i / 4].w[i & 3]);
       for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & (code & 31u)) == (code & 31u) && (s & 1)) a[i] = -a[i];
-    } else if (code < TC_SL) {
+        if ((i & arg) == arg && (s & 1)) a[i] = -a[i];
+    } else if (code == TC_PH) {
       if (!F32) ++q;
       const cd v = list(q, h.w[1], F32 ? turn(h.w[2]) : two);
       for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & (code & 31u)) == (code & 31u)) a[i] *= v;
-    } else if (code < TC_LEG) {
-      const uint32_t b = 1u << (code - TC_D);
+        if ((i & arg) == arg) a[i] *= v;
+    } else if (code == TC_D) {
+      const uint32_t b = 1u << arg;
       cd d0 = F32 ? turn(h.w[2]) : two, d1 = F32 ? turn(h.w[3]) : cget<double>(q, 1);
       if (!F32) q += 2;
       d0 = list(q, h.w[1] & 0xFFFFu, d0);
