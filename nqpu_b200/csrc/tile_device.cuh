@@ -79,6 +79,26 @@ __device__ __forceinline__ void rb_u1(C (&a)[NA], C m0, C m1, C m2, C m3) {
   }
 }
 
+// The same with the entries read again for every pair (volatile: the compiler
+// would keep all of them): complex128 at 128 registers has no room for them, and
+// the spills land on every instruction of the stage loop.
+template <typename Real, typename C, int NA, int B>
+__device__ __forceinline__ void rb_u1_reload(C (&a)[NA], const Real* p) {
+  const volatile Real* m = p;
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    if (i & (1 << B)) continue;
+    C &x = a[i], &y = a[i | (1 << B)];
+    C u, v;
+    { const Real r = m[0], s = m[1]; u.x = r * x.x - s * x.y; u.y = r * x.y + s * x.x; }
+    { const Real r = m[2], s = m[3]; u.x += r * y.x - s * y.y; u.y += r * y.y + s * y.x; }
+    { const Real r = m[4], s = m[5]; v.x = r * x.x - s * x.y; v.y = r * x.y + s * x.x; }
+    { const Real r = m[6], s = m[7]; v.x += r * y.x - s * y.y; v.y += r * y.y + s * y.x; }
+    x = u;
+    y = v;
+  }
+}
+
 // dense 2x2 with controls (generic: per-amplitude select)
 template <typename C, int NA, int B>
 __device__ __forceinline__ void rb_u1_ctrl(C (&a)[NA], C m0, C m1, C m2, C m3, bool tc, uint32_t creg) {
@@ -255,9 +275,10 @@ __device__ __forceinline__ void rb_u2(C (&a)[NA], const Real* __restrict__ mp, b
     } else {
       // one entry at a time: the 128-register build has no room for a row
       auto mac = [&](int k, const C& x, C& acc) {
-        const C m = reinterpret_cast<const C*>(mp)[k];
-        acc.x = fma(m.x, x.x, fma(-m.y, x.y, acc.x));
-        acc.y = fma(m.x, x.y, fma(m.y, x.x, acc.y));
+        const volatile Real* m = mp + 2 * k;  // read again per quad, not kept
+        const Real r = m[0], s = m[1];
+        acc.x = fma(r, x.x, fma(-s, x.y, acc.x));
+        acc.y = fma(r, x.y, fma(s, x.x, acc.y));
       };
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
@@ -507,12 +528,24 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
         default: break;
       }
     } else if (code == TC_G) {
-      C m0, m1, m2, m3;
-      ldc2<Real>(reinterpret_cast<const Real*>(q), m0, m1);
-      ldc2<Real>(reinterpret_cast<const Real*>(q) + 4, m2, m3);
+      const Real* m = reinterpret_cast<const Real*>(q);
       const bool tc = (vbase & h.y) == h.y;  // controls outside the registers
       switch (arg) {
-#define NQ_B(B, _) case B: if constexpr (B < NRB) { if (tc) rb_u1<C, NA, B>(a, m0, m1, m2, m3); } break;
+#define NQ_B(B, _) \
+        case B: \
+          if constexpr (B < NRB) { \
+            if (tc) { \
+              if constexpr (F32) { \
+                C m0, m1, m2, m3; \
+                ldc2<Real>(m, m0, m1); \
+                ldc2<Real>(m + 4, m2, m3); \
+                rb_u1<C, NA, B>(a, m0, m1, m2, m3); \
+              } else { \
+                rb_u1_reload<Real, C, NA, B>(a, m); \
+              } \
+            } \
+          } \
+          break;
         NQ_REG_CASES(NQ_B, 0)
 #undef NQ_B
         default: break;
