@@ -339,21 +339,13 @@ extern "C" NqpuError nqpu_gate_reset_qubit(NqpuState* state, uint32_t qubit) {
 // ---------------------------------------------------------------------------
 // Measurement and reductions
 // ---------------------------------------------------------------------------
-static NqpuError measure_one(StateImpl* s, uint32_t qubit, NqpuMeasurement* out) {
-  uint32_t outcome = 0;
-  double po = 0.0;
-  NQ_TRY(state_measure(s, qubit, &outcome, &po));
-  out->outcome = outcome;
-  out->probability = po;
-  return NQPU_OK;
-}
-
 extern "C" NqpuError nqpu_measure(NqpuState* state, uint32_t qubit, NqpuMeasurement* out) {
   if (!state) return NQPU_NULL_POINTER;
   if (!out) return NQPU_NULL_POINTER;
   StateImpl* s = S(state);
   if (qubit >= s->n) return NQPU_INVALID_QUBIT;
-  return measure_one(s, qubit, out);
+  NQ_TRY(state_measure(s, qubit, &out->outcome, &out->probability));
+  return NQPU_OK;
 }
 
 extern "C" NqpuError nqpu_measure_all(NqpuState* state, uint32_t* out, uint32_t num_qubits) {
@@ -361,12 +353,7 @@ extern "C" NqpuError nqpu_measure_all(NqpuState* state, uint32_t* out, uint32_t 
   if (!out) return NQPU_NULL_POINTER;
   StateImpl* s = S(state);
   if (num_qubits != s->n) return NQPU_INVALID_PARAMETER;
-  for (uint32_t q = 0; q < s->n; ++q) {
-    NqpuMeasurement m;
-    NqpuError e = measure_one(s, q, &m);
-    if (e != NQPU_OK) return e;
-    out[q] = m.outcome;
-  }
+  NQ_TRY(state_measure_all(s, out));
   return NQPU_OK;
 }
 

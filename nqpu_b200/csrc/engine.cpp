@@ -123,20 +123,34 @@ cudaError_t state_zsums(const StateImpl* s, double* zs, double* total) {
   return cudaSuccess;
 }
 
-cudaError_t state_measure(StateImpl* s, uint32_t qubit, uint32_t* outcome, double* probability) {
-  std::vector<double> z(s->n + 1);
-  cudaError_t e = state_zsums(s, z.data(), nullptr);
-  if (e != cudaSuccess) return e;
-  const double prob0 = z[0] - z[1 + qubit];  // sum over bit q == 0
-  const double prob1 = 1.0 - prob0;          // c_ffi.rs:546
+cudaError_t state_queue_measure(StateImpl* s, uint32_t qubit, bool flip, double* result) {
   const double r = next_random_f64();
-  const uint32_t out = r < prob0 ? 0u : 1u;
-  const double po = out == 0 ? prob0 : prob1;
-  const double renorm = 1.0 / std::sqrt(po);
-  e = launch_collapse(s->dt, s->amp, int(s->n), int(qubit), int(out), renorm, s->stream, device_sms());
+  cudaError_t e = launch_zsums(s->dt, s->amp, int(s->n), s->scratch, s->d_small, s->stream, device_sms());
   if (e != cudaSuccess) return e;
-  *outcome = out;
-  if (probability) *probability = po;
+  return launch_measure_collapse(s->dt, s->amp, int(s->n), int(qubit), s->d_small, r, flip, result, s->stream,
+                                 device_sms());
+}
+
+cudaError_t state_measure(StateImpl* s, uint32_t qubit, uint32_t* outcome, double* probability) {
+  double* res = s->h_small + kSmallTable;
+  cudaError_t e = state_queue_measure(s, qubit, false, res);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  if (e != cudaSuccess) return e;
+  *outcome = uint32_t(res[0]);
+  if (probability) *probability = res[1];
+  return cudaSuccess;
+}
+
+cudaError_t state_measure_all(StateImpl* s, uint32_t* outcomes) {
+  double* res = s->h_small + kSmallTable;
+  static_assert(kSmallTable + 2 * size_t(kMaxQubits) <= kSmallDoubles, "room for every qubit's result");
+  for (uint32_t q = 0; q < s->n; ++q) {
+    const cudaError_t e = state_queue_measure(s, q, false, res + 2 * q);
+    if (e != cudaSuccess) return e;
+  }
+  const cudaError_t e = cudaStreamSynchronize(s->stream);
+  if (e != cudaSuccess) return e;
+  for (uint32_t q = 0; q < s->n; ++q) outcomes[q] = uint32_t(res[2 * q]);
   return cudaSuccess;
 }
 
@@ -216,6 +230,19 @@ cudaError_t state_inner(const StateImpl* a, const StateImpl* b, double* out2) {
 cudaError_t state_sample(const StateImpl* sc, const double* uniforms, uint32_t shots, uint64_t* out) {
   StateImpl* s = const_cast<StateImpl*>(sc);
   cudaError_t e;
+  if (2 * size_t(shots) <= kSmallDoubles - kSmallTable) {
+    // uniforms staged in pinned memory, outcomes written there by the kernel: a
+    // copy from or to pageable memory costs about 10 us each way
+    double* hu = s->h_small + kSmallTable;
+    double* du = s->d_small + kSmallTable;
+    uint64_t* ho = reinterpret_cast<uint64_t*>(hu + shots);
+    std::memcpy(hu, uniforms, sizeof(double) * shots);
+    if ((e = cudaMemcpyAsync(du, hu, sizeof(double) * shots, cudaMemcpyHostToDevice, s->stream)) != cudaSuccess) return e;
+    if ((e = launch_sample(s->dt, s->amp, int(s->n), du, shots, s->scratch, ho, s->stream, device_sms())) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return e;
+    std::memcpy(out, ho, sizeof(uint64_t) * shots);
+    return cudaSuccess;
+  }
   if (s->shot_cap < shots) {
     e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return e;
@@ -470,30 +497,34 @@ cudaError_t circuit_run(CircuitImpl* c, StateImpl* s, int mode, std::vector<cuda
                         std::vector<uint32_t>* outcomes) {
   std::lock_guard<std::mutex> lk(c->mu);
   const std::vector<Segment> segs = circuit_segments(c->gates);
+  // measurements are queued like every other launch; their results gather in
+  // pinned memory and are read when it is full and at the end
+  constexpr size_t kSlots = (kSmallDoubles - kSmallTable) / 2;
+  size_t queued = 0;
+  auto drain = [&]() {
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return e;
+    for (size_t i = 0; i < queued; ++i) outcomes->push_back(uint32_t(s->h_small[kSmallTable + 2 * i]));
+    queued = 0;
+    return cudaSuccess;
+  };
   for (size_t si = 0; si < segs.size(); ++si) {
     const Segment& seg = segs[si];
     cudaError_t e = segment_run(c, seg, int(si), s, mode, events);
     if (e != cudaSuccess) return e;
     if (seg.mid < 0) break;
     const GateRec& g = c->gates[size_t(seg.mid)];
-    if (g.code == G_MEASURE) {
-      uint32_t out = 0;
-      if ((e = state_measure(s, uint32_t(g.q[0]), &out, nullptr)) != cudaSuccess) return e;
-      if (outcomes) outcomes->push_back(out);
-    } else {
-      // OpenQASM reset: measure (one RNG draw) and flip the qubit back to |0>
-      // when it came out 1 (the state API's nqpu_gate_reset_qubit keeps the
-      // reference's projection, GateOperations::reset_qubit)
-      uint32_t out = 0;
-      if ((e = state_measure(s, uint32_t(g.q[0]), &out, nullptr)) != cudaSuccess) return e;
-      if (out == 1) {
-        Op x;
-        x.kind = OP_X1;
-        x.t0 = int8_t(g.q[0]);
-        if ((e = launch_pergate(s->dt, s->amp, int(s->n), x, s->stream, device_sms())) != cudaSuccess) return e;
-      }
+    // OpenQASM reset: measure (one RNG draw) and flip the qubit back to |0>
+    // when it came out 1 (the state API's nqpu_gate_reset_qubit keeps the
+    // reference's projection, GateOperations::reset_qubit)
+    double* res = nullptr;
+    if (g.code == G_MEASURE && outcomes) {
+      if (queued == kSlots && (e = drain()) != cudaSuccess) return e;
+      res = s->h_small + kSmallTable + 2 * queued++;
     }
+    if ((e = state_queue_measure(s, uint32_t(g.q[0]), g.code == G_RESET, res)) != cudaSuccess) return e;
   }
+  if (queued) return drain();
   return cudaSuccess;
 }
 

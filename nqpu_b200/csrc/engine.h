@@ -21,7 +21,7 @@ double next_random_f64();
 bool device_ready();
 int device_sms();
 
-constexpr size_t kSmallDoubles = 2048, kSmallTable = 64;
+constexpr size_t kSmallDoubles = 4096, kSmallTable = 64;
 
 struct StateImpl {
   uint32_t n = 0;
@@ -110,6 +110,10 @@ NqpuError circuit_append_gates(CircuitImpl* c, const uint32_t* codes, const int3
 // Measure one qubit (collapse with the thread-local RNG draw, c_ffi.rs:537-560
 // rule) / project it onto |0> and renormalise (lib.rs:1705).
 cudaError_t state_measure(StateImpl* s, uint32_t qubit, uint32_t* outcome, double* probability);
+cudaError_t state_measure_all(StateImpl* s, uint32_t* outcomes);  // qubits 0..n-1 in order
+// Queue a measurement with the next draw of the thread-local RNG; `flip` moves
+// outcome 1 to |0>.  result (pinned, may be null): outcome, probability.
+cudaError_t state_queue_measure(StateImpl* s, uint32_t qubit, bool flip, double* result);
 cudaError_t state_reset_qubit(StateImpl* s, uint32_t qubit);
 
 void circuit_free(CircuitImpl* c);

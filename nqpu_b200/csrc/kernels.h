@@ -42,6 +42,11 @@ cudaError_t launch_scale(DType dt, void* amp, int n, double factor, cudaStream_t
 // zero amplitudes whose bit q differs from `keep`, scale the rest by `factor`
 cudaError_t launch_collapse(DType dt, void* amp, int n, int q, int keep, double factor,
                             cudaStream_t s, int num_sms);
+// Measure qubit q with the uniform draw r from launch_zsums' sums (device memory):
+// collapse, and with `flip` move outcome 1 to |0>.  result[0..1] (device or pinned
+// host memory, may be null) = outcome, its probability.
+cudaError_t launch_measure_collapse(DType dt, void* amp, int n, int q, const double* sums, double r, bool flip,
+                                    double* result, cudaStream_t s, int num_sms);
 // |a_i|^2 for `count` amplitudes starting at `amp` (already offset by the caller).
 cudaError_t launch_probabilities(DType dt, const void* amp, uint64_t count, double* out,
                                  cudaStream_t s, int num_sms);
@@ -87,7 +92,7 @@ struct PauliSet {
   uint16_t beg[17];
   uint16_t dbeg[17];
   uint16_t xused, dused;  // bit m: the list of X|Y (diagonal: Z) positions m is not empty
-  uint8_t rbit[4];
+  alignas(4) uint8_t rbit[4];
 };
 // One term: z = Z|Y positions outside the set's bits | those inside << 60 |
 // (odd number of Y's) << 59; c = coefficient with the pair factor and the sign

@@ -111,49 +111,55 @@ __global__ void __launch_bounds__(kRedThreads, 2)
   using C = typename Tr<Real>::C;
   const C* a = reinterpret_cast<const C*>(amp);
   const int hbits = n < kPauliChunkBits ? n : kPauliChunkBits;
-  // work units of kRedThreads threads: first (chunk, low set, tile), then (high set, tile)
-  const int lt_low = max(0, hbits - 4 - 8), lt_high = max(0, n - 4 - 8);
-  const uint64_t low_units = (uint64_t(nlow) << lt_low) << (n - hbits);
-  const uint64_t units = low_units + (uint64_t(nsets - nlow) << lt_high);
+  // work units of kRedThreads threads, one block after the other: first (chunk,
+  // low set, tile) with the tile running fastest, then (high set, tile).  The
+  // counters step instead of dividing the unit number (a 64-bit division costs
+  // as much as a whole unit's arithmetic).
+  const uint32_t low_tiles = 1u << max(0, hbits - 12), high_tiles = 1u << max(0, n - 12);
+  uint32_t tile = blockIdx.x, chunk = 0;
+  int si = 0;
   KSum acc;
-  for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
-    int si;
-    uint64_t w, chunk = 0;
-    int span;  // index bits the unit's threads run over
-    if (u < low_units) {
-      const uint64_t t = u >> lt_low;
-      chunk = t / unsigned(nlow);
-      si = int(t - chunk * unsigned(nlow));
-      w = ((u & ((1ull << lt_low) - 1)) << 8) + threadIdx.x;
-      span = hbits;
-    } else {
-      const uint64_t v = u - low_units;
-      si = nlow + int(v >> lt_high);
-      w = ((v & ((1ull << lt_high) - 1)) << 8) + threadIdx.x;
-      span = n;
+  for (;; tile += gridDim.x) {
+    while (si < nlow && tile >= low_tiles) {
+      tile -= low_tiles;
+      if (++si == nlow && ++chunk < (1u << (n - hbits))) si = 0;
     }
-    if (w >> (span - 4)) continue;  // fewer work items than threads
+    while (si >= nlow && si < nsets && tile >= high_tiles) {
+      tile -= high_tiles;
+      ++si;
+    }
+    if (si >= nsets) break;
+    const bool low = si < nlow;
+    const uint32_t w = tile * kRedThreads + threadIdx.x;
+    if (w >> ((low ? hbits : n) - 4)) continue;  // fewer work items than threads
     const PauliSet* S = sets + si;
     uint64_t base = w, off[4];
+    const uint32_t rb = *reinterpret_cast<const uint32_t*>(S->rbit);
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      base = insert_zero_bit(base, S->rbit[b]);
-      off[b] = 1ull << S->rbit[b];
+      const int q = int((rb >> (8 * b)) & 0xFF);
+      off[b] = 1ull << q;
+      const uint64_t lo = base & (off[b] - 1);
+      base += base - lo;  // insert a zero bit at q
     }
-    base += chunk << hbits;
+    if (low) base += uint64_t(chunk) << hbits;
     C v[16];
-    auto idx = [&](int r) {
-      return base + ((r & 1) ? off[0] : 0) + ((r & 2) ? off[1] : 0) + ((r & 4) ? off[2] : 0) + ((r & 8) ? off[3] : 0);
-    };
+    const C* p4[4];  // the four combinations of the upper two bits
+    p4[0] = a + base;
+    p4[1] = p4[0] + off[2];
+    p4[2] = p4[0] + off[3];
+    p4[3] = p4[1] + off[3];
+    const uint64_t off01 = off[0] + off[1];
+    auto at = [&](int r) { return p4[r >> 2] + ((r & 3) == 0 ? 0 : (r & 3) == 1 ? off[0] : (r & 3) == 2 ? off[1] : off01); };
     if (sizeof(Real) == 4 && off[0] == 1) {  // qubit 0 in the set: pairs as 128-bit loads
 #pragma unroll
       for (int r = 0; r < 16; r += 2) {
-        const float4 x = __ldg(reinterpret_cast<const float4*>(a + idx(r)));
+        const float4 x = __ldg(reinterpret_cast<const float4*>(at(r)));
         v[r].x = x.x; v[r].y = x.y; v[r + 1].x = x.z; v[r + 1].y = x.w;
       }
     } else {
 #pragma unroll
-      for (int r = 0; r < 16; ++r) v[r] = __ldg(a + idx(r));
+      for (int r = 0; r < 16; ++r) v[r] = __ldg(at(r));
     }
     double re[16], im[16];
 #pragma unroll
