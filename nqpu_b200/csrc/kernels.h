@@ -92,7 +92,9 @@ struct PauliSet {
   uint16_t beg[17];
   uint16_t dbeg[17];
   uint16_t xused, dused;  // bit m: the list of X|Y (diagonal: Z) positions m is not empty
+  uint16_t plain;         // bit b: a single X on bit b alone, its coefficient in cx[b] (not in the lists)
   alignas(4) uint8_t rbit[4];
+  double cx[4];
 };
 // One term: z = Z|Y positions outside the set's bits | those inside << 60 |
 // (odd number of Y's) << 59; c = coefficient with the pair factor and the sign

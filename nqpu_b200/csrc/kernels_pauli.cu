@@ -73,7 +73,16 @@ void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan
     };
     // (X positions, Z positions) within the set order the terms
     std::vector<std::pair<int, size_t>> order;
-    for (size_t t : g.idx) order.push_back({inside(strings[t].x) * 16 + inside(strings[t].z), t});
+    for (size_t t : g.idx) {
+      const PauliString& P = strings[t];
+      if (P.z == 0 && P.x != 0 && (P.x & (P.x - 1)) == 0) {
+        const int b = __builtin_ctz(unsigned(inside(P.x)));
+        S.plain |= uint16_t(1u << b);
+        S.cx[b] += 2.0 * P.c;
+        continue;
+      }
+      order.push_back({inside(P.x) * 16 + inside(P.z), t});
+    }
     std::stable_sort(order.begin(), order.end(),
                      [](const std::pair<int, size_t>& a, const std::pair<int, size_t>& b) { return a.first < b.first; });
     size_t k = 0;
@@ -201,6 +210,21 @@ __global__ void __launch_bounds__(kRedThreads, 2)
         item += W[m] * cs;
       }
     }
+    // a single X: no sign anywhere
+    const uint32_t plain = S->plain;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      if (!((plain >> b) & 1)) continue;
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (!(r & (1 << b))) {
+          s0 = fma(re[r], re[r | (1 << b)], s0);
+          s1 = fma(im[r], im[r | (1 << b)], s1);
+        }
+      item = fma(S->cx[b], s0 + s1, item);
+    }
+    if (xused)
 #pragma unroll
     for (int m = 1; m < 16; ++m) {
       if (!((xused >> m) & 1)) continue;
