@@ -191,6 +191,8 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   };
   if (tid == 0) s_pass = -1;
   __syncthreads();
+  using Copy = TileCopy<float, kBatchK>;
+  static_assert(Copy::kThreads == kTileThreads, "one vector per thread and step");
 
   for (;;) {
     if (tid == 0) {
@@ -239,20 +241,26 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       if (T.phase == 0) {
         init_tile(nvec, base == 0);
       } else {
-        for (uint32_t u = tid; u < nvec; u += blockDim.x) {
-          const uint32_t t = u << 1;
-          const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
-          cp_async16(sv + swz(u), state + g);
+        if (Copy::fits(P)) {
+          Copy::each(arena + 2 * C.amp_off, P, hi_off, base, [&](uint32_t slot, float4* g) { cp_async16(sv + slot, g); });
+        } else {
+          for (uint32_t u = tid; u < nvec; u += blockDim.x) {
+            const uint32_t t = u << 1;
+            cp_async16(sv + swz(u), state + base + (t & lowmask) + hi_off[t >> c]);
+          }
         }
         cp_async_commit();
         cp_async_wait0();
       }
       __syncthreads();
       run_stages(ext);
-      for (uint32_t u = tid; u < nvec; u += blockDim.x) {
-        const uint32_t t = u << 1;
-        const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
-        __stcg(reinterpret_cast<float4*>(state + g), sv[swz(u)]);
+      if (Copy::fits(P)) {
+        Copy::each(arena + 2 * C.amp_off, P, hi_off, base, [&](uint32_t slot, float4* g) { __stcg(g, sv[slot]); });
+      } else {
+        for (uint32_t u = tid; u < nvec; u += blockDim.x) {
+          const uint32_t t = u << 1;
+          __stcg(reinterpret_cast<float4*>(state + base + (t & lowmask) + hi_off[t >> c]), sv[swz(u)]);
+        }
       }
       __syncthreads();
       if (tid == 0) {

@@ -25,15 +25,19 @@ namespace nqpu {
 
 // Dynamic shared memory: [tile buffer 0 | tile buffer 1 | hi_off table
 // (2^(k-c) <= kHiOffEntries u64) | stage tables of the pass (kStageTabWords u32
-// each) | the pass's program, prog_smem words (0: read from global memory)].
+// each) | the pass's program].
+// WAY 0: the program stays in global memory (it does not fit); 1: it is in shared
+// memory; 2: that, and the tile has all of KMAX bits.  Kernels of their own,
+// because deciding it inside costs the stage loop spills (complex128 at 128
+// registers: 20-qubit brickwork 398 us against 385 without them).
 // MINB = 1: one persistent CTA per SM; while the stages of tile i run on one
 // buffer, the cp.async copies of tile i+1 stream into the other.  MINB > 1:
 // MINB CTAs per SM with one buffer each hide each other's copies.  Each thread
 // holds 16 vectors, so a CTA has 2^KMAX / (16 x amplitudes per vector) threads.
-template <typename Real, int KMAX, int MINB>
+template <typename Real, int KMAX, int MINB, int WAY>
 __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
     k_tile_pass(Real* __restrict__ amp, const __grid_constant__ PassRec P, const uint4* __restrict__ progs,
-                int prog_smem, uint64_t n_tiles) {
+                uint32_t n_tiles, uint64_t out_mask, uint64_t step) {
   using T = Tr<Real>;
   using V = typename T::V;
   constexpr int VB = T::kVecBit;
@@ -50,14 +54,14 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
   const int k = P.k, c = P.c;
   const uint32_t nvec = 1u << (k - VB);
   const int nhi = k - c;
-  load_pass_prog(P, progs, prog_smem, reinterpret_cast<uint4*>(tabs));
+  const int tab_words = (P.stage_end - P.stage_begin) * (kStageTabWords / 4);
+  load_pass_prog(P, progs, WAY ? P.prog_words - tab_words : 0, reinterpret_cast<uint4*>(tabs));
   for (int h = tid; h < (1 << nhi); h += blockDim.x) {
     uint64_t off = 0;
     for (int j = 0; j < nhi; ++j)
       if ((h >> j) & 1) off |= 1ull << P.qhi[j];
     hi_off[h] = off;
   }
-  const int tab_words = (P.stage_end - P.stage_begin) * (kStageTabWords / 4);
   const uint4* prog_s = reinterpret_cast<const uint4*>(tabs) + tab_words;
   const uint4* prog_g = progs + P.prog_begin + tab_words;
   cp_async_wait0();
@@ -67,59 +71,63 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t lowmask = (1u << c) - 1u;
+  using Copy = TileCopy<Real, KMAX>;
+  const bool full = WAY == 2 || Copy::fits(P);
 
   // HBM -> shared, asynchronous (consecutive threads take consecutive vectors).
-  auto issue_load = [&](uint64_t tile, V* dst) {
-    const uint64_t base = tile_base(P, tile);
-#pragma unroll
-    for (int i = 0; i < kVecPerThread; ++i) {
-      const uint32_t u = tid + i * kThreads;
-      if (u < nvec) {
-        const uint32_t t = u << VB;
-        const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
-        cp_async16(dst + swz(u), amp + 2 * g);
-      }
+  auto issue_load = [&](uint64_t base, V* dst) {
+    if (full) {
+      Copy::each(amp, P, hi_off, base, [&](uint32_t slot, V* g) { cp_async16(dst + slot, g); });
+      return;
+    }
+#pragma unroll 1
+    for (uint32_t u = tid; u < nvec; u += kThreads) {
+      const uint32_t t = u << VB;
+      cp_async16(dst + swz(u), amp + 2 * (base + (t & lowmask) + hi_off[t >> c]));
     }
   };
+  // the tile gridDim.x further on: an addition of `step`, the grid size laid out
+  // over the qubits outside the tile, with the carries running over the gaps
+  auto advance = [&](uint64_t base) { return ((base | ~out_mask) + step) & out_mask; };
 
-  uint64_t tile = blockIdx.x;
+  uint64_t base = tile_base(P, blockIdx.x);
   if (kDoubleBuffer) {
-    if (tile < n_tiles) issue_load(tile, buf0);
+    if (blockIdx.x < n_tiles) issue_load(base, buf0);
     cp_async_commit();
   }
-  for (int it = 0; tile < n_tiles; ++it, tile += gridDim.x) {
+  for (uint32_t it = 0, tile = blockIdx.x; tile < n_tiles; ++it, tile += gridDim.x) {
     V* sv = (it & 1) ? buf1 : buf0;
-    const uint64_t next = tile + gridDim.x;
     if (kDoubleBuffer) {
-      if (next < n_tiles) issue_load(next, (it & 1) ? buf0 : buf1);
+      if (tile + gridDim.x < n_tiles) issue_load(advance(base), (it & 1) ? buf0 : buf1);
     } else {
-      issue_load(tile, sv);  // single buffer: the other CTA on the SM hides the latency
+      issue_load(base, sv);  // single buffer: the other CTA on the SM hides the latency
     }
     cp_async_commit();
     if (kDoubleBuffer) cp_async_wait1();  // everything but the newest group (the prefetch) has landed
     else cp_async_wait0();
     __syncthreads();
 
-    const uint64_t base = tile_base(P, tile);
-    uint32_t ext = 0;
-    for (int j = 0; j < P.n_ext; ++j)
-      if ((base >> P.ext[j]) & 1ull) ext |= 1u << (k + j);
+    // lane j holds the bit of ext qubit j
+    int lane = threadIdx.x & 31;
+    asm volatile("" : "+r"(lane));  // worked out per tile: no registers held across the stages
+    const uint32_t ext =
+        __ballot_sync(0xffffffffu, lane < P.n_ext && ((base >> P.ext[lane]) & 1ull)) << k;
 
-    // two copies, so that the usual one reads the program by shared-memory loads
-    if (prog_smem) run_tile_stages<Real>(sv, P, tabs, prog_s, ext);
+    if constexpr (WAY > 0) run_tile_stages<Real>(sv, P, tabs, prog_s, ext);
     else run_tile_stages<Real>(sv, P, tabs, prog_g, ext);
 
     // shared -> HBM
-#pragma unroll
-    for (int i = 0; i < kVecPerThread; ++i) {
-      const uint32_t u = tid + i * kThreads;
-      if (u < nvec) {
+    if (full) {
+      Copy::each(amp, P, hi_off, base, [&](uint32_t slot, V* g) { __stcs(g, sv[slot]); });
+    } else {
+#pragma unroll 1
+      for (uint32_t u = tid; u < nvec; u += kThreads) {
         const uint32_t t = u << VB;
-        const uint64_t g = base + (t & lowmask) + hi_off[t >> c];
-        __stcs(reinterpret_cast<V*>(amp + 2 * g), sv[swz(u)]);
+        __stcs(reinterpret_cast<V*>(amp + 2 * (base + (t & lowmask) + hi_off[t >> c])), sv[swz(u)]);
       }
     }
     __syncthreads();  // this buffer is refilled by the prefetch issued next iteration
+    base = advance(base);
   }
 }
 
@@ -166,7 +174,7 @@ int tile_config_get(DType dt) {
   return c ? c : dt == DType::C64 ? 4 : 1;
 }
 
-template <typename Real, int KMAX, int MINB>
+template <typename Real, int KMAX, int MINB, int WAY>
 cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const ProgWord* d_prog,
                                  cudaStream_t stream, int num_sms) {
   // a plan built for larger tiles than this kernel holds must not run on it,
@@ -174,7 +182,7 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   if (host_pass.k > KMAX || host_pass.k < 1 || host_pass.k - host_pass.c > kHiOffBits ||
       host_pass.stage_end - host_pass.stage_begin > kMaxPassStages)
     return cudaErrorInvalidValue;
-  auto kern = k_tile_pass<Real, KMAX, MINB>;
+  auto kern = k_tile_pass<Real, KMAX, MINB, WAY>;
   constexpr int kThreads = (1 << (KMAX - Tr<Real>::kVecBit)) / kVecPerThread;
   // shared memory of this launch: the tile buffer(s), the high-offset table, the
   // stage tables of this pass and, where it fits beside them in MINB CTAs per
@@ -183,11 +191,13 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   const size_t smem_max = tile_smem_max<Real, KMAX>(MINB);
   size_t smem = tile_smem_base<Real, KMAX>(MINB) +
                 sizeof(uint32_t) * kStageTabWords * size_t(host_pass.stage_end - host_pass.stage_begin);
-  const int words = host_pass.prog_words - (host_pass.stage_end - host_pass.stage_begin) * (kStageTabWords / 4);
-  int prog_smem = 0;
-  if (smem + sizeof(ProgWord) * size_t(words) <= smem_max) {
-    prog_smem = words;
-    smem += sizeof(ProgWord) * size_t(prog_smem);
+  if constexpr (WAY == 2) {
+    if (!TileCopy<Real, KMAX>::fits(host_pass))
+      return launch_tile_pass_cfg<Real, KMAX, MINB, 1>(amp, host_pass, d_prog, stream, num_sms);
+  }
+  if constexpr (WAY > 0) {
+    smem = tile_smem_base<Real, KMAX>(MINB) + sizeof(ProgWord) * size_t(host_pass.prog_words);
+    if (smem > smem_max) return launch_tile_pass_cfg<Real, KMAX, MINB, 0>(amp, host_pass, d_prog, stream, num_sms);
   }
   // the shared-memory limit is a per-device attribute: set once per device
   static PerDeviceOnce<cudaError_t> attr;
@@ -197,9 +207,13 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   e = attr.get(dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max)); },
                cudaErrorInvalidDevice);
   if (e != cudaSuccess) return e;
-  const uint64_t n_tiles = 1ull << host_pass.n_out;
-  const uint64_t max_ctas = uint64_t(num_sms) * MINB;
-  const unsigned grid = unsigned(n_tiles < max_ctas ? n_tiles : max_ctas);
+  const uint32_t n_tiles = 1u << host_pass.n_out;
+  const unsigned grid = std::min<unsigned>(n_tiles, unsigned(num_sms) * MINB);
+  uint64_t out_mask = 0, step = 0;  // qubits outside the tile; the grid size over them
+  for (int j = 0; j < host_pass.n_out; ++j) {
+    out_mask |= 1ull << host_pass.qout[j];
+    step |= uint64_t((grid >> j) & 1u) << host_pass.qout[j];
+  }
   // The pass may start while the kernel before it on the stream drains (its CTAs
   // load their tables, then wait for that kernel to complete).
   cudaLaunchAttribute pdl{};
@@ -212,7 +226,8 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   cfg.stream = stream;
   cfg.attrs = &pdl;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, amp, host_pass, reinterpret_cast<const uint4*>(d_prog), prog_smem, n_tiles);
+  return cudaLaunchKernelEx(&cfg, kern, amp, host_pass, reinterpret_cast<const uint4*>(d_prog), n_tiles,
+                            out_mask, step);
 }
 
 template <typename Real>
@@ -224,10 +239,11 @@ static cudaError_t launch_tile_pass_t(Real* amp, const PassRec& host_pass, const
     if (sizeof(Real) == 4) cfg = host_pass.k == K ? 2 : 4;
     else cfg = (1ull << host_pass.n_out) <= uint64_t(num_sms) ? 1 : 2;
   }
+  constexpr int W = sizeof(Real) == 8 ? 2 : 1;
   switch (cfg) {
-    case 4: return launch_tile_pass_cfg<Real, K - 1, 4>(amp, host_pass, d_prog, stream, num_sms);
-    case 2: return launch_tile_pass_cfg<Real, K, 2>(amp, host_pass, d_prog, stream, num_sms);
-    default: return launch_tile_pass_cfg<Real, K, 1>(amp, host_pass, d_prog, stream, num_sms);
+    case 4: return launch_tile_pass_cfg<Real, K - 1, 4, W>(amp, host_pass, d_prog, stream, num_sms);
+    case 2: return launch_tile_pass_cfg<Real, K, 2, W>(amp, host_pass, d_prog, stream, num_sms);
+    default: return launch_tile_pass_cfg<Real, K, 1, 1>(amp, host_pass, d_prog, stream, num_sms);
   }
 }
 

@@ -600,6 +600,45 @@ __device__ __forceinline__ uint64_t tile_base(const PassRec& P, uint64_t tile) {
 }
 
 
+// Addressing of a full tile's copies between HBM and shared memory (KMAX tile
+// bits, the usual contiguous low block): vector tid + i * threads sits at slot
+// swz(tid) ^ swz(i * threads), and its HBM offset is the thread's part plus a
+// combination of the four highest tile qubits, so a vector costs about five
+// instructions beside the access (some twenty when every vector works out its
+// own index and swizzle; two of three instructions of a one-stage pass).
+template <typename Real, int KMAX>
+struct TileCopy {
+  static constexpr int VB = Tr<Real>::kVecBit;
+  static constexpr int C = sizeof(Real) == 4 ? 5 : 4;
+  static constexpr uint32_t kThreads = 1u << (KMAX - VB - 4);
+  using V = typename Tr<Real>::V;
+
+  static __host__ __device__ __forceinline__ bool fits(const PassRec& P) { return P.k == KMAX && P.c == C; }
+  // f(slot, pointer) for each of the thread's 16 vectors; `base` = amplitude
+  // index of the tile's first amplitude.
+  template <typename F>
+  static __device__ __forceinline__ void each(Real* amp, const PassRec& P, const uint64_t* hi_off, uint64_t base, F&& f) {
+    uint32_t tid = threadIdx.x;
+    asm volatile("" : "+r"(tid));  // worked out per tile: no registers held across the stages
+    const uint32_t t = tid << VB;
+    const uint32_t s0 = swz(tid);
+    char* g = reinterpret_cast<char*>(amp) +
+              (base + (t & ((1u << C) - 1u)) + hi_off[t >> C]) * (2 * sizeof(Real));
+    const int top = KMAX - C - 4;
+    const uint64_t d0 = uint64_t(2 * sizeof(Real)) << P.qhi[top], d1 = uint64_t(2 * sizeof(Real)) << P.qhi[top + 1];
+    const uint64_t d2 = uint64_t(2 * sizeof(Real)) << P.qhi[top + 2], d3 = uint64_t(2 * sizeof(Real)) << P.qhi[top + 3];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      char* gh = g + ((h & 1) ? d2 : 0) + ((h & 2) ? d3 : 0);
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        const uint32_t i = uint32_t(4 * h + l);
+        f(s0 ^ swz(i * kThreads), reinterpret_cast<V*>(gh + ((l & 1) ? d0 : 0) + ((l & 2) ? d1 : 0)));
+      }
+    }
+  }
+};
+
 // Copy a pass's stage tables (StageTab, tileprog.h) and, behind them, the first
 // `words` words of its program into shared memory, asynchronously: every thread
 // of the CTA calls it, then waits for its copies (cp_async_wait0) and the CTA
@@ -635,8 +674,7 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
   for (int si = 0; si < nst; ++si) {
     const uint32_t* Tb = tabs + si * kStageTabWords;
     if (uint32_t(tid & ~31) < active_threads) {
-      const bool writes = uint32_t(tid) < active_threads;
-      const int tid_ = writes ? tid : tid & int(active_threads - 1);
+      const int tid_ = tid & int(active_threads - 1);
       const uint32_t ub = Tb[StageTab::UL + (tid_ & 15)] | Tb[StageTab::UH + (tid_ >> 4)];
       // swz is linear over XOR and ub, vm_i have disjoint bits, so
       // swz(ub | sum vm_i) = swz(ub) ^ xor_i swz(vm_i).
@@ -652,7 +690,9 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
       }
       const uint32_t vbase = (ub << VB) | ext;
       apply_stage_prog<Real, NA, NRB>(a, prog + Tb[StageTab::OB], prog + min(Tb[StageTab::OE], words), vbase);
-      if (writes) {
+      int wtid = threadIdx.x;  // read again: no register held across the program
+      asm volatile("" : "+r"(wtid));
+      if (uint32_t(wtid) < active_threads) {
         // Write-back through the stage's deferred permutation pi(p) = A p ^ w:
         // register amplitude p goes to the slot of logical index pi(p).  Slot
         // offsets are linear in the free register bits (register bits
