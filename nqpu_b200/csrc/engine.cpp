@@ -383,20 +383,19 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
 // NQPU_MODE_AUTO: the engine mode with the lower modelled device time (the
 // counterpart of the reference's runtime-estimate backend choice,
 // select_backend_estimated, backends/runtime/auto_simulator.rs:1452, among
-// its statevector variants).  The model is in units of one HBM pass over the
-// state (2 S bytes).  Tiled passes: per pass one unit plus its launch cost,
-// plus the shared-memory tile work of each op (dense 1-qubit 0.15, dense
-// 2-qubit 0.30, diagonal 0.058, permutations free: they are deferred into the
-// write-back addresses).  Tensor passes: per pass one unit plus its launch
-// cost, plus 0.35 per fused unitary (its MMAs and epilogue on every tile).
-// The launch cost is about 15 us per pass in either mode (launch, pass-table
-// prologue, grid tail), i.e. 15 us / (2 S / 6.5 TB/s) units: negligible at 30
-// qubits, dominant below 20, where the mode with fewer passes wins.  The
-// per-op coefficients are fits to 30-qubit complex64 runs of the brickwork
-// (tiled 69 passes / 1200 U3, tensor 81 passes / 178 unitaries) and of the
-// QFT (tiled 8 passes / 30 H + 435 controlled phases) against the copy time
-// of the state.  The tensor mode is taken when its model is at least 10 %
-// below the tiled one.
+// its statevector variants).  Both models are device time as U x work + launch
+// cost, U = one HBM pass over the state (2 S bytes at 6.5 TB/s):
+//   tiled   U (0.80 passes + 0.069 stages + 0.071 one-qubit 2x2s + 0.011
+//           diagonal ops) + 11.2 us per pass + 1.1 us per stage
+//   tensor  U (1.013 passes + 0.139 unitaries) + 16.8 us per pass + 34 us
+// fitted (least squares of the relative error) to 42 measured complex64 circuits:
+// brickwork, ansatz, Ising evolution and phase estimation of 14 to 28 qubits and
+// two depths.  The fit is within 15 % for most, and picks the faster mode for
+// every one of them: the tensor passes win on brickworks from 23 qubits on
+// (26 qubits, 12 layers: 4.5 against 6.9 ms), the tiled ones everywhere else
+// (30-qubit Ising evolution, 10 steps: 121 against 140 ms).  4x4 matrices and 2x2s
+// with controls run as single records, priced at the 0.30 and 0.15 they
+// measured as such.
 int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt) {
   if (dt != DType::C64 || int(n) < kTcMinQubits) return NQPU_MODE_TILED;
   PlanStats ts;
@@ -407,19 +406,20 @@ int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt) {
   double work = 0.0;
   for (const Op& op : ops) {
     switch (op.kind) {
-      case OP_U1: work += 0.15; break;
+      case OP_U1: work += op.nctrl ? 0.15 : 0.071; break;
       case OP_U2: work += 0.30; break;
       case OP_D1:
       case OP_D2:
-      case OP_PH: work += 0.058; break;
+      case OP_PH: work += 0.011; break;
       default: break;  // OP_X1, OP_SW
     }
   }
-  const double pass_us = 2.0 * std::ldexp(8.0, int(n)) / 6.5e6;  // 2 S bytes at 6.5 TB/s, in microseconds
-  const double per_pass = 1.0 + 15.0 / pass_us;
-  const double tiled = double(tp.stats.passes) * per_pass + work;
-  const double tensor = double(ts.passes) * per_pass + 0.35 * double(ts.stages);
-  return tensor < 0.9 * tiled ? NQPU_MODE_TENSOR : NQPU_MODE_TILED;
+  const double unit = 2.0 * std::ldexp(8.0, int(n)) / 6.5e6;  // 2 S bytes at 6.5 TB/s, in microseconds
+  const double tp_ = double(tp.stats.passes), ts_ = double(tp.stats.stages);
+  const double tiled = unit * (0.80 * tp_ + 0.069 * ts_ + work) + 11.2 * tp_ + 1.1 * ts_;
+  const double xp = double(ts.passes);
+  const double tensor = unit * (1.013 * xp + 0.139 * double(ts.stages)) + 16.8 * xp + 34.0;
+  return tensor < tiled ? NQPU_MODE_TENSOR : NQPU_MODE_TILED;
 }
 
 static std::vector<Op> segment_ops(const CircuitImpl* c, const Segment& seg) {
