@@ -230,11 +230,39 @@ __device__ __forceinline__ void rb_table(C (&a)[NA], const uint4* q) {
   }
 }
 
-// diag(d0, d1) on register bit B
-template <typename C, int NA, int B>
-__device__ __forceinline__ void rb_d1(C (&a)[NA], C d0, C d1) {
+// a phase as three shears in place: p.x = tan(alpha / 2), p.y = sin(alpha)
+template <typename C>
+__device__ __forceinline__ void turn_in(C p, C& v) {
+  v.x = fma(-p.x, v.y, v.x);
+  v.y = fma(p.y, v.x, v.y);
+  v.x = fma(-p.x, v.y, v.x);
+}
+template <typename C, int NA, int CMASK>
+__device__ __forceinline__ void rb_turn(C (&a)[NA], C p) {
 #pragma unroll
-  for (int i = 0; i < NA; ++i) cmul_in((i & (1 << B)) ? d1 : d0, a[i]);
+  for (int i = 0; i < NA; ++i)
+    if ((i & CMASK) == CMASK) turn_in(p, a[i]);
+}
+template <typename Real, typename C, int NA>
+__device__ __forceinline__ void rb_turn_table(C (&a)[NA], const uint4* q) {
+  if constexpr (sizeof(Real) == 4) {
+#pragma unroll
+    for (int i = 0; i < NA; i += 2) {
+      C u, v;
+      ldc2<Real>(reinterpret_cast<const Real*>(q) + 2 * i, u, v);
+      turn_in(u, a[i]);
+      turn_in(v, a[i + 1]);
+    }
+  } else {
+    const volatile Real* m = reinterpret_cast<const volatile Real*>(q);  // not hoisted: no registers for it
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      C u;
+      u.x = m[2 * i];
+      u.y = m[2 * i + 1];
+      turn_in(u, a[i]);
+    }
+  }
 }
 
 // sign flip (s = 0 or the sign bit) of the register amplitudes with bits CMASK
@@ -251,6 +279,18 @@ __device__ __forceinline__ void rb_sign(C (&a)[NA], uint32_t s) {
       a[i].y = __hiloint2double(__double2hiint(a[i].y) ^ int(s), __double2loint(a[i].y));
     }
   }
+}
+
+// diag(d0, d1) on register bit B
+template <typename C, int NA, int B>
+__device__ __forceinline__ void rb_d1(C (&a)[NA], C d0, C d1) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i) cmul_in((i & (1 << B)) ? d1 : d0, a[i]);
+}
+template <typename C, int NA, int B>
+__device__ __forceinline__ void rb_turn1(C (&a)[NA], C p0, C p1) {
+#pragma unroll
+  for (int i = 0; i < NA; ++i) turn_in((i & (1 << B)) ? p1 : p0, a[i]);
 }
 
 // dense 4x4 on register bits (B0 = sub-index bit 0, B1 = bit 1); matrix rows
@@ -410,10 +450,17 @@ __device__ __forceinline__ uint32_t list_angle(const uint4*& p, uint32_t cnt, ui
   }
   return angle;
 }
-__device__ __forceinline__ float2 phase_of(uint32_t angle) {
-  float2 v;
-  sincospif(float(int32_t(angle)) * 0x1p-31f, &v.y, &v.x);
-  return v;
+// The phase of an angle for cmul_in or, where every lane of the warp is within a
+// quarter turn (*shear), for turn_in: a Trotter step's angles are, and there the
+// shears keep the norm from drifting with the rounding of one (cos, sin) step after
+// step.  Wider angles take the product: a shear would need a sign flip besides.
+__device__ __forceinline__ float2 phase_of(uint32_t angle, bool* shear) {
+  float s, c;
+  sincospif(float(int32_t(angle)) * 0x1p-31f, &s, &c);
+  *shear = __all_sync(0xffffffffu, c >= 0.0f);
+  // c >= 0: the quotient is good to two roundings; an error in it turns the angle
+  // by as much but leaves the shear's determinant
+  return *shear ? make_float2(__fdividef(s, 1.0f + c), s) : make_float2(c, s);
 }
 __device__ __forceinline__ double2 list_phase(const uint4*& p, uint32_t cnt, double2 v, uint32_t vbase) {
   for (uint32_t i = 0; i < cnt; ++i, p += 2) {
@@ -469,19 +516,31 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
       const uint32_t bits = __shfl_sync(0xffffffffu, h.y, 0);
       if (code == TC_R) rotate_bits<Real, NA, NRB>(a, bits, h, q, false);
       else rotate_bits<Real, NA, NRB>(a, bits, h, q, true);
-    } else if (code == TC_T) {
-      rb_table<Real, C, NA>(a, q);
-    } else if (code <= TC_PH) {
+    } else if (code <= TC_T) {
+      if (code == TC_TS) rb_turn_table<Real, C, NA>(a, q);
+      else rb_table<Real, C, NA>(a, q);
+    } else if (code <= TC_PU) {
       C d;
+      bool shear = code == TC_PS;  // (no PS in complex128: its registers)
       if constexpr (F32) {
-        if (code == TC_PU) d = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
-        else d = phase_of(list_angle(q, h.y, h.z, vbase));
+        if (code == TC_PH) d = phase_of(list_angle(q, h.y, h.z, vbase), &shear);
+        else d = make_float2(__uint_as_float(h.z), __uint_as_float(h.w));
       } else {
         d = *reinterpret_cast<const double2*>(q);
         if (code == TC_PH) d = list_phase(++q, h.y, d, vbase);
       }
       switch (arg) {
-#define NQ_A(V) case V: if constexpr (V < (1 << NRB)) rb_ph<C, NA, V>(a, d); break;
+#define NQ_A(V) \
+        case V: \
+          if constexpr (V < (1 << NRB)) { \
+            if constexpr (F32) { \
+              if (shear) rb_turn<C, NA, V>(a, d); \
+              else rb_ph<C, NA, V>(a, d); \
+            } else { \
+              rb_ph<C, NA, V>(a, d); \
+            } \
+          } \
+          break;
 #define NQ_SETS(M) M(0) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) \
         M(16) M(17) M(18) M(19) M(20) M(21) M(22) M(23) M(24) M(25) M(26) M(27) M(28) M(29) M(30) M(31)
         NQ_SETS(NQ_A)
@@ -510,10 +569,19 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
       }
     } else if (code == TC_D) {
       C d0, d1;
+      bool shear = false;
       if constexpr (F32) {
-        const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase);
-        d0 = phase_of(g);
-        d1 = phase_of(list_angle(q, h.y >> 16, g + h.w, vbase));
+        const uint32_t g = list_angle(q, h.y & 0xFFFFu, h.z, vbase), g1 = list_angle(q, h.y >> 16, g + h.w, vbase);
+        float s, c;  // both as shears or both as products
+        sincospif(float(int32_t(g)) * 0x1p-31f, &s, &c);
+        d0 = make_float2(c, s);
+        sincospif(float(int32_t(g1)) * 0x1p-31f, &s, &c);
+        d1 = make_float2(c, s);
+        shear = __all_sync(0xffffffffu, fminf(d0.x, d1.x) >= 0.0f);
+        if (shear) {
+          d0.x = __fdividef(d0.y, 1.0f + d0.x);
+          d1.x = __fdividef(d1.y, 1.0f + d1.x);
+        }
       } else {
         d0 = *reinterpret_cast<const double2*>(q);
         d1 = *reinterpret_cast<const double2*>(q + 1);
@@ -522,7 +590,13 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
         d1 = cmul(d0, list_phase(q, h.y >> 16, d1, vbase));
       }
       switch (arg) {
-#define NQ_B(B, _) case B: if constexpr (B < NRB) rb_d1<C, NA, B>(a, d0, d1); break;
+#define NQ_B(B, _) \
+        case B: \
+          if constexpr (B < NRB) { \
+            if (F32 && shear) rb_turn1<C, NA, B>(a, d0, d1); \
+            else rb_d1<C, NA, B>(a, d0, d1); \
+          } \
+          break;
         NQ_REG_CASES(NQ_B, 0)
 #undef NQ_B
         default: break;

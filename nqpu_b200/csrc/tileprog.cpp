@@ -101,6 +101,8 @@ class StageCompiler {
   // stage to stage and applied by the last one.
   void run(const StageRec& S, bool last, cplx* global, std::vector<ProgWord>* out) {
     W_ = Writer(out, sizeof(Real) == 4);
+    global_ = global;
+    final_ = false;
     items_.clear();
     for (Phase& p : pend_) p.clear();
     used_ = 0;
@@ -110,6 +112,7 @@ class StageCompiler {
     schedule();
     *global *= pend_[0].uniform;
     pend_[0].uniform = last ? *global : cplx(1.0, 0.0);
+    final_ = last;
     finish();
   }
 
@@ -350,15 +353,36 @@ class StageCompiler {
       pend_[A].uniform = cplx(1.0, 0.0);
       if (pend_[A].list.empty()) drop(A);
     }
-    double d[64];
+    // within half a turn of one another: shears around the middle, which goes to
+    // the phase common to all amplitudes
+    double d[64], lo = 0.0, hi = 0.0;
+    const cplx first = std::conj(v[0]);
     for (uint32_t r = 0; r < kAll; ++r) {
-      d[2 * r] = v[r].real();
-      d[2 * r + 1] = v[r].imag();
+      const cplx p = v[r] * first;
+      d[r] = std::atan2(p.imag(), p.real());
+      lo = std::min(lo, d[r]);
+      hi = std::max(hi, d[r]);
     }
-    W_.header(TC_T, 0);
+    if (!final_ && hi - lo <= kHalfTurn) {
+      const double mid = 0.5 * (lo + hi);
+      *global_ *= v[0] * cplx(std::cos(mid), std::sin(mid));
+      for (uint32_t r = kAll; r-- > 0;) {
+        const double a = d[r] - mid;
+        d[2 * r] = std::tan(0.5 * a);
+        d[2 * r + 1] = std::sin(a);
+      }
+      W_.header(TC_TS, 0);
+    } else {
+      for (uint32_t r = 0; r < kAll; ++r) {
+        d[2 * r] = v[r].real();
+        d[2 * r + 1] = v[r].imag();
+      }
+      W_.header(TC_T, 0);
+    }
     W_.reals(d, 2 * int(kAll));
     W_.end();
   }
+  static constexpr double kHalfTurn = 3.14159265358979;
   void drop(uint32_t A) {
     pend_[A].clear();
     used_ &= ~(1u << A);
@@ -411,8 +435,10 @@ class StageCompiler {
         W_.bytes(v.data(), v.size() * 4);
       }
     } else if (P.list.empty()) {
-      W_.header(TC_PU, A);
-      pair_of(u);
+      const double ts[2] = {u[1] / (1.0 + u[0]), u[1]};
+      const bool shear = kF32 && u[0] >= 0.0;
+      W_.header(shear ? TC_PS : TC_PU, A);
+      pair_of(shear ? ts : u);
     } else {
       W_.header(TC_PH, A, uint32_t(P.list.size()));
       if (kF32) W_.head().w[2] = turns(P.uniform);
@@ -488,6 +514,8 @@ class StageCompiler {
   std::vector<size_t> batch_;
   Phase pend_[32];
   uint32_t used_ = 0;  // pend_ entries in use
+  cplx* global_ = nullptr;  // phase common to all amplitudes
+  bool final_ = false;      // emitting the plan's last phases: nothing takes a common one any more
   cplx acc_[5][4];
   bool have_[5];
 };
@@ -567,8 +595,9 @@ void compile(const std::vector<Op>& ops, TilePlan* plan, const std::vector<TileO
   }
 }
 
-// A complex unitary 2x2 without controls that is neither real nor of RX's form.
-bool takes_carry(const Op& o) {
+// A unitary 2x2 without controls that is not real, diagonal or anti-diagonal: its
+// three Euler angles are all there.  `rx`: of RX's form.
+bool takes_carry(const Op& o, bool* rx = nullptr) {
   if (o.kind != OP_U1 || o.nctrl != 0) return false;
   const cplx* m = o.m;
   const double eps = 1e-12;
@@ -576,8 +605,8 @@ bool takes_carry(const Op& o) {
       std::abs(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) > eps)
     return false;
   const bool real = m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0;
-  const bool cross = m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
-  return !real && !cross && std::abs(m[0]) > 1e-6 && std::abs(m[2]) > 1e-6;
+  if (rx) *rx = m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
+  return !real && std::abs(m[0]) > 1e-6 && std::abs(m[2]) > 1e-6;
 }
 
 void times(const cplx* a, const cplx* b, cplx* out) {
@@ -614,7 +643,8 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
     return -1;
   };
   for (size_t i = 0; i < ops.size(); ++i) {
-    if (!takes_carry(ops[i])) continue;
+    bool rx = false;
+    if (!takes_carry(ops[i], &rx)) continue;
     const int q = ops[i].t0;
     bool z = true, x = true, found = false;
     size_t e = 0;
@@ -629,7 +659,9 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
       else if (o.kind == OP_X1 && o.t0 == q) z = false;
       else z = x = false;
     }
-    if (!found || z == x) continue;  // none, or nothing between: the compiler merges the two
+    // none, nothing between (the compiler merges the two), or an RX that would
+    // wander whole through X targets
+    if (!found || z == x || (rx && x)) continue;
     cplx* m = ops[i].m;
     cplx w[4] = {m[0], m[1], m[2], m[3]}, c[4] = {1.0, 0.0, 0.0, 1.0};
     if (z) {

@@ -14,6 +14,13 @@
 //   G b        any complex 2x2: header.y = virtual-index mask that must be set; the
 //              entries m00, m01, m10, m11 follow
 //   T          one constant phase per register amplitude: 2^(register bits) entries
+//   TS         the same as shears (t, s of every phase, all within a quarter turn
+//              either way): three operations per amplitude instead of four, and
+//              no drift of the norm (a shear has determinant 1 whatever its
+//              rounding; a rounded (cos, sin) scales what it turns, the same way
+//              in every step of an evolution)
+//   PS A       constant phase as a shear on the register amplitudes whose bits A
+//              are all set (complex64; t, s in header.z, .w)
 //   PU A       constant phase on the register amplitudes whose bits A are all set
 //              (re, im in header.z, .w or the next word)
 //   SG A       sign flip of those amplitudes
@@ -67,7 +74,7 @@ struct StageTab {
 };
 static_assert(StageTab::SH + 16 <= kStageTabWords && kStageTabWords % 4 == 0, "stage table layout");
 
-enum TileCode : uint32_t { TC_R, TC_X, TC_T, TC_PU, TC_PH, TC_SG, TC_SL, TC_D, TC_G, TC_LEG };
+enum TileCode : uint32_t { TC_R, TC_X, TC_TS, TC_T, TC_PS, TC_PH, TC_PU, TC_SG, TC_SL, TC_D, TC_G, TC_LEG };
 
 // The op list with every complex 2x2 reduced to rotation x phase where a later 2x2
 // on its qubit can take the rest: a phase passes through controls and diagonal

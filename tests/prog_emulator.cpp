@@ -73,6 +73,13 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
     const ProgWord& h = *p;
     if (len == 0 || p + len > end) return -2;
     const cd two = F32 ? cget<float>(p, 1) : cget<double>(q, 0);  // the instruction's two reals
+    auto turn_by = [](bool shear, cd p, cd& v) {
+      if (!shear) { v *= p; return; }
+      double x = v.real() - p.real() * v.imag();
+      const double y = v.imag() + p.imag() * x;
+      x -= p.real() * y;
+      v = cd(x, y);
+    };
     auto two_by_two = [&](uint32_t b, const cd* m) {
       for (uint32_t i = 0; i < a.size(); ++i) {
         if (i & b) continue;
@@ -96,11 +103,11 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
       cd m[4];
       for (int i = 0; i < 4; ++i) m[i] = cget<Real>(q, i);
       if (hit(h.w[1])) two_by_two(1u << arg, m);
-    } else if (code == TC_T) {
-      for (uint32_t i = 0; i < a.size(); ++i) a[i] *= cget<Real>(q, int(i));
-    } else if (code == TC_PU) {
+    } else if (code == TC_T || code == TC_TS) {
+      for (uint32_t i = 0; i < a.size(); ++i) turn_by(code == TC_TS, cget<Real>(q, int(i)), a[i]);
+    } else if (code == TC_PU || code == TC_PS) {
       for (uint32_t i = 0; i < a.size(); ++i)
-        if ((i & arg) == arg) a[i] *= two;
+        if ((i & arg) == arg) turn_by(code == TC_PS, two, a[i]);
     } else if (code == TC_SG || code == TC_SL) {
       uint32_t s = code == TC_SG ? 1u : h.w[2];
       for (uint32_t i = 0; code == TC_SL && i < h.w[1]; ++i) s += hit(q[i / 4].w[i & 3]);
