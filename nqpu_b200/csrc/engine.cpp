@@ -282,6 +282,17 @@ cudaError_t state_probabilities(const StateImpl* s, double* out) {
 
 cudaError_t state_download_c128(const StateImpl* s, NqpuComplex* out) {
   const uint64_t dim = 1ull << s->n;
+  if (dim * 16 <= (kSmallDoubles - kSmallTable) * sizeof(double)) {
+    // a small register through the pinned buffer (no allocation, and a copy to
+    // pageable memory costs several microseconds more)
+    double* h = s->h_small + kSmallTable;
+    cudaError_t e = s->dt == DType::C128
+                        ? cudaMemcpyAsync(h, s->amp, dim * 16, cudaMemcpyDeviceToHost, s->stream)
+                        : launch_convert(DType::C64, s->amp, DType::C128, h, dim, s->stream, device_sms());
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) std::memcpy(static_cast<void*>(out), h, dim * 16);
+    return e;
+  }
   if (s->dt == DType::C128) {
     cudaError_t e = cudaMemcpyAsync(out, s->amp, dim * 16, cudaMemcpyDeviceToHost, s->stream);
     if (e != cudaSuccess) return e;

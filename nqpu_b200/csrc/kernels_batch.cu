@@ -206,27 +206,12 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     const BatchTask T = tasks[ti];
     const BatchCirc C = circs[T.circ];
 
-    if (T.phase < 0) {
-      // ---- whole small circuit in shared memory ----
-      load_pass(C, 0);
-      const uint32_t nvec = 1u << (P.k - 1);
-      init_tile(nvec, true);
-      __syncthreads();
-      run_stages(0u);
-      double jtot;
-      load_obs(C, &jtot);
-      __syncthreads();
-      const double part = ising_tile(sv, C.n, C.n, 0, nullptr, lut, hq, jtot);
-      const double e = block_sum(part, red);
-      if (tid == 0) results[C.result] = e;
-      __syncthreads();
-      continue;
-    }
-
     float2* state = reinterpret_cast<float2*>(arena) + C.amp_off;
-    if (T.phase < C.n_passes) {
-      // ---- one tile of one pass ----
-      load_pass(C, T.phase);
+    const bool small = T.phase < 0;
+    if (small || T.phase < C.n_passes) {
+      // ---- whole small circuit in shared memory, or one tile of one pass (one
+      // call of the stage executor for both: it is most of the kernel's code) ----
+      load_pass(C, small ? 0 : T.phase);
       if (T.phase > 0) {
         const uint32_t need = 1u << passes[C.pass_base + T.phase - 1].n_out;
         if (!wait_counter(counters + C.done_base + T.phase - 1, need, spin_limit, err, &s_flag)) continue;
@@ -234,11 +219,11 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       const int k = P.k, c = P.c;
       const uint32_t nvec = 1u << (k - 1);
       const uint32_t lowmask = (1u << c) - 1u;
-      const uint64_t base = tile_base(P, T.tile);
+      const uint64_t base = small ? 0 : tile_base(P, T.tile);
       uint32_t ext = 0;
       for (int j = 0; j < P.n_ext; ++j)
         if ((base >> P.ext[j]) & 1ull) ext |= 1u << (k + j);
-      if (T.phase == 0) {
+      if (T.phase <= 0) {
         init_tile(nvec, base == 0);
       } else {
         if (Copy::fits(P)) {
@@ -254,6 +239,16 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       }
       __syncthreads();
       run_stages(ext);
+      if (small) {
+        double jtot;
+        load_obs(C, &jtot);
+        __syncthreads();
+        const double part = ising_tile(sv, C.n, C.n, 0, nullptr, lut, hq, jtot);
+        const double e = block_sum(part, red);
+        if (tid == 0) results[C.result] = e;
+        __syncthreads();
+        continue;
+      }
       if (Copy::fits(P)) {
         Copy::each(arena + 2 * C.amp_off, P, hi_off, base, [&](uint32_t slot, float4* g) { __stcg(g, sv[slot]); });
       } else {
