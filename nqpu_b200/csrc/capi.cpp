@@ -233,7 +233,7 @@ static NqpuError apply_rec(NqpuState* state, const GateRec& g) {
   for (int i = 0; i < 4; ++i)
     if (!is_finite_param(g.p[i])) return NQPU_INVALID_PARAMETER;
   const Op op = lower_gate(g);
-  NQ_TRY(launch_pergate(s->dt, s->amp, int(s->n), op, s->stream, device_sms()));
+  NQ_TRY(launch_pergate(s->dt, s->amp, int(s->n), op, s->next_sweep(), s->stream, device_sms()));
   return NQPU_OK;
 }
 

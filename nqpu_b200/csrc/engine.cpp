@@ -474,7 +474,7 @@ bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, Pl
 
 cudaError_t run_ops_pergate(StateImpl* s, const std::vector<Op>& ops) {
   for (const Op& op : ops) {
-    cudaError_t e = launch_pergate(s->dt, s->amp, int(s->n), op, s->stream, device_sms());
+    cudaError_t e = launch_pergate(s->dt, s->amp, int(s->n), op, s->next_sweep(), s->stream, device_sms());
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -577,7 +577,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   if (e != cudaSuccess) return e;
   if (effective == NQPU_MODE_PERGATE) {
     for (const Op& op : p->ops) {
-      if ((e = launch_pergate(s->dt, s->amp, int(s->n), op, s->stream, device_sms())) != cudaSuccess) return e;
+      if ((e = launch_pergate(s->dt, s->amp, int(s->n), op, s->next_sweep(), s->stream, device_sms())) != cudaSuccess) return e;
       if ((e = mark(events, s->stream)) != cudaSuccess) return e;
     }
     return cudaSuccess;

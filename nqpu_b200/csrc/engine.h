@@ -46,6 +46,8 @@ struct StateImpl {
   double* run_norm = nullptr;
   size_t run_norm_cap = 0;     // doubles
   int* run_err = nullptr;
+  bool sweep = false;          // direction of the last per-gate launch
+  bool next_sweep() { return sweep = !sweep; }
 };
 
 StateImpl* state_new(uint32_t n, DType dt);

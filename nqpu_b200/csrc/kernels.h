@@ -17,11 +17,13 @@ struct PGArgs {
   int32_t npos;       // zero-bit insert positions, ascending
   int32_t pos[8];
   int32_t t0, t1;
+  int32_t rev;        // run over the items from the far end
   double m[32];
 };
 
 // --- per-gate path -----------------------------------------------------------
-cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, cudaStream_t s, int num_sms);
+// `rev`: sweep the state from its far end (callers alternate from gate to gate).
+cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, bool rev, cudaStream_t s, int num_sms);
 
 // --- tiled pass path ---------------------------------------------------------
 // CTA configuration of the tiled pass kernel (1: one CTA per SM, double-buffered

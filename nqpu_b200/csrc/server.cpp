@@ -224,8 +224,8 @@ cudaError_t launch_request(ServerImpl* sv, Lane& L, Request& r) {
     for (const PassRec& P : r.plan.passes)
       if ((e = launch_tile_pass(DType::C64, amp, P, dprog, st, sv->sms)) != cudaSuccess) return e;
   } else {
-    for (const Op& op : r.ops)
-      if ((e = launch_pergate(DType::C64, amp, int(r.n), op, st, sv->sms)) != cudaSuccess) return e;
+    for (const Op& op : r.ops)  // a handful of qubits
+      if ((e = launch_pergate(DType::C64, amp, int(r.n), op, false, st, sv->sms)) != cudaSuccess) return e;
   }
   if (r.kind == NQPU_REQUEST_ZALL) {
     if ((e = launch_zsums(DType::C64, amp, int(r.n), L.scratch, L.d_small, st, sv->sms)) != cudaSuccess) return e;
