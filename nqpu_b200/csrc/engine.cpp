@@ -472,14 +472,6 @@ bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, Pl
   return true;
 }
 
-cudaError_t run_ops_pergate(StateImpl* s, const std::vector<Op>& ops) {
-  for (const Op& op : ops) {
-    cudaError_t e = launch_pergate(s->dt, s->amp, int(s->n), op, s->next_sweep(), s->stream, device_sms());
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
 // The copy is ordered on the stream the plan runs on first and has landed when
 // this returns, so every stream may run the plan afterwards (a plain cudaMemcpy
 // of pageable memory may return before its data reaches the device, and the

@@ -129,6 +129,5 @@ bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, Pl
 int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt);
 
 // Run a lowered op list on a state with the given mode (used by batch/server).
-cudaError_t run_ops_pergate(StateImpl* s, const std::vector<Op>& ops);
 
 }  // namespace nqpu

@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   auto tab_words = [&]() { return (P.stage_end - P.stage_begin) * (kStageTabWords / 4); };
   auto run_stages = [&](uint32_t ext) {
     if (P.prog_words <= kBatchProgWords)
-      run_tile_stages<float>(sv, P, tabs, reinterpret_cast<const uint4*>(tabs) + tab_words(), ext);
+      run_tile_stages<float, false>(sv, P, tabs, reinterpret_cast<const uint4*>(tabs) + tab_words(), ext);
     else
-      run_tile_stages<float>(sv, P, tabs, progs + P.prog_begin + tab_words(), ext);
+      run_tile_stages<float, false>(sv, P, tabs, progs + P.prog_begin + tab_words(), ext);
   };
   __shared__ int s_pass;  // global index of the pass whose tables are loaded (-1: none)
   __shared__ uint32_t s_task;

@@ -113,8 +113,9 @@ __global__ void __launch_bounds__(1 << (KMAX - Tr<Real>::kVecBit - 4), MINB)
     const uint32_t ext =
         __ballot_sync(0xffffffffu, lane < P.n_ext && ((base >> P.ext[lane]) & 1ull)) << k;
 
-    if constexpr (WAY > 0) run_tile_stages<Real>(sv, P, tabs, prog_s, ext);
-    else run_tile_stages<Real>(sv, P, tabs, prog_g, ext);
+    constexpr bool kFew = sizeof(Real) == 8 && MINB > 1;
+    if constexpr (WAY > 0) run_tile_stages<Real, kFew>(sv, P, tabs, prog_s, ext);
+    else run_tile_stages<Real, kFew>(sv, P, tabs, prog_g, ext);
 
     // shared -> HBM
     if (full) {
@@ -145,9 +146,9 @@ static size_t tile_smem_base(int minb) {
 // (1 KB each goes to the system, under 1 KB to the static arrays); enough for
 // the tables of the longest pass.
 template <typename Real, int KMAX>
-static size_t tile_smem_max(int minb) {
+static size_t tile_smem_max(int minb, int share_of) {
   const size_t need = tile_smem_base<Real, KMAX>(minb) + sizeof(uint32_t) * kMaxPassStages * kStageTabWords;
-  const size_t share = size_t(227 * 1024) / size_t(minb) - 2048;
+  const size_t share = size_t(227 * 1024) / size_t(share_of) - 2048;
   return std::max(need, share);
 }
 
@@ -188,7 +189,11 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   // stage tables of this pass and, where it fits beside them in MINB CTAs per
   // SM, its program (a single-tile CTA would wait for each op's first read
   // from L2 otherwise)
-  const size_t smem_max = tile_smem_max<Real, KMAX>(MINB);
+  // Fewer tiles than the GPU takes at once leave more of the SM's to each CTA (96
+  // 4x4 gates on 8 qubits: their program from global memory 201 us, from here 171).
+  const uint32_t n_tiles = 1u << host_pass.n_out;
+  const int per_sm = int(std::min<uint64_t>(uint64_t(MINB), (uint64_t(n_tiles) + num_sms - 1) / num_sms));
+  const size_t smem_max = tile_smem_max<Real, KMAX>(MINB, per_sm);
   size_t smem = tile_smem_base<Real, KMAX>(MINB) +
                 sizeof(uint32_t) * kStageTabWords * size_t(host_pass.stage_end - host_pass.stage_begin);
   if constexpr (WAY == 2) {
@@ -204,10 +209,10 @@ cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const Prog
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  e = attr.get(dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max)); },
+  e = attr.get(dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          int(tile_smem_max<Real, KMAX>(MINB, 1))); },
                cudaErrorInvalidDevice);
   if (e != cudaSuccess) return e;
-  const uint32_t n_tiles = 1u << host_pass.n_out;
   const unsigned grid = std::min<unsigned>(n_tiles, unsigned(num_sms) * MINB);
   uint64_t out_mask = 0, step = 0;  // qubits outside the tile; the grid size over them
   for (int j = 0; j < host_pass.n_out; ++j) {

@@ -60,24 +60,10 @@ __device__ __forceinline__ PackedC pack_coef(float2 m) {
   return PackedC{make_float2(m.x, m.x), make_float2(-m.y, m.y)};
 }
 __device__ __forceinline__ float2 swap_ri(float2 v) { return make_float2(v.y, v.x); }
-// m * x
-__device__ __forceinline__ float2 pcmul(const PackedC& m, float2 x) {
-  return __ffma2_rn(m.q, swap_ri(x), __fmul2_rn(m.p, x));
-}
-// m0 * x + m1 * y (the 2x2 row product)
-__device__ __forceinline__ float2 pcmac2(const PackedC& m0, float2 x, const PackedC& m1, float2 y) {
-  float2 t = __fmul2_rn(m0.p, x);
-  t = __ffma2_rn(m0.q, swap_ri(x), t);
-  t = __ffma2_rn(m1.p, y, t);
-  return __ffma2_rn(m1.q, swap_ri(y), t);
-}
 
 __device__ __forceinline__ uint64_t insert_zero_bit(uint64_t v, int bit) {
   uint64_t lo = v & ((1ull << bit) - 1);
   return lo | ((v >> bit) << (bit + 1));
 }
-
-template <typename V> __device__ __forceinline__ V ldg_v(const V* p) { return __ldg(p); }
-template <typename V> __device__ __forceinline__ V ldcs_v(const V* p) { return __ldcs(p); }
 
 }  // namespace nqpu

@@ -48,60 +48,71 @@ __device__ __forceinline__ void ldc2<double>(const double* __restrict__ p, doubl
   b = *(reinterpret_cast<const double2*>(p) + 1);
 }
 
-// dense 2x2, no controls
-template <typename C, int NA, int B>
-__device__ __forceinline__ void rb_u1(C (&a)[NA], C m0, C m1, C m2, C m3) {
-  if constexpr (sizeof(m0.x) == 4) {
-    const PackedC p0 = pack_coef(m0), p1 = pack_coef(m1), p2 = pack_coef(m2), p3 = pack_coef(m3);
-#pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      if (i & (1 << B)) continue;
-      const int j = i | (1 << B);
-      const float2 x = a[i], y = a[j];
-      const float2 sx = swap_ri(x), sy = swap_ri(y);
-      float2 ti = __fmul2_rn(p0.p, x), tj = __fmul2_rn(p2.p, x);
-      ti = __ffma2_rn(p0.q, sx, ti);
-      tj = __ffma2_rn(p2.q, sx, tj);
-      ti = __ffma2_rn(p1.p, y, ti);
-      tj = __ffma2_rn(p3.p, y, tj);
-      a[i] = __ffma2_rn(p1.q, sy, ti);
-      a[j] = __ffma2_rn(p3.q, sy, tj);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      if (i & (1 << B)) continue;
-      const int j = i | (1 << B);
-      const C x = a[i], y = a[j];
-      a[i] = cmac2(m0, x, m1, y);
-      a[j] = cmac2(m2, x, m3, y);
-    }
-  }
-}
-
-// The same with the entries read again for every pair (volatile: the compiler
-// would keep all of them): complex128 at 128 registers has no room for them, and
-// the spills land on every instruction of the stage loop.
-template <typename Real, typename C, int NA, int B>
-__device__ __forceinline__ void rb_u1_reload(C (&a)[NA], const Real* p) {
-  const volatile Real* m = p;
+// complex64 dense 2x2 on the pairs whose register bits CM (controls) are set
+template <int NA, int B, int CM>
+__device__ __forceinline__ void rb_u1(float2 (&a)[NA], float2 m0, float2 m1, float2 m2, float2 m3) {
+  const PackedC p0 = pack_coef(m0), p1 = pack_coef(m1), p2 = pack_coef(m2), p3 = pack_coef(m3);
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
-    if (i & (1 << B)) continue;
-    C &x = a[i], &y = a[i | (1 << B)];
-    C u, v;
-    { const Real r = m[0], s = m[1]; u.x = r * x.x - s * x.y; u.y = r * x.y + s * x.x; }
-    { const Real r = m[2], s = m[3]; u.x += r * y.x - s * y.y; u.y += r * y.y + s * y.x; }
-    { const Real r = m[4], s = m[5]; v.x = r * x.x - s * x.y; v.y = r * x.y + s * x.x; }
-    { const Real r = m[6], s = m[7]; v.x += r * y.x - s * y.y; v.y += r * y.y + s * y.x; }
-    x = u;
-    y = v;
+    if ((i & (1 << B)) || (i & CM) != CM) continue;
+    const int j = i | (1 << B);
+    const float2 x = a[i], y = a[j];
+    const float2 sx = swap_ri(x), sy = swap_ri(y);
+    float2 ti = __fmul2_rn(p0.p, x), tj = __fmul2_rn(p2.p, x);
+    ti = __ffma2_rn(p0.q, sx, ti);
+    tj = __ffma2_rn(p2.q, sx, tj);
+    ti = __ffma2_rn(p1.p, y, ti);
+    tj = __ffma2_rn(p3.p, y, tj);
+    a[i] = __ffma2_rn(p1.q, sy, ti);
+    a[j] = __ffma2_rn(p3.q, sy, tj);
   }
 }
 
-// dense 2x2 with controls (generic: per-amplitude select)
-template <typename C, int NA, int B>
-__device__ __forceinline__ void rb_u1_ctrl(C (&a)[NA], C m0, C m1, C m2, C m3, bool tc, uint32_t creg) {
+// The dense 2x2 on the pairs whose register bits CM (controls) are set.  FEW:
+// complex128 at 128 registers has no room for the entries, and the spills land on
+// every instruction of the stage loop: it reads them again for every pair
+// (volatile, or the compiler would keep them).
+template <typename Real, typename C, int NA, int B, int CM, bool FEW>
+__device__ __forceinline__ void rb_u1_at(C (&a)[NA], const Real* mp) {
+  if constexpr (FEW) {
+    const volatile Real* m = mp;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      if ((i & (1 << B)) || (i & CM) != CM) continue;
+      C &x = a[i], &y = a[i | (1 << B)];
+      C u, v;
+      { const Real r = m[0], s = m[1]; u.x = r * x.x - s * x.y; u.y = r * x.y + s * x.x; }
+      { const Real r = m[2], s = m[3]; u.x += r * y.x - s * y.y; u.y += r * y.y + s * y.x; }
+      { const Real r = m[4], s = m[5]; v.x = r * x.x - s * x.y; v.y = r * x.y + s * x.x; }
+      { const Real r = m[6], s = m[7]; v.x += r * y.x - s * y.y; v.y += r * y.y + s * y.x; }
+      x = u;
+      y = v;
+    }
+  } else {
+    C m0, m1, m2, m3;
+    ldc2<Real>(mp, m0, m1);
+    ldc2<Real>(mp + 4, m2, m3);
+    if constexpr (sizeof(Real) == 4) {
+      rb_u1<NA, B, CM>(a, m0, m1, m2, m3);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NA; ++i) {
+        if ((i & (1 << B)) || (i & CM) != CM) continue;
+        C &x = a[i], &y = a[i | (1 << B)];
+        const C u = cmac2(m0, x, m1, y);
+        y = cmac2(m2, x, m3, y);
+        x = u;
+      }
+    }
+  }
+}
+
+// The same with its control a run-time value: selects per amplitude.
+template <typename Real, typename C, int NA, int B>
+__device__ __forceinline__ void rb_u1_ctrl(C (&a)[NA], const Real* mp, bool tc, uint32_t creg) {
+  C m0, m1, m2, m3;
+  ldc2<Real>(mp, m0, m1);
+  ldc2<Real>(mp + 4, m2, m3);
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
     if (i & (1 << B)) continue;
@@ -295,7 +306,7 @@ __device__ __forceinline__ void rb_turn1(C (&a)[NA], C p0, C p1) {
 
 // dense 4x4 on register bits (B0 = sub-index bit 0, B1 = bit 1); matrix rows
 // are read from the op record (L1-resident) per quad to keep registers free.
-template <typename Real, typename C, int NA, int B0, int B1>
+template <typename Real, typename C, int NA, int B0, int B1, bool FEW>
 __device__ __forceinline__ void rb_u2(C (&a)[NA], const Real* __restrict__ mp, bool tc, uint32_t creg) {
   constexpr int M0 = 1 << B0, M1 = 1 << B1;
 #pragma unroll
@@ -304,7 +315,7 @@ __device__ __forceinline__ void rb_u2(C (&a)[NA], const Real* __restrict__ mp, b
     const bool cond = tc && ((uint32_t(i) & creg) == creg);
     const C x0 = a[i], x1 = a[i | M0], x2 = a[i | M1], x3 = a[i | M0 | M1];
     C y[4];
-    if constexpr (sizeof(Real) == 4) {
+    if constexpr (!FEW) {
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         C m[4];
@@ -313,7 +324,7 @@ __device__ __forceinline__ void rb_u2(C (&a)[NA], const Real* __restrict__ mp, b
         y[r] = cmac4(m, x0, x1, x2, x3);
       }
     } else {
-      // one entry at a time: the 128-register build has no room for a row
+      // one entry at a time: no room for a row
       auto mac = [&](int k, const C& x, C& acc) {
         const volatile Real* m = mp + 2 * k;  // read again per quad, not kept
         const Real r = m[0], s = m[1];
@@ -352,10 +363,10 @@ __device__ __forceinline__ void rb_sw(C (&a)[NA], bool tc, uint32_t creg) {
 // ---- dispatch helpers ------------------------------------------------------
 #define NQ_REG_CASES(M, ...) M(0, __VA_ARGS__) M(1, __VA_ARGS__) M(2, __VA_ARGS__) M(3, __VA_ARGS__) M(4, __VA_ARGS__)
 
-template <typename Real, typename C, int NA, int NRB, int B0>
+template <typename Real, typename C, int NA, int NRB, int B0, bool FEW>
 __device__ __forceinline__ void dispatch_u2_b(C (&a)[NA], int b1, const Real* mp, bool tc, uint32_t creg) {
   switch (b1) {
-#define NQ_U2B(V) case V: if constexpr (V < NRB && V != B0) rb_u2<Real, C, NA, B0, V>(a, mp, tc, creg); break;
+#define NQ_U2B(V) case V: if constexpr (V < NRB && V != B0) rb_u2<Real, C, NA, B0, V, FEW>(a, mp, tc, creg); break;
     NQ_U2B(0) NQ_U2B(1) NQ_U2B(2) NQ_U2B(3) NQ_U2B(4)
 #undef NQ_U2B
     default: break;
@@ -372,23 +383,40 @@ __device__ __forceinline__ void dispatch_sw_b(C (&a)[NA], int b1, bool tc, uint3
   }
 }
 
-// Ops a stage program holds as TileOp records: 1q gates with register controls,
-// X with register controls in the middle of a stage, SWAP and 4x4 matrices.
-template <typename Real, int NA, int NRB>
-__device__ __forceinline__ void apply_record(typename Tr<Real>::C (&a)[NA], const TileOp<Real>* op, uint32_t vbase) {
+// The other ops: 1q gates with register controls, X with register controls in
+// the middle of a stage, SWAP and 4x4 matrices.  Their fields come in the header
+// (warp-uniform, as the code): a record of its own behind it cost a second
+// dependent read per op and 160 bytes of a program that shared memory may not hold
+// (96 controlled unitaries on 8 qubits, complex64: 73 us, now 61).
+template <typename Real, int NA, int NRB, bool FEW>
+__device__ __forceinline__ void apply_op(typename Tr<Real>::C (&a)[NA], uint32_t kind, uint32_t fields, uint32_t cnr,
+                                         const Real* mp, uint32_t vbase) {
   using C = typename Tr<Real>::C;
-  const uint32_t rb0 = op->rb0, rb1 = op->rb1, creg = op->creg, cnr = op->cnr;
+  const uint32_t rb0 = fields & 0xFFu, rb1 = (fields >> 8) & 0xFFu, creg = fields >> 16;
   const bool tc = (vbase & cnr) == cnr;
-  const Real* mp = op->m;
-  switch (op->kind) {
+  switch (kind) {
     case OP_U1: {
-      C m0, m1, m2, m3;
-      ldc2<Real>(mp, m0, m1);
-      ldc2<Real>(mp + 4, m2, m3);
-      switch (rb0) {
-#define NQ_U1C(B, _) case B: if constexpr (B < NRB) rb_u1_ctrl<C, NA, B>(a, m0, m1, m2, m3, tc, creg); break;
+      if constexpr (FEW) {  // four variants per bit would spill 44 bytes: one-qubit gates on 23 qubits 666 against 613 us
+        switch (rb0) {
+#define NQ_U1C(B, _) case B: if constexpr (B < NRB) rb_u1_ctrl<Real, C, NA, B>(a, mp, tc, creg); break;
+          NQ_REG_CASES(NQ_U1C, 0)
+#undef NQ_U1C
+          default: break;
+        }
+        break;
+      }
+      // one register control (no gate has two on a dense target): only its half
+      // of the pairs (8-qubit complex64 controlled unitaries 69 -> 61 us)
+      if (!tc) break;
+      switch (rb0 << 5 | creg) {
+#define NQ_U1V(B, V) \
+        case B << 5 | 1 << V: \
+          if constexpr (B < NRB && V < NRB && B != V) rb_u1_at<Real, C, NA, B, 1 << V, FEW>(a, mp); \
+          break;
+#define NQ_U1C(B, _) NQ_U1V(B, 0) NQ_U1V(B, 1) NQ_U1V(B, 2) NQ_U1V(B, 3) NQ_U1V(B, 4)
         NQ_REG_CASES(NQ_U1C, 0)
 #undef NQ_U1C
+#undef NQ_U1V
         default: break;
       }
       break;
@@ -417,7 +445,7 @@ __device__ __forceinline__ void apply_record(typename Tr<Real>::C (&a)[NA], cons
     }
     case OP_U2: {
       switch (rb0) {
-#define NQ_U2A(B, _) case B: if constexpr (B < NRB) dispatch_u2_b<Real, C, NA, NRB, B>(a, rb1, mp, tc, creg); break;
+#define NQ_U2A(B, _) case B: if constexpr (B < NRB) dispatch_u2_b<Real, C, NA, NRB, B, FEW>(a, rb1, mp, tc, creg); break;
         NQ_REG_CASES(NQ_U2A, 0)
 #undef NQ_U2A
         default: break;
@@ -501,7 +529,7 @@ __device__ __forceinline__ void rotate_bits(typename Tr<Real>::C (&a)[NA], uint3
 // vbase = virtual index of register amplitude 0 (register bits are zero in it).
 // Whole warps run it: the headers are made warp-uniform values, so that the
 // dispatch compiles to uniform branches.
-template <typename Real, int NA, int NRB>
+template <typename Real, int NA, int NRB, bool FEW>
 __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], const uint4* p,
                                                  const uint4* const end, uint32_t vbase) {
   using C = typename Tr<Real>::C;
@@ -608,16 +636,7 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
 #define NQ_B(B, _) \
         case B: \
           if constexpr (B < NRB) { \
-            if (tc) { \
-              if constexpr (F32) { \
-                C m0, m1, m2, m3; \
-                ldc2<Real>(m, m0, m1); \
-                ldc2<Real>(m + 4, m2, m3); \
-                rb_u1<C, NA, B>(a, m0, m1, m2, m3); \
-              } else { \
-                rb_u1_reload<Real, C, NA, B>(a, m); \
-              } \
-            } \
+            if (tc) rb_u1_at<Real, C, NA, B, 0, FEW>(a, m); \
           } \
           break;
         NQ_REG_CASES(NQ_B, 0)
@@ -625,7 +644,7 @@ __device__ __forceinline__ void apply_stage_prog(typename Tr<Real>::C (&a)[NA], 
         default: break;
       }
     } else {
-      apply_record<Real, NA, NRB>(a, reinterpret_cast<const TileOp<Real>*>(q), vbase);
+      apply_op<Real, NA, NRB, FEW>(a, arg, __shfl_sync(0xffffffffu, h.y, 0), h.z, reinterpret_cast<const Real*>(q), vbase);
     }
   }
 }
@@ -730,8 +749,8 @@ __device__ __forceinline__ void load_pass_prog(const PassRec& P, const uint4* __
 // Every thread of the CTA must call it (it contains block barriers); warps
 // beyond nvec/16 threads only take part in them, and in a warp that is only partly
 // needed the other lanes run along on an earlier thread's amplitudes without
-// writing.
-template <typename Real>
+// writing.  FEW: complex128 with too few registers to keep matrices in (rb_u1_at).
+template <typename Real, bool FEW>
 __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict__ sv, const PassRec& P,
                                                 const uint32_t* __restrict__ tabs,
                                                 const uint4* prog, uint32_t ext) {
@@ -763,7 +782,7 @@ __device__ __forceinline__ void run_tile_stages(typename Tr<Real>::V* __restrict
         unpack_vec<Real>(sv[slot], a + r * APV);
       }
       const uint32_t vbase = (ub << VB) | ext;
-      apply_stage_prog<Real, NA, NRB>(a, prog + Tb[StageTab::OB], prog + min(Tb[StageTab::OE], words), vbase);
+      apply_stage_prog<Real, NA, NRB, FEW>(a, prog + Tb[StageTab::OB], prog + min(Tb[StageTab::OE], words), vbase);
       int wtid = threadIdx.x;  // read again: no register held across the program
       asm volatile("" : "+r"(wtid));
       if (uint32_t(wtid) < active_threads) {

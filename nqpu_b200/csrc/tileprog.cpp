@@ -498,8 +498,11 @@ class StageCompiler {
       W_.reals(v, 8);
       W_.end();
     } else if (I.kind == Item::RECORD) {
-      W_.header(TC_LEG, 0);
-      W_.bytes(&enc_[I.op], sizeof(TileOp<Real>));
+      const TileOp<Real>& t = enc_[I.op];
+      W_.header(TC_OP, t.kind, uint32_t(t.rb0) | uint32_t(t.rb1) << 8 | uint32_t(t.creg) << 16);
+      W_.head().w[2] = t.cnr;
+      const size_t entries = t.kind == OP_U2 ? 16 : t.kind == OP_U1 ? 4 : 0;
+      W_.bytes(t.m, 2 * sizeof(Real) * entries);
       W_.end();
     }
   }

@@ -35,7 +35,9 @@
 //              << 16; constant parts in header.z, .w (complex64) or two words
 //   SL A       sign flips: header.y = masks, header.z = constant parity; four
 //              masks per word
-//   LEG        any other op: its TileOp record follows
+//   OP A       any other op of kind A: header.y = register target bits, the second
+//              in the second byte, and register controls in the third, header.z =
+//              its controls elsewhere; the matrix of a 1q or 2q gate follows
 //
 // Why a program and not the ops themselves: the tile kernels are bound by
 // instructions (every one costs a warp about seven cycles at any occupancy the
@@ -74,7 +76,7 @@ struct StageTab {
 };
 static_assert(StageTab::SH + 16 <= kStageTabWords && kStageTabWords % 4 == 0, "stage table layout");
 
-enum TileCode : uint32_t { TC_R, TC_X, TC_TS, TC_T, TC_PS, TC_PH, TC_PU, TC_SG, TC_SL, TC_D, TC_G, TC_LEG };
+enum TileCode : uint32_t { TC_R, TC_X, TC_TS, TC_T, TC_PS, TC_PH, TC_PU, TC_SG, TC_SL, TC_D, TC_G, TC_OP };
 
 // The op list with every complex 2x2 reduced to rotation x phase where a later 2x2
 // on its qubit can take the rest: a phase passes through controls and diagonal

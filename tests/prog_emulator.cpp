@@ -127,7 +127,13 @@ int run_words(const ProgWord* p, const ProgWord* end, std::vector<cd>& a, uint32
       for (uint32_t i = 0; i < a.size(); ++i) a[i] *= (i & b) ? d1 : d0;
     } else {
       TileOp<Real> t;
-      std::memcpy(&t, q, sizeof(t));
+      t.kind = uint8_t(arg);
+      t.rb0 = uint8_t(h.w[1]);
+      t.rb1 = uint8_t(h.w[1] >> 8);
+      t.creg = uint8_t(h.w[1] >> 16);
+      t.cnr = h.w[2];
+      if (size_t(len) * 16 != 16 + 2 * sizeof(Real) * (arg == OP_U2 ? 16 : arg == OP_U1 ? 4 : 0)) return -5;
+      std::memcpy(t.m, q, size_t(len - 1) * 16);
       record(F32 ? reinterpret_cast<TileOp<float>*>(&t) : nullptr, F32 ? nullptr : reinterpret_cast<TileOp<double>*>(&t),
              a, vbase);
     }
