@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <vector>
 #include "planner.h"
 #include "sv_types.h"
@@ -33,7 +34,9 @@ void tile_config_set(DType dt, int minb);
 int tile_config_get(DType dt);
 int tile_config_raw(DType dt);
 // Tiled plan of the tile size in force for the dtype.
-bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err);
+// (`enough`: asked with the first plan, true spares the search for a better one)
+bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
+                         const std::function<bool(const TilePlan&)>& enough = nullptr);
 // One pass; d_prog is the plan's program table in device memory.
 cudaError_t launch_tile_pass(DType dt, void* amp, const PassRec& host_pass, const ProgWord* d_prog,
                              cudaStream_t stream, int num_sms);

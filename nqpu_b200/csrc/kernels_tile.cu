@@ -273,9 +273,11 @@ constexpr int kWideTileMinQubits = 22;
 // estimation 7 instead of 10 passes, 7.5 against 8.3 ms; 25-qubit Ising
 // evolution 7 instead of 9, 3.35 against 3.53 ms; a 26-qubit brickwork, 13
 // instead of 15, would lose 2.5 %).
-bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err) {
+bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
+                         const std::function<bool(const TilePlan&)>& enough) {
   if (!build_tile_plan(ops, n, dt, tile_kmax_for(dt), out, err)) return false;
   if (dt != DType::C64 || tile_config_raw(dt) != 0 || n < kWideTileMinQubits || out->passes.size() < 2) return true;
+  if (enough && enough(*out)) return true;
   TilePlan wide;
   if (build_tile_plan(ops, n, dt, 13, &wide, err) && 5 * wide.passes.size() <= 4 * out->passes.size())
     *out = std::move(wide);
