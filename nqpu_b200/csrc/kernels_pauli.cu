@@ -20,7 +20,8 @@
 // all but the first of them find the chunk in L2.  FP64 conversion (two per
 // complex64 amplitude and set) comes second.  Before, each string was a launch
 // of its own that read the state with 4-byte loads (and its partner amplitudes
-// again) and ended in a host synchronisation.
+// again) and ended in a host synchronisation.  Measured: the 24-qubit Ising
+// Hamiltonian (47 strings, complex64) 3140 -> 190 us.
 #include "reduce_device.cuh"
 
 namespace nqpu {

@@ -43,7 +43,8 @@ cudaError_t launch_sum_rows(const double* part, int nvals, int nblk, double* out
 // operations per 128-bit vector here.  The earlier form took 22 (a compensated
 // add per vector bit and vector), wrote one total per 4096 vectors and folded
 // those in one block, which alone cost about 30 us of the 38 us of a 10-qubit
-// call.
+// call.  Measured (a call): 10 qubits complex64 37 -> 18 us, 20 qubits complex128
+// 50 -> 28, 25 qubits complex64 (256 MB, 41 us at the copy rate) 98 -> 64.
 template <typename Real>
 __global__ void __launch_bounds__(kRedThreads)
     k_zsums(const Real* __restrict__ amp, int n, uint64_t nchunks, double* __restrict__ part,
@@ -162,6 +163,8 @@ __device__ __forceinline__ void load_pair(const double* p, uint64_t pair, double
 // Bound: HBM (both states are read once).  Four pairs of amplitudes per state
 // in flight per thread as 128-bit loads; the eight products of a step are
 // summed plainly and go through the compensated accumulators as one value.
+// Measured (a call): 25 qubits complex64 (512 MB) 111 -> 100 us, 20 qubits
+// complex128 36 -> 26, 10 qubits 24 -> 17.
 template <typename RA, typename RB>
 __global__ void __launch_bounds__(kRedThreads)
     k_inner(const RA* __restrict__ a, const RB* __restrict__ b, uint64_t npairs,
@@ -373,7 +376,9 @@ __global__ void __launch_bounds__(1024)
 // loads 8 consecutive vectors at once, sums its probabilities serially, and the
 // warp scans the 32 lane totals; the lane whose range holds r then picks the
 // amplitude from its own prefix.  A segment is 8 (complex64) or 16 (complex128)
-// dependent steps instead of 128 of one amplitude per lane.
+// dependent steps instead of 128 of one amplitude per lane.  Measured (1024
+// shots, the whole call): 25 qubits complex64 202 -> 97 us, 20 qubits complex128
+// 99 -> 59, 10 qubits 56 -> 44.
 template <typename Real>
 __global__ void __launch_bounds__(256, 2)
     k_sample(const Real* __restrict__ amp, uint64_t dim, int segbits, uint64_t nseg,

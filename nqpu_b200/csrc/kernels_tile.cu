@@ -160,10 +160,12 @@ static size_t tile_smem_max(int minb, int share_of) {
 //      the price of more passes;
 //   0: not set: chosen per plan and launch.
 //     complex64: 4, or 2 for a plan on 13-bit tiles (build_tile_plan_for).
-//     complex128: 1 while there is at most one tile per SM (no spills at 218
-//     registers: a 13-qubit ansatz takes 123 us against 134), else 2 (four warps
-//     per scheduler instead of two hide the dependency waits: 25-qubit ansatz
-//     6.6 against 9.1 ms, 20-qubit brickwork 618 against 718 us).
+//     complex128: 1 while there is at most one tile per SM (no spills, matrices
+//     in registers: a 13-qubit ansatz takes 72 us against 74; 8 qubits of 4x4s 95
+//     against 122), else 2 (four warps per scheduler instead of two hide the
+//     dependency waits: 25-qubit ansatz of 8 layers 5.1 against 6.6 ms, 20-qubit
+//     brickwork 383 against 461 us; 4 takes 4.7 ms and 389 us, with 12 and 21
+//     passes for 10 and 14).
 static int g_tile_minb[2] = {0, 0};
 
 void tile_config_set(DType dt, int minb) {
