@@ -270,18 +270,20 @@ static int tile_kmax_for(DType dt) {
 constexpr int kWideTileMinQubits = 22;
 
 // Complex64 tiles of 2^12 amplitudes are the better ones per pass (four CTAs of
-// 128 threads against two of 256: 3 % on a 24-qubit brickwork of 13 / 12 passes),
-// 2^13 save passes: taken when they save at least a fifth (27-qubit phase
-// estimation 7 instead of 10 passes, 7.5 against 8.3 ms; 25-qubit Ising
-// evolution 7 instead of 9, 3.35 against 3.53 ms; a 26-qubit brickwork, 13
-// instead of 15, would lose 2.5 %).
+// 128 threads against two of 256: 24-qubit brickwork 574 against 631 us on 4 passes
+// either way), 2^13 save passes.  Taken when they save at least a fifth of the
+// passes and stages too: 27-qubit phase estimation (7 passes and 19 stages instead
+// of 10 and 22) 5.55 against 7.48 ms.  With the passes alone fewer they lose:
+// 25-qubit Ising evolution of 10 steps (12 and 40 instead of 15 and 38) 3.30 against
+// 3.17 ms, of 5 steps (6 and 21 instead of 8 and 20) 1.70 against 1.54.
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>& enough) {
   if (!build_tile_plan(ops, n, dt, tile_kmax_for(dt), out, err)) return false;
   if (dt != DType::C64 || tile_config_raw(dt) != 0 || n < kWideTileMinQubits || out->passes.size() < 2) return true;
   if (enough && enough(*out)) return true;
   TilePlan wide;
-  if (build_tile_plan(ops, n, dt, 13, &wide, err) && 5 * wide.passes.size() <= 4 * out->passes.size())
+  if (build_tile_plan(ops, n, dt, 13, &wide, err) && 5 * wide.passes.size() <= 4 * out->passes.size() &&
+      wide.stats.stages < out->stats.stages)
     *out = std::move(wide);
   return true;
 }
