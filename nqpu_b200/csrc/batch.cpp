@@ -79,16 +79,8 @@ static void batch_release(BatchImpl* b) {
 }
 
 template <typename T>
-static cudaError_t upload(T** d, const T* h, size_t count) {
-  const size_t bytes = std::max<size_t>(1, count) * sizeof(T);
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(d), bytes);
-  if (e != cudaSuccess) return e;
-  if (count) e = cudaMemcpy(*d, h, count * sizeof(T), cudaMemcpyHostToDevice);
-  return e;
-}
-template <typename T>
-static cudaError_t upload(T** d, const std::vector<T>& h) {
-  return upload(d, h.data(), h.size());
+static cudaError_t upload(T** d, const std::vector<T>& h, cudaStream_t st) {
+  return upload_table(reinterpret_cast<void**>(d), h.data(), h.size() * sizeof(T), st);
 }
 
 // Host staging of the batch tables: one pinned buffer per process, grown on
@@ -261,8 +253,8 @@ static cudaError_t batch_build(BatchImpl* b) {
   b->prep_us[1] = since_us(clk);
   cudaError_t e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_arena), std::max<size_t>(16, b->arena_bytes))) != cudaSuccess) return e;
-  if ((e = upload(&b->d_circs, circs)) != cudaSuccess) return e;
-  if ((e = upload(&b->d_tasks, tasks)) != cudaSuccess) return e;
+  if ((e = upload(&b->d_circs, circs, b->stream)) != cudaSuccess) return e;
+  if ((e = upload(&b->d_tasks, tasks, b->stream)) != cudaSuccess) return e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_tables), table_bytes)) != cudaSuccess) return e;
   b->d_passes = reinterpret_cast<PassRec*>(b->d_tables);
   b->d_prog = reinterpret_cast<ProgWord*>(b->d_tables + off_o);

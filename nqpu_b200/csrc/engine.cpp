@@ -46,6 +46,13 @@ int device_sms() {
   }, 148);
 }
 
+cudaError_t upload_table(void** dev, const void* host, size_t bytes, cudaStream_t st) {
+  cudaError_t e = cudaMalloc(dev, std::max<size_t>(16, bytes));
+  if (e != cudaSuccess || bytes == 0) return e;
+  e = cudaMemcpyAsync(*dev, host, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 StateImpl* state_new(uint32_t n, DType dt) {
   if (!device_ready()) return nullptr;
   auto* s = new (std::nothrow) StateImpl();
@@ -369,7 +376,10 @@ std::vector<Segment> circuit_segments(const std::vector<GateRec>& gates) {
   return segs;
 }
 
-static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DType dt, int mode, DevicePlan* p) {
+// The segment's plan; the tables of the fused and tensor modes are uploaded on `st`
+// (those of the tiled mode by the caller; without a stream no mode uploads).
+static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DType dt, int mode, cudaStream_t st,
+                      DevicePlan* p) {
   p->ops = lower_circuit(std::vector<GateRec>(c->gates.begin() + long(seg.begin), c->gates.begin() + long(seg.end)));
   p->stats = PlanStats{};
   if (mode == NQPU_MODE_TILED && int(n) >= tile_min_qubits(dt)) {
@@ -381,9 +391,9 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
     p->stats = p->tile.stats;
   } else if (mode == NQPU_MODE_FUSED) {
     p->stats.ops = p->ops.size();
-    return fused_plan_build(p->ops, int(n), dt, &p->fused, &p->stats);
+    return fused_plan_build(p->ops, int(n), dt, st, &p->fused, &p->stats);
   } else if (mode == NQPU_MODE_TENSOR) {
-    return tc_plan_build(p->ops, int(n), dt, &p->tc, &p->stats);
+    return tc_plan_build(p->ops, int(n), dt, st, &p->tc, &p->stats);
   } else {
     p->stats.passes = p->ops.size();
     p->stats.ops = p->ops.size();
@@ -468,7 +478,7 @@ bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, Pl
                                               : tc_plan_stats(p.ops, int(n), dt, &st);
       if (!ok) return false;
     } else {
-      if (!plan_host(c, seg, n, dt, mode, &p)) return false;
+      if (!plan_host(c, seg, n, dt, mode, nullptr, &p)) return false;
       st = p.stats;
     }
     out->passes += st.passes;
@@ -477,18 +487,6 @@ bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, Pl
     out->upload_bytes += st.upload_bytes;
   }
   return true;
-}
-
-// The copy is ordered on the stream the plan runs on first and has landed when
-// this returns, so every stream may run the plan afterwards (a plain cudaMemcpy
-// of pageable memory may return before its data reaches the device, and the
-// states' non-blocking streams do not wait for the default stream).
-static cudaError_t upload_tile(DevicePlan* p, cudaStream_t st) {
-  const size_t bytes = p->tile.prog.size() * sizeof(ProgWord);
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p->d_prog), std::max<size_t>(16, bytes));
-  if (e != cudaSuccess || bytes == 0) return e;
-  e = cudaMemcpyAsync(p->d_prog, p->tile.prog.data(), bytes, cudaMemcpyHostToDevice, st);
-  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
 static cudaError_t mark(std::vector<cudaEvent_t>* ev, cudaStream_t st) {
@@ -557,13 +555,14 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   }
   if (!p) {
     p = new DevicePlan();
-    if (!plan_host(c, seg, s->n, s->dt, effective, p)) {
+    if (!plan_host(c, seg, s->n, s->dt, effective, s->stream, p)) {
       plan_free(p);
       p = nullptr;
       return cudaErrorInvalidValue;
     }
     if (effective == NQPU_MODE_TILED) {
-      cudaError_t e = upload_tile(p, s->stream);
+      const std::vector<ProgWord>& prog = p->tile.prog;
+      cudaError_t e = upload_table(reinterpret_cast<void**>(&p->d_prog), prog.data(), prog.size() * sizeof(ProgWord), s->stream);
       if (e != cudaSuccess) {
         plan_free(p);
         p = nullptr;

@@ -50,6 +50,14 @@ struct StateImpl {
   bool next_sweep() { return sweep = !sweep; }
 };
 
+// Allocate *dev and copy a plan's table into it.  The copy is ordered on `st`, the
+// stream the plan runs on first, and has landed when this returns, so every
+// stream may run the plan afterwards.  (A plain cudaMemcpy of pageable memory may
+// return before its data reaches the device, and neither the states' nor the
+// batch's non-blocking streams wait for the default stream it is ordered on: a
+// first run could read an unwritten table, whose qubit positions are addresses.)
+cudaError_t upload_table(void** dev, const void* host, size_t bytes, cudaStream_t st);
+
 StateImpl* state_new(uint32_t n, DType dt);
 void state_free(StateImpl* s);
 // The state's run scratch with room for `doubles` norm partials (grown on

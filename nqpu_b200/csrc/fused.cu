@@ -531,7 +531,7 @@ bool fused_plan_stats(const std::vector<Op>& ops, int n, DType dt, PlanStats* st
   return true;
 }
 
-bool fused_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, PlanStats* stats) {
+bool fused_plan_build(const std::vector<Op>& ops, int n, DType dt, cudaStream_t st, void** plan, PlanStats* stats) {
   *plan = nullptr;
   // complex64 only; 12 qubits minimum (5 fused + 7 group bits per 128-row tile)
   if (dt != DType::C64 || n < 12) return false;
@@ -544,8 +544,8 @@ bool fused_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, 
     real_embedding(p->gates[i], host.data() + i * 8192, host.data() + i * 8192 + 4096);
     p->args.push_back(make_args(p->gates[i], n));
   }
-  bool ok = cudaMalloc(reinterpret_cast<void**>(&p->d_bmats), host.size() * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMemcpy(p->d_bmats, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess;
+  const bool ok = upload_table(reinterpret_cast<void**>(&p->d_bmats), host.data(), host.size() * sizeof(float), st) ==
+                  cudaSuccess;
   p->norm_slots = device_sms() * kFusedCtasPerSm;
   if (!ok) {
     fused_plan_free(p);

@@ -7,7 +7,8 @@
 
 namespace nqpu {
 struct StateImpl;
-bool fused_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, PlanStats* stats);
+// Plan and upload (ordered on `st`, landed on return); false for complex128 or n < 12.
+bool fused_plan_build(const std::vector<Op>& ops, int n, DType dt, cudaStream_t st, void** plan, PlanStats* stats);
 bool fused_plan_stats(const std::vector<Op>& ops, int n, DType dt, PlanStats* stats);
 void fused_plan_free(void* plan);
 // Queue the plan's launches on the state's stream; its norm partials and

@@ -637,7 +637,7 @@ struct TcPlanImpl {
   uint16_t* d_bmats = nullptr;
 };
 
-bool tc_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, PlanStats* stats) {
+bool tc_plan_build(const std::vector<Op>& ops, int n, DType dt, cudaStream_t st, void** plan, PlanStats* stats) {
   *plan = nullptr;
   if (dt != DType::C64) return false;
   auto* p = new TcPlanImpl();
@@ -651,15 +651,10 @@ bool tc_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, Pla
     p->bmat_off.push_back(off);
     off += size_t(P.m) * kTcBmatHalves;
   }
-  const size_t np = std::max<size_t>(1, p->plan.passes.size());
-  bool ok = cudaMalloc(reinterpret_cast<void**>(&p->d_passes), np * sizeof(TcPassRec)) == cudaSuccess;
-  ok = ok && cudaMalloc(reinterpret_cast<void**>(&p->d_bmats), std::max<size_t>(8, off) * sizeof(uint16_t)) ==
-                 cudaSuccess;
-  if (ok && !p->plan.passes.empty())
-    ok = cudaMemcpy(p->d_passes, p->plan.passes.data(), p->plan.passes.size() * sizeof(TcPassRec),
-                    cudaMemcpyHostToDevice) == cudaSuccess;
-  if (ok && off)
-    ok = cudaMemcpy(p->d_bmats, p->plan.bmats.data(), off * sizeof(uint16_t), cudaMemcpyHostToDevice) == cudaSuccess;
+  const bool ok = upload_table(reinterpret_cast<void**>(&p->d_passes), p->plan.passes.data(),
+                               p->plan.passes.size() * sizeof(TcPassRec), st) == cudaSuccess &&
+                  upload_table(reinterpret_cast<void**>(&p->d_bmats), p->plan.bmats.data(), off * sizeof(uint16_t),
+                               st) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     tc_plan_free(p);

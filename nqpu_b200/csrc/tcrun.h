@@ -7,8 +7,9 @@
 
 namespace nqpu {
 struct StateImpl;
-// Plan (host, tcplan.cpp) and upload; false for complex128 or n < 12.
-bool tc_plan_build(const std::vector<Op>& ops, int n, DType dt, void** plan, PlanStats* stats);
+// Plan (host, tcplan.cpp) and upload (ordered on `st`, landed on return); false for
+// complex128 or n < 12.
+bool tc_plan_build(const std::vector<Op>& ops, int n, DType dt, cudaStream_t st, void** plan, PlanStats* stats);
 bool tc_plan_stats(const std::vector<Op>& ops, int n, DType dt, PlanStats* stats);
 void tc_plan_free(void* plan);
 // Queue every pass of the plan on the state's stream (one launch per pass).

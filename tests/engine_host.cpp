@@ -1,0 +1,127 @@
+// Test infrastructure: the engine's host code (engine.cpp) on a CUDA runtime of
+// this file's own, without a GPU.  Device memory is host memory; work queued on a
+// stream runs as late as the runtime allows, when the stream is waited for.  The
+// kernels' launchers only record what the checks below ask about.
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "engine.h"
+#include "fused.h"
+#include "tcrun.h"
+
+using namespace nqpu;
+
+namespace {
+std::map<cudaStream_t, std::deque<std::function<void()>>> g_queue;
+int g_fail_malloc = -1;  // the allocation that fails, counted from now on
+void run(cudaStream_t st) {
+  auto& q = g_queue[st];
+  while (!q.empty()) {
+    q.front()();
+    q.pop_front();
+  }
+}
+cudaStream_t new_stream() { return reinterpret_cast<cudaStream_t>(new int(0)); }
+}  // namespace
+
+// ---- CUDA runtime -----------------------------------------------------------
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) {
+  if (g_fail_malloc >= 0 && g_fail_malloc-- == 0) return cudaErrorMemoryAllocation;
+  *p = std::calloc(1, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void** p, size_t n) { *p = std::calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = new_stream(); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { g_queue.erase(s); delete reinterpret_cast<int*>(s); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { run(s); return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() {
+  for (auto& kv : g_queue) run(kv.first);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* h, size_t n, cudaMemcpyKind, cudaStream_t s) {
+  g_queue[s].push_back([=] { std::memcpy(d, h, n); });
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* h, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, h, n, k, nullptr); }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t s) {
+  g_queue[s].push_back([=] { std::memset(d, v, n); });
+  return cudaSuccess;
+}
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t*) { return cudaErrorNotSupported; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaErrorNotSupported; }
+}
+
+// ---- launchers --------------------------------------------------------------
+namespace nqpu {
+double next_random_f64() { return 0.5; }
+size_t reduce_scratch_bytes(int) { return 4096; }
+int tile_config_raw(DType) { return 0; }
+bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
+                         const std::function<bool(const TilePlan&)>&) {
+  return build_tile_plan(ops, n, dt, 12, out, err);
+}
+cudaError_t launch_tile_pass(DType, void*, const PassRec&, const ProgWord*, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_pergate(DType, void*, int, const Op&, bool, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_set_basis(DType, void*, int, uint64_t, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_scale(DType, void*, int, double, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_collapse(DType, void*, int, int, int, double, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_measure_collapse(DType, void*, int, int, const double*, double, bool, double* result, cudaStream_t s,
+                                    int) {
+  if (result) g_queue[s].push_back([=] { result[0] = 1.0; });
+  return cudaSuccess;
+}
+cudaError_t launch_probabilities(DType, const void*, uint64_t, double*, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_convert(DType, const void*, DType, void*, uint64_t, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_zsums(DType, const void*, int, double*, double*, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_inner(DType, const void*, DType, const void*, int, double*, double*, cudaStream_t, int) {
+  return cudaSuccess;
+}
+cudaError_t launch_pauli(DType, const void*, int, uint64_t, uint64_t, uint64_t, double*, double*, cudaStream_t, int) {
+  return cudaSuccess;
+}
+void pauli_plan(const PauliString*, size_t, int, PauliPlan*, std::vector<PauliString>*) {}
+cudaError_t launch_pauli_sum(DType, const void*, int, const PauliSet*, const PauliPlan&, const PauliTerm*, double*, double*,
+                             cudaStream_t, int) {
+  return cudaSuccess;
+}
+cudaError_t launch_sample(DType, const void*, int, const double*, uint32_t, double*, uint64_t*, cudaStream_t, int) {
+  return cudaSuccess;
+}
+bool fused_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void**, PlanStats*) { return false; }
+bool fused_plan_stats(const std::vector<Op>&, int, DType, PlanStats*) { return false; }
+void fused_plan_free(void*) {}
+cudaError_t fused_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
+bool tc_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void**, PlanStats*) { return false; }
+bool tc_plan_stats(const std::vector<Op>&, int, DType, PlanStats*) { return false; }
+void tc_plan_free(void*) {}
+cudaError_t tc_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
+}  // namespace nqpu
+
+// ---- checks (0: as it should be) ---------------------------------------------
+// A plan table is in device memory when its upload returns, whatever its size.
+extern "C" int check_upload(int bytes) {
+  std::vector<unsigned char> h(size_t(bytes) + 1, 0xA5);
+  cudaStream_t st = new_stream();
+  void* d = nullptr;
+  if (upload_table(&d, h.data(), size_t(bytes), st) != cudaSuccess || !d) return 1;
+  if (std::memcmp(d, h.data(), size_t(bytes)) != 0) return 2;
+  for (auto& kv : g_queue)
+    if (!kv.second.empty()) return 3;
+  cudaFree(d);
+  cudaStreamDestroy(st);
+  return 0;
+}
