@@ -153,7 +153,10 @@ cudaError_t state_measure_all(StateImpl* s, uint32_t* outcomes) {
   static_assert(kSmallTable + 2 * size_t(kMaxQubits) <= kSmallDoubles, "room for every qubit's result");
   for (uint32_t q = 0; q < s->n; ++q) {
     const cudaError_t e = state_queue_measure(s, q, false, res + 2 * q);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(s->stream);  // the queued ones write to the staging buffer
+      return e;
+    }
   }
   const cudaError_t e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return e;
@@ -516,10 +519,16 @@ cudaError_t circuit_run(CircuitImpl* c, StateImpl* s, int mode, std::vector<cuda
     queued = 0;
     return cudaSuccess;
   };
+  // no error leaves a kernel behind that still writes there: the next call stages
+  // its own tables in the same memory
+  auto fail = [&](cudaError_t e) {
+    if (queued) drain();
+    return e;
+  };
   for (size_t si = 0; si < segs.size(); ++si) {
     const Segment& seg = segs[si];
     cudaError_t e = segment_run(c, seg, int(si), s, mode, events);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) return fail(e);
     if (seg.mid < 0) break;
     const GateRec& g = c->gates[size_t(seg.mid)];
     // OpenQASM reset: measure (one RNG draw) and flip the qubit back to |0>
@@ -528,9 +537,10 @@ cudaError_t circuit_run(CircuitImpl* c, StateImpl* s, int mode, std::vector<cuda
     double* res = nullptr;
     if (g.code == G_MEASURE && outcomes) {
       if (queued == kSlots && (e = drain()) != cudaSuccess) return e;
-      res = s->h_small + kSmallTable + 2 * queued++;
+      res = s->h_small + kSmallTable + 2 * queued;
     }
-    if ((e = state_queue_measure(s, uint32_t(g.q[0]), g.code == G_RESET, res)) != cudaSuccess) return e;
+    if ((e = state_queue_measure(s, uint32_t(g.q[0]), g.code == G_RESET, res)) != cudaSuccess) return fail(e);
+    if (res) ++queued;
   }
   if (queued) return drain();
   return cudaSuccess;

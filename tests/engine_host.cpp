@@ -20,7 +20,8 @@ using namespace nqpu;
 
 namespace {
 std::map<cudaStream_t, std::deque<std::function<void()>>> g_queue;
-int g_fail_malloc = -1;  // the allocation that fails, counted from now on
+int g_fail_malloc = -1;   // the allocation that fails, counted from now on
+int g_fail_measure = -1;  // the measurement launch that fails
 void run(cudaStream_t st) {
   auto& q = g_queue[st];
   while (!q.empty()) {
@@ -81,6 +82,7 @@ cudaError_t launch_scale(DType, void*, int, double, cudaStream_t, int) { return 
 cudaError_t launch_collapse(DType, void*, int, int, int, double, cudaStream_t, int) { return cudaSuccess; }
 cudaError_t launch_measure_collapse(DType, void*, int, int, const double*, double, bool, double* result, cudaStream_t s,
                                     int) {
+  if (g_fail_measure >= 0 && g_fail_measure-- == 0) return cudaErrorLaunchOutOfResources;
   if (result) g_queue[s].push_back([=] { result[0] = 1.0; });
   return cudaSuccess;
 }
@@ -123,5 +125,36 @@ extern "C" int check_upload(int bytes) {
     if (!kv.second.empty()) return 3;
   cudaFree(d);
   cudaStreamDestroy(st);
+  return 0;
+}
+
+static bool idle(StateImpl* s) { return g_queue[s->stream].empty(); }
+
+// H, measurement, H, measurement, H: the third segment's plan upload fails (what
+// = 0) or the second measurement's launch (1); then one of a whole register's
+// measurements (2).  Nothing may stay queued that writes to the state's buffers, and
+// the first error is what the call returns.
+extern "C" int check_measure_error(int what) {
+  StateImpl* s = state_new(6, DType::C64);
+  CircuitImpl c;
+  c.n = 6;
+  for (int i = 0; i < 5; ++i) {
+    GateRec g;
+    g.code = i % 2 ? G_MEASURE : G_H;
+    c.gates.push_back(g);
+  }
+  std::vector<uint32_t> out(6);
+  g_fail_malloc = what == 0 ? 2 : -1;
+  g_fail_measure = what == 1 ? 1 : what == 2 ? 3 : -1;
+  const cudaError_t e = what == 2 ? state_measure_all(s, out.data())
+                                  : circuit_run(&c, s, NQPU_MODE_TILED, nullptr, &out);
+  g_fail_malloc = g_fail_measure = -1;
+  if (e != (what == 0 ? cudaErrorMemoryAllocation : cudaErrorLaunchOutOfResources)) return 1;
+  if (!idle(s)) return 2;
+  // without a failure the same circuit's outcomes all arrive
+  out.clear();
+  if (circuit_run(&c, s, NQPU_MODE_TILED, nullptr, &out) != cudaSuccess || out.size() != 2) return 3;
+  if (out[0] != 1 || out[1] != 1) return 4;
+  state_free(s);
   return 0;
 }

@@ -36,3 +36,8 @@ def test_no_copy_on_the_default_stream():
     found = [f"{p.name}:{i}" for p in sorted(CSRC.iterdir()) if p.suffix in (".cu", ".cpp", ".h", ".cuh")
              for i, line in enumerate(p.read_text().splitlines(), 1) if plain.search(line.split("//")[0])]
     assert not found, found
+
+
+@pytest.mark.parametrize("what", [0, 1, 2])
+def test_no_measurement_outlives_an_error(eng, what):
+    assert eng.check_measure_error(what) == 0
