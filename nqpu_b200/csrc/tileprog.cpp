@@ -1,5 +1,6 @@
 // Compiler of the tiled passes' stage programs (encoding: tileprog.h).
 #include "tileprog.h"
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -37,7 +38,6 @@ struct Item {
   cplx m[4];                     // PHASE: m[0]; GENERIC: the matrix
   double t = 0, s = 0;           // ROT, CROSS
   size_t op = 0;                 // RECORD: index into the plan's ops
-  bool done = false;
 };
 
 // Angle in 2^-32 turns of a unit complex number.
@@ -277,41 +277,65 @@ class StageCompiler {
   // Rounds of: take every phase that no earlier open dense item blocks, then emit
   // every dense item with nothing open before it on its bits.  Phases gather
   // as long as they can, so that a layer's join in one instruction.
+  //
+  // An item waits for the last dense item before it on each of its bits and, where
+  // it is dense, for the items since then that read the bit; a round takes what
+  // waits for nothing any more, in circuit order.  So the work is linear in the
+  // items: walking all of them in every round took 4.4 s for 32000 gates on five
+  // qubits, which are one stage.
   void schedule() {
-    size_t left = items_.size();
-    while (left) {
-      uint32_t open = 0;
-      for (Item& I : items_) {
-        if (I.done) continue;
-        if (I.kind == Item::PHASE && !(I.diag & open)) {
-          pend(I.diag, I.cnr, I.m[0]);
-          I.done = true;
-          --left;
-        } else {
-          open |= I.dense;
-        }
+    const size_t n = items_.size();
+    wait_.assign(n, 0);
+    first_.assign(n, -1);
+    edges_.clear();
+    phases_.clear();
+    dense_.clear();
+    int last[kBits];
+    for (int b = 0; b < kBits; ++b) {
+      last[b] = -1;
+      readers_[b].clear();
+    }
+    auto edge = [&](int from, int to) {
+      edges_.push_back({to, first_[size_t(from)]});
+      first_[size_t(from)] = int(edges_.size()) - 1;
+      ++wait_[size_t(to)];
+    };
+    auto ready = [&](int i) { (items_[size_t(i)].kind == Item::PHASE ? phases_ : dense_).push_back(i); };
+    for (int i = 0; i < int(n); ++i) {
+      const Item& I = items_[size_t(i)];
+      for (uint32_t w = I.diag | I.dense; w; w &= w - 1)
+        if (last[ctz(w)] >= 0) edge(last[ctz(w)], i);
+      for (uint32_t w = I.dense; w; w &= w - 1) {
+        for (int r : readers_[ctz(w)]) edge(r, i);
+        readers_[ctz(w)].clear();
+        last[ctz(w)] = i;
       }
-      uint32_t dense_open = 0, diag_open = 0, bits = 0;
-      std::vector<size_t>& batch = batch_;
-      batch.clear();
-      for (size_t i = 0; i < items_.size(); ++i) {
-        const Item& I = items_[i];
-        if (I.done) continue;
-        if (I.kind != Item::PHASE && !(I.dense & (dense_open | diag_open)) && !(I.diag & dense_open)) {
-          batch.push_back(i);
-          bits |= I.dense;
-        }
-        dense_open |= I.dense;
-        diag_open |= I.diag;
+      for (uint32_t w = I.diag; w; w &= w - 1) readers_[ctz(w)].push_back(i);
+      if (wait_[size_t(i)] == 0) ready(i);
+    }
+    auto release = [&](int i) {
+      for (int e = first_[size_t(i)]; e >= 0; e = edges_[size_t(e)].next)
+        if (--wait_[size_t(edges_[size_t(e)].to)] == 0) ready(edges_[size_t(e)].to);
+    };
+    for (;;) {
+      std::sort(phases_.begin(), phases_.end());
+      for (int i : phases_) {  // frees dense items only
+        pend(items_[size_t(i)].diag, items_[size_t(i)].cnr, items_[size_t(i)].m[0]);
+        release(i);
       }
-      if (batch.empty()) break;  // only phases were left
+      phases_.clear();
+      if (dense_.empty()) break;
+      batch_.swap(dense_);
+      dense_.clear();
+      std::sort(batch_.begin(), batch_.end());
+      uint32_t bits = 0;
+      for (int i : batch_) bits |= items_[size_t(i)].dense;
       flush(bits);
       emit_rotations(Item::ROT);
       emit_rotations(Item::CROSS);
-      for (size_t i : batch) {
-        emit(items_[i]);
-        items_[i].done = true;
-        --left;
+      for (int i : batch_) {
+        emit(items_[size_t(i)]);
+        release(i);
       }
     }
   }
@@ -476,8 +500,8 @@ class StageCompiler {
   void emit_rotations(Item::Kind kind) {
     uint32_t bits = 0;
     double v[5][2] = {};
-    for (size_t i : batch_) {
-      const Item& I = items_[i];
+    for (int i : batch_) {
+      const Item& I = items_[size_t(i)];
       if (I.kind != kind) continue;
       bits |= I.dense;
       v[ctz(I.dense)][0] = I.t;
@@ -514,7 +538,13 @@ class StageCompiler {
   const std::vector<TileOp<Real>>& enc_;
   Writer W_;
   std::vector<Item> items_;
-  std::vector<size_t> batch_;
+  struct Edge {
+    int to, next;
+  };
+  std::vector<int> wait_, first_;  // per item: items it waits for; its first edge
+  std::vector<Edge> edges_;
+  std::vector<int> phases_, dense_, batch_;  // items that wait for nothing; those being emitted
+  std::vector<int> readers_[kBits];
   Phase pend_[32];
   uint32_t used_ = 0;  // pend_ entries in use
   cplx* global_ = nullptr;  // phase common to all amplitudes

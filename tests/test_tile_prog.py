@@ -92,3 +92,23 @@ def test_workloads(emu, n, c64):
         prep = [("u3", (q,), (0.3 + q, 0.2 * q, 1.0)) for q in range(n)]
         got, _ = run(emu, n, c64, prep + gates)
         check(got, prep + gates, n, c64)
+
+
+@pytest.mark.parametrize("n,dtype", [(5, "c64"), (4, "c128")])
+def test_compile_time_is_linear_in_the_gates(n, dtype):
+    # a circuit on as many qubits as a stage has register bits is one stage: 8 times the gates may take 8 times as
+    # long (64 times if every round walked all of them); a factor of 3 for noise
+    import time
+
+    from nqpu_b200.state import Circuit
+
+    def best(steps):
+        c = Circuit(n, circuits.tfim_trotter(n, steps, 1)[0])
+        times = []
+        for _ in range(3):
+            t = time.perf_counter()
+            c.plan_stats(n, dtype, "tiled")
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    assert best(2000) <= 24 * best(250)
