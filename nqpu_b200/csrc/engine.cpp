@@ -380,7 +380,8 @@ std::vector<Segment> circuit_segments(const std::vector<GateRec>& gates) {
 }
 
 // The segment's plan; the tables of the fused and tensor modes are uploaded on `st`
-// (those of the tiled mode by the caller; without a stream no mode uploads).
+// (those of the tiled mode by the caller; without a stream no mode uploads).  A
+// tiled plan made for the same ops may be in p->tile already (auto_mode_for).
 static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DType dt, int mode, cudaStream_t st,
                       DevicePlan* p) {
   p->ops = lower_circuit(std::vector<GateRec>(c->gates.begin() + long(seg.begin), c->gates.begin() + long(seg.end)));
@@ -389,7 +390,7 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
     std::string err;
     p->ops = carry_phases(std::move(p->ops));
     p->tile_cfg = tile_config_raw(dt);
-    if (!build_tile_plan_for(p->ops, int(n), dt, &p->tile, &err)) return false;
+    if (p->tile.passes.empty() && !build_tile_plan_for(p->ops, int(n), dt, &p->tile, &err)) return false;
     build_tile_prog(p->ops, &p->tile);
     p->stats = p->tile.stats;
   } else if (mode == NQPU_MODE_FUSED) {
@@ -420,7 +421,7 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
 // (30-qubit Ising evolution, 10 steps: 121 against 140 ms).  4x4 matrices and 2x2s
 // with controls run as single records, priced at the 0.30 and 0.15 they
 // measured as such.
-int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt) {
+int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt, TilePlan* plan) {
   if (dt != DType::C64 || int(n) < kTcMinQubits) return NQPU_MODE_TILED;
   PlanStats ts;
   if (!tc_plan_stats(ops, int(n), dt, &ts)) return NQPU_MODE_TILED;
@@ -450,7 +451,9 @@ int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt) {
   std::string err;
   if (!build_tile_plan_for(ops, int(n), dt, &tp, &err, [&](const TilePlan& p) { return tensor < 0.8 * tiled(p); }))
     return NQPU_MODE_TENSOR;
-  return tensor < tiled(tp) ? NQPU_MODE_TENSOR : NQPU_MODE_TILED;
+  if (tensor < tiled(tp)) return NQPU_MODE_TENSOR;
+  if (plan) *plan = std::move(tp);
+  return NQPU_MODE_TILED;
 }
 
 static std::vector<Op> segment_ops(const CircuitImpl* c, const Segment& seg) {
@@ -549,9 +552,10 @@ cudaError_t circuit_run(CircuitImpl* c, StateImpl* s, int mode, std::vector<cuda
 static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, StateImpl* s, int mode,
                                std::vector<cudaEvent_t>* events) {
   if (seg.begin == seg.end) return cudaSuccess;
+  TilePlan ready;
   if (mode == NQPU_MODE_AUTO) {
     std::pair<uint64_t, int>& am = c->auto_modes[std::make_tuple(s->n, int(s->dt), si)];
-    if (am.first != c->version + 1) am = {c->version + 1, auto_mode_for(segment_ops(c, seg), s->n, s->dt)};
+    if (am.first != c->version + 1) am = {c->version + 1, auto_mode_for(segment_ops(c, seg), s->n, s->dt, &ready)};
     mode = am.second;
   }
   const int effective = (mode == NQPU_MODE_TILED && int(s->n) < tile_min_qubits(s->dt)) ? int(NQPU_MODE_PERGATE) : mode;
@@ -565,6 +569,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   }
   if (!p) {
     p = new DevicePlan();
+    p->tile = std::move(ready);
     if (!plan_host(c, seg, s->n, s->dt, effective, s->stream, p)) {
       plan_free(p);
       p = nullptr;

@@ -133,9 +133,10 @@ cudaError_t circuit_run(CircuitImpl* c, StateImpl* s, int mode,
                         std::vector<cudaEvent_t>* events = nullptr,
                         std::vector<uint32_t>* outcomes = nullptr);
 bool circuit_plan_stats(const CircuitImpl* c, uint32_t n, DType dt, int mode, PlanStats* out);
-// The mode NQPU_MODE_AUTO runs a lowered gate run in on an n-qubit state.
-int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt);
-
-// Run a lowered op list on a state with the given mode (used by batch/server).
+// The mode NQPU_MODE_AUTO runs a lowered gate run in on an n-qubit state.  With
+// `plan`, the tiled plan that the choice was made on is left there where the tiled
+// mode won (no passes: none was needed); carry_phases changes neither kinds nor
+// qubits of the ops, so it is their plan too.
+int auto_mode_for(const std::vector<Op>& ops, uint32_t n, DType dt, TilePlan* plan = nullptr);
 
 }  // namespace nqpu

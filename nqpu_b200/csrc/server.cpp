@@ -468,7 +468,7 @@ extern "C" NqpuError nqpu_server_submit(NqpuServer* server, const NqpuCircuit* c
   r->seed = seed;
   r->large = c->n >= sv->cfg.large_qubits;
   std::vector<Op> ops = lower_circuit(c->gates);
-  if (auto_mode_for(ops, c->n, DType::C64) == NQPU_MODE_TENSOR) {
+  if (auto_mode_for(ops, c->n, DType::C64, &r->plan) == NQPU_MODE_TENSOR) {
     // the engine's own choice (NQPU_MODE_AUTO): tensor-core passes; tables =
     // pass records | B operands
     std::string err;
@@ -487,7 +487,7 @@ extern "C" NqpuError nqpu_server_submit(NqpuServer* server, const NqpuCircuit* c
   } else if (int(c->n) >= tile_min_qubits(DType::C64)) {
     std::string err;
     ops = carry_phases(std::move(ops));
-    if (!build_tile_plan_for(ops, int(c->n), DType::C64, &r->plan, &err))
+    if (r->plan.passes.empty() && !build_tile_plan_for(ops, int(c->n), DType::C64, &r->plan, &err))
       return NQPU_INVALID_PARAMETER;
     build_tile_prog(ops, &r->plan);
     r->tiled = true;

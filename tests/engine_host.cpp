@@ -22,6 +22,9 @@ namespace {
 std::map<cudaStream_t, std::deque<std::function<void()>>> g_queue;
 int g_fail_malloc = -1;   // the allocation that fails, counted from now on
 int g_fail_measure = -1;  // the measurement launch that fails
+int g_plans = 0;          // tiled plans built
+uint64_t g_tc_passes = 0;  // of the tensor plan (0: the tensor mode does not take the circuit)
+std::vector<uint32_t> g_words;  // program words of the tiled passes launched
 void run(cudaStream_t st) {
   auto& q = g_queue[st];
   while (!q.empty()) {
@@ -73,9 +76,14 @@ size_t reduce_scratch_bytes(int) { return 4096; }
 int tile_config_raw(DType) { return 0; }
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>&) {
+  ++g_plans;
   return build_tile_plan(ops, n, dt, 12, out, err);
 }
-cudaError_t launch_tile_pass(DType, void*, const PassRec&, const ProgWord*, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t launch_tile_pass(DType, void*, const PassRec& P, const ProgWord* prog, cudaStream_t, int) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(prog + P.prog_begin);
+  g_words.insert(g_words.end(), w, w + 4 * P.prog_words);
+  return cudaSuccess;
+}
 cudaError_t launch_pergate(DType, void*, int, const Op&, bool, cudaStream_t, int) { return cudaSuccess; }
 cudaError_t launch_set_basis(DType, void*, int, uint64_t, cudaStream_t, int) { return cudaSuccess; }
 cudaError_t launch_scale(DType, void*, int, double, cudaStream_t, int) { return cudaSuccess; }
@@ -108,7 +116,10 @@ bool fused_plan_stats(const std::vector<Op>&, int, DType, PlanStats*) { return f
 void fused_plan_free(void*) {}
 cudaError_t fused_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
 bool tc_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void**, PlanStats*) { return false; }
-bool tc_plan_stats(const std::vector<Op>&, int, DType, PlanStats*) { return false; }
+bool tc_plan_stats(const std::vector<Op>&, int, DType, PlanStats* st) {
+  st->passes = st->stages = g_tc_passes;
+  return g_tc_passes > 0;
+}
 void tc_plan_free(void*) {}
 cudaError_t tc_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
 }  // namespace nqpu
@@ -155,6 +166,40 @@ extern "C" int check_measure_error(int what) {
   out.clear();
   if (circuit_run(&c, s, NQPU_MODE_TILED, nullptr, &out) != cudaSuccess || out.size() != 2) return 3;
   if (out[0] != 1 || out[1] != 1) return 4;
+  state_free(s);
+  return 0;
+}
+
+// AUTO builds one tiled plan for a circuit that it runs in the tiled mode, none for
+// its second run, and the programs are the tiled mode's own.
+extern "C" int check_auto_plans_once(int n) {
+  StateImpl* s = state_new(uint32_t(n), DType::C64);
+  std::vector<GateRec> gates;
+  for (int l = 0; l < 6; ++l)
+    for (int q = 0; q < n; ++q) {
+      GateRec g;
+      g.code = G_U3;
+      g.q[0] = q;
+      g.p[0] = 0.3 + q + l, g.p[1] = 0.7 * q - l, g.p[2] = 1.1 + l * q;
+      gates.push_back(g);
+      g.code = G_CX;
+      g.nq = 2;
+      g.q[1] = (q + 1) % n;
+      gates.push_back(g);
+    }
+  CircuitImpl a, b;
+  a.n = b.n = uint32_t(n);
+  a.gates = b.gates = gates;
+  g_tc_passes = 1000;
+  g_plans = 0;
+  g_words.clear();
+  if (circuit_run(&a, s, NQPU_MODE_AUTO) != cudaSuccess || g_plans != 1 || g_words.empty()) return 1;
+  const std::vector<uint32_t> words = std::move(g_words);
+  g_words.clear();
+  if (circuit_run(&a, s, NQPU_MODE_AUTO) != cudaSuccess || g_plans != 1 || g_words != words) return 2;
+  g_words.clear();
+  if (circuit_run(&b, s, NQPU_MODE_TILED) != cudaSuccess || g_plans != 2 || g_words != words) return 3;
+  g_tc_passes = 0;
   state_free(s);
   return 0;
 }

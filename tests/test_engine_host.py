@@ -41,3 +41,8 @@ def test_no_copy_on_the_default_stream():
 @pytest.mark.parametrize("what", [0, 1, 2])
 def test_no_measurement_outlives_an_error(eng, what):
     assert eng.check_measure_error(what) == 0
+
+
+@pytest.mark.parametrize("n", [12, 17, 22])
+def test_auto_plans_a_tiled_circuit_once(eng, n):
+    assert eng.check_auto_plans_once(n) == 0
