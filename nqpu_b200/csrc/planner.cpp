@@ -259,7 +259,9 @@ static TileOp<Real> encode_op(const Op& o, const int* tile_pos, const int* reg_o
   };
   if (o.kind == OP_D1) diag(o.t0, &t.dreg0, &t.dv0);
   if (o.kind == OP_D2) { diag(o.t0, &t.dreg0, &t.dv0); diag(o.t1, &t.dreg1, &t.dv1); }
-  for (int i = 0; i < 16; ++i) {
+  // the entries the kind uses (the rest are zero in the op, too)
+  static constexpr int kEntries[] = {4, 2, 0, 16, 4, 0, 1};  // by OpKind
+  for (int i = 0; i < kEntries[o.kind]; ++i) {
     t.m[2 * i] = Real(o.m[i].real());
     t.m[2 * i + 1] = Real(o.m[i].imag());
   }
@@ -281,6 +283,9 @@ bool build_tile_plan(const std::vector<Op>& ops, int n, DType dt, int kmax, Tile
     if (err) *err = "state too small for the tiled kernel";
     return false;
   }
+  if (dt == DType::C64) out->ops_f.reserve(ops.size());
+  else out->ops_d.reserve(ops.size());
+  out->op_src.reserve(ops.size());
   const int k = std::min(kmax, n);
   const int c = std::min(k, dt == DType::C64 ? 5 : 4);
   const uint64_t all = (n >= 64) ? ~0ull : ((1ull << n) - 1);
@@ -293,7 +298,12 @@ bool build_tile_plan(const std::vector<Op>& ops, int n, DType dt, int kmax, Tile
     uint64_t Q = (n <= kmax) ? all : lowc;
     uint64_t blocked = 0, used_val = 0;
     std::vector<int> taken, rest;
-    for (int idx : remaining) {
+    for (size_t at = 0; at < remaining.size(); ++at) {
+      const int idx = remaining[at];
+      if (blocked == all) {  // nothing after this op can join the pass
+        rest.insert(rest.end(), remaining.begin() + long(at), remaining.end());
+        break;
+      }
       const Op& o = ops[idx];
       const uint64_t qm = o.qubit_mask();
       if (qm & blocked) { blocked |= qm; rest.push_back(idx); continue; }
@@ -378,20 +388,24 @@ bool build_tile_plan(const std::vector<Op>& ops, int n, DType dt, int kmax, Tile
         const int tb = tile_pos[q];
         return tb;
       };
-      for (int idx : pending) {
+      for (size_t at = 0; at < pending.size(); ++at) {
+        const int idx = pending[at];
+        if (sblocked == all) {  // nothing after this op can join the stage
+          srest.insert(srest.end(), pending.begin() + long(at), pending.end());
+          break;
+        }
         const Op& o = ops[idx];
         const uint64_t qm = o.qubit_mask();
         if (qm & sblocked) { sblocked |= qm; srest.push_back(idx); continue; }
         uint64_t need = 0;
         const uint64_t dt_ = dense_targets(o);
         bool bad = false;
-        for (int q = 0; q < n; ++q)
-          if ((dt_ >> q) & 1) {
-            const int tb = reg_tile_bit(q);
-            if (vb == 1 && tb == 0) continue;  // complex64: tile bit 0 is always in registers
-            if ((no_reg >> tb) & 1) bad = true;
-            need |= 1ull << tb;
-          }
+        for (uint64_t w = dt_; w; w &= w - 1) {
+          const int tb = reg_tile_bit(__builtin_ctzll(w));
+          if (vb == 1 && tb == 0) continue;  // complex64: tile bit 0 is always in registers
+          if ((no_reg >> tb) & 1) bad = true;
+          need |= 1ull << tb;
+        }
         const bool fits = !bad && popc(R | need) <= kRegFree;
         // deferrable permutation: X/CNOT with <= 1 control, SWAP without controls
         bool deferrable = false;

@@ -149,17 +149,25 @@ class StageCompiler {
     dense(b, 0, acc_[b]);
   }
 
+  // Magnitudes and quotients of unitaries' entries and phases.  The operands of
+  // complex64 programs are rounded to 2^-24, so hypot, the full complex division and
+  // (join_constant) an angle per table entry buy nothing there: a circuit that runs
+  // once pays for its program (17-qubit brickwork, 375 gates: build_tile_prog 165 ->
+  // 95 us; complex128 keeps them, its results are 1e-15 off).
+  static double mag(cplx z) { return kF32 ? std::sqrt(std::norm(z)) : std::abs(z); }
+  static cplx unit(cplx z) { return z / mag(z); }
+  static cplx quot(cplx z, cplx w) { return kF32 ? z * std::conj(w) / std::norm(w) : z / w; }
+
   // A 2x2 as items: phase x rotation x phase where it is unitary, else as it is.
   void dense(int b, uint32_t cnr, const cplx* m) {
     Item I;
     I.dense = 1u << b;
     I.cnr = cnr;
     const double eps = 1e-12;
-    const cplx m11 = std::abs(m[0]) > std::abs(m[1]) ? std::conj(m[0]) * det(m) : m[3];
-    const bool unitary = std::abs(std::norm(m[0]) + std::norm(m[2]) - 1.0) < eps &&
+    const bool unitary = cnr == 0 && std::abs(std::norm(m[0]) + std::norm(m[2]) - 1.0) < eps &&
                          std::abs(std::norm(m[1]) + std::norm(m[3]) - 1.0) < eps &&
-                         std::abs(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) < eps && std::abs(m11 - m[3]) < 1e-9;
-    if (!unitary || cnr != 0) {
+                         std::norm(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) < eps * eps;
+    if (!unitary) {
       I.kind = Item::GENERIC;
       for (int i = 0; i < 4; ++i) I.m[i] = m[i];
       items_.push_back(I);
@@ -175,28 +183,27 @@ class StageCompiler {
       if (I.s != 0.0) items_.push_back(I);
       return;
     }
-    const double c = std::abs(m[0]), s = std::abs(m[2]);
+    const double c = mag(m[0]), s = mag(m[2]);
     const cplx one(1.0, 0.0);
     if (s < kTiny || c < kTiny) {  // a phase, or a rotation by pi/2 with phases
-      const cplx p0 = s < kTiny ? m[0] : -m[1], p1 = s < kTiny ? m[3] / m[0] : m[2] / -m[1];
-      push_phase(0, 0, p0 / std::abs(p0));
+      const cplx p0 = s < kTiny ? m[0] : -m[1], p1 = s < kTiny ? quot(m[3], m[0]) : quot(m[2], -m[1]);
+      push_phase(0, 0, unit(p0));
       if (c < kTiny) {
         shears(0.0, 1.0, &I);
         I.kind = Item::ROT;
         items_.push_back(I);
       }
-      push_phase(1u << b, 0, clean(p1 / std::abs(p1)));
+      push_phase(1u << b, 0, clean(unit(p1)));
       return;
     }
     // e^{ia} diag(1, after) [[c, -s], [s, c]] diag(1, before)
-    const cplx a = m[0] / c;
+    const cplx a = m[0] / c, ia = std::conj(a);
     // (`before` from the larger of the entries that fix it: a small off-diagonal
     // has no precise phase, and only its product with `after` matters then)
-    cplx after = (m[2] / s) / a, before = s > c ? (-m[1] / s) / a : (m[3] / c) / a / after;
-    after /= std::abs(after);
-    before /= std::abs(before);
+    cplx after = unit((m[2] / s) * ia);
+    cplx before = unit(s > c ? (-m[1] / s) * ia : (m[3] / c) * ia * std::conj(after));
     double sn = s;
-    if (std::abs(after + one) < kTiny) {  // a rotation the other way
+    if (std::norm(after + one) < kTiny * kTiny) {  // a rotation the other way
       sn = -s;
       after = -after;
       before = -before;
@@ -211,12 +218,11 @@ class StageCompiler {
   // A phase that is 1 or -1 up to the rounding of its making.
   static constexpr double kTiny = 1e-15;
   static cplx clean(cplx p) {
-    if (std::abs(p - cplx(1.0, 0.0)) < kTiny) return cplx(1.0, 0.0);
-    return std::abs(p + cplx(1.0, 0.0)) < kTiny ? cplx(-1.0, 0.0) : p;
+    if (std::norm(p - cplx(1.0, 0.0)) < kTiny * kTiny) return cplx(1.0, 0.0);
+    return std::norm(p + cplx(1.0, 0.0)) < kTiny * kTiny ? cplx(-1.0, 0.0) : p;
   }
-  static cplx det(const cplx* m) { return m[0] * m[3] - m[1] * m[2]; }
   static void shears(double c, double s, Item* I) {  // c >= 0
-    const double h = std::hypot(c, s);
+    const double h = mag(cplx(c, s));
     I->t = (s / h) / (1.0 + c / h);
     I->s = s / h;
   }
@@ -231,15 +237,15 @@ class StageCompiler {
       case OP_D1: {
         const uint32_t a = t.dreg0 != 0xFF ? 1u << t.dreg0 : 0u;
         phase(t.creg, t.cnr, o.m[0]);
-        phase(t.creg | a, t.cnr | t.dv0, o.m[1] / o.m[0]);
+        phase(t.creg | a, t.cnr | t.dv0, quot(o.m[1], o.m[0]));
         return;
       }
       case OP_D2: {
         const uint32_t a = t.dreg0 != 0xFF ? 1u << t.dreg0 : 0u, b = t.dreg1 != 0xFF ? 1u << t.dreg1 : 0u;
         phase(t.creg, t.cnr, o.m[0]);
-        phase(t.creg | a, t.cnr | t.dv0, o.m[1] / o.m[0]);
-        phase(t.creg | b, t.cnr | t.dv1, o.m[2] / o.m[0]);
-        phase(t.creg | a | b, t.cnr | t.dv0 | t.dv1, (o.m[3] * o.m[0]) / (o.m[1] * o.m[2]));
+        phase(t.creg | a, t.cnr | t.dv0, quot(o.m[1], o.m[0]));
+        phase(t.creg | b, t.cnr | t.dv1, quot(o.m[2], o.m[0]));
+        phase(t.creg | a | b, t.cnr | t.dv0 | t.dv1, quot(o.m[3] * o.m[0], o.m[1] * o.m[2]));
         return;
       }
       case OP_U1:
@@ -381,19 +387,41 @@ class StageCompiler {
     // the phase common to all amplitudes
     double d[64], lo = 0.0, hi = 0.0;
     const cplx first = std::conj(v[0]);
-    for (uint32_t r = 0; r < kAll; ++r) {
-      const cplx p = v[r] * first;
-      d[r] = std::atan2(p.imag(), p.real());
-      lo = std::min(lo, d[r]);
-      hi = std::max(hi, d[r]);
+    if (!kF32) {
+      for (uint32_t r = 0; r < kAll; ++r) {
+        const cplx p = v[r] * first;
+        d[r] = std::atan2(p.imag(), p.real());
+        lo = std::min(lo, d[r]);
+        hi = std::max(hi, d[r]);
+      }
+    } else if (!final_) {
+      // the outermost by y / (|x| + |y|), which grows with the angle on each half turn
+      cplx plo(1.0, 0.0), phi(1.0, 0.0);
+      double olo = 0.0, ohi = 0.0;
+      for (uint32_t r = 0; r < kAll; ++r) {
+        const cplx p = v[r] * first;
+        const double q = p.imag() / (std::fabs(p.real()) + std::fabs(p.imag()));
+        const double o = p.real() >= 0.0 ? q : std::signbit(p.imag()) ? -2.0 - q : 2.0 - q;
+        if (o < olo) olo = o, plo = p;
+        if (o > ohi) ohi = o, phi = p;
+      }
+      lo = std::atan2(plo.imag(), plo.real());
+      hi = std::atan2(phi.imag(), phi.real());
     }
     if (!final_ && hi - lo <= kHalfTurn) {
       const double mid = 0.5 * (lo + hi);
-      *global_ *= v[0] * cplx(std::cos(mid), std::sin(mid));
+      const cplx m = v[0] * cplx(std::cos(mid), std::sin(mid));
+      *global_ *= m;
       for (uint32_t r = kAll; r-- > 0;) {
-        const double a = d[r] - mid;
-        d[2 * r] = std::tan(0.5 * a);
-        d[2 * r + 1] = std::sin(a);
+        if (kF32) {  // tan(a / 2) = sin a / (1 + cos a) without an angle
+          const cplx p = v[r] * std::conj(m);
+          d[2 * r] = p.imag() / (1.0 + p.real());
+          d[2 * r + 1] = p.imag();
+        } else {
+          const double a = d[r] - mid;
+          d[2 * r] = std::tan(0.5 * a);
+          d[2 * r + 1] = std::sin(a);
+        }
       }
       W_.header(TC_TS, 0);
     } else {
@@ -591,16 +619,17 @@ void stage_tab(const StageRec& S, int vb, uint32_t (&t)[kStageTabWords]) {
     t[StageTab::CS + i] = regslot(w);
     t[StageTab::CH + i] = half(w);
   }
-  for (int v = 0; v < 16; ++v) {
-    uint32_t lo = 0, hi = 0;
-    for (int j = 0; j < 4; ++j) {
-      if (j < S.n_tbits && ((v >> j) & 1)) lo |= 1u << S.tpos[j];
-      if (j + 4 < S.n_tbits && ((v >> j) & 1)) hi |= 1u << S.tpos[j + 4];
+  t[StageTab::UL] = t[StageTab::UH] = t[StageTab::SL] = t[StageTab::SH] = 0;
+  for (int j = 0; j < 4; ++j) {  // each bit on top of the combinations of those below it
+    const uint32_t lo = j < S.n_tbits ? 1u << S.tpos[j] : 0u, hi = j + 4 < S.n_tbits ? 1u << S.tpos[j + 4] : 0u;
+    const uint32_t slo = swz(lo), shi = swz(hi);
+    for (int v = 0; v < 1 << j; ++v) {
+      const int w = v | 1 << j;
+      t[StageTab::UL + w] = t[StageTab::UL + v] | lo;
+      t[StageTab::UH + w] = t[StageTab::UH + v] | hi;
+      t[StageTab::SL + w] = t[StageTab::SL + v] ^ slo;
+      t[StageTab::SH + w] = t[StageTab::SH + v] ^ shi;
     }
-    t[StageTab::UL + v] = lo;
-    t[StageTab::UH + v] = hi;
-    t[StageTab::SL + v] = swz(lo);
-    t[StageTab::SH + v] = swz(hi);
   }
 }
 
@@ -609,6 +638,8 @@ void compile(const std::vector<Op>& ops, TilePlan* plan, const std::vector<TileO
   StageCompiler<Real> C(ops, *plan, enc);
   cplx global(1.0, 0.0);
   const size_t last = plan->stages.empty() ? 0 : plan->stages.size() - 1;
+  // the tables, and about what an op's share of the instructions takes
+  plan->prog.reserve(plan->stages.size() * (kStageTabWords / 4 + 8) + 2 * plan->op_src.size() + 64);
   for (PassRec& P : plan->passes) {
     P.prog_begin = int32_t(plan->prog.size());
     const size_t tabs = plan->prog.size(), base = tabs + size_t(P.stage_end - P.stage_begin) * (kStageTabWords / 4);
@@ -630,16 +661,16 @@ void compile(const std::vector<Op>& ops, TilePlan* plan, const std::vector<TileO
 
 // A unitary 2x2 without controls that is not real, diagonal or anti-diagonal: its
 // three Euler angles are all there.  `rx`: of RX's form.
-bool takes_carry(const Op& o, bool* rx = nullptr) {
+bool takes_carry(const Op& o, bool* rx) {
   if (o.kind != OP_U1 || o.nctrl != 0) return false;
   const cplx* m = o.m;
   const double eps = 1e-12;
   if (std::abs(std::norm(m[0]) + std::norm(m[2]) - 1.0) > eps || std::abs(std::norm(m[1]) + std::norm(m[3]) - 1.0) > eps ||
-      std::abs(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) > eps)
+      std::norm(std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3]) > eps * eps)
     return false;
   const bool real = m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0;
-  if (rx) *rx = m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
-  return !real && std::abs(m[0]) > 1e-6 && std::abs(m[2]) > 1e-6;
+  *rx = m[0].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[3].imag() == 0;
+  return !real && std::norm(m[0]) > 1e-12 && std::norm(m[2]) > 1e-12;
 }
 
 void times(const cplx* a, const cplx* b, cplx* out) {
@@ -652,7 +683,11 @@ void times(const cplx* a, const cplx* b, cplx* out) {
 
 std::vector<Op> carry_phases(std::vector<Op> ops) {
   size_t takers = 0;
-  for (const Op& o : ops) takers += takes_carry(o);
+  struct Takes {
+    bool any, rx;
+  };
+  std::vector<Takes> takes(ops.size());
+  for (size_t i = 0; i < ops.size(); ++i) takers += takes[i].any = takes_carry(ops[i], &takes[i].rx);
   if (takers < 2) return ops;
   // the op after op i on each of its (at most five) qubits, from a backward walk
   struct Next {
@@ -676,14 +711,14 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
     return -1;
   };
   for (size_t i = 0; i < ops.size(); ++i) {
-    bool rx = false;
-    if (!takes_carry(ops[i], &rx)) continue;
+    if (!takes[i].any) continue;
+    const bool rx = takes[i].rx;
     const int q = ops[i].t0;
     bool z = true, x = true, found = false;
     size_t e = 0;
     for (int32_t k = after(i, q); k >= 0 && (z || x); k = after(size_t(k), q)) {
       const Op& o = ops[size_t(k)];
-      if (takes_carry(o)) {
+      if (takes[size_t(k)].any) {
         e = size_t(k);
         found = true;
         break;
@@ -698,10 +733,11 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
     cplx* m = ops[i].m;
     cplx w[4] = {m[0], m[1], m[2], m[3]}, c[4] = {1.0, 0.0, 0.0, 1.0};
     if (z) {
-      const cplx p = (m[2] / std::abs(m[2])) / (m[0] / std::abs(m[0]));
+      cplx p = m[2] * std::conj(m[0]);
+      p /= std::abs(p);
       c[3] = p;
-      w[2] = m[2] / p;
-      w[3] = m[3] / p;
+      w[2] = m[2] * std::conj(p);
+      w[3] = m[3] * std::conj(p);
     } else {
       // RX(al) rotation phase: RX(-al) m has a real ratio in its first column
       const double al = std::atan2(-2.0 * (std::conj(m[0]) * m[2]).imag(), std::norm(m[0]) - std::norm(m[2]));
@@ -712,6 +748,7 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
     }
     std::memcpy(static_cast<void*>(m), w, sizeof(w));
     times(ops[e].m, c, ops[e].m);
+    takes[e].any = takes_carry(ops[e], &takes[e].rx);
   }
   return ops;
 }

@@ -112,3 +112,24 @@ def test_compile_time_is_linear_in_the_gates(n, dtype):
         return min(times)
 
     assert best(2000) <= 24 * best(250)
+
+
+def test_compile_time_against_lowering():
+    # a circuit that runs once pays for its programs: planning and compiling a
+    # 17-qubit brickwork takes 9 times as long as lowering its gates (15 times with
+    # an angle per phase table entry and the matrices tested at every look)
+    import time
+
+    from nqpu_b200.state import Circuit
+
+    c = Circuit(17, circuits.brickwork(17, 15, 1))
+
+    def best(mode):
+        times = []
+        for _ in range(100):
+            t = time.perf_counter()
+            c.plan_stats(17, "c64", mode)
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    assert best("tiled") <= 12 * best("pergate")
