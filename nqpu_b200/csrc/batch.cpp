@@ -124,12 +124,13 @@ static cudaError_t batch_build(BatchImpl* b) {
   uint64_t arena_amps = 0;
   uint32_t counters = 0, partials = 0;
   b->n_small = 0;
-  // per-circuit tiled plans (independent: built on host threads), then
-  // concatenated with rebased program offsets
+  // per-circuit tiled plans (independent: built on host threads, 16 to each at least:
+  // 256 circuits take 2.2 ms on sixteen, 5 on the four that 64 to each would be),
+  // then concatenated with rebased program offsets
   const size_t nc = b->entries.size();
   std::vector<TilePlan> plans(nc);
   std::vector<char> plan_ok(nc, 0);
-  parallel_ranges(nc, 64, [&](size_t lo, size_t hi) {
+  parallel_ranges(nc, 16, [&](size_t lo, size_t hi) {
     for (size_t ci = lo; ci < hi; ++ci) {
       const BatchEntry& E = b->entries[ci];
       const bool small = E.n <= b->small_max;
