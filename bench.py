@@ -459,7 +459,7 @@ def run_engine(args):
                        "engine_mode_chosen_by": "NQPU_MODE_AUTO" if getattr(args, "auto", False) else "--mode",
                        "engine": MODE_DESCRIPTIONS[args.mode],
                        "plan": {"passes": stats["passes"], "stages": stats["stages"]},
-                       "tile_ctas_per_sm": int(lib.nqpu_tile_config_get(1 if args.dtype == "c64" else 0)),
+                       "tile_ctas_per_sm": int(lib.nqpu_tile_config_get(1 if args.dtype == "c64" else 0)) or "chosen per plan",
                        "l2": f"state {S / 2**30:.2f} GiB vs 126 MB L2; no flush", "parallelism": f"replicas{world}"},
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
             "gpu_launches": launches_per_step * args.steps, "clocks": clk,

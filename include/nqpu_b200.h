@@ -302,11 +302,11 @@ NqpuError    nqpu_circuit_profile(const NqpuCircuit* circuit, NqpuState* state, 
                                   float* launch_ms, uint32_t len, uint32_t* count);
 /* Tiled-pass kernel configuration per dtype: ctas_per_sm = 1 (one CTA per SM,
  * double-buffered 64 KB tiles), 2 (two CTAs per SM, single-buffered 64 KB
- * tiles) or 4 (four CTAs per SM on 32 KB tiles, one tile qubit fewer).  Until it
- * is set the library chooses per plan and launch (complex64 4, or 2 where larger
- * tiles save a fifth of the passes; complex128 1 up to one tile per SM, else 2),
- * and nqpu_tile_config_get reports 4 and 1.  Plans
- * are built for the configuration in force when a circuit is first run on a
+ * tiles), 4 (four CTAs per SM on 32 KB tiles, one tile qubit fewer) or 0, the
+ * default: the library chooses per plan and launch (complex64 4, or 2 where larger
+ * tiles save a fifth of the passes and some of the stages; complex128 1 up to one
+ * tile per SM, else 2).  nqpu_tile_config_get returns what is set, so a caller that
+ * saves and restores it leaves the library as it was.  Plans are built for the configuration in force when a circuit is first run on a
  * state size (a plan built for larger tiles is rebuilt, never run on smaller). */
 NqpuError    nqpu_tile_config_set(NqpuDtype dtype, uint32_t ctas_per_sm);
 /* Diagnostics (no counterpart in the reference): how many times a tensor-pass

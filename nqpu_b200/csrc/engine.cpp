@@ -389,7 +389,7 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
   if (mode == NQPU_MODE_TILED && int(n) >= tile_min_qubits(dt)) {
     std::string err;
     p->ops = carry_phases(std::move(p->ops));
-    p->tile_cfg = tile_config_raw(dt);
+    p->tile_cfg = tile_config_get(dt);
     if (p->tile.passes.empty() && !build_tile_plan_for(p->ops, int(n), dt, &p->tile, &err)) return false;
     build_tile_prog(p->ops, &p->tile);
     p->stats = p->tile.stats;
@@ -562,7 +562,7 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   const auto key = std::make_tuple(s->n, int(s->dt), effective, si);
   DevicePlan*& p = c->plans[key];
   // rebuild when the circuit changed or the tiled kernel's tile size did
-  if (p && (p->version != c->version || (effective == NQPU_MODE_TILED && p->tile_cfg != tile_config_raw(s->dt)))) {
+  if (p && (p->version != c->version || (effective == NQPU_MODE_TILED && p->tile_cfg != tile_config_get(s->dt)))) {
     cudaStreamSynchronize(s->stream);
     plan_free(p);
     p = nullptr;

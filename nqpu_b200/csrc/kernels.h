@@ -28,11 +28,10 @@ cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, bool rev, c
 
 // --- tiled pass path ---------------------------------------------------------
 // CTA configuration of the tiled pass kernel (1: one CTA per SM, double-buffered
-// tiles; 2: two CTAs per SM, single-buffered; 4: four on half-size tiles).  get
-// names the default while none is set; raw is 0 then.
+// tiles; 2: two CTAs per SM, single-buffered; 4: four on half-size tiles; 0, the
+// default: chosen per plan and launch).
 void tile_config_set(DType dt, int minb);
 int tile_config_get(DType dt);
-int tile_config_raw(DType dt);
 // Tiled plan of the tile size in force for the dtype.
 // (`enough`: asked with the first plan, true spares the search for a better one)
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,

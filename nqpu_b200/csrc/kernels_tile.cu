@@ -169,13 +169,9 @@ static size_t tile_smem_max(int minb, int share_of) {
 static int g_tile_minb[2] = {0, 0};
 
 void tile_config_set(DType dt, int minb) {
-  g_tile_minb[dt == DType::C64 ? 0 : 1] = (minb == 4) ? 4 : (minb == 2) ? 2 : 1;
+  g_tile_minb[dt == DType::C64 ? 0 : 1] = minb;
 }
-int tile_config_raw(DType dt) { return g_tile_minb[dt == DType::C64 ? 0 : 1]; }
-int tile_config_get(DType dt) {
-  const int c = tile_config_raw(dt);
-  return c ? c : dt == DType::C64 ? 4 : 1;
-}
+int tile_config_get(DType dt) { return g_tile_minb[dt == DType::C64 ? 0 : 1]; }
 
 template <typename Real, int KMAX, int MINB, int WAY>
 cudaError_t launch_tile_pass_cfg(Real* amp, const PassRec& host_pass, const ProgWord* d_prog,
@@ -261,8 +257,8 @@ cudaError_t launch_tile_pass(DType dt, void* amp, const PassRec& host_pass, cons
 }
 
 static int tile_kmax_for(DType dt) {
-  const int full = dt == DType::C64 ? 13 : 12;
-  return tile_config_get(dt) == 4 ? full - 1 : full;
+  const int full = dt == DType::C64 ? 13 : 12, set = tile_config_get(dt);
+  return set == 4 || (set == 0 && dt == DType::C64) ? full - 1 : full;
 }
 
 // From this size on a complex64 pass is long enough (32 MB of state) for its HBM
@@ -279,7 +275,7 @@ constexpr int kWideTileMinQubits = 22;
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>& enough) {
   if (!build_tile_plan(ops, n, dt, tile_kmax_for(dt), out, err)) return false;
-  if (dt != DType::C64 || tile_config_raw(dt) != 0 || n < kWideTileMinQubits || out->passes.size() < 2) return true;
+  if (dt != DType::C64 || tile_config_get(dt) != 0 || n < kWideTileMinQubits || out->passes.size() < 2) return true;
   if (enough && enough(*out)) return true;
   TilePlan wide;
   if (build_tile_plan(ops, n, dt, 13, &wide, err) && 5 * wide.passes.size() <= 4 * out->passes.size() &&

@@ -73,7 +73,7 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaErrorNotSupp
 namespace nqpu {
 double next_random_f64() { return 0.5; }
 size_t reduce_scratch_bytes(int) { return 4096; }
-int tile_config_raw(DType) { return 0; }
+int tile_config_get(DType) { return 0; }
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>&) {
   ++g_plans;
