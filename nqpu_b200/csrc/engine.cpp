@@ -554,9 +554,10 @@ static cudaError_t segment_run(CircuitImpl* c, const Segment& seg, int si, State
   if (seg.begin == seg.end) return cudaSuccess;
   TilePlan ready;
   if (mode == NQPU_MODE_AUTO) {
-    std::pair<uint64_t, int>& am = c->auto_modes[std::make_tuple(s->n, int(s->dt), si)];
-    if (am.first != c->version + 1) am = {c->version + 1, auto_mode_for(segment_ops(c, seg), s->n, s->dt, &ready)};
-    mode = am.second;
+    CircuitImpl::AutoMode& am = c->auto_modes[std::make_tuple(s->n, int(s->dt), si)];
+    if (am.version != c->version || am.tile_cfg != tile_config_get(s->dt))
+      am = {c->version, tile_config_get(s->dt), auto_mode_for(segment_ops(c, seg), s->n, s->dt, &ready)};
+    mode = am.mode;
   }
   const int effective = (mode == NQPU_MODE_TILED && int(s->n) < tile_min_qubits(s->dt)) ? int(NQPU_MODE_PERGATE) : mode;
   const auto key = std::make_tuple(s->n, int(s->dt), effective, si);

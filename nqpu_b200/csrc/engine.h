@@ -96,9 +96,13 @@ struct CircuitImpl {
   // cached plans per (state qubits, dtype, mode, segment); segments are the
   // gate runs between mid-circuit measurements / resets
   std::map<std::tuple<uint32_t, int, int, int>, DevicePlan*> plans;
-  // NQPU_MODE_AUTO's choice per (state qubits, dtype, segment): (circuit
-  // version + 1, mode); version + 1 so that a default entry reads as unset
-  std::map<std::tuple<uint32_t, int, int>, std::pair<uint64_t, int>> auto_modes;
+  // NQPU_MODE_AUTO's choice per (state qubits, dtype, segment), and what it was made
+  // for: the circuit's version and the tile configuration that its tiled plan had
+  struct AutoMode {
+    uint64_t version = ~0ull;
+    int tile_cfg = 0, mode = 0;
+  };
+  std::map<std::tuple<uint32_t, int, int>, AutoMode> auto_modes;
   std::mutex mu;
 };
 

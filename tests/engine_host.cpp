@@ -22,7 +22,9 @@ namespace {
 std::map<cudaStream_t, std::deque<std::function<void()>>> g_queue;
 int g_fail_malloc = -1;   // the allocation that fails, counted from now on
 int g_fail_measure = -1;  // the measurement launch that fails
+int g_tile_cfg = 0;       // tile configuration; 1: plans on 11 bits here, else 12
 int g_plans = 0;          // tiled plans built
+int g_tc_runs = 0;        // circuits run in the tensor mode
 uint64_t g_tc_passes = 0;  // of the tensor plan (0: the tensor mode does not take the circuit)
 std::vector<uint32_t> g_words;  // program words of the tiled passes launched
 void run(cudaStream_t st) {
@@ -73,11 +75,11 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaErrorNotSupp
 namespace nqpu {
 double next_random_f64() { return 0.5; }
 size_t reduce_scratch_bytes(int) { return 4096; }
-int tile_config_get(DType) { return 0; }
+int tile_config_get(DType) { return g_tile_cfg; }
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>&) {
   ++g_plans;
-  return build_tile_plan(ops, n, dt, 12, out, err);
+  return build_tile_plan(ops, n, dt, g_tile_cfg == 1 ? 11 : 12, out, err);
 }
 cudaError_t launch_tile_pass(DType, void*, const PassRec& P, const ProgWord* prog, cudaStream_t, int) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(prog + P.prog_begin);
@@ -115,13 +117,19 @@ bool fused_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void**, 
 bool fused_plan_stats(const std::vector<Op>&, int, DType, PlanStats*) { return false; }
 void fused_plan_free(void*) {}
 cudaError_t fused_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
-bool tc_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void**, PlanStats*) { return false; }
+bool tc_plan_build(const std::vector<Op>&, int, DType, cudaStream_t, void** plan, PlanStats*) {
+  *plan = nullptr;
+  return true;
+}
 bool tc_plan_stats(const std::vector<Op>&, int, DType, PlanStats* st) {
   st->passes = st->stages = g_tc_passes;
   return g_tc_passes > 0;
 }
 void tc_plan_free(void*) {}
-cudaError_t tc_run(void*, StateImpl*, std::vector<cudaEvent_t>*) { return cudaSuccess; }
+cudaError_t tc_run(void*, StateImpl*, std::vector<cudaEvent_t>*) {
+  ++g_tc_runs;
+  return cudaSuccess;
+}
 }  // namespace nqpu
 
 // ---- checks (0: as it should be) ---------------------------------------------
@@ -170,10 +178,8 @@ extern "C" int check_measure_error(int what) {
   return 0;
 }
 
-// AUTO builds one tiled plan for a circuit that it runs in the tiled mode, none for
-// its second run, and the programs are the tiled mode's own.
-extern "C" int check_auto_plans_once(int n) {
-  StateImpl* s = state_new(uint32_t(n), DType::C64);
+// Six layers of U3s and CNOTs in a ring.
+static std::vector<GateRec> layers(int n) {
   std::vector<GateRec> gates;
   for (int l = 0; l < 6; ++l)
     for (int q = 0; q < n; ++q) {
@@ -187,6 +193,14 @@ extern "C" int check_auto_plans_once(int n) {
       g.q[1] = (q + 1) % n;
       gates.push_back(g);
     }
+  return gates;
+}
+
+// AUTO builds one tiled plan for a circuit that it runs in the tiled mode, none for
+// its second run, and the programs are the tiled mode's own.
+extern "C" int check_auto_plans_once(int n) {
+  StateImpl* s = state_new(uint32_t(n), DType::C64);
+  const std::vector<GateRec> gates = layers(n);
   CircuitImpl a, b;
   a.n = b.n = uint32_t(n);
   a.gates = b.gates = gates;
@@ -202,4 +216,39 @@ extern "C" int check_auto_plans_once(int n) {
   g_tc_passes = 0;
   state_free(s);
   return 0;
+}
+
+// AUTO chooses again when the tile configuration that the choice was made for has
+// changed, and keeps its choice while it has not: a tensor plan priced between the
+// tiled plans of two tile sizes.
+extern "C" int check_auto_follows_tiles() {
+  const int n = 22;
+  StateImpl* s = state_new(n, DType::C64);
+  CircuitImpl c;
+  c.n = n;
+  c.gates = layers(n);
+  const std::vector<Op> ops = lower_circuit(c.gates);
+  auto mode_at = [&](int cfg) {
+    g_tile_cfg = cfg;
+    return auto_mode_for(ops, n, DType::C64);
+  };
+  g_tc_passes = 0;
+  do ++g_tc_passes;
+  while (g_tc_passes < 1000 && mode_at(0) == NQPU_MODE_TENSOR);  // dearer than the 12-bit plan,
+  if (mode_at(0) != NQPU_MODE_TILED || mode_at(1) != NQPU_MODE_TENSOR) return 1;  // cheaper than the 11-bit one
+  auto tensor_runs = [&](int cfg) {
+    g_tile_cfg = cfg;
+    g_tc_runs = 0;
+    return circuit_run(&c, s, NQPU_MODE_AUTO) == cudaSuccess ? g_tc_runs : -1;
+  };
+  int rc = 0;
+  if (tensor_runs(0) != 0) rc = 2;
+  else if (tensor_runs(1) != 1) rc = 3;
+  else if (tensor_runs(0) != 0) rc = 4;
+  g_plans = 0;
+  if (!rc && (tensor_runs(0) != 0 || g_plans != 0)) rc = 5;
+  g_tile_cfg = 0;
+  g_tc_passes = 0;
+  state_free(s);
+  return rc;
 }

@@ -46,3 +46,7 @@ def test_no_measurement_outlives_an_error(eng, what):
 @pytest.mark.parametrize("n", [12, 17, 22])
 def test_auto_plans_a_tiled_circuit_once(eng, n):
     assert eng.check_auto_plans_once(n) == 0
+
+
+def test_auto_chooses_again_for_another_tile_size(eng):
+    assert eng.check_auto_follows_tiles() == 0
