@@ -32,6 +32,16 @@ cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, bool rev, c
 // default: chosen per plan and launch).
 void tile_config_set(DType dt, int minb);
 int tile_config_get(DType dt);
+// The configuration (1, 2 or 4) that a pass of 2^k-amplitude tiles over 2^n_out of
+// them runs in where `set` is set.  One that was planned on larger tiles than 4
+// takes runs in 2: the setting may change after a plan was made, under a request
+// that waits for its launch or in another thread.
+inline int tile_launch_config(DType dt, int set, int k, int n_out, int num_sms) {
+  const int full = dt == DType::C64 ? 13 : 12;
+  if (set == 0 && dt == DType::C128) return (uint64_t(1) << n_out) <= uint64_t(num_sms) ? 1 : 2;
+  if (set == 0 || set == 4) return k == full ? 2 : 4;
+  return set;
+}
 // Tiled plan of the tile size in force for the dtype.
 // (`enough`: asked with the first plan, true spares the search for a better one)
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,

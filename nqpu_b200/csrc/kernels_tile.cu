@@ -17,6 +17,7 @@
 // Shared-memory layout: vector u (16 B) lives at slot swz(u) = u ^ fold3(u>>3)
 // so that the 8 lanes of a quarter-warp that the planner maps to vector bits of
 // distinct residue mod 3 hit 8 distinct 16-byte bank groups.
+#include <atomic>
 #include "device_once.h"
 #include "kernels.h"
 #include "tile_device.cuh"
@@ -166,11 +167,9 @@ static size_t tile_smem_max(int minb, int share_of) {
 //     dependency waits: 25-qubit ansatz of 8 layers 5.1 against 6.6 ms, 20-qubit
 //     brickwork 383 against 461 us; 4 takes 4.7 ms and 389 us, with 12 and 21
 //     passes for 10 and 14).
-static int g_tile_minb[2] = {0, 0};
+static std::atomic<int> g_tile_minb[2];
 
-void tile_config_set(DType dt, int minb) {
-  g_tile_minb[dt == DType::C64 ? 0 : 1] = minb;
-}
+void tile_config_set(DType dt, int minb) { g_tile_minb[dt == DType::C64 ? 0 : 1] = minb; }
 int tile_config_get(DType dt) { return g_tile_minb[dt == DType::C64 ? 0 : 1]; }
 
 template <typename Real, int KMAX, int MINB, int WAY>
@@ -237,13 +236,9 @@ template <typename Real>
 static cudaError_t launch_tile_pass_t(Real* amp, const PassRec& host_pass, const ProgWord* d_prog,
                                       cudaStream_t stream, int num_sms) {
   constexpr int K = tile_kmax_full<Real>();
-  int cfg = g_tile_minb[sizeof(Real) == 4 ? 0 : 1];
-  if (cfg == 0) {
-    if (sizeof(Real) == 4) cfg = host_pass.k == K ? 2 : 4;
-    else cfg = (1ull << host_pass.n_out) <= uint64_t(num_sms) ? 1 : 2;
-  }
+  constexpr DType dt = sizeof(Real) == 4 ? DType::C64 : DType::C128;
   constexpr int W = sizeof(Real) == 8 ? 2 : 1;
-  switch (cfg) {
+  switch (tile_launch_config(dt, tile_config_get(dt), host_pass.k, host_pass.n_out, num_sms)) {
     case 4: return launch_tile_pass_cfg<Real, K - 1, 4, W>(amp, host_pass, d_prog, stream, num_sms);
     case 2: return launch_tile_pass_cfg<Real, K, 2, W>(amp, host_pass, d_prog, stream, num_sms);
     default: return launch_tile_pass_cfg<Real, K, 1, 1>(amp, host_pass, d_prog, stream, num_sms);

@@ -252,3 +252,20 @@ extern "C" int check_auto_follows_tiles() {
   state_free(s);
   return rc;
 }
+
+// The configuration a pass is launched in holds its tiles whatever is set, and is the
+// set one wherever that holds them.
+extern "C" int check_launch_config() {
+  for (DType dt : {DType::C64, DType::C128}) {
+    const int full = dt == DType::C64 ? 13 : 12;
+    for (int set : {0, 1, 2, 4})
+      for (int k = 5; k <= full; ++k)
+        for (int n_out : {0, 3, 7, 8, 20}) {
+          const int cfg = tile_launch_config(dt, set, k, n_out, 148);
+          if (cfg != 1 && cfg != 2 && cfg != 4) return 1;
+          if (k > (cfg == 4 ? full - 1 : full)) return 2;
+          if (set != 0 && cfg != set && !(set == 4 && k == full)) return 3;
+        }
+  }
+  return 0;
+}

@@ -50,3 +50,7 @@ def test_auto_plans_a_tiled_circuit_once(eng, n):
 
 def test_auto_chooses_again_for_another_tile_size(eng):
     assert eng.check_auto_follows_tiles() == 0
+
+
+def test_a_pass_is_launched_where_its_tiles_fit(eng):
+    assert eng.check_launch_config() == 0
