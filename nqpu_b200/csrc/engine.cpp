@@ -181,7 +181,26 @@ static cudaError_t pauli_direct(const StateImpl* s, const PauliString& p, double
   return e;
 }
 
+static cudaError_t pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out);
+
+// The kernel adds coefficients up before they meet the amplitudes and doubles those
+// of pairs: near the ends of the type's range it works on coefficients scaled by a
+// power of two, so that a sum overflows or vanishes only where its value does.
 cudaError_t state_pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out) {
+  double most = 0.0;
+  for (const PauliString& p : strings) most = std::max(most, std::fabs(p.c));
+  constexpr int kRoom = 900;  // of 1023: 2^123 for the sum of 2^32 terms and for the doubling
+  const int e = most > 0.0 ? std::ilogb(most) : 0;
+  const int shift = e > kRoom ? e - kRoom : e < -kRoom ? e + kRoom : 0;
+  if (shift == 0) return pauli_sum(s, strings, out);
+  std::vector<PauliString> scaled = strings;
+  for (PauliString& p : scaled) p.c = std::ldexp(p.c, -shift);
+  const cudaError_t r = pauli_sum(s, scaled, out);
+  *out = std::ldexp(*out, shift);
+  return r;
+}
+
+static cudaError_t pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out) {
   *out = 0.0;
   cudaError_t e;
   if (s->n < 4) {

@@ -95,3 +95,20 @@ def test_pauli_sum(n, count, dtype):
         assert abs(sv.expectation_pauli_string(s) - w) <= 1e-13
     assert abs(sv.expectation_x(n - 1) - want[-1]) <= 1e-13
     sv.close()
+
+
+# finite coefficients whose double or sum is not, and ones whose share of an
+# amplitude would be subnormal; the sum is scaled exactly, so the bound is that of
+# coefficients near 1
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [2, 5, 13])
+@pytest.mark.parametrize("size", [1.7e308, 1e305, 1e-303])
+def test_pauli_sum_of_extreme_coefficients(size, n, dtype):
+    a, sv = random_state(n, dtype, n)
+    strings = ["X" + "I" * (n - 1), "Z" * n, "Y" + "Z" * (n - 1), "I" * (n - 1) + "Z", "ZZ" + "I" * (n - 2)]
+    unit = np.array([1.0, 0.9, -0.8, 0.7, 0.6])
+    want = unit @ np.array([pauli_value(a, s) for s in strings])
+    assert abs(want) < 1.05  # and 1.05 * 1.7e308 is finite
+    got = sv.expectation_pauli_sum(list(zip(unit * size, strings)))
+    assert abs(got / size - want) <= 1e-13 * unit.size
+    sv.close()
