@@ -32,7 +32,7 @@ struct Phase {
 
 // An op of a stage, or a part of one, before scheduling.
 struct Item {
-  enum Kind { PHASE, ROT, CROSS, GENERIC, RECORD } kind = PHASE;
+  enum Kind { PHASE, ROT, CROSS, FLIP, GENERIC, RECORD } kind = PHASE;
   uint32_t diag = 0, dense = 0;  // register bits it reads (commutes with phases) / changes
   uint32_t cnr = 0;              // virtual-index mask: a phase's condition, a 2x2's control
   cplx m[4];                     // PHASE: m[0]; GENERIC: the matrix
@@ -173,6 +173,14 @@ class StageCompiler {
       items_.push_back(I);
       return;
     }
+    const double c = mag(m[0]), s = mag(m[2]);
+    if (c < kFlip) {  // Y, RX(pi), RY(pi): the amplitudes change places, with phases
+      I.kind = Item::FLIP;
+      items_.push_back(I);
+      push_phase(0, 0, unit(m[1]));
+      push_phase(1u << b, 0, clean(unit(quot(m[2], m[1]))));
+      return;
+    }
     // RX: cos and -i sin
     if (m[0].imag() == 0 && m[3].imag() == 0 && m[1].real() == 0 && m[2].real() == 0 && m[0].real() == m[3].real() &&
         m[1].imag() == m[2].imag()) {
@@ -183,17 +191,10 @@ class StageCompiler {
       if (I.s != 0.0) items_.push_back(I);
       return;
     }
-    const double c = mag(m[0]), s = mag(m[2]);
     const cplx one(1.0, 0.0);
-    if (s < kTiny || c < kTiny) {  // a phase, or a rotation by pi/2 with phases
-      const cplx p0 = s < kTiny ? m[0] : -m[1], p1 = s < kTiny ? quot(m[3], m[0]) : quot(m[2], -m[1]);
-      push_phase(0, 0, unit(p0));
-      if (c < kTiny) {
-        shears(0.0, 1.0, &I);
-        I.kind = Item::ROT;
-        items_.push_back(I);
-      }
-      push_phase(1u << b, 0, clean(unit(p1)));
+    if (s < kTiny) {  // a phase
+      push_phase(0, 0, unit(m[0]));
+      push_phase(1u << b, 0, clean(unit(quot(m[3], m[0]))));
       return;
     }
     // e^{ia} diag(1, after) [[c, -s], [s, c]] diag(1, before)
@@ -217,6 +218,11 @@ class StageCompiler {
   }
   // A phase that is 1 or -1 up to the rounding of its making.
   static constexpr double kTiny = 1e-15;
+  // |cos| below which a rotation is an exchange.  Three shears by a quarter turn add
+  // either amplitude to the other and take it off again, which costs a small one its
+  // digits beside a large one; leaving out less than half an ulp of the large one
+  // does not cost more.
+  static constexpr double kFlip = kF32 ? 1e-15 : 0x1p-53;
   static cplx clean(cplx p) {
     if (std::norm(p - cplx(1.0, 0.0)) < kTiny * kTiny) return cplx(1.0, 0.0);
     return std::norm(p + cplx(1.0, 0.0)) < kTiny * kTiny ? cplx(-1.0, 0.0) : p;
@@ -548,6 +554,9 @@ class StageCompiler {
       for (int i = 0; i < 4; ++i) { v[2 * i] = I.m[i].real(); v[2 * i + 1] = I.m[i].imag(); }
       W_.header(TC_G, uint32_t(ctz(I.dense)), I.cnr);
       W_.reals(v, 8);
+      W_.end();
+    } else if (I.kind == Item::FLIP) {
+      W_.header(TC_OP, OP_X1, uint32_t(ctz(I.dense)));
       W_.end();
     } else if (I.kind == Item::RECORD) {
       const TileOp<Real>& t = enc_[I.op];

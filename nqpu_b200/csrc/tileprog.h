@@ -35,9 +35,10 @@
 //              << 16; constant parts in header.z, .w (complex64) or two words
 //   SL A       sign flips: header.y = masks, header.z = constant parity; four
 //              masks per word
-//   OP A       any other op of kind A: header.y = register target bits, the second
-//              in the second byte, and register controls in the third, header.z =
-//              its controls elsewhere; the matrix of a 1q or 2q gate follows
+//   OP A       any other op of kind A (X also for a 2x2 without a diagonal):
+//              header.y = register target bits, the second in the second byte, and
+//              register controls in the third, header.z = its controls elsewhere;
+//              the matrix of a 1q or 2q gate follows
 //
 // Why a program and not the ops themselves: the tile kernels are bound by
 // instructions (every one costs a warp about seven cycles at any occupancy the

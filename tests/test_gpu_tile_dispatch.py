@@ -97,3 +97,28 @@ def test_many_shots(shots):
     with StateVector(12, "c128") as sv:
         sv.set_amplitudes(a)
         np.testing.assert_array_equal(sv.sample_with_uniforms(u), pick.astype(np.uint64))
+
+
+# A gate without a diagonal moves amplitudes and turns their phases: a small one keeps
+# its digits beside a large one.  Per amplitude: 2^-22 (complex64: entries, a phase and
+# the state's own rounding, 2^-24 each) and 2^-50 of its own size.
+@pytest.mark.parametrize("n", [5, 9, 14])
+@pytest.mark.parametrize("dtype,gate", [
+    ("c64", ("y", ())), ("c64", ("rx", (np.pi,))), ("c64", ("ry", (np.pi,))), ("c64", ("u3", (np.pi, 0.4, 0.9))),
+    ("c128", ("y", ())), ("c128", ("custom1", ()))])
+def test_exchanged_amplitudes_keep_their_digits(n, dtype, gate):
+    name, params = gate
+    rng = np.random.default_rng(n)
+    a = np.exp(2j * np.pi * rng.random(1 << n)) * 10.0 ** -rng.integers(0, 9, 1 << n)
+    a = a.astype(np.complex64 if dtype == "c64" else np.complex128).astype(np.complex128)
+    m = {"y": [[0, -1j], [1j, 0]], "rx": [[0, -1j], [-1j, 0]], "ry": [[0, -1], [1, 0]],
+         "u3": [[0, -np.exp(0.9j)], [np.exp(0.4j), 0]], "custom1": [[0, np.exp(0.3j)], [np.exp(-1.1j), 0]]}[name]
+    for q in {0, 2, n - 1}:
+        g = (name, (q,), params) if name != "custom1" else (name, (q,), (), np.array(m))
+        with StateVector(n, dtype) as sv:
+            sv.set_amplitudes(a)
+            Circuit(n, [g]).execute(sv, "tiled")
+            got = sv.amplitudes()
+        v = a.reshape(-1, 2, 1 << q)
+        want = np.stack([m[0][1] * v[:, 1], m[1][0] * v[:, 0]], axis=1).reshape(-1)
+        assert (np.abs(got - want) <= (2.0 ** -20 if dtype == "c64" else 2.0 ** -49) * np.abs(want)).all()
