@@ -560,6 +560,20 @@ class StageCompiler {
       W_.end();
     } else if (I.kind == Item::RECORD) {
       const TileOp<Real>& t = enc_[I.op];
+      if (t.kind == OP_U1 && (t.creg & (t.creg - 1))) {
+        // the kernel's 2x2 takes one register control: the first of several becomes
+        // the second bit of a 4x4 that is the identity where it is 0
+        const uint32_t c = uint32_t(ctz(t.creg));
+        W_.header(TC_OP, OP_U2, uint32_t(t.rb0) | c << 8 | (t.creg & (t.creg - 1u)) << 16);
+        W_.head().w[2] = t.cnr;
+        Real m[32] = {};
+        m[0] = m[2 * 5] = Real(1);
+        for (int r = 0; r < 2; ++r)
+          for (int e = 0; e < 4; ++e) m[2 * (4 * (2 + r) + 2) + e] = t.m[4 * r + e];
+        W_.bytes(m, sizeof(m));
+        W_.end();
+        return;
+      }
       W_.header(TC_OP, t.kind, uint32_t(t.rb0) | uint32_t(t.rb1) << 8 | uint32_t(t.creg) << 16);
       W_.head().w[2] = t.cnr;
       const size_t entries = t.kind == OP_U2 ? 16 : t.kind == OP_U1 ? 4 : 0;
