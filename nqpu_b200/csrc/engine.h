@@ -22,6 +22,7 @@ bool device_ready();
 int device_sms();
 
 constexpr size_t kSmallDoubles = 4096, kSmallTable = 64;
+constexpr size_t kSweepBytes = size_t(128) << 20;
 
 struct StateImpl {
   uint32_t n = 0;
@@ -47,7 +48,9 @@ struct StateImpl {
   size_t run_norm_cap = 0;     // doubles
   int* run_err = nullptr;
   bool sweep = false;          // direction of the last per-gate launch
-  bool next_sweep() { return sweep = !sweep; }
+  // Direction of the next one: alternating on states that the L2 does not hold
+  // (kernels_gate.cu), else always the same.
+  bool next_sweep() { return sweep = bytes >= kSweepBytes && !sweep; }
 };
 
 // Allocate *dev and copy a plan's table into it.  The copy is ordered on `st`, the

@@ -14,11 +14,11 @@ namespace nqpu {
 struct PGArgs {
   uint64_t n_items;   // work items (index sets) of the launch
   uint64_t setmask;   // bits forced to one (controls)
+  uint64_t flip;      // n_items - 1 in a launch that runs from the far end, else 0
   uint64_t cmask;     // controls checked per amplitude (elementwise kernels)
   int32_t npos;       // zero-bit insert positions, ascending
   int32_t pos[8];
   int32_t t0, t1;
-  int32_t rev;        // run over the items from the far end
   double m[32];
 };
 

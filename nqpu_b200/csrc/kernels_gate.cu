@@ -11,12 +11,14 @@
 //     are 128-bit double2 accesses;
 //   * grid-stride loops with two items in flight per thread, grid sized to
 //     the SM count;
-//   * successive gates on a state sweep it in alternate directions, so a launch
-//     begins with the part that the one before it left in L2 (126 MB); accesses
-//     carry no streaming hint that would evict it.  A U3 and CNOT layer,
-//     complex64: 24 qubits 1425 -> 1254 us, 25 qubits 3048 -> 2879, 28 qubits 27.1
-//     -> 26.6 ms; complex128, 23 qubits 1408 -> 1188 us; no change below 23
-//     (complex64), where L2 holds the whole state.
+//   * on states of 128 MB and more successive gates sweep in alternate directions,
+//     so a launch begins with the part that the one before it left in L2 (126 MB);
+//     accesses carry no streaming hint that would evict it.  A U3 and CNOT layer,
+//     complex64: 24 qubits 1370 -> 1210 us, 25 qubits 2934 -> 2794, 26 qubits 6165 ->
+//     5948; complex128, 23 qubits 1362 -> 1139.  Below, the L2 holds the state, and
+//     turning round moves every address to another SM's half of it (complex64, 20
+//     qubits: 20 RY gates 115 us, in alternate directions 121; 23 qubits: 355
+//     against 363).
 #include "sv_device.cuh"
 #include "kernels.h"
 
@@ -30,10 +32,15 @@ __device__ __forceinline__ void load_m(const PGArgs& A, typename Tr<Real>::C* m,
   }
 }
 
-// Index set of work item w, counted from the far end when the launch runs
-// backwards (launch_pergate).
+// Index set of work item w (n_items is a power of two, so the far end is a flip of
+// all its bits).  The direction is compiled in: as a run-time value it took
+// registers or instructions from every launch (4x4s on 21 qubits of complex128 199 ->
+// 233 us, RZ on 21 qubits of complex64 142 -> 173), except for X, whose run-time form
+// is the faster code (23 qubits of complex128, 23 gates: 915 us, compiled in 1000).
+enum Dir { FORWARD, BACKWARD, RUNTIME };
+template <Dir DIR>
 __device__ __forceinline__ uint64_t pg_expand(uint64_t w, const PGArgs& A) {
-  uint64_t i = A.rev ? A.n_items - 1 - w : w;
+  uint64_t i = DIR == FORWARD ? w : w ^ A.flip;
 #pragma unroll 1
   for (int j = 0; j < A.npos; ++j) i = insert_zero_bit(i, A.pos[j]);
   return i | A.setmask;
@@ -45,7 +52,7 @@ __device__ __forceinline__ uint64_t pg_expand(uint64_t w, const PGArgs& A) {
 // MODE 1: complex64, target t >= 1, qubit 0 free: item -> float4 at i and at
 //         i|2^t (two pairs).
 // MODE 2: complex64, target 0: item -> one float4 holding the pair.
-template <typename Real, int KIND, int MODE>
+template <typename Real, int KIND, int MODE, Dir DIR>
 __global__ void __launch_bounds__(256) k_pg_1t(Real* __restrict__ amp, PGArgs A) {
   using C = typename Tr<Real>::C;
   C m[4];
@@ -55,8 +62,8 @@ __global__ void __launch_bounds__(256) k_pg_1t(Real* __restrict__ amp, PGArgs A)
   for (uint64_t w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; w < A.n_items; w += 2 * stride) {
     const uint64_t w2 = w + stride;
     const bool has2 = w2 < A.n_items;
-    const uint64_t i0 = pg_expand(w, A);
-    const uint64_t i1 = has2 ? pg_expand(w2, A) : 0;
+    const uint64_t i0 = pg_expand<DIR>(w, A);
+    const uint64_t i1 = has2 ? pg_expand<DIR>(w2, A) : 0;
     if constexpr (MODE == 1) {
       float4* p = reinterpret_cast<float4*>(amp);
       float4 x0 = p[i0 >> 1], y0 = p[(i0 | tbit) >> 1];
@@ -116,7 +123,7 @@ __global__ void __launch_bounds__(256) k_pg_1t(Real* __restrict__ amp, PGArgs A)
 
 // ---- dense / swap on two targets ------------------------------------------
 // VEC: complex64 with qubit 0 free: four float4 per item (two quads).
-template <typename Real, int KIND, bool VEC>
+template <typename Real, int KIND, bool VEC, Dir DIR>
 __global__ void __launch_bounds__(256) k_pg_2t(Real* __restrict__ amp, PGArgs A) {
   using C = typename Tr<Real>::C;
   C m[16];
@@ -124,7 +131,7 @@ __global__ void __launch_bounds__(256) k_pg_2t(Real* __restrict__ amp, PGArgs A)
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t b0 = 1ull << A.t0, b1 = 1ull << A.t1;
   for (uint64_t w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; w < A.n_items; w += stride) {
-    const uint64_t i = pg_expand(w, A);
+    const uint64_t i = pg_expand<DIR>(w, A);
     if constexpr (VEC) {
       float4* p = reinterpret_cast<float4*>(amp);
       float4 v0 = p[i >> 1], v1 = p[(i | b0) >> 1];
@@ -167,8 +174,10 @@ __global__ void __launch_bounds__(256) k_pg_2t(Real* __restrict__ amp, PGArgs A)
 
 // ---- elementwise phases (D1, D2 over all amplitudes; PH on a masked subset)
 // PH: items enumerate only amplitudes with all mask bits set.
-template <typename Real, int KIND, bool VEC>
-__global__ void __launch_bounds__(256) k_pg_elem(Real* __restrict__ amp, PGArgs A) {
+// Backwards: eight blocks per SM, one register over 32 would cost a quarter of the warps (RZ
+// on 26 qubits of complex64, 26 gates: 5140 us at 33 registers, 4505 so bounded).
+template <typename Real, int KIND, bool VEC, Dir DIR>
+__global__ void __launch_bounds__(256, DIR == BACKWARD ? 8 : 0) k_pg_elem(Real* __restrict__ amp, PGArgs A) {
   using C = typename Tr<Real>::C;
   C m[4];
   load_m<Real>(A, m, KIND == OP_D2 ? 4 : (KIND == OP_D1 ? 2 : 1));
@@ -184,21 +193,30 @@ __global__ void __launch_bounds__(256) k_pg_elem(Real* __restrict__ amp, PGArgs 
   for (uint64_t w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; w < A.n_items; w += 2 * stride) {
     const uint64_t w2 = w + stride;
     const bool has2 = w2 < A.n_items;
-    const uint64_t i0 = pg_expand(w, A);
-    const uint64_t i1 = has2 ? pg_expand(w2, A) : 0;
+    const uint64_t i0 = pg_expand<DIR>(w, A);
+    const uint64_t i1 = has2 ? pg_expand<DIR>(w2, A) : 0;
     if constexpr (VEC) {
+      // one diagonal on a state that the L2 holds: streaming (RZ, complex64, 20 and 21
+      // qubits: 111 and 143 us, plain accesses 124 and 159; plain ones win or tie
+      // for every other gate, 4x4s on 23 qubits 440 -> 407 us)
+      constexpr bool kStream = KIND == OP_D1 && DIR == FORWARD;
       float4* p = reinterpret_cast<float4*>(amp);
-      float4 x0 = p[i0 >> 1];
+      auto load = [&](uint64_t i) { return kStream ? __ldcs(p + (i >> 1)) : p[i >> 1]; };
+      auto store = [&](uint64_t i, const float4& x) {
+        if (kStream) __stcs(p + (i >> 1), x);
+        else p[i >> 1] = x;
+      };
+      float4 x0 = load(i0);
       float4 x1;
-      if (has2) x1 = p[i1 >> 1];
+      if (has2) x1 = load(i1);
       auto op = [&](uint64_t i, float4& x) {
         float2 a = phase(i, make_float2(x.x, x.y));
         float2 b = phase(i | 1, make_float2(x.z, x.w));
         x = make_float4(a.x, a.y, b.x, b.y);
       };
       op(i0, x0);
-      p[i0 >> 1] = x0;
-      if (has2) { op(i1, x1); p[i1 >> 1] = x1; }
+      store(i0, x0);
+      if (has2) { op(i1, x1); store(i1, x1); }
     } else {
       C* p = reinterpret_cast<C*>(amp);
       C a0 = p[i0];
@@ -218,10 +236,9 @@ static unsigned pg_grid(uint64_t items, int num_sms) {
 }
 
 // Host-side lowering of one op to a per-gate launch.
-template <typename Real>
-static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStream_t s, int num_sms) {
+template <typename Real, Dir DIR>
+static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, cudaStream_t s, int num_sms) {
   PGArgs A{};
-  A.rev = rev;
   for (int i = 0; i < 16; ++i) {
     A.m[2 * i] = op.m[i].real();
     A.m[2 * i + 1] = op.m[i].imag();
@@ -238,6 +255,7 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
     A.npos = int(pos.size());
     for (int i = 0; i < A.npos; ++i) A.pos[i] = pos[i];
     A.n_items = (1ull << n) >> A.npos;
+    A.flip = DIR == BACKWARD ? A.n_items - 1 : 0;
   };
   const unsigned blk = 256;
   switch (op.kind) {
@@ -250,23 +268,23 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
         if (op.t0 == 0 && !(ctrl & 1)) {
           finish(false);
           unsigned g = pg_grid(A.n_items, num_sms);
-          if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 2><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_1t<Real, OP_X1, 2><<<g, blk, 0, s>>>(amp, A);
+          if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 2, DIR><<<g, blk, 0, s>>>(amp, A);
+          else k_pg_1t<Real, OP_X1, 2, RUNTIME><<<g, blk, 0, s>>>(amp, A);
           break;
         }
         if (!(ctrl & 1) && n >= 2) {
           finish(true);
           unsigned g = pg_grid(A.n_items, num_sms);
-          if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 1><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_1t<Real, OP_X1, 1><<<g, blk, 0, s>>>(amp, A);
+          if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 1, DIR><<<g, blk, 0, s>>>(amp, A);
+          else k_pg_1t<Real, OP_X1, 1, RUNTIME><<<g, blk, 0, s>>>(amp, A);
           break;
         }
       }
       {
         finish(false);
         unsigned g = pg_grid(A.n_items, num_sms);
-        if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 0><<<g, blk, 0, s>>>(amp, A);
-        else k_pg_1t<Real, OP_X1, 0><<<g, blk, 0, s>>>(amp, A);
+        if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 0, DIR><<<g, blk, 0, s>>>(amp, A);
+        else k_pg_1t<Real, OP_X1, 0, RUNTIME><<<g, blk, 0, s>>>(amp, A);
       }
       break;
     }
@@ -281,13 +299,13 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
       unsigned g = pg_grid(A.n_items, num_sms);
       if constexpr (sizeof(Real) == 4) {
         if (vec) {
-          if (op.kind == OP_U2) k_pg_2t<Real, OP_U2, true><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_2t<Real, OP_SW, true><<<g, blk, 0, s>>>(amp, A);
+          if (op.kind == OP_U2) k_pg_2t<Real, OP_U2, true, DIR><<<g, blk, 0, s>>>(amp, A);
+          else k_pg_2t<Real, OP_SW, true, DIR><<<g, blk, 0, s>>>(amp, A);
           break;
         }
       }
-      if (op.kind == OP_U2) k_pg_2t<Real, OP_U2, false><<<g, blk, 0, s>>>(amp, A);
-      else k_pg_2t<Real, OP_SW, false><<<g, blk, 0, s>>>(amp, A);
+      if (op.kind == OP_U2) k_pg_2t<Real, OP_U2, false, DIR><<<g, blk, 0, s>>>(amp, A);
+      else k_pg_2t<Real, OP_SW, false, DIR><<<g, blk, 0, s>>>(amp, A);
       break;
     }
     case OP_PH: {
@@ -299,9 +317,9 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
       finish(vec);
       unsigned g = pg_grid(A.n_items, num_sms);
       if constexpr (sizeof(Real) == 4) {
-        if (vec) { k_pg_elem<Real, OP_PH, true><<<g, blk, 0, s>>>(amp, A); break; }
+        if (vec) { k_pg_elem<Real, OP_PH, true, DIR><<<g, blk, 0, s>>>(amp, A); break; }
       }
-      k_pg_elem<Real, OP_PH, false><<<g, blk, 0, s>>>(amp, A);
+      k_pg_elem<Real, OP_PH, false, DIR><<<g, blk, 0, s>>>(amp, A);
       break;
     }
     case OP_D1:
@@ -315,13 +333,13 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
       unsigned g = pg_grid(A.n_items, num_sms);
       if constexpr (sizeof(Real) == 4) {
         if (vec) {
-          if (op.kind == OP_D1) k_pg_elem<Real, OP_D1, true><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_elem<Real, OP_D2, true><<<g, blk, 0, s>>>(amp, A);
+          if (op.kind == OP_D1) k_pg_elem<Real, OP_D1, true, DIR><<<g, blk, 0, s>>>(amp, A);
+          else k_pg_elem<Real, OP_D2, true, DIR><<<g, blk, 0, s>>>(amp, A);
           break;
         }
       }
-      if (op.kind == OP_D1) k_pg_elem<Real, OP_D1, false><<<g, blk, 0, s>>>(amp, A);
-      else k_pg_elem<Real, OP_D2, false><<<g, blk, 0, s>>>(amp, A);
+      if (op.kind == OP_D1) k_pg_elem<Real, OP_D1, false, DIR><<<g, blk, 0, s>>>(amp, A);
+      else k_pg_elem<Real, OP_D2, false, DIR><<<g, blk, 0, s>>>(amp, A);
       break;
     }
     default:
@@ -331,8 +349,11 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, bool rev, cudaStr
 }
 
 cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, bool rev, cudaStream_t s, int num_sms) {
-  if (dt == DType::C64) return launch_pg_t<float>(static_cast<float*>(amp), n, op, rev, s, num_sms);
-  return launch_pg_t<double>(static_cast<double*>(amp), n, op, rev, s, num_sms);
+  if (dt == DType::C64)
+    return rev ? launch_pg_t<float, BACKWARD>(static_cast<float*>(amp), n, op, s, num_sms)
+               : launch_pg_t<float, FORWARD>(static_cast<float*>(amp), n, op, s, num_sms);
+  return rev ? launch_pg_t<double, BACKWARD>(static_cast<double*>(amp), n, op, s, num_sms)
+             : launch_pg_t<double, FORWARD>(static_cast<double*>(amp), n, op, s, num_sms);
 }
 
 }  // namespace nqpu

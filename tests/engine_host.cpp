@@ -269,3 +269,23 @@ extern "C" int check_launch_config() {
   }
   return 0;
 }
+
+// Per-gate launches alternate their direction from 128 MB of state on, and not below.
+extern "C" int check_sweeps() {
+  StateImpl s;
+  for (size_t mb : {1, 64, 127}) {
+    s.bytes = mb << 20;
+    for (int i = 0; i < 4; ++i)
+      if (s.next_sweep()) return 1;
+  }
+  for (size_t mb : {128, 4096}) {
+    s.bytes = mb << 20;
+    bool last = s.sweep;
+    for (int i = 0; i < 4; ++i) {
+      const bool now = s.next_sweep();
+      if (now == last) return 2;
+      last = now;
+    }
+  }
+  return 0;
+}

@@ -54,3 +54,7 @@ def test_auto_chooses_again_for_another_tile_size(eng):
 
 def test_a_pass_is_launched_where_its_tiles_fit(eng):
     assert eng.check_launch_config() == 0
+
+
+def test_sweeps_alternate_where_the_l2_does_not_hold_the_state(eng):
+    assert eng.check_sweeps() == 0

@@ -80,3 +80,24 @@ def test_library_takes_13_bit_tiles(tile_config):
         passes[cfg] = c.plan_stats(n, "c64", "tiled")["passes"]
     assert passes[0] == passes[2] < passes[4]
     check(n, "c64", c, gates)
+
+
+# per-gate launches in both directions: 128 MB of state, every kind of gate
+@pytest.mark.parametrize("n,dtype", [(24, "c64"), (23, "c128")])
+def test_pergate_both_directions(n, dtype):
+    rng = np.random.default_rng(n)
+    gates = [("u3", (q,), tuple(rng.uniform(0, 6, 3))) for q in range(0, n, 3)]
+    for name in EVERY + ["x", "x", "rz", "rz", "swap", "cx"]:
+        qs = tuple(int(x) for x in rng.choice(n, size=circuits.ARITY[name], replace=False))
+        d = {"custom1": 2, "custom2": 4}.get(name)
+        gates.append((name, qs, (), unitary(rng, d)) if d else (name, qs, tuple(rng.uniform(-6, 6, 4))))
+    gates += [("x", (0,), ()), ("rz", (0,), (0.3,)), ("h", (0,), ()), ("cz", (0, n - 1), ()), ("cp", (1, 0), (0.4,))]
+    with StateVector(n, dtype) as sv:
+        Circuit(n, gates).execute(sv, "pergate")
+        got = sv.amplitudes()
+    o = O.OracleState(n)
+    o.apply(gates)
+    ref = o.amplitudes()
+    if dtype == "c128":
+        assert np.abs(got - ref).max() <= 1e-12
+    assert 1 - abs(np.vdot(got, ref)) ** 2 / (np.vdot(got, got).real * np.vdot(ref, ref).real) <= 1e-5
