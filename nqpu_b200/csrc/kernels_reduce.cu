@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
-// One warp per shot.  In a segment a step covers 32 lanes x 8 vectors: each lane
+// One warp per shot, for few shots.  In a segment a step covers 32 lanes x 8 vectors: each lane
 // loads 8 consecutive vectors at once, sums its probabilities serially, and the
 // warp scans the 32 lane totals; the lane whose range holds r then picks the
 // amplitude from its own prefix.  A segment is 8 (complex64) or 16 (complex128)
@@ -452,6 +452,117 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
+// The same for many shots, where the loads of the form above count (eight consecutive
+// vectors per lane: every load touches 32 lines).  A step covers NV rows of 32
+// vectors, a vector per lane and row.  A step that r lies beyond costs one sum over
+// the warp; in the one that holds r every row is scanned, all rows at once, and the
+// first amplitude whose prefix exceeds r is taken.  Without SKIP (states of a few rows)
+// every step is scanned.
+// Measured (100000 shots, the whole call; one amplitude per lane and step, the form
+// above, this one):
+//   13 qubits   complex64   877  705  379 us     complex128   860 1185  391
+//   25 qubits   complex64  1126  713  480        complex128  1142 1197  534
+template <typename Real, int NV, bool SKIP>
+__global__ void __launch_bounds__(256, 2)
+    k_sample_rows(const Real* __restrict__ amp, uint64_t dim, int segbits, uint64_t nseg,
+             const double* __restrict__ seg_sum, const double* __restrict__ seg_incl,
+             const double* __restrict__ u, uint32_t shots, uint64_t* __restrict__ out) {
+  using V = typename Tr<Real>::V;
+  constexpr int VB = Tr<Real>::kVecBit;
+  const V* vp = reinterpret_cast<const V*>(amp);
+  const int lane = threadIdx.x & 31;
+  const uint64_t warp_id = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
+  const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  const uint64_t nvec = dim >> VB;
+  for (uint64_t sh = warp_id; sh < shots; sh += nwarps) {
+    const double r = u[sh];
+    // first segment whose inclusive prefix exceeds r
+    uint64_t lo = 0, hi = nseg;
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (seg_incl[mid] > r) hi = mid; else lo = mid + 1;
+    }
+    uint64_t result = dim - 1;
+    bool found = false;
+    for (uint64_t sg = lo; sg < nseg && !found; ++sg) {
+      double run = seg_incl[sg] - seg_sum[sg];
+      const uint64_t v0 = (sg << segbits) >> VB;
+      const uint64_t seg_end = v0 + ((1ull << segbits) >> VB);
+      const uint64_t v1 = seg_end < nvec ? seg_end : nvec;
+      for (uint64_t b = v0; b < v1 && !found; b += 32 * NV) {
+        const uint64_t k = b + lane;
+        V v[NV];
+        if (b + 32 * NV <= v1) {
+#pragma unroll
+          for (int j = 0; j < NV; ++j) v[j] = __ldg(vp + k + 32 * j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NV; ++j) {
+            v[j] = V{};
+            if (k + 32 * j < v1) v[j] = __ldg(vp + k + 32 * j);
+          }
+        }
+        double p0[NV], sc[NV], t = 0.0;  // the vector's first amplitude, all of it
+        uint32_t some = 0, later = 0;    // bit j: row j's vector, its second amplitude is not 0
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          double p[2];
+          vec_probs<Real>(v[j], p);
+          p0[j] = p[0];
+          sc[j] = VB == 1 ? p[0] + p[1] : p[0];
+          t += sc[j];
+          some |= uint32_t(sc[j] > 0.0) << j;
+          if (VB == 1) later |= uint32_t(p[1] > 0.0) << j;
+        }
+        if (SKIP) {
+          t = warp_sum(t);
+          if (!(r < run + t)) {
+            run += t;
+            continue;
+          }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+          for (int j = 0; j < NV; ++j) {
+            const double x = __shfl_up_sync(0xffffffffu, sc[j], o);
+            if (lane >= o) sc[j] += x;
+          }
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          // (only what has a probability: two lanes' prefixes may differ by a rounding)
+          const unsigned hit = __ballot_sync(0xffffffffu, ((some >> j) & 1u) && r < run + sc[j]);
+          if (hit && !found) {
+            const double excl = __shfl_up_sync(0xffffffffu, sc[j], 1);
+            const bool second = ((later >> j) & 1u) && !(r < run + (lane ? excl : 0.0) + p0[j]);
+            result = __shfl_sync(0xffffffffu, ((k + 32 * j) << VB) + (second ? 1 : 0), __ffs(hit) - 1);
+            found = true;
+          }
+          run += __shfl_sync(0xffffffffu, sc[j], 31);
+        }
+      }
+    }
+    if (lane == 0) out[sh] = result < dim ? result : dim - 1;
+  }
+}
+
+// From this many shots on by rows: below, a call's latency counts and either form
+// takes about as long.
+constexpr uint32_t kRowShots = 2017;
+
+template <typename Real>
+static void sample_t(const Real* amp, uint64_t dim, int segbits, uint64_t nseg, const double* seg_sum,
+                     const double* seg_incl, const double* u, uint32_t shots, uint64_t* out, int grid, cudaStream_t s) {
+  auto go = [&](auto kernel) {
+    kernel<<<grid, 256, 0, s>>>(amp, dim, segbits, nseg, seg_sum, seg_incl, u, shots, out);
+  };
+  const uint64_t rows = (dim >> Tr<Real>::kVecBit) >> 5;
+  if (shots < kRowShots) go(k_sample<Real>);
+  else if (rows <= 4) go(k_sample_rows<Real, 1, false>);
+  else if (rows <= 8) go(k_sample_rows<Real, 4, true>);
+  else go(k_sample_rows<Real, 8, true>);
+}
+
 cudaError_t launch_sample(DType dt, const void* amp, int n, const double* d_uniforms,
                           uint32_t shots, double* scratch, uint64_t* d_out, cudaStream_t s,
                           int num_sms) {
@@ -470,9 +581,9 @@ cudaError_t launch_sample(DType dt, const void* amp, int n, const double* d_unif
   const uint64_t warps = shots;
   const int g2 = int(std::max<uint64_t>(1, std::min<uint64_t>((warps * 32 + 255) / 256, uint64_t(num_sms) * 8)));
   if (dt == DType::C64)
-    k_sample<float><<<g2, 256, 0, s>>>(static_cast<const float*>(amp), dim, segbits, nseg, seg_sum, seg_incl, d_uniforms, shots, d_out);
+    sample_t(static_cast<const float*>(amp), dim, segbits, nseg, seg_sum, seg_incl, d_uniforms, shots, d_out, g2, s);
   else
-    k_sample<double><<<g2, 256, 0, s>>>(static_cast<const double*>(amp), dim, segbits, nseg, seg_sum, seg_incl, d_uniforms, shots, d_out);
+    sample_t(static_cast<const double*>(amp), dim, segbits, nseg, seg_sum, seg_incl, d_uniforms, shots, d_out, g2, s);
   return cudaGetLastError();
 }
 

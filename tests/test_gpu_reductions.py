@@ -112,3 +112,38 @@ def test_pauli_sum_of_extreme_coefficients(size, n, dtype):
     got = sv.expectation_pauli_sum(list(zip(unit * size, strings)))
     assert abs(got / size - want) <= 1e-13 * unit.size
     sv.close()
+
+
+# many shots: one row and less, each number of rows of a single step, several steps,
+# several segments.  The middle of a bin of at least 1e-9 is far from any rounding.
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("n", [1, 2, 5, 6, 7, 8, 9, 10, 12, 13, 18])
+def test_many_shots_pick_the_bin(n, dtype):
+    a, sv = random_state(n, dtype, n)
+    p = np.abs(a) ** 2
+    cum = np.cumsum(p)
+    pick = np.random.default_rng(n).choice(np.nonzero(p > 1e-9)[0], size=4000)
+    u = cum[pick] - 0.5 * p[pick]
+    np.testing.assert_array_equal(sv.sample_with_uniforms(u), pick.astype(np.uint64))
+    beyond = np.full(2017, 2.0)
+    np.testing.assert_array_equal(sv.sample_with_uniforms(beyond), [(1 << n) - 1] * 2017)
+    sv.close()
+
+
+def test_many_shots_read_whole_lines():
+    # both types read a segment's vectors alike: complex128, twice the bytes, takes
+    # little longer (1.7 times as long with eight consecutive vectors per lane)
+    import time
+
+    best = {}
+    u = np.random.default_rng(0).random(100000)
+    for dtype in ("c64", "c128"):
+        _, sv = random_state(13, dtype, 13)
+        times = []
+        for _ in range(10):
+            t = time.perf_counter()
+            sv.sample_with_uniforms(u)
+            times.append(time.perf_counter() - t)
+        best[dtype] = min(times)
+        sv.close()
+    assert best["c128"] <= 1.3 * best["c64"]
