@@ -211,7 +211,7 @@ static cudaError_t pauli_sum(StateImpl* s, const std::vector<PauliString>& strin
   PauliPlan plan;
   std::vector<PauliString> wide;
   for (size_t lo = 0; lo < strings.size(); lo += kPauliMaxTerms) {
-    pauli_plan(strings.data() + lo, std::min<size_t>(kPauliMaxTerms, strings.size() - lo), int(s->n), &plan, &wide);
+    pauli_plan(s->dt, strings.data() + lo, std::min<size_t>(kPauliMaxTerms, strings.size() - lo), int(s->n), &plan, &wide);
     for (const PauliString& p : wide)
       if ((e = pauli_direct(s, p, out)) != cudaSuccess) return e;
     if (plan.sets.empty()) continue;

@@ -72,7 +72,7 @@ cudaError_t state_run_error(StateImpl* s);
 // out (n+1 values): [0] = sum|a|^2, [1+q] = sum over bit q set; either pointer may be null.
 cudaError_t state_zsums(const StateImpl* s, double* zs, double* total);
 // sum_t c_t <P_t> (one launch per kPauliMaxTerms strings plus one per string
-// that spans more than four X|Y positions).
+// that pauli_plan leaves to run by itself).
 cudaError_t state_pauli_sum(StateImpl* s, const std::vector<PauliString>& strings, double* out);
 cudaError_t state_inner(const StateImpl* a, const StateImpl* b, double* out2);
 cudaError_t state_sample(const StateImpl* s, const double* uniforms, uint32_t shots, uint64_t* out);

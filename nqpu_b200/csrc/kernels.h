@@ -122,10 +122,11 @@ struct PauliPlan {
   std::vector<PauliSet> sets;
   std::vector<PauliTerm> terms;
 };
-// Split a Pauli sum on n >= 4 qubits into register sets; terms whose X|Y
-// positions span more than four qubits are left in `wide` (at most
+// Split a Pauli sum on n >= 4 qubits into register sets; terms that run better by
+// themselves (X|Y positions on more than four qubits, or on the lowest ones of a
+// large complex128 state and alone there) are left in `wide` (at most
 // kPauliMaxTerms strings per call).
-void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan,
+void pauli_plan(DType dt, const PauliString* strings, size_t count, int n, PauliPlan* plan,
                 std::vector<PauliString>* wide);
 // out[0] = the plan's sum over the state; d_sets / d_terms are the plan's tables
 // in device memory.

@@ -29,7 +29,12 @@ namespace nqpu {
 // 2^22 amplitudes are 32 MB (complex64) / 64 MB (complex128): well inside the L2.
 constexpr int kPauliChunkBits = 22;
 
-void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan,
+// Complex128 from this size on (128 MB of state): a set that holds qubits 0, 1 and 2
+// reads 128 bytes per lane, a line each, and for one string alone the scalar kernel
+// is the faster one (25 qubits, X on 0, 1, 2: 108 us, 154 from a set; on 3, 4, 5: 104).
+constexpr int kPauliAloneQubits = 23;
+
+void pauli_plan(DType dt, const PauliString* strings, size_t count, int n, PauliPlan* plan,
                 std::vector<PauliString>* wide) {
   plan->sets.clear();
   plan->terms.clear();
@@ -51,6 +56,12 @@ void pauli_plan(const PauliString* strings, size_t count, int n, PauliPlan* plan
     g->bits |= x;
     g->idx.push_back(t);
   }
+  if (dt == DType::C128 && n >= kPauliAloneQubits)
+    for (size_t i = groups.size(); i-- > 0;)
+      if (groups[i].idx.size() == 1 && (groups[i].bits & 7) == 7) {
+        wide->push_back(strings[groups[i].idx[0]]);
+        groups.erase(groups.begin() + long(i));
+      }
   if (!diag.empty()) {
     if (groups.empty()) groups.emplace_back();
     groups[0].idx.insert(groups[0].idx.end(), diag.begin(), diag.end());

@@ -105,7 +105,7 @@ cudaError_t launch_inner(DType, const void*, DType, const void*, int, double*, d
 cudaError_t launch_pauli(DType, const void*, int, uint64_t, uint64_t, uint64_t, double*, double*, cudaStream_t, int) {
   return cudaSuccess;
 }
-void pauli_plan(const PauliString*, size_t, int, PauliPlan*, std::vector<PauliString>*) {}
+void pauli_plan(DType, const PauliString*, size_t, int, PauliPlan*, std::vector<PauliString>*) {}
 cudaError_t launch_pauli_sum(DType, const void*, int, const PauliSet*, const PauliPlan&, const PauliTerm*, double*, double*,
                              cudaStream_t, int) {
   return cudaSuccess;

@@ -147,3 +147,39 @@ def test_many_shots_read_whole_lines():
         best[dtype] = min(times)
         sv.close()
     assert best["c128"] <= 1.3 * best["c64"]
+
+
+# strings on the lowest qubits of a large complex128 state, alone, two in one set, and
+# among others; every value against numpy
+def test_pauli_strings_on_the_lowest_qubits():
+    n = 23
+    a, sv = random_state(n, "c128", n)
+
+    def on(**q):
+        return "".join(q.get(f"q{i}", "I") for i in range(n))
+
+    strings = [on(q0="X", q1="X", q2="X"), on(q0="X", q1="Y", q2="Y", q9="Z"), on(q0="Y", q1="X", q2="X", q20="X"),
+               on(q5="X", q6="Y"), on(q0="Z", q22="Z"), on(q0="X", q1="X", q2="Y", q3="Z")]
+    want = np.array([pauli_value(a, s) for s in strings])
+    for s, w in zip(strings, want):
+        assert abs(sv.expectation_pauli_string(s) - w) <= 1e-13
+    c = np.array([0.3, -1.2, 0.8, 0.5, -0.9, 1.1])
+    for k in range(2, 7):
+        assert abs(sv.expectation_pauli_sum(list(zip(c[:k], strings[:k]))) - c[:k] @ want[:k]) <= 1e-13 * np.abs(c).sum()
+    sv.close()
+
+
+def test_a_string_on_the_lowest_qubits_takes_no_longer():
+    import time
+
+    n = 25
+    best = []
+    with StateVector(n, "c128") as sv:
+        for s in ("XXX" + "I" * (n - 3), "IIIXXX" + "I" * (n - 6)):
+            times = []
+            for _ in range(20):
+                t = time.perf_counter()
+                sv.expectation_pauli_string(s)
+                times.append(time.perf_counter() - t)
+            best.append(min(times))
+    assert best[0] <= 1.25 * best[1]  # 1.5 times as long from a register set
