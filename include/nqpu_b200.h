@@ -242,7 +242,7 @@ NqpuError    nqpu_circuit_add_custom_2q(NqpuCircuit* c, uint32_t q1, uint32_t q2
  * the CALLER's device memory, for callers that cannot allocate device memory:
  * plugins whose host runtime owns the device memory pool, and real-time loops
  * that must not wait on the allocator.  It allocates nothing: the reduction's
- * scratch is a fixed array in this library's device module (about 0.3 MB on
+ * scratch is a fixed array in this library's device module (about 0.24 MB on
  * every GPU that loads the library, kept until exit).  d_amplitudes: 2^n
  * interleaved (re, im) amplitudes of `dtype`, 16-byte aligned; d_out: n doubles
  * in device memory; cuda_stream: a cudaStream_t (NULL = legacy default

@@ -434,8 +434,9 @@ static bool plan_host(const CircuitImpl* c, const Segment& seg, uint32_t n, DTyp
 //   tensor  U (1.013 passes + 0.139 unitaries) + 16.8 us per pass + 34 us
 // fitted (least squares of the relative error) to 42 measured complex64 circuits:
 // brickwork, ansatz, Ising evolution and phase estimation of 14 to 28 qubits and
-// two depths.  The fit is within 15 % for most, and picks the faster mode for
-// every one of them: the tensor passes win on brickworks from 23 qubits on
+// two depths, none held out, with the kernels of that time (later ones took a few
+// per cent off either side).  The fit is within 15 % for most, and picks the faster
+// mode for every one of them: the tensor passes win on brickworks from 23 qubits on
 // (26 qubits, 12 layers: 4.5 against 6.9 ms), the tiled ones everywhere else
 // (30-qubit Ising evolution, 10 steps: 121 against 140 ms).  4x4 matrices and 2x2s
 // with controls run as single records, priced at the 0.30 and 0.15 they

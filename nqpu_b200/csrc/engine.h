@@ -21,6 +21,9 @@ double next_random_f64();
 bool device_ready();
 int device_sms();
 
+// (32 KB: a complex128 register of 10 qubits, or the uniforms and outcomes of 2016
+// shots.  A copy from or to pageable memory costs about 10 us more at any size;
+// the line is this buffer's size, not where that stops.)
 constexpr size_t kSmallDoubles = 4096, kSmallTable = 64;
 constexpr size_t kSweepBytes = size_t(128) << 20;
 

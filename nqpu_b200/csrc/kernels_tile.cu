@@ -30,7 +30,8 @@ namespace nqpu {
 // WAY 0: the program stays in global memory (it does not fit); 1: it is in shared
 // memory; 2: that, and the tile has all of KMAX bits.  Kernels of their own,
 // because deciding it inside costs the stage loop spills (complex128 at 128
-// registers: 20-qubit brickwork 398 us against 385 without them).
+// registers: 20-qubit brickwork 398 us against 385; the forms apart spill 8 to 40
+// bytes there, complex64 none but 76 where the program is in global memory).
 // MINB = 1: one persistent CTA per SM; while the stages of tile i run on one
 // buffer, the cp.async copies of tile i+1 stream into the other.  MINB > 1:
 // MINB CTAs per SM with one buffer each hide each other's copies.  Each thread
@@ -166,7 +167,8 @@ static size_t tile_smem_max(int minb, int share_of) {
 //     against 122), else 2 (four warps per scheduler instead of two hide the
 //     dependency waits: 25-qubit ansatz of 8 layers 5.1 against 6.6 ms, 20-qubit
 //     brickwork 383 against 461 us; 4 takes 4.7 ms and 389 us, with 12 and 21
-//     passes for 10 and 14).
+//     passes for 10 and 14: the better one on large states, which no rule here
+//     separates yet).
 static std::atomic<int> g_tile_minb[2];
 
 void tile_config_set(DType dt, int minb) { g_tile_minb[dt == DType::C64 ? 0 : 1] = minb; }
@@ -266,7 +268,10 @@ constexpr int kWideTileMinQubits = 22;
 // passes and stages too: 27-qubit phase estimation (7 passes and 19 stages instead
 // of 10 and 22) 5.55 against 7.48 ms.  With the passes alone fewer they lose:
 // 25-qubit Ising evolution of 10 steps (12 and 40 instead of 15 and 38) 3.30 against
-// 3.17 ms, of 5 steps (6 and 21 instead of 8 and 20) 1.70 against 1.54.
+// 3.17 ms, of 5 steps (6 and 21 instead of 8 and 20) 1.70 against 1.54.  A ratio of
+// passes does not separate every case: phase estimation of 24 and 25 qubits (6
+// passes for 7, 7 for 8) is refused and would take 0.65 for 0.85 ms and 1.36 for
+// 1.81, that of 26 qubits would lose 6 %.
 bool build_tile_plan_for(const std::vector<Op>& ops, int n, DType dt, TilePlan* out, std::string* err,
                          const std::function<bool(const TilePlan&)>& enough) {
   if (!build_tile_plan(ops, n, dt, tile_kmax_for(dt), out, err)) return false;

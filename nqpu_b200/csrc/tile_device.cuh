@@ -143,9 +143,9 @@ __device__ __forceinline__ void rb_x1_generic(C (&a)[NA], int b, bool tc, uint32
 }
 
 // X on register bit B, controlled by the register bits CM (compile time) and
-// by controls outside the registers (tc): per-thread selects (TC_ALWAYS would
-// make it a register renaming, which only straight-line code can afford).
-template <typename C, int NA, int B, int CM, bool TC_ALWAYS>
+// by controls outside the registers (tc): per-thread selects (a register renaming
+// where tc is always true is what only straight-line code can afford).
+template <typename C, int NA, int B, int CM>
 __device__ __forceinline__ void rb_x1_fixed(C (&a)[NA], bool tc) {
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
@@ -153,21 +153,16 @@ __device__ __forceinline__ void rb_x1_fixed(C (&a)[NA], bool tc) {
     if ((i & CM) != CM) continue;
     const int j = i | (1 << B);
     const C x = a[i], y = a[j];
-    if constexpr (TC_ALWAYS) {
-      a[i] = y;
-      a[j] = x;
-    } else {
-      a[i] = csel(tc, y, x);
-      a[j] = csel(tc, x, y);
-    }
+    a[i] = csel(tc, y, x);
+    a[j] = csel(tc, x, y);
   }
 }
 
-template <typename C, int NA, int NRB, int B, bool TC_ALWAYS>
+template <typename C, int NA, int NRB, int B>
 __device__ __forceinline__ void dispatch_x1_ctrl(C (&a)[NA], uint32_t creg, bool tc) {
   switch (creg) {
 #define NQ_X1C(V) case (V == 0 ? 0 : (1 << (V - 1))): \
-    if constexpr (V == 0 || (V - 1 < NRB && V - 1 != B)) rb_x1_fixed<C, NA, B, (V == 0 ? 0 : (1 << (V - 1))), TC_ALWAYS>(a, tc); break;
+    if constexpr (V == 0 || (V - 1 < NRB && V - 1 != B)) rb_x1_fixed<C, NA, B, (V == 0 ? 0 : (1 << (V - 1)))>(a, tc); break;
     NQ_X1C(0) NQ_X1C(1) NQ_X1C(2) NQ_X1C(3) NQ_X1C(4) NQ_X1C(5)
 #undef NQ_X1C
     default: break;
@@ -435,7 +430,7 @@ __device__ __forceinline__ void apply_op(typename Tr<Real>::C (&a)[NA], uint32_t
       // register block on every other op's path
       switch (rb0) {
 #define NQ_X1(B, _) case B: \
-        if constexpr (B < NRB) dispatch_x1_ctrl<C, NA, NRB, B, false>(a, creg, tc); \
+        if constexpr (B < NRB) dispatch_x1_ctrl<C, NA, NRB, B>(a, creg, tc); \
         break;
         NQ_REG_CASES(NQ_X1, 0)
 #undef NQ_X1

@@ -677,7 +677,6 @@ void compile(const std::vector<Op>& ops, TilePlan* plan, const std::vector<TileO
       std::memcpy(static_cast<void*>(plan->prog.data() + tabs + size_t(s - P.stage_begin) * (kStageTabWords / 4)), tab,
                   sizeof(tab));
     }
-    plan->prog.push_back(ProgWord{{0, 0, 0, 0}});  // the kernel reads one word past a header
     P.prog_words = int32_t(plan->prog.size() - tabs);
   }
 }
