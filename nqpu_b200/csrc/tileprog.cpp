@@ -157,6 +157,7 @@ class StageCompiler {
   static double mag(cplx z) { return kF32 ? std::sqrt(std::norm(z)) : std::abs(z); }
   static cplx unit(cplx z) { return z / mag(z); }
   static cplx quot(cplx z, cplx w) { return kF32 ? z * std::conj(w) / std::norm(w) : z / w; }
+  static cplx over(cplx z, cplx w) { return kF32 ? z * std::conj(w) : z / w; }  // w a unit
 
   // A 2x2 as items: phase x rotation x phase where it is unitary, else as it is.
   void dense(int b, uint32_t cnr, const cplx* m) {
@@ -198,11 +199,11 @@ class StageCompiler {
       return;
     }
     // e^{ia} diag(1, after) [[c, -s], [s, c]] diag(1, before)
-    const cplx a = m[0] / c, ia = std::conj(a);
+    const cplx a = m[0] / c;
     // (`before` from the larger of the entries that fix it: a small off-diagonal
     // has no precise phase, and only its product with `after` matters then)
-    cplx after = unit((m[2] / s) * ia);
-    cplx before = unit(s > c ? (-m[1] / s) * ia : (m[3] / c) * ia * std::conj(after));
+    const cplx after0 = over(m[2] / s, a);
+    cplx after = unit(after0), before = unit(s > c ? over(-m[1] / s, a) : over(over(m[3] / c, a), after0));
     double sn = s;
     if (std::norm(after + one) < kTiny * kTiny) {  // a rotation the other way
       sn = -s;
@@ -755,11 +756,10 @@ std::vector<Op> carry_phases(std::vector<Op> ops) {
     cplx* m = ops[i].m;
     cplx w[4] = {m[0], m[1], m[2], m[3]}, c[4] = {1.0, 0.0, 0.0, 1.0};
     if (z) {
-      cplx p = m[2] * std::conj(m[0]);
-      p /= std::abs(p);
+      const cplx p = (m[2] / std::abs(m[2])) / (m[0] / std::abs(m[0]));
       c[3] = p;
-      w[2] = m[2] * std::conj(p);
-      w[3] = m[3] * std::conj(p);
+      w[2] = m[2] / p;
+      w[3] = m[3] / p;
     } else {
       // RX(al) rotation phase: RX(-al) m has a real ratio in its first column
       const double al = std::atan2(-2.0 * (std::conj(m[0]) * m[2]).imag(), std::norm(m[0]) - std::norm(m[2]));
