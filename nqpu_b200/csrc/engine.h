@@ -25,7 +25,6 @@ int device_sms();
 // shots.  A copy from or to pageable memory costs about 10 us more at any size;
 // the line is this buffer's size, not where that stops.)
 constexpr size_t kSmallDoubles = 4096, kSmallTable = 64;
-constexpr size_t kSweepBytes = size_t(128) << 20;
 
 struct StateImpl {
   uint32_t n = 0;

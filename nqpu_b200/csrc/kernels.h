@@ -14,8 +14,10 @@ namespace nqpu {
 struct PGArgs {
   uint64_t n_items;   // work items (index sets) of the launch
   uint64_t setmask;   // bits forced to one (controls)
-  uint64_t flip;      // n_items - 1 in a launch that runs from the far end, else 0
-  uint64_t cmask;     // controls checked per amplitude (elementwise kernels)
+  union {
+    uint64_t cmask;   // controls checked per amplitude (elementwise kernels)
+    uint64_t flip;    // X: n_items - 1 in a launch that runs from the far end, else 0
+  };
   int32_t npos;       // zero-bit insert positions, ascending
   int32_t pos[8];
   int32_t t0, t1;
@@ -23,6 +25,8 @@ struct PGArgs {
 };
 
 // --- per-gate path -----------------------------------------------------------
+// State size from which successive launches sweep in alternate directions.
+constexpr size_t kSweepBytes = size_t(128) << 20;
 // `rev`: sweep the state from its far end (callers alternate from gate to gate).
 cudaError_t launch_pergate(DType dt, void* amp, int n, const Op& op, bool rev, cudaStream_t s, int num_sms);
 

@@ -35,12 +35,13 @@ __device__ __forceinline__ void load_m(const PGArgs& A, typename Tr<Real>::C* m,
 // Index set of work item w (n_items is a power of two, so the far end is a flip of
 // all its bits).  The direction is compiled in: as a run-time value it took
 // registers or instructions from every launch (4x4s on 21 qubits of complex128 199 ->
-// 233 us, RZ on 21 qubits of complex64 142 -> 173), except for X, whose run-time form
-// is the faster code (23 qubits of complex128, 23 gates: 915 us, compiled in 1000).
+// 233 us, RZ on 21 qubits of complex64 142 -> 173), except for X on large states,
+// whose run-time form is the faster code (23 qubits of complex128, 23 gates: 915 us,
+// compiled in 1000).
 enum Dir { FORWARD, BACKWARD, RUNTIME };
 template <Dir DIR>
 __device__ __forceinline__ uint64_t pg_expand(uint64_t w, const PGArgs& A) {
-  uint64_t i = DIR == FORWARD ? w : w ^ A.flip;
+  uint64_t i = DIR == FORWARD ? w : DIR == BACKWARD ? w ^ (A.n_items - 1) : w ^ A.flip;
 #pragma unroll 1
   for (int j = 0; j < A.npos; ++j) i = insert_zero_bit(i, A.pos[j]);
   return i | A.setmask;
@@ -255,9 +256,16 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, cudaStream_t s, i
     A.npos = int(pos.size());
     for (int i = 0; i < A.npos; ++i) A.pos[i] = pos[i];
     A.n_items = (1ull << n) >> A.npos;
-    A.flip = DIR == BACKWARD ? A.n_items - 1 : 0;
   };
   const unsigned blk = 256;
+  auto x1 = [&](auto small, auto large, unsigned g) {
+    if ((sizeof(Real) << (n + 1)) < kSweepBytes) {
+      small<<<g, blk, 0, s>>>(amp, A);
+    } else {
+      A.flip = DIR == BACKWARD ? A.n_items - 1 : 0;
+      large<<<g, blk, 0, s>>>(amp, A);
+    }
+  };
   switch (op.kind) {
     case OP_U1:
     case OP_X1: {
@@ -269,14 +277,14 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, cudaStream_t s, i
           finish(false);
           unsigned g = pg_grid(A.n_items, num_sms);
           if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 2, DIR><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_1t<Real, OP_X1, 2, RUNTIME><<<g, blk, 0, s>>>(amp, A);
+          else x1(k_pg_1t<Real, OP_X1, 2, FORWARD>, k_pg_1t<Real, OP_X1, 2, RUNTIME>, g);
           break;
         }
         if (!(ctrl & 1) && n >= 2) {
           finish(true);
           unsigned g = pg_grid(A.n_items, num_sms);
           if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 1, DIR><<<g, blk, 0, s>>>(amp, A);
-          else k_pg_1t<Real, OP_X1, 1, RUNTIME><<<g, blk, 0, s>>>(amp, A);
+          else x1(k_pg_1t<Real, OP_X1, 1, FORWARD>, k_pg_1t<Real, OP_X1, 1, RUNTIME>, g);
           break;
         }
       }
@@ -284,7 +292,7 @@ static cudaError_t launch_pg_t(Real* amp, int n, const Op& op, cudaStream_t s, i
         finish(false);
         unsigned g = pg_grid(A.n_items, num_sms);
         if (op.kind == OP_U1) k_pg_1t<Real, OP_U1, 0, DIR><<<g, blk, 0, s>>>(amp, A);
-        else k_pg_1t<Real, OP_X1, 0, RUNTIME><<<g, blk, 0, s>>>(amp, A);
+        else x1(k_pg_1t<Real, OP_X1, 0, FORWARD>, k_pg_1t<Real, OP_X1, 0, RUNTIME>, g);
       }
       break;
     }
