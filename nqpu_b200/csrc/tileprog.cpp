@@ -104,6 +104,7 @@ class StageCompiler {
     global_ = global;
     final_ = false;
     items_.clear();
+    dense_bits_ = 0;
     for (Phase& p : pend_) p.clear();
     used_ = 0;
     for (bool& h : have_) h = false;
@@ -136,10 +137,19 @@ class StageCompiler {
   }
   void push_phase(uint32_t A, uint32_t B, cplx p) {
     if (p == cplx(1.0, 0.0)) return;
+    if (!(A & dense_bits_)) {  // nothing to wait for
+      pend(A, B, p);
+      return;
+    }
     Item I;
     I.diag = A;
     I.cnr = B;
     I.m[0] = p;
+    items_.push_back(I);
+  }
+
+  void push_dense(const Item& I) {
+    dense_bits_ |= I.dense;
     items_.push_back(I);
   }
 
@@ -171,13 +181,13 @@ class StageCompiler {
     if (!unitary) {
       I.kind = Item::GENERIC;
       for (int i = 0; i < 4; ++i) I.m[i] = m[i];
-      items_.push_back(I);
+      push_dense(I);
       return;
     }
     const double c = mag(m[0]), s = mag(m[2]);
     if (c < kFlip) {  // Y, RX(pi), RY(pi): the amplitudes change places, with phases
       I.kind = Item::FLIP;
-      items_.push_back(I);
+      push_dense(I);
       push_phase(0, 0, unit(m[1]));
       push_phase(1u << b, 0, clean(unit(quot(m[2], m[1]))));
       return;
@@ -189,7 +199,7 @@ class StageCompiler {
       push_phase(0, 0, cplx(sg, 0.0));
       shears(sg * m[0].real(), -sg * m[1].imag(), &I);
       I.kind = Item::CROSS;
-      if (I.s != 0.0) items_.push_back(I);
+      if (I.s != 0.0) push_dense(I);
       return;
     }
     const cplx one(1.0, 0.0);
@@ -214,7 +224,7 @@ class StageCompiler {
     push_phase(1u << b, 0, clean(before));
     shears(c, sn, &I);
     I.kind = Item::ROT;
-    items_.push_back(I);
+    push_dense(I);
     push_phase(1u << b, 0, clean(after));
   }
   // A phase that is 1 or -1 up to the rounding of its making.
@@ -283,7 +293,7 @@ class StageCompiler {
     I.diag = t.creg;
     for (int b = 0; b < kBits; ++b)
       if (((I.dense | I.diag) >> b) & 1) settle(b);
-    items_.push_back(I);
+    push_dense(I);
   }
 
   // ---- scheduling ---------------------------------------------------------
@@ -590,6 +600,7 @@ class StageCompiler {
   const std::vector<TileOp<Real>>& enc_;
   Writer W_;
   std::vector<Item> items_;
+  uint32_t dense_bits_ = 0;  // register bits some item changes
   struct Edge {
     int to, next;
   };
