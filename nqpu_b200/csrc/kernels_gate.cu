@@ -15,10 +15,10 @@
 //     so a launch begins with the part that the one before it left in L2 (126 MB);
 //     accesses carry no streaming hint that would evict it.  A U3 and CNOT layer,
 //     complex64: 24 qubits 1370 -> 1210 us, 25 qubits 2934 -> 2794, 26 qubits 6165 ->
-//     5948; complex128, 23 qubits 1362 -> 1139.  Below, the L2 holds the state, and
-//     turning round moves every address to another SM's half of it (complex64, 20
-//     qubits: 20 RY gates 115 us, in alternate directions 121; 23 qubits: 355
-//     against 363).
+//     5948; complex128, 23 qubits 1362 -> 1139.  Below, the L2 holds the state and
+//     alternation costs (another SM touches an address than the launch before):
+//     complex64, 20 qubits, 20 RY gates 115 us, in alternate directions 121; 23
+//     qubits, 23 of them 355 against 363.
 #include "sv_device.cuh"
 #include "kernels.h"
 

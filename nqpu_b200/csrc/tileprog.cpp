@@ -163,7 +163,8 @@ class StageCompiler {
   // complex64 programs are rounded to 2^-24, so hypot, the full complex division and
   // (join_constant) an angle per table entry buy nothing there: a circuit that runs
   // once pays for its program (17-qubit brickwork, 375 gates: build_tile_prog 165 ->
-  // 95 us; complex128 keeps them, its results are 1e-15 off).
+  // 95 us, 77 with phases that wait for nothing taken at once; complex128 keeps
+  // them, its results are 1e-15 off).
   static double mag(cplx z) { return kF32 ? std::sqrt(std::norm(z)) : std::abs(z); }
   static cplx unit(cplx z) { return z / mag(z); }
   static cplx quot(cplx z, cplx w) { return kF32 ? z * std::conj(w) / std::norm(w) : z / w; }
@@ -304,8 +305,8 @@ class StageCompiler {
   // An item waits for the last dense item before it on each of its bits and, where
   // it is dense, for the items since then that read the bit; a round takes what
   // waits for nothing any more, in circuit order.  So the work is linear in the
-  // items: walking all of them in every round took 4.4 s for 32000 gates on five
-  // qubits, which are one stage.
+  // items: walking all of them in every round took 580 ms for 18000 gates of an
+  // Ising evolution on five qubits, which are one stage (now 9).
   void schedule() {
     const size_t n = items_.size();
     wait_.assign(n, 0);
